@@ -17,6 +17,7 @@
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <memory>
 #include <vector>
 
@@ -45,6 +46,7 @@ struct mg_mlp {
   float* dA = nullptr;  // nh-wide scratch
   float* dB = nullptr;
   float* loss = nullptr;
+  float* part = nullptr;  // partial weight gradients of the split batch, all layers
   // BF16 activations of the tensor-core inference path, up to tc_cap rows,
   // and its error flag (a bounded wait that gave up).
   int64_t tc_cap = 0;
@@ -59,7 +61,6 @@ struct mg_mlp {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int BM = 64, BN = 64, BK = 16;
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigmoidf_(z); }
@@ -76,105 +77,232 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p) { ret
 // C[m, n] = sum_k opA(m, k) opB(k, n) with
 //   opA(m, k) = TA ? A[k*lda + m] : A[m*lda + k]
 //   opB(k, n) = TB ? B[k*ldb + n] : B[n*ldb + k]
-// then epi(m, n, acc).  64 x 64 tiles, 16-deep K steps, 4 x 4 per thread.
-template <bool TA, bool TB, typename TAe, typename TBe, typename Epi>
-__global__ void __launch_bounds__(kThreads) gemm_kernel(int M, int N, int K, const TAe* __restrict__ A, int lda,
-                                                        const TBe* __restrict__ B, int ldb, Epi epi) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int e = tid; e < BM * BK; e += kThreads) {
-      int m, k;
-      if (TA) { m = e % BM; k = e / BM; } else { k = e % BK; m = e / BK; }
-      const int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < M && gk < K) ? ld(TA ? &A[(int64_t)gk * lda + gm] : &A[(int64_t)gm * lda + gk]) : 0.0f;
+// then epi(m, n, acc).  BM x BN tiles, 16-deep K steps, TM x TN per thread
+// (256 threads).  What bounded the first version was the latency of one K
+// step (scalar loads, two barriers, nothing in flight): 4 us each, 256 of
+// them in a row for a weight gradient.  A K step's operands are therefore
+// fetched as float4 (four consecutive elements of the contiguous index)
+// into registers while the previous step computes, and a long K is split
+// over gridDim.z: CTA z sums k in [z kz, (z + 1) kz) and hands its sum to
+// epi as partial z.  rowsum (weight gradients): partial z of
+// sum_k A[k, m], the bias gradient, from the tiles already in shared memory.
+// Loss and gradients of a 4096-row batch (64-256-256-16): 2.10 -> 0.20 ms.
+constexpr int BK = 16;
+
+// Four consecutive elements p[0..3] (n of them valid), as float.
+__device__ __forceinline__ float4 ld4(const float* p, int n, bool vec) {
+  if (vec && n >= 4) return *reinterpret_cast<const float4*>(p);
+  return make_float4(n > 0 ? p[0] : 0.0f, n > 1 ? p[1] : 0.0f, n > 2 ? p[2] : 0.0f, n > 3 ? p[3] : 0.0f);
+}
+__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p, int n, bool vec) {
+  if (vec && n >= 4) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+  }
+  return make_float4(n > 0 ? ld(p) : 0.0f, n > 1 ? ld(p + 1) : 0.0f, n > 2 ? ld(p + 2) : 0.0f,
+                     n > 3 ? ld(p + 3) : 0.0f);
+}
+
+// One operand's share of a K step: ROWS x BK elements, element (r, k) at
+// T ? P[k*ld + r] : P[r*ld + k], four of the contiguous index per item.
+template <bool T, int ROWS, typename E>
+struct Fetch {
+  static constexpr int ITEMS = ROWS * BK / 4, PER = (ITEMS + kThreads - 1) / kThreads;
+  static __device__ __forceinline__ void item(int it, int& r, int& k) {
+    if (T) { r = (it % (ROWS / 4)) * 4; k = it / (ROWS / 4); } else { k = (it % (BK / 4)) * 4; r = it / (BK / 4); }
+  }
+  static __device__ __forceinline__ void load(float4 (&v)[PER], const E* P, int ld_, int r0, int R, int k0, int K1,
+                                              bool vec) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int it = threadIdx.x + u * kThreads;
+      int r, k;
+      item(it, r, k);
+      const int gr = r0 + r, gk = k0 + k;
+      v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (it < ITEMS && gr < R && gk < K1)
+        v[u] = T ? ld4(P + (int64_t)gk * ld_ + gr, R - gr, vec) : ld4(P + (int64_t)gr * ld_ + gk, K1 - gk, vec);
     }
-    for (int e = tid; e < BN * BK; e += kThreads) {
-      int n, k;
-      if (TB) { n = e % BN; k = e / BN; } else { k = e % BK; n = e / BK; }
-      const int gn = n0 + n, gk = k0 + k;
-      Bs[k][n] = (gn < N && gk < K) ? ld(TB ? &B[(int64_t)gk * ldb + gn] : &B[(int64_t)gn * ldb + gk]) : 0.0f;
+  }
+  template <int LDS>
+  static __device__ __forceinline__ void store(const float4 (&v)[PER], float (*S)[LDS]) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int it = threadIdx.x + u * kThreads;
+      int r, k;
+      item(it, r, k);
+      if (it >= ITEMS) continue;
+      if (T) {
+        *reinterpret_cast<float4*>(&S[k][r]) = v[u];
+      } else {
+        S[k][r] = v[u].x;
+        S[k + 1][r] = v[u].y;
+        S[k + 2][r] = v[u].z;
+        S[k + 3][r] = v[u].w;
+      }
     }
-    __syncthreads();
+  }
+};
+
+template <int BM, int BN, int TM, int TN, bool TA, bool TB, typename TAe, typename TBe, typename Epi>
+__global__ void __launch_bounds__(kThreads) gemm_kernel(int M, int N, int K, int kz, const TAe* __restrict__ A,
+                                                        int lda, const TBe* __restrict__ B, int ldb, bool vecA,
+                                                        bool vecB, Epi epi) {
+  static_assert(BM * BN == TM * TN * kThreads, "one TM x TN block per thread");
+  using FA = Fetch<TA, BM, TAe>;
+  using FB = Fetch<TB, BN, TBe>;
+  __shared__ __align__(16) float As[2][BK][BM + 4];
+  __shared__ __align__(16) float Bs[2][BK][BN + 4];
+  constexpr int TX = BN / TN;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, z = blockIdx.z;
+  const int kb = z * kz, ke = min(K, kb + kz);
+  const bool rs = Epi::ROWSUM && blockIdx.x == 0 && tid < BM;
+  float acc[TM][TN] = {}, rsum = 0.0f;
+  float4 va[FA::PER], vb[FB::PER];
+  FA::load(va, A, lda, m0, M, kb, ke, vecA);
+  FB::load(vb, B, ldb, n0, N, kb, ke, vecB);
+  FA::store(va, As[0]);
+  FB::store(vb, Bs[0]);
+  __syncthreads();
+  int cur = 0;
+  for (int k0 = kb; k0 < ke; k0 += BK, cur ^= 1) {
+    const bool more = k0 + BK < ke;
+    if (more) {
+      FA::load(va, A, lda, m0, M, k0 + BK, ke, vecA);
+      FB::load(vb, B, ldb, n0, N, k0 + BK, ke, vecB);
+    }
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      float a[4], b[4];
+      float a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+      for (int i = 0; i < TM; ++i) a[i] = As[cur][kk][ty * TM + i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
+      for (int j = 0; j < TN; ++j) b[j] = Bs[cur][kk][tx * TN + j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
+        for (int j = 0; j < TN; ++j) acc[i][j] += a[i] * b[j];
+      if (Epi::ROWSUM && rs) rsum += As[cur][kk][tid];
+    }
+    if (more) {
+      FA::store(va, As[cur ^ 1]);
+      FB::store(vb, Bs[cur ^ 1]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m < M && n < N) epi(m, n, acc[i][j]);
+    for (int j = 0; j < TN; ++j) {
+      const int m = m0 + ty * TM + i, n = n0 + tx * TN + j;
+      if (m < M && n < N) epi(m, n, z, acc[i][j]);
     }
+  if constexpr (Epi::ROWSUM) {
+    if (rs && m0 + tid < M) epi.rowsum(m0 + tid, z, rsum);
+  }
 }
 
 // Epilogues.
 struct EpiBiasSilu {  // Z = acc + b, H = SiLU(Z)
+  static constexpr bool ROWSUM = false;
   const float* b;
   float* Z;
   float* H;
   int ld;
-  __device__ void operator()(int m, int n, float acc) const {
+  __device__ void operator()(int m, int n, int, float acc) const {
     const float z = acc + b[n];
     Z[(int64_t)m * ld + n] = z;
     H[(int64_t)m * ld + n] = silu(z);
   }
 };
 struct EpiBias {  // Y = acc + b
+  static constexpr bool ROWSUM = false;
   const float* b;
   float* Y;
   int ld;
-  __device__ void operator()(int m, int n, float acc) const { Y[(int64_t)m * ld + n] = acc + b[n]; }
+  __device__ void operator()(int m, int n, int, float acc) const { Y[(int64_t)m * ld + n] = acc + b[n]; }
 };
 struct EpiSiluGrad {  // dZ = acc * SiLU'(Z)
+  static constexpr bool ROWSUM = false;
   const float* Z;
   float* dZ;
   int ld;
-  __device__ void operator()(int m, int n, float acc) const {
+  __device__ void operator()(int m, int n, int, float acc) const {
     dZ[(int64_t)m * ld + n] = acc * silu_grad(Z[(int64_t)m * ld + n]);
   }
 };
-struct EpiStore {  // G = acc
-  float* G;
-  int ld;
-  __device__ void operator()(int m, int n, float acc) const { G[(int64_t)m * ld + n] = acc; }
+struct EpiPart {  // partial z of a layer's gradients, laid out as its parameters: [W (M x ld), b (M)]
+  static constexpr bool ROWSUM = true;
+  float* part;
+  int M, ld;
+  __device__ void operator()(int m, int n, int z, float acc) const {
+    part[z * ((int64_t)M * ld + M) + (int64_t)m * ld + n] = acc;
+  }
+  __device__ void rowsum(int m, int z, float s) const {
+    part[z * ((int64_t)M * ld + M) + (int64_t)M * ld + m] = s;
+  }
 };
 
+template <typename T>
+bool vec4_ok(const T* p, int ld_) {
+  return ld_ % 4 == 0 && reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0;
+}
+
+// The tile follows the narrow side: an output side of at most 16 (nout)
+// would leave three quarters of a 64-wide tile idle.
 template <bool TA, bool TB, typename TAe, typename TBe, typename Epi>
-cudaError_t gemm(cudaStream_t s, int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, Epi epi) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  gemm_kernel<TA, TB, TAe, TBe, Epi><<<grid, kThreads, 0, s>>>(M, N, K, A, lda, B, ldb, epi);
+cudaError_t gemm(cudaStream_t s, int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, Epi epi,
+                 int splits = 1, int kz = 0) {
+  if (splits == 1) kz = K;
+  const bool va = vec4_ok(A, lda), vb = vec4_ok(B, ldb);
+  if (N <= 16) {
+    const dim3 grid((N + 15) / 16, (M + 63) / 64, splits);
+    gemm_kernel<64, 16, 4, 1, TA, TB><<<grid, kThreads, 0, s>>>(M, N, K, kz, A, lda, B, ldb, va, vb, epi);
+  } else if (M <= 16) {
+    const dim3 grid((N + 63) / 64, (M + 15) / 16, splits);
+    gemm_kernel<16, 64, 1, 4, TA, TB><<<grid, kThreads, 0, s>>>(M, N, K, kz, A, lda, B, ldb, va, vb, epi);
+  } else {
+    const dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
+    gemm_kernel<64, 64, 4, 4, TA, TB><<<grid, kThreads, 0, s>>>(M, N, K, kz, A, lda, B, ldb, va, vb, epi);
+  }
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
-// Column sums of a B x N matrix into out (bias gradients).
-__global__ void colsum_kernel(const float* __restrict__ D, int64_t B, int N, float* __restrict__ out) {
-  const int n = blockIdx.x;
-  float s = 0.0f;
-  for (int64_t b = threadIdx.x; b < B; b += blockDim.x) s += D[b * N + n];
-  __shared__ float red[kThreads];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[n] = red[0];
+// Split of a weight gradient's K = B rows: about two CTAs per SM over the
+// M x N tiles, each with at least 64 rows (four K steps); max_splits grows
+// with B, so buffers for a batch also hold every smaller one's partials.
+int64_t max_splits(int M, int N, int64_t B, int num_sms) {
+  const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
+  return std::min<int64_t>(std::max<int64_t>(1, 2 * (int64_t)num_sms / tiles), std::max<int64_t>(1, B / 64));
+}
+struct Split {
+  int splits, kz;
+};
+Split split_rows(int M, int N, int64_t B, int num_sms) {
+  const int64_t z = max_splits(M, N, B, num_sms);
+  int64_t kz = (B + z - 1) / z;
+  kz = (kz + BK - 1) / BK * BK;
+  return {(int)((B + kz - 1) / kz), (int)kz};
+}
+
+// Gradient of each parameter: its layer's partials summed in order.
+struct PartLayers {
+  const float* part[3];
+  int64_t start[4];  // parameter ranges of the layers
+  int splits[3];
+};
+__global__ void __launch_bounds__(kThreads) reduce_grad_kernel(PartLayers L, float* __restrict__ grad) {
+  const int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (e >= L.start[3]) return;
+  const int l = e < L.start[1] ? 0 : (e < L.start[2] ? 1 : 2);
+  const int64_t len = L.start[l + 1] - L.start[l];
+  const float* p = L.part[l] + (e - L.start[l]);
+  float t = 0.0f;
+  for (int z = 0; z < L.splits[l]; ++z) t += p[z * len];
+  grad[e] = t;
 }
 
 // dY = 2 (Y - (Yt - shift)/scale) / (B nout); loss += sum of squares.
@@ -342,7 +470,7 @@ inline unsigned grid_for(int64_t n, int threads = kThreads) {
 
 int ensure_capacity(mg_context* ctx, mg_mlp* m, int64_t B) {
   if (B <= m->cap) return MG_OK;
-  float* bufs[] = {m->Z1, m->H1, m->Z2, m->H2, m->Y, m->dY, m->dA, m->dB};
+  float* bufs[] = {m->Z1, m->H1, m->Z2, m->H2, m->Y, m->dY, m->dA, m->dB, m->part};
   for (float* p : bufs)
     if (p) cudaFree(p);
   const int64_t hw = (int64_t)B * m->nh, ow = (int64_t)B * m->nout;
@@ -353,7 +481,11 @@ int ensure_capacity(mg_context* ctx, mg_mlp* m, int64_t B) {
       return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: activation allocation failed");
     }
   }
-  if (cudaMalloc(&m->Y, sizeof(float) * ow) != cudaSuccess || cudaMalloc(&m->dY, sizeof(float) * ow) != cudaSuccess) {
+  const int64_t np = max_splits(m->nh, m->nin, B, ctx->num_sms) * m->oW2 +
+                     max_splits(m->nh, m->nh, B, ctx->num_sms) * (m->oW3 - m->oW2) +
+                     max_splits(m->nout, m->nh, B, ctx->num_sms) * (m->nparam - m->oW3);
+  if (cudaMalloc(&m->Y, sizeof(float) * ow) != cudaSuccess || cudaMalloc(&m->dY, sizeof(float) * ow) != cudaSuccess ||
+      cudaMalloc(&m->part, sizeof(float) * np) != cudaSuccess) {
     cudaGetLastError();
     return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: activation allocation failed");
   }
@@ -417,22 +549,22 @@ int backward(mg_context* ctx, mg_mlp* m, const float* X, const float* Yt, int64_
   const __nv_bfloat16* W = m->wbf;
   float* G = m->grad;
   const int nin = m->nin, nh = m->nh, no = m->nout;
+  const Split sp[3] = {split_rows(nh, nin, B, ctx->num_sms), split_rows(nh, nh, B, ctx->num_sms),
+                       split_rows(no, nh, B, ctx->num_sms)};
+  const int64_t len[3] = {m->oW2, m->oW3 - m->oW2, m->nparam - m->oW3};
+  float* const part[3] = {m->part, m->part + sp[0].splits * len[0],
+                          m->part + sp[0].splits * len[0] + sp[1].splits * len[1]};
   MG_TRY_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), s));
   loss_grad_kernel<<<grid_for(B * no), kThreads, 0, s>>>(m->Y, Yt, B, no, m->out_shift, m->out_scale, m->dY, m->loss);
   MG_COUNT_LAUNCH();
-  // layer 3: dW3 = dY^T H2, db3 = colsum dY, dH2 = dY W3 (then * SiLU'(Z2))
-  MG_TRY_CUDA((gemm<true, true>(s, no, nh, (int)B, m->dY, no, m->H2, nh, EpiStore{G + m->oW3, nh})));
-  colsum_kernel<<<no, kThreads, 0, s>>>(m->dY, B, no, G + m->ob3);
-  MG_COUNT_LAUNCH();
+  // layer 3: dW3 = dY^T H2, db3 = column sums of dY, dH2 = dY W3 (then * SiLU'(Z2)); layers 2 and 1 alike
+  MG_TRY_CUDA((gemm<true, true>(s, no, nh, (int)B, m->dY, no, m->H2, nh, EpiPart{part[2], no, nh}, sp[2].splits, sp[2].kz)));
   MG_TRY_CUDA((gemm<false, true>(s, (int)B, nh, no, m->dY, no, W + m->oW3, nh, EpiSiluGrad{m->Z2, m->dA, nh})));
-  // layer 2
-  MG_TRY_CUDA((gemm<true, true>(s, nh, nh, (int)B, m->dA, nh, m->H1, nh, EpiStore{G + m->oW2, nh})));
-  colsum_kernel<<<nh, kThreads, 0, s>>>(m->dA, B, nh, G + m->ob2);
-  MG_COUNT_LAUNCH();
+  MG_TRY_CUDA((gemm<true, true>(s, nh, nh, (int)B, m->dA, nh, m->H1, nh, EpiPart{part[1], nh, nh}, sp[1].splits, sp[1].kz)));
   MG_TRY_CUDA((gemm<false, true>(s, (int)B, nh, nh, m->dA, nh, W + m->oW2, nh, EpiSiluGrad{m->Z1, m->dB, nh})));
-  // layer 1
-  MG_TRY_CUDA((gemm<true, true>(s, nh, nin, (int)B, m->dB, nh, X, nin, EpiStore{G + m->oW1, nin})));
-  colsum_kernel<<<nh, kThreads, 0, s>>>(m->dB, B, nh, G + m->ob1);
+  MG_TRY_CUDA((gemm<true, true>(s, nh, nin, (int)B, m->dB, nh, X, nin, EpiPart{part[0], nh, nin}, sp[0].splits, sp[0].kz)));
+  const PartLayers L{{part[0], part[1], part[2]}, {0, m->oW2, m->oW3, m->nparam}, {sp[0].splits, sp[1].splits, sp[2].splits}};
+  reduce_grad_kernel<<<(unsigned)((m->nparam + kThreads - 1) / kThreads), kThreads, 0, s>>>(L, G);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   return MG_OK;
@@ -551,7 +683,7 @@ int mg_mlp_create(mg_context* ctx, int32_t nin, int32_t nh, int32_t nout, mg_mlp
 void mg_mlp_destroy(mg_mlp* m) {
   if (!m) return;
   void* ps[] = {m->master, m->m1, m->m2, m->grad, m->wbf, m->out_shift, m->out_scale, m->loss,
-                m->Z1, m->H1, m->Z2, m->H2, m->Y, m->dY, m->dA, m->dB,
+                m->Z1, m->H1, m->Z2, m->H2, m->Y, m->dY, m->dA, m->dB, m->part,
                 m->Xb, m->H1b, m->H2b, m->tc_err};
   for (void* p : ps)
     if (p) cudaFree(p);
