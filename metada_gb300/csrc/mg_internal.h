@@ -80,6 +80,9 @@ cudaError_t launch_obs_prior(const double* HX, const double* yo, const double* r
                              int k, double* Y64, float* Y32, double* d, double* rinv,
                              cudaStream_t s);
 
+// Workspace that mg_select_grid takes (from the start of the context's) for npt grid points.
+size_t select_grid_bytes(int64_t npt);
+
 // Tensor-core GEMM (tcgen05): C = A B^T + bias, SiLU if act != 0; A (M x K)
 // and B (N x K) BF16 row-major, 16-byte aligned, 1 <= N <= 256, K % 8 == 0.
 // Writes C32 (FP32) and/or C16 (BF16) with leading dimension ldc; *err is

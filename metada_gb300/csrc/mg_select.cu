@@ -1,6 +1,6 @@
 // Local observation search (LETKF.hpp:159-165 with Location::distance_to).
 //
-// Grid coordinates: exact integer distances, one warp per grid point, obs
+// Grid coordinates: exact integer distances, a CTA per 8 x 8 points, obs
 // scanned in order and compacted with warp ballots so every list comes out
 // in obs order, as the reference builds it.
 //
@@ -62,6 +62,103 @@ __global__ void select_grid_kernel(int nx, int ny, const int32_t* __restrict__ o
     w += __popc(b);
   }
   if (!offsets && lane == 0) counts[g] = w;
+}
+
+// The same lists for 0 <= radius < 2^26 without FP64 (two lanes per clock per
+// SM) and without testing every obs at every point: the squared distance is
+// an integer below 2^53, exact in the reference's double arithmetic, and
+// sqrt is monotone, so sqrt(m) <= radius is m <= r2, r2 the largest integer
+// whose rounded square root is within the radius.  One CTA owns 8 x 8
+// points: the obs inside its box widened by the radius are compacted in obs
+// order (slabs of 256), then each warp tests that short list for the 8
+// points of one row.  (144 x 72 points, 2592 obs, radius 6: 12 us a pass, 734 us
+// over all pairs.)
+constexpr int kSelTile = 8, kSelCap = 1024;
+__global__ void __launch_bounds__(256) select_grid_tile_kernel(int nx, int ny, const int32_t* __restrict__ obs_xy,
+                                                               int64_t p, int64_t ri, int64_t r2,
+                                                               const int64_t* __restrict__ offsets,
+                                                               int64_t* __restrict__ counts,
+                                                               int32_t* __restrict__ idx) {
+  __shared__ int cx[kSelCap], cy[kSelCap], co[kSelCap];
+  __shared__ int wcnt[2][8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int x0 = blockIdx.x * kSelTile, y0 = blockIdx.y * kSelTile;
+  const int gy = y0 + warp;
+  int64_t w[kSelTile];
+#pragma unroll
+  for (int q = 0; q < kSelTile; ++q)
+    w[q] = (offsets && x0 + q < nx && gy < ny) ? offsets[(int64_t)gy * nx + x0 + q] : 0;
+  int n = 0, ph = 0;
+  for (int64_t o0 = 0; o0 < p; o0 += 256, ph ^= 1) {
+    const int64_t o = o0 + tid;
+    int x = 0, y = 0;
+    bool in = false;
+    if (o < p) {
+      x = obs_xy[2 * o];
+      y = obs_xy[2 * o + 1];
+      in = x >= x0 - ri && x <= x0 + kSelTile - 1 + ri && y >= y0 - ri && y <= y0 + kSelTile - 1 + ri;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) wcnt[ph][warp] = __popc(b);
+    __syncthreads();
+    int pos = n + __popc(b & ((1u << lane) - 1u));
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (q < warp) pos += wcnt[ph][q];
+      n += wcnt[ph][q];
+    }
+    if (in) {
+      cx[pos] = x;
+      cy[pos] = y;
+      co[pos] = (int)o;
+    }
+    if (n <= kSelCap - 256 && o0 + 256 < p) continue;
+    __syncthreads();
+    if (gy < ny) {
+      for (int c0 = 0; c0 < n; c0 += 32) {
+        const int c = c0 + lane;
+        int64_t dx0 = 0, d2y = INT64_MAX;
+        int ob = 0;
+        if (c < n) {
+          dx0 = (int64_t)x0 - cx[c];
+          const int64_t dy = (int64_t)gy - cy[c];
+          d2y = dy * dy;
+          ob = co[c];
+        }
+#pragma unroll
+        for (int q = 0; q < kSelTile; ++q) {
+          const int64_t dx = dx0 + q;
+          const bool hit = d2y <= r2 && dx * dx <= r2 - d2y && x0 + q < nx;
+          const unsigned m = __ballot_sync(0xffffffffu, hit);
+          if (idx && hit) idx[w[q] + __popc(m & ((1u << lane) - 1u))] = ob;
+          w[q] += __popc(m);
+        }
+      }
+    }
+    n = 0;
+    __syncthreads();
+  }
+  if (!offsets && lane == 0 && gy < ny) {
+#pragma unroll
+    for (int q = 0; q < kSelTile; ++q)
+      if (x0 + q < nx) counts[(int64_t)gy * nx + x0 + q] = w[q];
+  }
+}
+
+cudaError_t launch_select_grid(int nx, int ny, const int32_t* obs_xy, int64_t p, double radius,
+                               const int64_t* offsets, int64_t* counts, int32_t* idx, cudaStream_t s) {
+  const int64_t ty = (ny + kSelTile - 1) / kSelTile;
+  if (radius >= 0.0 && radius < (double)(1 << 26) && ty <= 65535) {
+    int64_t r2 = (int64_t)(radius * radius) + 4;
+    while (std::sqrt((double)r2) > radius) --r2;
+    const dim3 grid((nx + kSelTile - 1) / kSelTile, (unsigned)ty);
+    select_grid_tile_kernel<<<grid, 256, 0, s>>>(nx, ny, obs_xy, p, (int64_t)radius, r2, offsets, counts, idx);
+  } else {
+    const unsigned blocks = (unsigned)(((int64_t)nx * ny + 7) / 8);
+    select_grid_kernel<<<blocks, 256, 0, s>>>(nx, ny, obs_xy, p, radius, offsets, counts, idx);
+  }
+  MG_COUNT_LAUNCH();
+  return cudaGetLastError();
 }
 
 // ----------------------------------------------------------- geographic ---
@@ -384,6 +481,17 @@ double haversine_host(double lat1, double lon1, double lat2, double lon2) {
 
 }  // namespace
 
+namespace mg {
+
+size_t select_grid_bytes(int64_t npt) {
+  Carver cv;
+  cv.reserve<int64_t>(npt + 1);
+  cv.reserve<char>(scan_temp_bytes(npt));
+  return cv.off;
+}
+
+}  // namespace mg
+
 extern "C" {
 
 int mg_select_grid(mg_context* ctx, int32_t nx, int32_t ny, const int32_t* obs_xy, int64_t p,
@@ -393,32 +501,21 @@ int mg_select_grid(mg_context* ctx, int32_t nx, int32_t ny, const int32_t* obs_x
                "mg_select_grid: bad arguments");
   const int64_t npt = (int64_t)nx * ny;
   const size_t tmpb = mg::scan_temp_bytes(npt);
-  mg::Carver cv;
-  cv.reserve<int64_t>(npt + 1);
-  cv.reserve<char>(tmpb);
-  void* ws = mg::workspace(ctx, cv.off);
+  void* ws = mg::workspace(ctx, mg::select_grid_bytes(npt));
   if (!ws) return MG_ERR_NOMEM;
-  cv = mg::Carver{static_cast<char*>(ws), 0};
+  mg::Carver cv{static_cast<char*>(ws), 0};
   int64_t* counts = cv.take<int64_t>(npt + 1);
   void* tmp = cv.take<char>(tmpb);
-  const unsigned blocks = (unsigned)((npt + 7) / 8);
-  MG_TRY_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * (npt + 1), ctx->stream));
-  select_grid_kernel<<<blocks, 256, 0, ctx->stream>>>(nx, ny, obs_xy, p, radius, nullptr, counts,
-                                                      nullptr);
-  MG_COUNT_LAUNCH();
-  MG_TRY_CUDA(cudaGetLastError());
+  MG_TRY_CUDA(cudaMemsetAsync(counts + npt, 0, sizeof(int64_t), ctx->stream));
+  MG_TRY_CUDA(launch_select_grid(nx, ny, obs_xy, p, radius, nullptr, counts, nullptr, ctx->stream));
   MG_TRY_CUDA(mg::exclusive_scan(counts, offsets, npt, tmp, tmpb, ctx->stream));
   MG_TRY_CUDA(cudaMemcpyAsync(total, offsets + npt, sizeof(int64_t), cudaMemcpyDeviceToHost,
                               ctx->stream));
   MG_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
   if (*total > cap || (*total > 0 && !idx))
     return mg::fail(ctx, MG_ERR_CAPACITY, "mg_select_grid: index buffer too small");
-  if (*total > 0) {
-    select_grid_kernel<<<blocks, 256, 0, ctx->stream>>>(nx, ny, obs_xy, p, radius, offsets, nullptr,
-                                                        idx);
-    MG_COUNT_LAUNCH();
-    MG_TRY_CUDA(cudaGetLastError());
-  }
+  if (*total > 0)
+    MG_TRY_CUDA(launch_select_grid(nx, ny, obs_xy, p, radius, offsets, nullptr, idx, ctx->stream));
   return MG_OK;
 }
 
