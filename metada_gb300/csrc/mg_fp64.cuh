@@ -1,0 +1,34 @@
+// FP64 arithmetic in few FP64 instructions.  GB300 runs two FP64 lanes per
+// clock per SM (a warp instruction takes its scheduler's FP64 unit 64
+// cycles), and conversions between FP32 and FP64 run at the same rate, so
+// divisions are replaced by a reciprocal and corrections.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace mg {
+
+// 1 / d for d > 0 to FP64 rounding (about one ulp): an FP32 reciprocal of
+// d's leading 24 bits, moved between the formats with integer operations,
+// and r (1 + e + e^2) with e = 1 - d r, whose error is e^3 < 2^-66.
+// Outside FP32's normal range the plain division.
+__device__ __forceinline__ double recip_fp64(double d) {
+  const int hi = __double2hiint(d);
+  const int ex = (hi >> 20) - 1023;
+  if (ex < -120 || ex > 120) return 1.0 / d;
+  const float f = __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)__double2loint(d) >> 29));
+  const int rb = __float_as_int(__frcp_rn(f));
+  const double r = __hiloint2double((rb >> 3) + (896 << 20), rb << 29);
+  const double e = __fma_rn(-d, r, 1.0);
+  return __fma_rn(r, __fma_rn(e, e, e), r);
+}
+
+// a / b given r = 1 / b correctly rounded: one correction of a r by its exact
+// remainder gives the correctly rounded quotient (Markstein, 1990) while no
+// term leaves the normal range.
+__device__ __forceinline__ double div_refined(double a, double b, double r) {
+  const double q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+}  // namespace mg

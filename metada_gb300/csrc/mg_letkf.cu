@@ -1015,6 +1015,9 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
       MG_TRY_CUDA(cudaMemsetAsync(cnt + 6, 0, sizeof(unsigned long long), s));
       rc = (k <= 64) ? launch_batched<float, 64>(ctx, fb) : launch_batched<float, 96>(ctx, fb);
     }
+  } else if (fp64 && (d->flags & MG_SQRT_CHOLESKY)) {
+    MG_TRY_CUDA(mg::letkf_chol_launch(prm, ctx->num_sms, s));
+    rc = MG_OK;
   } else if (fp64) {
     if (k <= 32) rc = launch_batched<double, 32>(ctx, prm);
     else if (k <= 64) rc = launch_batched<double, 64>(ctx, prm);

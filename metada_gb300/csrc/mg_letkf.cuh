@@ -100,4 +100,7 @@ bool letkf_tc_supported(const LetkfParams& prm);
 // and the CTA count.
 int letkf_tc_launch(const LetkfParams& prm, int num_sms, void* stream, int* ctas);
 
+// FP64 local analyses with the Cholesky square root (MG_SQRT_CHOLESKY), k <= 96.
+cudaError_t letkf_chol_launch(const LetkfParams& prm, int num_sms, cudaStream_t s);
+
 }  // namespace mg
