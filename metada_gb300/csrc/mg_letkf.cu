@@ -1,5 +1,6 @@
 // Batched LETKF local analyses (replaces LETKF.hpp:101 grid loop and
-// updateGridPoint :152-243) and the sequential reference-order LETKF.
+// updateGridPoint :152-243).  The reference's sequential order is in
+// mg_letkf_seq.cu.
 //
 // One CTA (256 threads) runs one local analysis at a time, inside a
 // persistent grid that pulls analysis points from a work counter in the
@@ -694,147 +695,6 @@ int launch_batched(mg_context* ctx, LetkfParams& prm) {
   return MG_OK;
 }
 
-// ------------------------------------------------------------------------
-// Sequential LETKF in the reference's order (LETKF.hpp:101), one CTA.
-// ------------------------------------------------------------------------
-struct CompatSeqParams {
-  double* X;
-  int k, nx, ny;
-  int64_t ld;
-  const int32_t* obs_xy;
-  const uint8_t* valid;
-  const double* yo;
-  const int64_t* loc_off;
-  const int32_t* loc_idx;
-  double rho;
-  int* status;
-};
-
-__device__ __forceinline__ double idw4_seq(const double* x, int nx, int ny, int ox, int oy) {
-  const double xx = fmax(0.0, fmin((double)(nx - 1), (double)ox));
-  const double yy = fmax(0.0, fmin((double)(ny - 1), (double)oy));
-  const long long i0 = (long long)floor(xx), j0 = (long long)floor(yy);
-  const long long i1 = min(i0 + 1, (long long)nx - 1), j1 = min(j0 + 1, (long long)ny - 1);
-  const long long ii[4] = {i0, i1, i0, i1}, jj[4] = {j0, j0, j1, j1};
-  double ws = 0.0, wsum = 0.0;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const double dx = __dsub_rn(xx, (double)ii[t]), dy = __dsub_rn(yy, (double)jj[t]);
-    const double dist = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-    const double w = (dist == 0.0) ? 1e12 : __ddiv_rn(1.0, dist);
-    ws = __dadd_rn(ws, __dmul_rn(w, x[jj[t] * nx + ii[t]]));
-    wsum = __dadd_rn(wsum, w);
-  }
-  return __ddiv_rn(ws, wsum);
-}
-
-template <int KMAX>
-__global__ void __launch_bounds__(kThreads) letkf_compat_seq_kernel(CompatSeqParams prm) {
-  constexpr int LDA = KMAX + 1, CH = 64;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* A = reinterpret_cast<double*>(smem_raw);
-  double* V = A + KMAX * LDA;
-  double* Ys = V + KMAX * LDA;  // CH x KMAX
-  double* dd = Ys + CH * KMAX;  // CH
-  double* bvec = dd + CH;       // KMAX
-  double* wa = bvec + KMAX;     // KMAX
-  double* xb = wa + KMAX;       // KMAX
-  int* misc = reinterpret_cast<int*>(xb + KMAX);
-  __shared__ double s_xm;
-  const int tid = threadIdx.x, k = prm.k;
-  const int npt = prm.nx * prm.ny;
-  const double sqk = sqrt((double)(k - 1));
-  for (int g = 0; g < npt; ++g) {
-    const int64_t e0 = prm.loc_off[g], e1 = prm.loc_off[g + 1];
-    double acc[KMAX / 16][KMAX / 16];
-    constexpr int R = KMAX / 16;
-    const int ti = tid / 16, tj = tid % 16;
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-      for (int b = 0; b < R; ++b) acc[a][b] = 0.0;
-    double bacc = 0.0;
-    for (int64_t c0 = e0; c0 < e1; c0 += CH) {
-      const int cnt = (int)(e1 - c0 < (int64_t)CH ? e1 - c0 : (int64_t)CH);
-      // H_local rows from the CURRENT members (LETKF.hpp:197-206).
-      for (int e = tid; e < cnt * KMAX; e += kThreads) {
-        const int r = e / KMAX, j = e - r * KMAX;
-        double v = 0.0;
-        if (j < k) {
-          const int o = prm.loc_idx[c0 + r];
-          if (!prm.valid || prm.valid[o])
-            v = idw4_seq(prm.X + (int64_t)j * prm.ld, prm.nx, prm.ny, prm.obs_xy[2 * o],
-                         prm.obs_xy[2 * o + 1]);
-        }
-        Ys[e] = v;
-      }
-      __syncthreads();
-      if (tid < cnt) {  // row mean, anomalies, innovation (:209-211)
-        double s = 0.0;
-        for (int j = 0; j < k; ++j) s += Ys[tid * KMAX + j];
-        const double ym = s / (double)k;
-        for (int j = 0; j < k; ++j) Ys[tid * KMAX + j] -= ym;
-        dd[tid] = prm.yo[prm.loc_idx[c0 + tid]] - ym;
-      }
-      __syncthreads();
-      for (int r = 0; r < cnt; ++r) {
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = 0; b < R; ++b)
-            acc[a][b] += Ys[r * KMAX + ti + 16 * a] * Ys[r * KMAX + tj + 16 * b];
-      }
-      if (tid < k)
-        for (int r = 0; r < cnt; ++r) bacc += Ys[r * KMAX + tid] * dd[r];
-      __syncthreads();
-    }
-    if (tid < k) xb[tid] = prm.X[(int64_t)tid * prm.ld + g];
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      for (int i = 0; i < k; ++i) s += xb[i];
-      s_xm = s / (double)k;
-    }
-    __syncthreads();
-    const double xm = s_xm;
-    if (e1 == e0) {  // LETKF.hpp:167-190
-      const double sr = sqrt(prm.rho);
-      if (tid < k) prm.X[(int64_t)tid * prm.ld + g] = xm + (xb[tid] - xm) * sr;
-      __syncthreads();
-      continue;
-    }
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-      for (int b = 0; b < R; ++b) {
-        const int i = ti + 16 * a, j = tj + 16 * b;
-        if (i < k && j < k) A[i * LDA + j] = acc[a][b] + (i == j ? (double)(k - 1) : 0.0);
-      }
-    if (tid < k) bvec[tid] = bacc;
-    __syncthreads();
-    bool ok = mg::cta_cholesky<double>(A, k, LDA, misc);
-    mg::cta_lower_inverse<double>(A, V, k, LDA);
-    mg::cta_gram_of_lower<double>(V, A, k, LDA);
-    for (int e = tid; e < k * k; e += kThreads) A[(e / k) * LDA + e % k] *= prm.rho;
-    __syncthreads();
-    if (tid < k) {
-      double s = 0.0;
-      for (int j = 0; j < k; ++j) s += A[tid * LDA + j] * bvec[j];
-      wa[tid] = s;
-    }
-    __syncthreads();
-    ok = mg::cta_cholesky<double>(A, k, LDA, misc) && ok;
-    if (!ok && tid == 0) atomicExch(prm.status, 1);
-    if (tid < k) {  // :227-242, in place
-      const double xp = xb[tid] - xm;
-      double rs = 0.0;
-      for (int j = 0; j < k; ++j) rs += xp * (sqk * A[tid * LDA + j]);
-      prm.X[(int64_t)tid * prm.ld + g] = (xm + xp * wa[tid]) + rs;
-    }
-    __syncthreads();
-  }
-}
-
 }  // namespace
 
 extern "C" {
@@ -1071,74 +931,6 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   if ((int)(host_cnt[4] & 0xffffffffull) != 0)
     return mg::fail(ctx, MG_ERR_NUMERIC, "mg_letkf_batched: a local k x k system was not positive definite");
   return MG_OK;
-}
-
-int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,
-                         const int32_t* obs_xy, const uint8_t* valid, const double* yo, int64_t p,
-                         double radius, double rho, double* mean_out) {
-  if (!ctx) return MG_ERR_ARG;
-  MG_CHECK_ARG(X && k >= 2 && k <= 64 && nx > 0 && ny > 0 && ld >= (int64_t)nx * ny && p >= 0 &&
-                   (p == 0 || (obs_xy && yo)) && rho > 0.0,
-               "mg_letkf_compat_grid: bad arguments (k must be 2..64)");
-  const int64_t npt = (int64_t)nx * ny;
-  // Local lists by grid distance (independent of the in-place updates).
-  // mg_select_grid uses the context workspace, so these live apart from it.
-  int64_t total = 0;
-  int64_t* off_tmp = nullptr;
-  int32_t* idx = nullptr;
-  int* status = nullptr;
-  MG_TRY_CUDA(cudaMalloc(&off_tmp, sizeof(int64_t) * (npt + 1)));
-  int rc = mg_select_grid(ctx, nx, ny, obs_xy, p, radius, off_tmp, nullptr, 0, &total);
-  if (rc != MG_OK && rc != MG_ERR_CAPACITY) {
-    cudaFree(off_tmp);
-    return rc;
-  }
-  if (cudaMalloc(&idx, sizeof(int32_t) * (total + 1)) != cudaSuccess ||
-      cudaMalloc(&status, sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(off_tmp);
-    cudaFree(idx);
-    return mg::fail(ctx, MG_ERR_NOMEM, "mg_letkf_compat_grid: allocation failed");
-  }
-  rc = mg_select_grid(ctx, nx, ny, obs_xy, p, radius, off_tmp, idx, total, &total);
-  if (rc == MG_OK) {
-    MG_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(int), ctx->stream));
-    CompatSeqParams prm{X, k, nx, ny, ld, obs_xy, valid, yo, off_tmp, idx, rho, status};
-    const int kmax = k <= 32 ? 32 : 64;
-    const size_t smem = sizeof(double) * (2 * (size_t)kmax * (kmax + 1) + 64 * (size_t)kmax + 64 +
-                                          3 * (size_t)kmax) + 64;
-    cudaError_t e;
-    if (kmax == 32) {
-      e = cudaFuncSetAttribute(letkf_compat_seq_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-      if (e == cudaSuccess) letkf_compat_seq_kernel<32><<<1, kThreads, smem, ctx->stream>>>(prm);
-      if (e == cudaSuccess) MG_COUNT_LAUNCH();
-    } else {
-      e = cudaFuncSetAttribute(letkf_compat_seq_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-      if (e == cudaSuccess) letkf_compat_seq_kernel<64><<<1, kThreads, smem, ctx->stream>>>(prm);
-      if (e == cudaSuccess) MG_COUNT_LAUNCH();
-    }
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) rc = mg::fail(ctx, MG_ERR_CUDA, std::string("letkf_compat_seq: ") + cudaGetErrorString(e));
-    if (rc == MG_OK && mean_out) {
-      e = mg::launch_mean_pert_members(X, npt, k, ld, mean_out, nullptr, nullptr, 0, ctx->stream);
-      if (e != cudaSuccess) rc = mg::fail(ctx, MG_ERR_CUDA, cudaGetErrorString(e));
-    }
-    int hs = 0;
-    if (rc == MG_OK) {
-      e = cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-      if (e != cudaSuccess) rc = mg::fail(ctx, MG_ERR_CUDA, cudaGetErrorString(e));
-      else if (hs != 0)
-        rc = mg::fail(ctx, MG_ERR_NUMERIC, "mg_letkf_compat_grid: a local k x k system was not positive definite");
-    }
-  }
-  cudaStreamSynchronize(ctx->stream);
-  cudaFree(idx);
-  cudaFree(status);
-  cudaFree(off_tmp);
-  return rc;
 }
 
 }  // extern "C"
