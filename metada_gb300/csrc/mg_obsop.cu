@@ -2,41 +2,69 @@
 // innovation).  Arithmetic that must be bit-identical to the reference uses
 // explicitly rounded intrinsics so the compiler cannot contract a multiply
 // and an add into one FMA.
+#include <algorithm>
+#include <cmath>
+
+#include "mg_fp64.cuh"
 #include "mg_internal.h"
 
 namespace {
 
-// IdentityObsOperator.hpp:594-617 (2-D branch) and :643-676 for an obs at
-// integer grid coordinates (ox, oy) on member x.
-__device__ __forceinline__ double idw4(const double* __restrict__ x, int nx, int ny, int ox,
-                                       int oy) {
-  const double xx = fmax(0.0, fmin((double)(nx - 1), (double)ox));
-  const double yy = fmax(0.0, fmin((double)(ny - 1), (double)oy));
-  const long long i0 = (long long)floor(xx), j0 = (long long)floor(yy);
-  const long long i1 = min(i0 + 1, (long long)nx - 1), j1 = min(j0 + 1, (long long)ny - 1);
-  const long long ii[4] = {i0, i1, i0, i1}, jj[4] = {j0, j0, j1, j1};
-  double ws = 0.0, wsum = 0.0;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const double dx = __dsub_rn(xx, (double)ii[t]), dy = __dsub_rn(yy, (double)jj[t]);
-    const double dist = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-    const double w = (dist == 0.0) ? 1e12 : __ddiv_rn(1.0, dist);
-    ws = __dadd_rn(ws, __dmul_rn(w, __ldg(x + jj[t] * nx + ii[t])));
-    wsum = __dadd_rn(wsum, w);
+// IDW4 at integer grid coordinates (IdentityObsOperator.hpp:594-617, 2-D
+// branch, and :643-676).  The four neighbours lie at distance 0, 1 or
+// sqrt(2), or collapse onto each other at the grid's last column and row, so
+// there are four weight sets, by (last column, last row); the host computes
+// them with the reference's operations (IEEE square root and division).
+struct Idw4Weights {
+  double w[4][4];
+  double wsum[4], rinv[4];  // rinv: 1 / wsum rounded
+};
+
+Idw4Weights idw4_weights() {
+  Idw4Weights t;
+  for (int c = 0; c < 4; ++c) {
+    t.wsum[c] = 0.0;
+    for (int q = 0; q < 4; ++q) {
+      const double dx = (c & 1) ? 0.0 : (double)(q & 1), dy = (c & 2) ? 0.0 : (double)(q >> 1);
+      const double dist = std::sqrt(dx * dx + dy * dy);
+      t.w[c][q] = dist == 0.0 ? 1e12 : 1.0 / dist;
+      t.wsum[c] += t.w[c][q];
+    }
+    t.rinv[c] = 1.0 / t.wsum[c];
   }
-  return __ddiv_rn(ws, wsum);
+  return t;
 }
 
-__global__ void hx_idw4_kernel(const double* __restrict__ X, int k, int64_t ld, int nx, int ny,
-                               const int32_t* __restrict__ obs_xy, const uint8_t* __restrict__ valid,
-                               int64_t p, double* __restrict__ HX) {
+// One thread per (obs, member).  Eight separately rounded FP64 operations for
+// the weighted sum and a division: by Markstein's theorem (1990) one
+// correction of ws * RN(1 / wsum) by its exact remainder is the correctly
+// rounded quotient away from the ends of the exponent range, where the plain
+// division is taken.  (The weights' square roots and divisions per value
+// took 250 us for 20,000 obs x 64 members, now 34 us.)
+__global__ void __launch_bounds__(256) hx_idw4_kernel(const double* __restrict__ X, int k, int64_t ld, int nx, int ny,
+                                                      const int32_t* __restrict__ obs_xy,
+                                                      const uint8_t* __restrict__ valid, int64_t p, Idw4Weights wt,
+                                                      double* __restrict__ HX) {
   const int64_t total = p * k;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
     const int64_t o = e / k;
     const int i = (int)(e - o * k);
     double v = 0.0;
-    if (!valid || valid[o]) v = idw4(X + (int64_t)i * ld, nx, ny, obs_xy[2 * o], obs_xy[2 * o + 1]);
+    if (!valid || valid[o]) {
+      const int i0 = max(0, min(nx - 1, obs_xy[2 * o])), j0 = max(0, min(ny - 1, obs_xy[2 * o + 1]));
+      const int i1 = min(i0 + 1, nx - 1), j1 = min(j0 + 1, ny - 1);
+      const int c = (i1 == i0) | (j1 == j0) << 1;
+      const double* x = X + (int64_t)i * ld;
+      const double x0 = __ldg(x + (int64_t)j0 * nx + i0), x1 = __ldg(x + (int64_t)j0 * nx + i1);
+      const double x2 = __ldg(x + (int64_t)j1 * nx + i0), x3 = __ldg(x + (int64_t)j1 * nx + i1);
+      double ws = __dadd_rn(0.0, __dmul_rn(wt.w[c][0], x0));
+      ws = __dadd_rn(ws, __dmul_rn(wt.w[c][1], x1));
+      ws = __dadd_rn(ws, __dmul_rn(wt.w[c][2], x2));
+      ws = __dadd_rn(ws, __dmul_rn(wt.w[c][3], x3));
+      const unsigned ex = ((unsigned)__double2hiint(ws) >> 20) & 0x7ff;
+      v = (ex > 200 && ex < 2000) ? mg::div_refined(ws, wt.wsum[c], wt.rinv[c]) : __ddiv_rn(ws, wt.wsum[c]);
+    }
     HX[e] = v;
   }
 }
@@ -141,30 +169,62 @@ __global__ void __launch_bounds__(256) hx_latlon_kernel(const TX* __restrict__ X
   }
 }
 
-// One warp per observation: ym = (sum_i HX[o,i]) / k (rowwise().mean()),
-// Y' = HX - ym, d = yo - ym, rinv = 1 / rvar.
-__global__ void obs_prior_kernel(const double* __restrict__ HX, const double* __restrict__ yo,
-                                 const double* __restrict__ rvar, int64_t p, int k,
-                                 double* __restrict__ Y64, float* __restrict__ Y32,
-                                 double* __restrict__ d, double* __restrict__ rinv) {
+// ym = (sum_i HX[o,i]) / k (rowwise().mean()), Y' = HX - ym, d = yo - ym,
+// rinv = 1 / rvar.  A warp takes `rows` obs (32, fewer when that would leave
+// SMs without a warp per scheduler): 1 / rvar for all of them at once,
+// then the rows four at a time, their lane sums reduced together (each
+// exchange halves the rows a lane carries, so four rows take six additions
+// instead of twenty, in the same tree) and one division for the four means.
+// FP64 warp instructions are what bounds this (64 cycles each): about six a
+// row instead of fifty; 500,000 obs x 64 members 737 -> 289 us.
+__global__ void __launch_bounds__(256) obs_prior_kernel(const double* __restrict__ HX, const double* __restrict__ yo,
+                                                        const double* __restrict__ rvar, int64_t p, int k, int rows,
+                                                        double* __restrict__ Y64, float* __restrict__ Y32,
+                                                        double* __restrict__ d, double* __restrict__ rinv) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t o = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); o < p; o += warps) {
-    const double* h = HX + o * k;
-    double s = 0.0;
-    for (int i = lane; i < k; i += 32) s += h[i];
+  const double dk = (double)k, rk = 1.0 / dk;
+  for (int64_t ob = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rows; ob < p;
+       ob += warps * rows) {
+    const int nob = p - ob < rows ? (int)(p - ob) : rows;
+    if (rinv && lane < nob) rinv[ob + lane] = 1.0 / rvar[ob + lane];
+    const double yl = (d && lane < nob) ? yo[ob + lane] : 0.0;
+    double dl = 0.0;  // d of obs ob + lane
+    for (int q0 = 0; q0 < nob; q0 += 4) {
+      double s[4];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    const double ym = s / (double)k;
-    for (int i = lane; i < k; i += 32) {
-      const double v = h[i] - ym;
-      if (Y64) Y64[o * k + i] = v;
-      if (Y32) Y32[o * k + i] = (float)v;
+      for (int q = 0; q < 4; ++q) {
+        s[q] = 0.0;
+        if (q0 + q < nob) {
+          const double* h = HX + (ob + q0 + q) * k;
+          for (int i = lane; i < k; i += 32) s[q] += h[i];
+        }
+      }
+      // lane bit 4 keeps rows {0, 1} or {2, 3}, bit 3 one of the two
+      const bool up = lane & 16, up2 = lane & 8;
+      double a = up ? s[2] : s[0], b = up ? s[3] : s[1];
+      a += __shfl_xor_sync(0xffffffffu, up ? s[0] : s[2], 16);
+      b += __shfl_xor_sync(0xffffffffu, up ? s[1] : s[3], 16);
+      double t = up2 ? b : a;
+      t += __shfl_xor_sync(0xffffffffu, up2 ? a : b, 8);
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+      const unsigned ex = ((unsigned)__double2hiint(t) >> 20) & 0x7ff;
+      const double ym = (ex > 200 && ex < 2000) ? mg::div_refined(t, dk, rk) : t / dk;  // row 2 (lane >> 4) + bit 3
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double m = __shfl_sync(0xffffffffu, ym, (q >> 1) * 16 + (q & 1) * 8);
+        if (q0 + q >= nob) break;
+        if (lane == q0 + q) dl = m;
+        const int64_t r = (ob + q0 + q) * k;
+        for (int i = lane; i < k; i += 32) {
+          const double v = HX[r + i] - m;
+          if (Y64) Y64[r + i] = v;
+          if (Y32) Y32[r + i] = (float)v;
+        }
+      }
     }
-    if (lane == 0) {
-      if (d) d[o] = yo[o] - ym;
-      if (rinv) rinv[o] = 1.0 / rvar[o];
-    }
+    if (d && lane < nob) d[ob + lane] = yl - dl;
   }
 }
 
@@ -183,7 +243,9 @@ cudaError_t launch_obs_prior(const double* HX, const double* yo, const double* r
                              int k, double* Y64, float* Y32, double* d, double* rinv,
                              cudaStream_t s) {
   if (p <= 0) return cudaSuccess;
-  obs_prior_kernel<<<grid_for(p * 32, 256), 256, 0, s>>>(HX, yo, rvar, p, k, Y64, Y32, d, rinv);
+  const int rows = (int)std::max<int64_t>(4, std::min<int64_t>(32, p / (152 * 16) / 4 * 4));
+  obs_prior_kernel<<<grid_for((p + rows - 1) / rows * 32, 256), 256, 0, s>>>(HX, yo, rvar, p, k, rows, Y64, Y32, d,
+                                                                             rinv);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -199,7 +261,7 @@ int mg_hx_idw4(mg_context* ctx, const double* X, int32_t k, int64_t ld, int32_t 
                "mg_hx_idw4: bad arguments");
   if (p == 0) return MG_OK;
   hx_idw4_kernel<<<grid_for(p * k, 256), 256, 0, ctx->stream>>>(X, k, ld, nx, ny, obs_xy, valid, p,
-                                                                HX);
+                                                                idw4_weights(), HX);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   return MG_OK;
