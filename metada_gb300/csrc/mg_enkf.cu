@@ -18,7 +18,6 @@
 #include <algorithm>
 #include <cmath>
 
-#include "mg_dense.cuh"
 #include "mg_internal.h"
 #include "mg_update.cuh"
 
@@ -26,6 +25,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kRedBlocks = 304;
+constexpr int kSpreadBlocks = 152 * 8;
 
 // C = sum_o rinv_o U[o]^T W[o] over this CTA's obs range (U, W: p x k
 // row-major); with bout, also b = sum_o rinv_o d_o U[o].  TE is the
@@ -100,84 +100,33 @@ __global__ void __launch_bounds__(kThreads) reduce_partials_kernel(const TE* __r
   out[e] = t;
 }
 
-// T = sqrt(rho) (I + A^-1 (b 1^T + F - G)), A = G + (k-1) I, by Cholesky
-// A = L L^T and two triangular solves on the k right-hand sides.
-__global__ void __launch_bounds__(kThreads) enkf_solve_kernel(const double* __restrict__ Gpart,
-                                                              const double* __restrict__ Fpart,
-                                                              const double* __restrict__ bpart, int nblk, int k,
-                                                              double rho, double* __restrict__ T,
-                                                              float* __restrict__ T32, int* status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lda = k + 1;
-  double* A = reinterpret_cast<double*>(smem_raw);  // k x lda
-  double* B = A + (size_t)k * lda;                 // k x lda
-  __shared__ int flag;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < k * k; e += kThreads) {
-    const int i = e / k, j = e - i * k;
-    double g = 0.0, f = 0.0;
-    for (int b = 0; b < nblk; ++b) {
-      g += Gpart[(size_t)b * k * k + e];
-      f += Fpart[(size_t)b * k * k + e];
+// Mean over the members (member order, as the analyses' other means) and the
+// CTA's partial of the sum of squared perturbations, in one pass over X; the
+// second read of a state's members comes from cache.
+__global__ void __launch_bounds__(kThreads) mean_spread_kernel(const double* __restrict__ X, int64_t n, int k,
+                                                               int64_t ld, double inv_k, double* __restrict__ mean,
+                                                               double* __restrict__ partial) {
+  __shared__ double red[kThreads / 32];
+  double sq = 0.0;
+  for (int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x; s < n; s += (int64_t)gridDim.x * kThreads) {
+    double m = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < k; ++i) m = __dadd_rn(m, X[(int64_t)i * ld + s]);
+    m = __dmul_rn(m, inv_k);
+    mean[s] = m;
+#pragma unroll 8
+    for (int i = 0; i < k; ++i) {
+      const double x = X[(int64_t)i * ld + s] - m;
+      sq = __fma_rn(x, x, sq);
     }
-    double bi = 0.0;
-    for (int b = 0; b < nblk; ++b) bi += bpart[(size_t)b * k + i];
-    A[i * lda + j] = g + (i == j ? (double)(k - 1) : 0.0);
-    B[i * lda + j] = (bi + f) - g;
   }
+  for (int off = 16; off > 0; off >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, off);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
   __syncthreads();
-  const bool ok = mg::cta_cholesky<double>(A, k, lda, &flag);
-  for (int i = 0; i < k; ++i) {  // B <- L^-1 B, all columns at once
-    for (int c = tid; c < k; c += kThreads) {
-      double s = B[i * lda + c];
-      for (int m = 0; m < i; ++m) s -= A[i * lda + m] * B[m * lda + c];
-      B[i * lda + c] = s / A[i * lda + i];
-    }
-    __syncthreads();
-  }
-  for (int i = k - 1; i >= 0; --i) {  // B <- L^-T B
-    for (int c = tid; c < k; c += kThreads) {
-      double s = B[i * lda + c];
-      for (int m = i + 1; m < k; ++m) s -= A[m * lda + i] * B[m * lda + c];
-      B[i * lda + c] = s / A[i * lda + i];
-    }
-    __syncthreads();
-  }
-  const double sr = sqrt(rho);
-  for (int e = tid; e < k * k; e += kThreads) {
-    const int i = e / k, j = e - i * k;
-    const double t = sr * ((i == j ? 1.0 : 0.0) + B[i * lda + j]);
-    T[i * k + j] = t;
-    if (T32) T32[i * k + j] = (float)t;
-  }
-  if (tid == 0 && !ok) *status = 1;
-}
-
-// Xa_i[s] = xm[s] + sum_j X'_j[s] T_ji for a tile of 32 state indices.
-template <typename TE>
-__global__ void __launch_bounds__(kThreads) enkf_update_kernel(const TE* __restrict__ Xp, int64_t ldp,
-                                                               const double* __restrict__ mean,
-                                                               const double* __restrict__ T, int64_t n, int k,
-                                                               double* __restrict__ X, int64_t ld) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TE* Ts = reinterpret_cast<TE*>(smem_raw);  // k x k
-  TE* Xt = Ts + k * k;                       // 32 x (k + 1)
-  const int64_t s0 = (int64_t)blockIdx.x * 32;
-  for (int e = threadIdx.x; e < k * k; e += kThreads) Ts[e] = (TE)T[e];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int j = warp; j < k; j += kThreads / 32) {
-    const int64_t s = s0 + lane;
-    Xt[lane * (k + 1) + j] = (s < n) ? Xp[(int64_t)j * ldp + s] : TE(0);
-  }
-  __syncthreads();
-  const int64_t s = s0 + lane;
-  if (s < n) {
-    const double m = mean[s];
-    for (int i = warp; i < k; i += kThreads / 32) {
-      TE acc = TE(0);
-      for (int j = 0; j < k; ++j) acc += Xt[lane * (k + 1) + j] * Ts[j * k + i];
-      X[(int64_t)i * ld + s] = m + (double)acc;
-    }
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
+    partial[blockIdx.x] = t;
   }
 }
 
@@ -251,11 +200,18 @@ int reduce_partials(mg_context* ctx, const TE* part, int nblk, int64_t len, doub
   return MG_OK;
 }
 
-int launch_solve(mg_context* ctx, const double* G, const double* F, const double* b, int k, double rho, double* T,
-                 float* T32, int* status) {
-  const size_t smem = sizeof(double) * 2 * (size_t)k * (k + 1);
-  MG_TRY_CUDA(cudaFuncSetAttribute(enkf_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  enkf_solve_kernel<<<1, kThreads, smem, ctx->stream>>>(G, F, b, 1, k, rho, T, T32, status);
+// Mean and, when sum is given, the sum of squared perturbations.
+int mean_spread(mg_context* ctx, const double* X, int64_t n, int k, int64_t ld, double* mean, double* partial,
+                double* sum) {
+  cudaStream_t s = ctx->stream;
+  if (!sum) {
+    MG_TRY_CUDA(mg::launch_mean_pert_members(X, n, k, ld, mean, nullptr, nullptr, 0, s));
+    return MG_OK;
+  }
+  const int nb = (int)std::min<int64_t>((n + kThreads - 1) / kThreads, kSpreadBlocks);
+  mean_spread_kernel<<<nb, kThreads, 0, s>>>(X, n, k, ld, 1.0 / (double)k, mean, partial);
+  MG_COUNT_LAUNCH();
+  sum_partials_kernel<<<1, kThreads, 0, s>>>(partial, nb, sum);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   return MG_OK;
@@ -280,69 +236,51 @@ int finish(mg_context* ctx, int64_t n, int k, double rho, const double* mean, do
   return MG_OK;
 }
 
-// FP64 path: every stage in FP64, the analysis mean and spread recomputed
-// from the analysed members in member order.
+// FP64 path: every stage in FP64 (the contractions by exact splitting on the
+// tensor cores), the analysis mean and spread recomputed from the analysed
+// members in member order.
 int run_enkf_fp64(mg_context* ctx, double* X, int64_t n, int k, int64_t ld, const double* HX, const double* yo,
                   const double* rvar, const double* eps, int64_t p, double rho, double* mean_out,
                   mg_enkf_diag* diag) {
-  const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((p + 255) / 256, 2 * ctx->num_sms));
-  const int64_t per_block = (p + nblk - 1) / nblk;
+  const int nblk = mg::cross_blocks(p, ctx->num_sms);
   const int64_t kk = (int64_t)k * k;
   mg::Carver cv;
-  cv.reserve<double>(n);
-  cv.reserve<double>((size_t)n * k);
-  cv.reserve<double>((size_t)(p + 1) * k);
-  cv.reserve<double>(p + 1);
-  cv.reserve<double>(p + 1);
-  cv.reserve<double>((size_t)nblk * kk);
-  cv.reserve<double>((size_t)nblk * kk);
-  cv.reserve<double>((size_t)nblk * k);
-  cv.reserve<double>(2 * kk + k);
-  cv.reserve<double>(kk);
-  cv.reserve<double>(kRedBlocks);
-  cv.reserve<double>(4);
-  cv.reserve<int>(4);
-  void* ws = mg::workspace(ctx, cv.off);
-  if (!ws) return MG_ERR_NOMEM;
-  cv = mg::Carver{static_cast<char*>(ws), 0};
-  double* mean = cv.take<double>(n);
-  double* Xp = cv.take<double>((size_t)n * k);
-  double* Y = cv.take<double>((size_t)(p + 1) * k);
-  double* dinn = cv.take<double>(p + 1);
-  double* rinv = cv.take<double>(p + 1);
-  double* Gpart = cv.take<double>((size_t)nblk * kk);
-  double* Fpart = cv.take<double>((size_t)nblk * kk);
-  double* bpart = cv.take<double>((size_t)nblk * k);
-  double* GFb = cv.take<double>(2 * kk + k);
-  double* T = cv.take<double>(kk);
-  double* red = cv.take<double>(kRedBlocks);
-  double* sums = cv.take<double>(4);
-  int* status = cv.take<int>(4);
+  double *mean = nullptr, *Y = nullptr, *dinn = nullptr, *rinv = nullptr, *Gpart = nullptr, *Fpart = nullptr;
+  double *T = nullptr, *red = nullptr, *sums = nullptr;
+  int* status = nullptr;
+  for (int pass = 0; pass < 2; ++pass) {
+    mean = cv.take<double>(n);
+    Y = cv.take<double>((size_t)(p + 1) * k);
+    dinn = cv.take<double>(p + 1);
+    rinv = cv.take<double>(p + 1);
+    Gpart = cv.take<double>((size_t)nblk * (kk + k));
+    Fpart = cv.take<double>((size_t)nblk * kk);
+    T = cv.take<double>(kk);
+    red = cv.take<double>(kSpreadBlocks);
+    sums = cv.take<double>(4);
+    status = cv.take<int>(4);
+    if (pass == 1) break;
+    void* ws = mg::workspace(ctx, cv.off);
+    if (!ws) return MG_ERR_NOMEM;
+    cv = mg::Carver{static_cast<char*>(ws), 0};
+  }
   cudaStream_t s = ctx->stream;
   int rc;
-  MG_TRY_CUDA(mg::launch_mean_pert_members(X, n, k, ld, mean, Xp, nullptr, n, s));
+  if ((rc = mean_spread(ctx, X, n, k, ld, mean, red, diag ? sums + 1 : nullptr)) != MG_OK) return rc;
   MG_TRY_CUDA(mg::launch_obs_prior(HX, yo, rvar, p, k, Y, nullptr, dinn, rinv, s));
-  if (diag) {
-    if ((rc = sumsq<double>(ctx, dinn, p, red, sums + 0)) != MG_OK) return rc;
-    if ((rc = sumsq<double>(ctx, Xp, (int64_t)n * k, red, sums + 1)) != MG_OK) return rc;
+  if (diag && (rc = sumsq<double>(ctx, dinn, p, red, sums + 0)) != MG_OK) return rc;
+  MG_TRY_CUDA(mg::launch_gram_fp64(Y, rinv, dinn, p, k, nblk, Gpart, s));
+  MG_TRY_CUDA(mg::launch_cross_fp64(Y, eps, rinv, p, k, nblk, Fpart, s));
+  if (nblk > 1) {
+    MG_TRY_CUDA(mg::launch_reduce_parts(Gpart, nblk, kk + k, Gpart, s));
+    MG_TRY_CUDA(mg::launch_reduce_parts(Fpart, nblk, kk, Fpart, s));
   }
-  if ((rc = launch_cross<double>(ctx, Y, Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart)) != MG_OK ||
-      (rc = launch_cross<double>(ctx, Y, eps, rinv, dinn, p, k, nblk, per_block, Fpart, nullptr)) != MG_OK ||
-      (rc = reduce_partials<double>(ctx, Gpart, nblk, kk, GFb)) != MG_OK ||
-      (rc = reduce_partials<double>(ctx, Fpart, nblk, kk, GFb + kk)) != MG_OK ||
-      (rc = reduce_partials<double>(ctx, bpart, nblk, k, GFb + 2 * kk)) != MG_OK)
-    return rc;
   MG_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * 4, s));
-  if ((rc = launch_solve(ctx, GFb, GFb + kk, GFb + 2 * kk, k, rho, T, nullptr, status)) != MG_OK) return rc;
-  const size_t usmem = sizeof(double) * ((size_t)k * k + 32 * (size_t)(k + 1));
-  MG_TRY_CUDA(cudaFuncSetAttribute(enkf_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)usmem));
-  enkf_update_kernel<double><<<(unsigned)((n + 31) / 32), kThreads, usmem, s>>>(Xp, n, mean, T, n, k, X, ld);
-  MG_COUNT_LAUNCH();
-  MG_TRY_CUDA(cudaGetLastError());
+  MG_TRY_CUDA(mg::launch_enkf_chol(Gpart, Fpart, Gpart + kk, k, rho, T, nullptr, status, s));
+  // X' carries sqrt(rho) in T, whose columns also hold the identity.
+  MG_TRY_CUDA(mg::launch_update_fp64(X, ld, n, k, mean, T, ctx->num_sms, s));
   // Analysis mean and perturbations (Ensemble::RecomputeMean/Perturbations).
-  MG_TRY_CUDA(mg::launch_mean_pert_members(X, n, k, ld, mean, diag ? Xp : nullptr, nullptr, n, s));
-  if (diag && (rc = sumsq<double>(ctx, Xp, (int64_t)n * k, red, sums + 2)) != MG_OK) return rc;
+  if ((rc = mean_spread(ctx, X, n, k, ld, mean, red, diag ? sums + 2 : nullptr)) != MG_OK) return rc;
   return finish(ctx, n, k, rho, mean, mean_out, status, sums, diag);
 }
 
@@ -520,7 +458,7 @@ int run_enkf_mixed(mg_context* ctx, double* X, int64_t n, int k, int64_t ld, con
       (rc = reduce_partials<float>(ctx, bpart, nblk, k, GFb + 2 * kk)) != MG_OK)
     return rc;
   MG_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * 4, s));
-  if ((rc = launch_solve(ctx, GFb, GFb + kk, GFb + 2 * kk, k, rho, T, T32, status)) != MG_OK) return rc;
+  MG_TRY_CUDA(mg::launch_enkf_chol(GFb, GFb + kk, GFb + 2 * kk, k, rho, T, T32, status, s));
   const size_t usmem = mg::upd_bytes(k);
   MG_TRY_CUDA(cudaFuncSetAttribute(enkf_update_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)usmem));

@@ -2,18 +2,16 @@
 //
 //   1. mean + perturbations (Ensemble.hpp:105-151), member-major;
 //   2. obs-space prior ym, Y' = HX - ym, d = yo - ym (ETKF.hpp:128-141);
-//   3. Gram G = Y'^T R^-1 Y' and b = Y'^T R^-1 d: every CTA reduces a
-//      contiguous obs range into register tiles, partials summed in a fixed
-//      order (deterministic) in FP64;
-//   4. one CTA solves the k x k system (Cholesky path = the reference's
-//      inverse + llt; or the Jacobi symmetric square root) into the
+//   3. Gram G = Y'^T R^-1 Y' and b = Y'^T R^-1 d by obs ranges, partials
+//      summed in a fixed order (deterministic), FP64 by exact splitting on
+//      the tensor cores (mg_fp64gemm.cu);
+//   4. the k x k system: the reference's inverse + llt by one factorisation
+//      (mg_solve.cu), or one CTA's Jacobi symmetric square root, into the
 //      transform T (T_ji = rho (wa_j + W_ji) for the reference, whose
 //      perturbations carry the inflation, ETKF.hpp:125);
-//   5. Xa_i = xm + sum_j X'_j T_ji, streamed over state tiles.
-// The Gram, its reduction and the k x k solve are FP64 on both paths (one
-// system per analysis, negligible cost; the small eigenvalues of
-// (k-1)I + Y'^T R^-1 Y' need it); the mixed path stores X' in FP32 and runs
-// the O(n k^2) update in FP32.
+//   5. Xa_i = xm + sum_j X'_j T_ji over state tiles (mg_fp64gemm.cu).
+// The Gram and the k x k solve are FP64 on both paths; the mixed path stores
+// X' in FP32 and runs the O(n k^2) update in FP32.
 // The reference never recomputes the ensemble mean after the update
 // (ETKF.hpp:190-191); mean_out receives that background mean.
 #include <algorithm>
@@ -26,66 +24,10 @@ namespace {
 
 constexpr int kThreads = 256;
 
-template <typename TE, int KMAX>
-__global__ void __launch_bounds__(kThreads) gram_partial_kernel(
-    const TE* __restrict__ Y, const double* __restrict__ rinv, const double* __restrict__ dinn,
-    int64_t p, int k, int64_t per_block, double* __restrict__ Gpart, double* __restrict__ bpart) {
-  constexpr int CH = (KMAX * sizeof(TE) > 512) ? 32 : 64, R = KMAX / 16;
-  __shared__ TE Ys[CH * KMAX];
-  __shared__ TE sr[CH], sd[CH];
-  const int tid = threadIdx.x, ti = tid / 16, tj = tid % 16;
-  const int64_t o0 = (int64_t)blockIdx.x * per_block;
-  const int64_t o1 = min(p, o0 + per_block);
-  TE acc[R][R];
-#pragma unroll
-  for (int a = 0; a < R; ++a)
-#pragma unroll
-    for (int b = 0; b < R; ++b) acc[a][b] = TE(0);
-  TE bacc = TE(0);
-  for (int64_t c0 = o0; c0 < o1; c0 += CH) {
-    const int cnt = (int)(o1 - c0 < (int64_t)CH ? o1 - c0 : (int64_t)CH);
-    for (int e = tid; e < cnt * KMAX; e += kThreads) {
-      const int r = e / KMAX, j = e - r * KMAX;
-      Ys[e] = (j < k) ? Y[(c0 + r) * k + j] : TE(0);
-    }
-    if (tid < cnt) {
-      sr[tid] = (TE)rinv[c0 + tid];
-      sd[tid] = (TE)dinn[c0 + tid];
-    }
-    __syncthreads();
-    for (int r = 0; r < cnt; ++r) {
-      const TE w = sr[r];
-      TE av[R], bv[R];
-#pragma unroll
-      for (int a = 0; a < R; ++a) av[a] = Ys[r * KMAX + ti * R + a] * w;
-#pragma unroll
-      for (int b = 0; b < R; ++b) bv[b] = Ys[r * KMAX + tj * R + b];
-#pragma unroll
-      for (int a = 0; a < R; ++a)
-#pragma unroll
-        for (int b = 0; b < R; ++b) acc[a][b] += av[a] * bv[b];
-    }
-    if (tid < k)
-      for (int r = 0; r < cnt; ++r) bacc += (Ys[r * KMAX + tid] * sr[r]) * sd[r];
-    __syncthreads();
-  }
-  double* G = Gpart + (size_t)blockIdx.x * k * k;
-#pragma unroll
-  for (int a = 0; a < R; ++a)
-#pragma unroll
-    for (int b = 0; b < R; ++b) {
-      const int i = ti * R + a, j = tj * R + b;
-      if (i < k && j < k) G[i * k + j] = (double)acc[a][b];
-    }
-  if (tid < k) bpart[(size_t)blockIdx.x * k + tid] = (double)bacc;
-}
-
-// Sums the partials (fixed order), adds the diagonal, solves, writes T.
+// Hunt: the symmetric square root (Jacobi) of the reduced system [G, b].
 template <typename TE>
-__global__ void __launch_bounds__(kThreads) etkf_solve_kernel(const double* __restrict__ Gpart,
-                                                              const double* __restrict__ bpart,
-                                                              int nblk, int k, int flags, double rho,
-                                                              double tol, int sweep_cap,
+__global__ void __launch_bounds__(kThreads) etkf_solve_kernel(const double* __restrict__ Gb, int k, int flags,
+                                                              double rho, double tol, int sweep_cap,
                                                               TE* __restrict__ Tout, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int kp = k + (k & 1), lda = kp + 1;
@@ -107,23 +49,18 @@ __global__ void __launch_bounds__(kThreads) etkf_solve_kernel(const double* __re
     const int i = e / kp, j = e % kp;
     double s = 0.0;
     if (i < k && j < k) {
-      for (int b = 0; b < nblk; ++b) s += Gpart[(size_t)b * k * k + i * k + j];
+      s = Gb[i * k + j];
       if (i == j) s += diag;
     } else if (i == j) {
       s = 1.0;
     }
     A[i * lda + j] = (TE)s;
   }
-  for (int i = tid; i < k; i += kThreads) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += bpart[(size_t)b * k + i];
-    bvec[i] = (TE)s;
-  }
+  for (int i = tid; i < k; i += kThreads) bvec[i] = (TE)Gb[k * k + i];
   __syncthreads();
   int sweeps = 0;
   // In the reference form the inflation is applied to X' rather than Pa.
-  const bool ok = mg::solve_transform<TE, 128, kThreads>(A, V, bvec, wa, lam, uvec, rot, pairbuf, misc, k, kp, lda,
-                                          flags & MG_SQRT_CHOLESKY, false, rho, (TE)tol, sweep_cap,
+  const bool ok = mg::solve_transform<TE, 128, kThreads>(A, V, bvec, wa, lam, uvec, rot, pairbuf, misc, k, kp, lda, false, false, rho, (TE)tol, sweep_cap,
                                           &sweeps);
   const TE scale = compat_infl ? (TE)rho : TE(1);
   for (int e = tid; e < k * k; e += kThreads) {
@@ -133,7 +70,7 @@ __global__ void __launch_bounds__(kThreads) etkf_solve_kernel(const double* __re
   if (tid == 0 && !ok) *status = 1;
 }
 
-// Xa_i[s] = xm[s] + sum_j X'_j[s] T_ji for a tile of 32 state indices.
+// Mixed path: Xa_i[s] = xm[s] + sum_j X'_j[s] T_ji in FP32 for a tile of 32 state indices.
 template <typename TE>
 __global__ void __launch_bounds__(kThreads) etkf_update_kernel(const TE* __restrict__ Xp, int64_t ldp,
                                                                const double* __restrict__ mean,
@@ -162,69 +99,85 @@ __global__ void __launch_bounds__(kThreads) etkf_update_kernel(const TE* __restr
   }
 }
 
-template <typename TE, int KMAX>
-cudaError_t launch_gram(const TE* Y, const double* rinv, const double* d, int64_t p, int k,
-                        int nblk, int64_t per_block, double* Gpart, double* bpart, cudaStream_t s) {
-  gram_partial_kernel<TE, KMAX><<<nblk, kThreads, 0, s>>>(Y, rinv, d, p, k, per_block, Gpart, bpart);
+// Device buffers of one analysis.
+struct EtkfBuffers {
+  double* mean;   // n
+  float* Xp;      // n x k perturbations (mixed path)
+  double* Y;      // p x k
+  double* dinn;   // p
+  double* rinv;   // p
+  double* part;   // nblk x (k x k + k)
+  double* T;      // k x k
+  int* status;
+  int nblk;
+};
+
+// Enqueues the analysis; *status is set when the k x k system fails.
+cudaError_t enqueue_etkf(const EtkfBuffers& w, bool mixed, int num_sms, double* X, int64_t n, int k, int64_t ld,
+                         const double* HX, const double* yo, const double* rvar, int64_t p, double rho, int flags,
+                         cudaStream_t s) {
+  const int64_t len = (int64_t)k * k + k;
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(w.status, 0, sizeof(int), s)) != cudaSuccess ||
+      (e = mg::launch_mean_pert_members(X, n, k, ld, w.mean, nullptr, mixed ? w.Xp : nullptr, n, s)) != cudaSuccess ||
+      (e = mg::launch_obs_prior(HX, yo, rvar, p, k, w.Y, nullptr, w.dinn, w.rinv, s)) != cudaSuccess ||
+      (e = mg::launch_gram_fp64(w.Y, w.rinv, w.dinn, p, k, w.nblk, w.part, s)) != cudaSuccess)
+    return e;
+  const bool chol = flags & MG_SQRT_CHOLESKY;
+  // The Cholesky solve sums a few partials itself; more are summed on many SMs first.
+  int nparts = w.nblk;
+  if (nparts > (chol ? 8 : 1)) {
+    if ((e = mg::launch_reduce_parts(w.part, nparts, len, w.part, s)) != cudaSuccess) return e;
+    nparts = 1;
+  }
+  if (chol) {
+    const bool compat_infl = flags & MG_INFL_COMPAT;
+    e = mg::launch_etkf_chol(w.part, nparts, k, compat_infl ? (double)(k - 1) : (double)(k - 1) / rho,
+                             compat_infl ? rho : 1.0, w.T, w.status, s);
+    if (e != cudaSuccess) return e;
+  } else {
+    const int kp = k + (k & 1);
+    const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
+    if ((e = cudaFuncSetAttribute(etkf_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem)) != cudaSuccess)
+      return e;
+    etkf_solve_kernel<double><<<1, kThreads, smem, s>>>(w.part, k, flags, rho, 1e-14, 30, w.T, w.status);
+    MG_COUNT_LAUNCH();
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (!mixed) return mg::launch_update_fp64(X, ld, n, k, w.mean, w.T, num_sms, s);
+  const size_t usmem = sizeof(float) * ((size_t)k * k + 32 * (size_t)(k + 1));
+  if ((e = cudaFuncSetAttribute(etkf_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)usmem)) != cudaSuccess)
+    return e;
+  etkf_update_kernel<float><<<(unsigned)((n + 31) / 32), kThreads, usmem, s>>>(w.Xp, n, w.mean, w.T, n, k, X, ld);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
-template <typename TE>
-int run_etkf(mg_context* ctx, double* X, int64_t n, int k, int64_t ld, const double* HX,
-             const double* yo, const double* rvar, int64_t p, double rho, int flags,
-             double* mean_out) {
-  const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((p + 255) / 256, 2 * ctx->num_sms));
-  const int64_t per_block = (p + nblk - 1) / nblk;
+int run_etkf(mg_context* ctx, bool mixed, double* X, int64_t n, int k, int64_t ld, const double* HX, const double* yo,
+             const double* rvar, int64_t p, double rho, int flags, double* mean_out) {
+  EtkfBuffers w{};
+  w.nblk = mg::cross_blocks(p, ctx->num_sms);
   mg::Carver cv;
-  cv.reserve<double>(n);
-  cv.reserve<TE>((size_t)n * k);
-  cv.reserve<double>((size_t)(p + 1) * k);
-  cv.reserve<double>(p + 1);
-  cv.reserve<double>(p + 1);
-  cv.reserve<double>((size_t)nblk * k * k);
-  cv.reserve<double>((size_t)nblk * k);
-  cv.reserve<double>((size_t)k * k);
-  cv.reserve<int>(4);
-  void* ws = mg::workspace(ctx, cv.off);
-  if (!ws) return MG_ERR_NOMEM;
-  cv = mg::Carver{static_cast<char*>(ws), 0};
-  double* mean = cv.take<double>(n);
-  TE* Xp = cv.take<TE>((size_t)n * k);
-  double* Y = cv.take<double>((size_t)(p + 1) * k);
-  double* dinn = cv.take<double>(p + 1);
-  double* rinv = cv.take<double>(p + 1);
-  double* Gpart = cv.take<double>((size_t)nblk * k * k);
-  double* bpart = cv.take<double>((size_t)nblk * k);
-  double* T = cv.take<double>((size_t)k * k);
-  int* status = cv.take<int>(4);
+  for (int pass = 0; pass < 2; ++pass) {
+    w.mean = mean_out ? mean_out : cv.take<double>(n);
+    w.Xp = cv.take<float>(mixed ? (size_t)n * k : 1);
+    w.Y = cv.take<double>((size_t)(p + 1) * k);
+    w.dinn = cv.take<double>(p + 1);
+    w.rinv = cv.take<double>(p + 1);
+    w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
+    w.T = cv.take<double>((size_t)k * k);
+    w.status = cv.take<int>(4);
+    if (pass == 1) break;
+    void* ws = mg::workspace(ctx, cv.off);
+    if (!ws) return MG_ERR_NOMEM;
+    cv = mg::Carver{static_cast<char*>(ws), 0};
+  }
   cudaStream_t s = ctx->stream;
-  const bool f64 = sizeof(TE) == 8;
-  MG_TRY_CUDA(mg::launch_mean_pert_members(X, n, k, ld, mean, f64 ? (double*)Xp : nullptr,
-                                           f64 ? nullptr : (float*)Xp, n, s));
-  MG_TRY_CUDA(mg::launch_obs_prior(HX, yo, rvar, p, k, Y, nullptr, dinn, rinv, s));
-  if (k <= 32) MG_TRY_CUDA((launch_gram<double, 32>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s)));
-  else if (k <= 64) MG_TRY_CUDA((launch_gram<double, 64>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s)));
-  else MG_TRY_CUDA((launch_gram<double, 128>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s)));
-  MG_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * 4, s));
-  const int kp = k + (k & 1);
-  const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
-  if (smem > 227 * 1024) return mg::fail(ctx, MG_ERR_ARG, "mg_etkf: k too large");
-  MG_TRY_CUDA(cudaFuncSetAttribute(etkf_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-  etkf_solve_kernel<double><<<1, kThreads, smem, s>>>(Gpart, bpart, nblk, k, flags, rho, 1e-14, 30, T, status);
-  MG_COUNT_LAUNCH();
-  MG_TRY_CUDA(cudaGetLastError());
-  const size_t usmem = sizeof(TE) * ((size_t)k * k + 32 * (size_t)(k + 1));
-  MG_TRY_CUDA(cudaFuncSetAttribute(etkf_update_kernel<TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)usmem));
-  etkf_update_kernel<TE><<<(unsigned)((n + 31) / 32), kThreads, usmem, s>>>(Xp, n, mean, T, n, k, X, ld);
-  MG_COUNT_LAUNCH();
-  MG_TRY_CUDA(cudaGetLastError());
-  if (mean_out)
-    MG_TRY_CUDA(cudaMemcpyAsync(mean_out, mean, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  MG_TRY_CUDA(enqueue_etkf(w, mixed, ctx->num_sms, X, n, k, ld, HX, yo, rvar, p, rho, flags, s));
   int hs = 0;
-  MG_TRY_CUDA(cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MG_TRY_CUDA(cudaMemcpyAsync(&hs, w.status, sizeof(int), cudaMemcpyDeviceToHost, s));
   MG_TRY_CUDA(cudaStreamSynchronize(s));
   if (hs) return mg::fail(ctx, MG_ERR_NUMERIC, "mg_etkf: the k x k system was not positive definite");
   return MG_OK;
@@ -240,8 +193,7 @@ extern "C" int mg_etkf(mg_context* ctx, double* X, int64_t n, int32_t k, int64_t
                "mg_etkf: bad arguments (k must be 2..128, p >= 1)");
   MG_CHECK_ARG(precision == MG_PREC_FP64 || precision == MG_PREC_MIXED, "mg_etkf: bad precision");
   MG_CHECK_ARG(k <= 112, "mg_etkf: k must be <= 112 (FP64 k x k solve in shared memory)");
-  if (precision == MG_PREC_FP64) return run_etkf<double>(ctx, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
-  return run_etkf<float>(ctx, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
+  return run_etkf(ctx, precision == MG_PREC_MIXED, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -299,21 +251,20 @@ cudaError_t static_scratch_for_current_device(void** addr, int* sms) {
   return cudaSuccess;
 }
 
-template <typename TE>
-int run_etkf_static(cudaStream_t s, double* X, int64_t n, int k, int64_t ld, const double* HX,
-                    const double* yo, const double* rvar, int64_t p, double rho, int flags,
-                    double* mean_out) {
+int run_etkf_static(cudaStream_t s, bool mixed, double* X, int64_t n, int k, int64_t ld, const double* HX,
+                    const double* yo, const double* rvar, int64_t p, double rho, int flags, double* mean_out) {
   void* base = nullptr;
   int num_sms = 0;
   if (static_scratch_for_current_device(&base, &num_sms) != cudaSuccess) {
     cudaGetLastError();
     return MG_ERR_CUDA;
   }
+  // The sizes that the entry point documents: what fits does not depend on
+  // how the kernels divide the work (the FP64 path needs no X' buffer).
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((p + 255) / 256, 2 * num_sms));
-  const int64_t per_block = (p + nblk - 1) / nblk;
   mg::Carver cv;
   cv.reserve<double>(n);
-  cv.reserve<TE>((size_t)n * k);
+  cv.reserve<char>((mixed ? sizeof(float) : sizeof(double)) * n * k);
   cv.reserve<double>((size_t)(p + 1) * k);
   cv.reserve<double>(p + 1);
   cv.reserve<double>(p + 1);
@@ -323,47 +274,20 @@ int run_etkf_static(cudaStream_t s, double* X, int64_t n, int k, int64_t ld, con
   cv.reserve<int>(4);
   if (cv.off > kStaticScratchBytes) return MG_ERR_CAPACITY;
   cv = mg::Carver{static_cast<char*>(base), 0};
-  double* mean = cv.take<double>(n);
-  TE* Xp = cv.take<TE>((size_t)n * k);
-  double* Y = cv.take<double>((size_t)(p + 1) * k);
-  double* dinn = cv.take<double>(p + 1);
-  double* rinv = cv.take<double>(p + 1);
-  double* Gpart = cv.take<double>((size_t)nblk * k * k);
-  double* bpart = cv.take<double>((size_t)nblk * k);
-  double* T = cv.take<double>((size_t)k * k);
-  int* status = cv.take<int>(4);
-  const bool f64 = sizeof(TE) == 8;
+  EtkfBuffers w{};
+  w.nblk = std::min(nblk, mg::cross_blocks(p, num_sms));
+  w.mean = mean_out ? mean_out : cv.take<double>(n);
+  w.Xp = cv.take<float>(mixed ? (size_t)n * k : 1);
+  w.Y = cv.take<double>((size_t)(p + 1) * k);
+  w.dinn = cv.take<double>(p + 1);
+  w.rinv = cv.take<double>(p + 1);
+  w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
+  w.T = cv.take<double>((size_t)k * k);
+  w.status = cv.take<int>(4);
   auto cuda = [](cudaError_t e) { return e == cudaSuccess ? MG_OK : (cudaGetLastError(), MG_ERR_CUDA); };
-  int rc;
-  if ((rc = cuda(mg::launch_mean_pert_members(X, n, k, ld, mean, f64 ? (double*)Xp : nullptr,
-                                              f64 ? nullptr : (float*)Xp, n, s))) != MG_OK) return rc;
-  if ((rc = cuda(mg::launch_obs_prior(HX, yo, rvar, p, k, Y, nullptr, dinn, rinv, s))) != MG_OK) return rc;
-  cudaError_t e;
-  if (k <= 32) e = launch_gram<double, 32>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s);
-  else if (k <= 64) e = launch_gram<double, 64>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s);
-  else e = launch_gram<double, 128>(Y, rinv, dinn, p, k, nblk, per_block, Gpart, bpart, s);
-  if ((rc = cuda(e)) != MG_OK) return rc;
-  // The status word carries the previous call's value: clear it.
-  if ((rc = cuda(cudaMemsetAsync(status, 0, sizeof(int) * 4, s))) != MG_OK) return rc;
-  const int kp = k + (k & 1);
-  const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
-  if (smem > 227 * 1024) return MG_ERR_ARG;
-  if ((rc = cuda(cudaFuncSetAttribute(etkf_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem))) != MG_OK) return rc;
-  etkf_solve_kernel<double><<<1, kThreads, smem, s>>>(Gpart, bpart, nblk, k, flags, rho, 1e-14, 30, T, status);
-  MG_COUNT_LAUNCH();
-  if ((rc = cuda(cudaGetLastError())) != MG_OK) return rc;
-  const size_t usmem = sizeof(TE) * ((size_t)k * k + 32 * (size_t)(k + 1));
-  if ((rc = cuda(cudaFuncSetAttribute(etkf_update_kernel<TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)usmem))) != MG_OK) return rc;
-  etkf_update_kernel<TE><<<(unsigned)((n + 31) / 32), kThreads, usmem, s>>>(Xp, n, mean, T, n, k, X, ld);
-  MG_COUNT_LAUNCH();
-  if ((rc = cuda(cudaGetLastError())) != MG_OK) return rc;
-  if (mean_out &&
-      (rc = cuda(cudaMemcpyAsync(mean_out, mean, sizeof(double) * n, cudaMemcpyDeviceToDevice, s))) != MG_OK)
-    return rc;
-  int hs = 0;
-  if ((rc = cuda(cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, s))) != MG_OK) return rc;
+  int rc, hs = 0;
+  if ((rc = cuda(enqueue_etkf(w, mixed, num_sms, X, n, k, ld, HX, yo, rvar, p, rho, flags, s))) != MG_OK) return rc;
+  if ((rc = cuda(cudaMemcpyAsync(&hs, w.status, sizeof(int), cudaMemcpyDeviceToHost, s))) != MG_OK) return rc;
   if ((rc = cuda(cudaStreamSynchronize(s))) != MG_OK) return rc;
   return hs ? MG_ERR_NUMERIC : MG_OK;
 }
@@ -377,7 +301,5 @@ extern "C" int mg_etkf_noalloc(void* stream, double* X, int64_t n, int32_t k, in
     return MG_ERR_ARG;
   if (precision != MG_PREC_FP64 && precision != MG_PREC_MIXED) return MG_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (precision == MG_PREC_FP64)
-    return run_etkf_static<double>(s, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
-  return run_etkf_static<float>(s, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
+  return run_etkf_static(s, precision == MG_PREC_MIXED, X, n, k, ld, HX, yo, rvar, p, rho, flags, mean_out);
 }

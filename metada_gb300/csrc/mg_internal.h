@@ -83,6 +83,29 @@ cudaError_t launch_obs_prior(const double* HX, const double* yo, const double* r
 // Workspace that mg_select_grid takes (from the start of the context's) for npt grid points.
 size_t select_grid_bytes(int64_t npt);
 
+// FP64 contractions on the tensor cores by exact splitting, k <= 112
+// (mg_fp64gemm.cu).  gram: nblk partials of [Y^T diag(rinv) Y (k x k),
+// Y^T diag(rinv) d (k)]; cross: nblk partials of U^T diag(rinv) V; reduce:
+// out[e] = sum over partials (out == part allowed); update: X_i <- mean +
+// sum_j (X_j - mean) T_ji in place, member-major.
+int cross_blocks(int64_t p, int num_sms);
+cudaError_t launch_gram_fp64(const double* Y, const double* rinv, const double* dinn, int64_t p, int k, int nblk,
+                             double* part, cudaStream_t s);
+cudaError_t launch_cross_fp64(const double* U, const double* V, const double* rinv, int64_t p, int k, int nblk,
+                              double* part, cudaStream_t s);
+cudaError_t launch_reduce_parts(const double* part, int nblk, int64_t len, double* out, cudaStream_t s);
+cudaError_t launch_update_fp64(double* X, int64_t ld, int64_t n, int k, const double* mean, const double* T,
+                               int num_sms, cudaStream_t s);
+
+// k x k systems by one factorisation (mg_solve.cu).  etkf: from nblk
+// partials of [G, b], T_ji = scale (wa_j + W_ji) with A = diag I + G,
+// W = sqrt(k-1) chol_L(A^-1); enkf: T = sqrt(rho) (I + A^-1 (b 1^T + F - G)).
+// *status is set to 1 (not cleared) when A is not positive definite.
+cudaError_t launch_etkf_chol(const double* part, int nblk, int k, double diag, double scale, double* T, int* status,
+                             cudaStream_t s);
+cudaError_t launch_enkf_chol(const double* G, const double* F, const double* b, int k, double rho, double* T,
+                             float* T32, int* status, cudaStream_t s);
+
 // Tensor-core GEMM (tcgen05): C = A B^T + bias, SiLU if act != 0; A (M x K)
 // and B (N x K) BF16 row-major, 16-byte aligned, 1 <= N <= 256, K % 8 == 0.
 // Writes C32 (FP32) and/or C16 (BF16) with leading dimension ldc; *err is
