@@ -422,8 +422,8 @@ typedef struct mg_letkf_stats {
   double ms_writeback;   /* device time: write-back to members and mean */
   int64_t total_sweeps;  /* Jacobi sweeps (tensor-core path: Newton-Schulz iterations)
                             summed over all analyses */
-  int64_t n_fallback;    /* tensor-core path: analyses whose residual test failed and
-                            that the SIMT Jacobi kernel re-ran */
+  int64_t n_fallback;    /* analyses that the first kernel (tensor-core, or FP64 symmetric
+                            square root) handed back and the SIMT Jacobi kernel re-ran */
   double max_residual;   /* tensor-core path: largest max |Z A Z - P| accepted */
   int32_t tensor_path;   /* 1 when the tensor-core kernel ran the analyses */
   int32_t tensor_ctas;   /* CTAs of its persistent grid */

@@ -6,8 +6,8 @@
 //      summed in a fixed order (deterministic), FP64 by exact splitting on
 //      the tensor cores (mg_fp64gemm.cu);
 //   4. the k x k system: the reference's inverse + llt by one factorisation
-//      (mg_solve.cu), or one CTA's Jacobi symmetric square root, into the
-//      transform T (T_ji = rho (wa_j + W_ji) for the reference, whose
+//      (mg_solve.cu), or the symmetric square root (mg_letkf_hunt.cu, FP64
+//      Jacobi where that does not apply), into the transform T (T_ji = rho (wa_j + W_ji) for the reference, whose
 //      perturbations carry the inflation, ETKF.hpp:125);
 //   5. Xa_i = xm + sum_j X'_j T_ji over state tiles (mg_fp64gemm.cu).
 // The Gram and the k x k solve are FP64 on both paths; the mixed path stores
@@ -24,11 +24,14 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Hunt: the symmetric square root (Jacobi) of the reduced system [G, b].
+// Hunt: the symmetric square root by FP64 Jacobi of the reduced system
+// [G, b], unless *solved says that launch_hunt_global has written T.
 template <typename TE>
 __global__ void __launch_bounds__(kThreads) etkf_solve_kernel(const double* __restrict__ Gb, int k, int flags,
                                                               double rho, double tol, int sweep_cap,
+                                                              const double* __restrict__ solved,
                                                               TE* __restrict__ Tout, int* status) {
+  if (solved && *solved != 0.0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int kp = k + (k & 1), lda = kp + 1;
   TE* A = reinterpret_cast<TE*>(smem_raw);
@@ -109,6 +112,7 @@ struct EtkfBuffers {
   double* part;   // nblk x (k x k + k)
   double* T;      // k x k
   int* status;
+  void* hunt;     // hunt_global_bytes(k), or null: the FP64 Jacobi solves every system
   int nblk;
 };
 
@@ -136,12 +140,20 @@ cudaError_t enqueue_etkf(const EtkfBuffers& w, bool mixed, int num_sms, double* 
                              compat_infl ? rho : 1.0, w.T, w.status, s);
     if (e != cudaSuccess) return e;
   } else {
+    if (w.hunt) {
+      const bool compat_infl = flags & MG_INFL_COMPAT;
+      e = mg::launch_hunt_global(w.part, k, compat_infl ? (double)(k - 1) : (double)(k - 1) / rho,
+                                 compat_infl ? rho : 1.0, w.hunt, w.T, s);
+      if (e != cudaSuccess) return e;
+    }
     const int kp = k + (k & 1);
     const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
     if ((e = cudaFuncSetAttribute(etkf_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem)) != cudaSuccess)
       return e;
-    etkf_solve_kernel<double><<<1, kThreads, smem, s>>>(w.part, k, flags, rho, 1e-14, 30, w.T, w.status);
+    etkf_solve_kernel<double><<<1, kThreads, smem, s>>>(w.part, k, flags, rho, 1e-14, 30,
+                                                             w.hunt ? mg::hunt_global_info(w.hunt, k) : nullptr, w.T,
+                                                             w.status);
     MG_COUNT_LAUNCH();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -169,6 +181,7 @@ int run_etkf(mg_context* ctx, bool mixed, double* X, int64_t n, int k, int64_t l
     w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
     w.T = cv.take<double>((size_t)k * k);
     w.status = cv.take<int>(4);
+    w.hunt = (flags & MG_SQRT_CHOLESKY) ? nullptr : cv.take<char>(mg::hunt_global_bytes(k));
     if (pass == 1) break;
     void* ws = mg::workspace(ctx, cv.off);
     if (!ws) return MG_ERR_NOMEM;
@@ -284,6 +297,8 @@ int run_etkf_static(cudaStream_t s, bool mixed, double* X, int64_t n, int k, int
   w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
   w.T = cv.take<double>((size_t)k * k);
   w.status = cv.take<int>(4);
+  if (!(flags & MG_SQRT_CHOLESKY) && cv.off + 256 + mg::hunt_global_bytes(k) <= kStaticScratchBytes)
+    w.hunt = cv.take<char>(mg::hunt_global_bytes(k));
   auto cuda = [](cudaError_t e) { return e == cudaSuccess ? MG_OK : (cudaGetLastError(), MG_ERR_CUDA); };
   int rc, hs = 0;
   if ((rc = cuda(enqueue_etkf(w, mixed, num_sms, X, n, k, ld, HX, yo, rvar, p, rho, flags, s))) != MG_OK) return rc;

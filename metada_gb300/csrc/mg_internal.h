@@ -97,6 +97,15 @@ cudaError_t launch_reduce_parts(const double* part, int nblk, int64_t len, doubl
 cudaError_t launch_update_fp64(double* X, int64_t ld, int64_t n, int k, const double* mean, const double* T,
                                int num_sms, cudaStream_t s);
 
+// The global ETKF's transform with the symmetric square root
+// (mg_letkf_hunt.cu): T_ji = out_scale (wa_j + W_ji) from Gb = [G, b],
+// A = diag I + G.  ws: hunt_global_bytes(k) of device memory; afterwards
+// *hunt_global_info(ws, k) is zero when the system was left to the FP64 Jacobi.
+size_t hunt_global_bytes(int k);
+const double* hunt_global_info(const void* ws, int k);
+cudaError_t launch_hunt_global(const double* Gb, int k, double diag, double out_scale, void* ws, double* T,
+                               cudaStream_t s);
+
 // k x k systems by one factorisation (mg_solve.cu).  etkf: from nblk
 // partials of [G, b], T_ji = scale (wa_j + W_ji) with A = diag I + G,
 // W = sqrt(k-1) chol_L(A^-1); enkf: T = sqrt(rho) (I + A^-1 (b 1^T + F - G)).

@@ -746,7 +746,7 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   cv.reserve<double>((size_t)p + 1);               // rinv
   cv.reserve<int32_t>((size_t)d->ncol);            // column order
   cv.reserve<unsigned long long>(8);               // counters
-  cv.reserve<int32_t>((size_t)npoints);            // points handed back by the tensor-core path
+  cv.reserve<int32_t>((size_t)npoints);            // points handed back by the first kernel
   cv.reserve<float4>((size_t)p + 1);               // per-obs FP32 pack (tensor-core path)
   cv.reserve<uint8_t>(bucket ? (size_t)p + 1 : 1);                          // obs level buckets
   cv.reserve<int32_t>(bucket ? (size_t)d->ncol * (d->nlev + 1) : 1);       // bucket starts
@@ -833,6 +833,7 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   const bool tensor = !fp64 && !(d->flags & MG_SOLVE_SIMT) && mg::letkf_tc_supported(prm);
   int64_t n_fallback = 0;
   int tc_ctas = 0;
+  const bool hunt64 = fp64 && !(d->flags & MG_SQRT_CHOLESKY) && !prm.warm_start;
   if (tensor) {
     // Tensor-core local analyses; the few whose residual test fails are
     // re-run by the SIMT kernel over the list the first kernel wrote.
@@ -860,11 +861,16 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
     const int e = mg::letkf_tc_launch(prm, ctx->num_sms, s, &tc_ctas);
     if (e != 0)
       return mg::fail(ctx, MG_ERR_CUDA, std::string("letkf_tc_kernel: ") + cudaGetErrorString((cudaError_t)e));
+  } else if (hunt64) {
+    // The same with the FP64 kernel that corrects an FP32 eigenbasis.
+    MG_TRY_CUDA(mg::letkf_hunt_launch(prm, ctx->num_sms, s));
+  }
+  rc = MG_OK;
+  if (tensor || hunt64) {
     unsigned long long hr = 0;
     MG_TRY_CUDA(cudaMemcpyAsync(&hr, cnt + 6, sizeof(hr), cudaMemcpyDeviceToHost, s));
     MG_TRY_CUDA(cudaStreamSynchronize(s));
     n_fallback = (int64_t)hr;
-    rc = MG_OK;
     if (n_fallback > 0) {
       LetkfParams fb = prm;
       fb.redo_in = redo;
@@ -873,11 +879,16 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
       fb.next = cnt + 6;  // reused as the work counter of the re-run
       fb.lev_boff = nullptr;  // the SIMT kernel walks the column lists as given
       MG_TRY_CUDA(cudaMemsetAsync(cnt + 6, 0, sizeof(unsigned long long), s));
-      rc = (k <= 64) ? launch_batched<float, 64>(ctx, fb) : launch_batched<float, 96>(ctx, fb);
+      if (fp64) {
+        if (k <= 32) rc = launch_batched<double, 32>(ctx, fb);
+        else if (k <= 64) rc = launch_batched<double, 64>(ctx, fb);
+        else rc = launch_batched<double, 96>(ctx, fb);
+      } else {
+        rc = (k <= 64) ? launch_batched<float, 64>(ctx, fb) : launch_batched<float, 96>(ctx, fb);
+      }
     }
   } else if (fp64 && (d->flags & MG_SQRT_CHOLESKY)) {
     MG_TRY_CUDA(mg::letkf_chol_launch(prm, ctx->num_sms, s));
-    rc = MG_OK;
   } else if (fp64) {
     if (k <= 32) rc = launch_batched<double, 32>(ctx, prm);
     else if (k <= 64) rc = launch_batched<double, 64>(ctx, prm);

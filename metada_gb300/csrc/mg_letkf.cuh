@@ -102,5 +102,8 @@ int letkf_tc_launch(const LetkfParams& prm, int num_sms, void* stream, int* ctas
 
 // FP64 local analyses with the Cholesky square root (MG_SQRT_CHOLESKY), k <= 96.
 cudaError_t letkf_chol_launch(const LetkfParams& prm, int num_sms, cudaStream_t s);
+// FP64 local analyses with the symmetric square root, k <= 96; points that
+// it leaves to the FP64 Jacobi go to prm.redo_out / n_redo.
+cudaError_t letkf_hunt_launch(const LetkfParams& prm, int num_sms, cudaStream_t s);
 
 }  // namespace mg
