@@ -24,7 +24,6 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRedBlocks = 304;
 constexpr int kSpreadBlocks = 152 * 8;
 
 // C = sum_o rinv_o U[o]^T W[o] over this CTA's obs range (U, W: p x k
@@ -130,27 +129,6 @@ __global__ void __launch_bounds__(kThreads) mean_spread_kernel(const double* __r
   }
 }
 
-// Deterministic sum of squares: fixed grid, per-CTA partials, one CTA sums
-// them in order into *out.
-template <typename TE>
-__global__ void __launch_bounds__(kThreads) sumsq_partial_kernel(const TE* __restrict__ v, int64_t n,
-                                                                 double* __restrict__ partial) {
-  __shared__ double red[kThreads / 32];
-  double s = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
-    const double x = (double)v[i];
-    s += x * x;
-  }
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    partial[blockIdx.x] = t;
-  }
-}
-
 // *out = sum of nb partials by one CTA: thread t sums t, t + kThreads, ...
 // in order, then a fixed-order tree (deterministic).
 __global__ void __launch_bounds__(kThreads) sum_partials_kernel(const double* __restrict__ partial, int nb,
@@ -165,16 +143,6 @@ __global__ void __launch_bounds__(kThreads) sum_partials_kernel(const double* __
     __syncthreads();
   }
   if (threadIdx.x == 0) *out = red[0];
-}
-
-template <typename TE>
-int sumsq(mg_context* ctx, const TE* v, int64_t n, double* partial, double* out) {
-  sumsq_partial_kernel<TE><<<kRedBlocks, kThreads, 0, ctx->stream>>>(v, n, partial);
-  MG_COUNT_LAUNCH();
-  sum_partials_kernel<<<1, kThreads, 0, ctx->stream>>>(partial, kRedBlocks, out);
-  MG_COUNT_LAUNCH();
-  MG_TRY_CUDA(cudaGetLastError());
-  return MG_OK;
 }
 
 template <typename TE>
@@ -242,21 +210,16 @@ int finish(mg_context* ctx, int64_t n, int k, double rho, const double* mean, do
 int run_enkf_fp64(mg_context* ctx, double* X, int64_t n, int k, int64_t ld, const double* HX, const double* yo,
                   const double* rvar, const double* eps, int64_t p, double rho, double* mean_out,
                   mg_enkf_diag* diag) {
-  const int nblk = mg::cross_blocks(p, ctx->num_sms);
+  const int nblk = mg::obs_blocks(p, ctx->num_sms);
   const int64_t kk = (int64_t)k * k;
   mg::Carver cv;
-  double *mean = nullptr, *Y = nullptr, *dinn = nullptr, *rinv = nullptr, *Gpart = nullptr, *Fpart = nullptr;
-  double *T = nullptr, *red = nullptr, *sums = nullptr;
+  double *mean = nullptr, *part = nullptr, *T = nullptr, *red = nullptr, *sums = nullptr;
   int* status = nullptr;
   for (int pass = 0; pass < 2; ++pass) {
     mean = cv.take<double>(n);
-    Y = cv.take<double>((size_t)(p + 1) * k);
-    dinn = cv.take<double>(p + 1);
-    rinv = cv.take<double>(p + 1);
-    Gpart = cv.take<double>((size_t)nblk * (kk + k));
-    Fpart = cv.take<double>((size_t)nblk * kk);
+    part = cv.take<double>((size_t)nblk * (2 * kk + k));
     T = cv.take<double>(kk);
-    red = cv.take<double>(kSpreadBlocks);
+    red = cv.take<double>(std::max(kSpreadBlocks, nblk));
     sums = cv.take<double>(4);
     status = cv.take<int>(4);
     if (pass == 1) break;
@@ -267,16 +230,16 @@ int run_enkf_fp64(mg_context* ctx, double* X, int64_t n, int k, int64_t ld, cons
   cudaStream_t s = ctx->stream;
   int rc;
   if ((rc = mean_spread(ctx, X, n, k, ld, mean, red, diag ? sums + 1 : nullptr)) != MG_OK) return rc;
-  MG_TRY_CUDA(mg::launch_obs_prior(HX, yo, rvar, p, k, Y, nullptr, dinn, rinv, s));
-  if (diag && (rc = sumsq<double>(ctx, dinn, p, red, sums + 0)) != MG_OK) return rc;
-  MG_TRY_CUDA(mg::launch_gram_fp64(Y, rinv, dinn, p, k, nblk, Gpart, s));
-  MG_TRY_CUDA(mg::launch_cross_fp64(Y, eps, rinv, p, k, nblk, Fpart, s));
-  if (nblk > 1) {
-    MG_TRY_CUDA(mg::launch_reduce_parts(Gpart, nblk, kk + k, Gpart, s));
-    MG_TRY_CUDA(mg::launch_reduce_parts(Fpart, nblk, kk, Fpart, s));
+  const mg::ObsProducts op{HX, eps, yo, rvar, p, k, nblk, part, diag ? red : nullptr, nullptr, 0, 0, nullptr};
+  MG_TRY_CUDA(mg::launch_obs_products(op, s));
+  if (diag) {
+    sum_partials_kernel<<<1, kThreads, 0, s>>>(red, nblk, sums + 0);
+    MG_COUNT_LAUNCH();
+    MG_TRY_CUDA(cudaGetLastError());
   }
+  if (nblk > 1) MG_TRY_CUDA(mg::launch_reduce_parts(part, nblk, 2 * kk + k, part, s));
   MG_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * 4, s));
-  MG_TRY_CUDA(mg::launch_enkf_chol(Gpart, Fpart, Gpart + kk, k, rho, T, nullptr, status, s));
+  MG_TRY_CUDA(mg::launch_enkf_chol(part, part + kk + k, part + kk, k, rho, T, nullptr, status, s));
   // X' carries sqrt(rho) in T, whose columns also hold the identity.
   MG_TRY_CUDA(mg::launch_update_fp64(X, ld, n, k, mean, T, ctx->num_sms, s));
   // Analysis mean and perturbations (Ensemble::RecomputeMean/Perturbations).

@@ -1,7 +1,7 @@
 // Global ETKF (ETKF.hpp:100-179).
 //
 //   1. mean + perturbations (Ensemble.hpp:105-151), member-major;
-//   2. obs-space prior ym, Y' = HX - ym, d = yo - ym (ETKF.hpp:128-141);
+//   2. obs-space prior ym, Y' = HX - ym, d = yo - ym (ETKF.hpp:128-141) and
 //   3. Gram G = Y'^T R^-1 Y' and b = Y'^T R^-1 d by obs ranges, partials
 //      summed in a fixed order (deterministic), FP64 by exact splitting on
 //      the tensor cores (mg_fp64gemm.cu);
@@ -106,9 +106,6 @@ __global__ void __launch_bounds__(kThreads) etkf_update_kernel(const TE* __restr
 struct EtkfBuffers {
   double* mean;   // n
   float* Xp;      // n x k perturbations (mixed path)
-  double* Y;      // p x k
-  double* dinn;   // p
-  double* rinv;   // p
   double* part;   // nblk x (k x k + k)
   double* T;      // k x k
   int* status;
@@ -122,15 +119,16 @@ cudaError_t enqueue_etkf(const EtkfBuffers& w, bool mixed, int num_sms, double* 
                          cudaStream_t s) {
   const int64_t len = (int64_t)k * k + k;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(w.status, 0, sizeof(int), s)) != cudaSuccess ||
-      (e = mg::launch_mean_pert_members(X, n, k, ld, w.mean, nullptr, mixed ? w.Xp : nullptr, n, s)) != cudaSuccess ||
-      (e = mg::launch_obs_prior(HX, yo, rvar, p, k, w.Y, nullptr, w.dinn, w.rinv, s)) != cudaSuccess ||
-      (e = mg::launch_gram_fp64(w.Y, w.rinv, w.dinn, p, k, w.nblk, w.part, s)) != cudaSuccess)
-    return e;
   const bool chol = flags & MG_SQRT_CHOLESKY;
+  const bool along = !mixed && mg::mean_rides_along(n);
+  if (!along && (e = mg::launch_mean_pert_members(X, n, k, ld, w.mean, nullptr, mixed ? w.Xp : nullptr, n, s)) !=
+                    cudaSuccess)
+    return e;
+  const mg::ObsProducts op{HX, nullptr, yo, rvar, p, k, w.nblk, w.part, nullptr, X, n, ld, along ? w.mean : nullptr};
+  if ((e = mg::launch_obs_products(op, s)) != cudaSuccess) return e;
   // The Cholesky solve sums a few partials itself; more are summed on many SMs first.
   int nparts = w.nblk;
-  if (nparts > (chol ? 8 : 1)) {
+  if (nparts > (chol ? mg::etkf_chol_parts() : 1)) {
     if ((e = mg::launch_reduce_parts(w.part, nparts, len, w.part, s)) != cudaSuccess) return e;
     nparts = 1;
   }
@@ -140,6 +138,7 @@ cudaError_t enqueue_etkf(const EtkfBuffers& w, bool mixed, int num_sms, double* 
                              compat_infl ? rho : 1.0, w.T, w.status, s);
     if (e != cudaSuccess) return e;
   } else {
+    if ((e = cudaMemsetAsync(w.status, 0, sizeof(int), s)) != cudaSuccess) return e;
     if (w.hunt) {
       const bool compat_infl = flags & MG_INFL_COMPAT;
       e = mg::launch_hunt_global(w.part, k, compat_infl ? (double)(k - 1) : (double)(k - 1) / rho,
@@ -170,14 +169,11 @@ cudaError_t enqueue_etkf(const EtkfBuffers& w, bool mixed, int num_sms, double* 
 int run_etkf(mg_context* ctx, bool mixed, double* X, int64_t n, int k, int64_t ld, const double* HX, const double* yo,
              const double* rvar, int64_t p, double rho, int flags, double* mean_out) {
   EtkfBuffers w{};
-  w.nblk = mg::cross_blocks(p, ctx->num_sms);
+  w.nblk = mg::obs_blocks(p, ctx->num_sms);
   mg::Carver cv;
   for (int pass = 0; pass < 2; ++pass) {
     w.mean = mean_out ? mean_out : cv.take<double>(n);
     w.Xp = cv.take<float>(mixed ? (size_t)n * k : 1);
-    w.Y = cv.take<double>((size_t)(p + 1) * k);
-    w.dinn = cv.take<double>(p + 1);
-    w.rinv = cv.take<double>(p + 1);
     w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
     w.T = cv.take<double>((size_t)k * k);
     w.status = cv.take<int>(4);
@@ -189,10 +185,11 @@ int run_etkf(mg_context* ctx, bool mixed, double* X, int64_t n, int k, int64_t l
   }
   cudaStream_t s = ctx->stream;
   MG_TRY_CUDA(enqueue_etkf(w, mixed, ctx->num_sms, X, n, k, ld, HX, yo, rvar, p, rho, flags, s));
-  int hs = 0;
-  MG_TRY_CUDA(cudaMemcpyAsync(&hs, w.status, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int* hs = static_cast<int*>(mg::host_stage(ctx, sizeof(int)));  // pinned
+  if (!hs) return MG_ERR_NOMEM;
+  MG_TRY_CUDA(cudaMemcpyAsync(hs, w.status, sizeof(int), cudaMemcpyDeviceToHost, s));
   MG_TRY_CUDA(cudaStreamSynchronize(s));
-  if (hs) return mg::fail(ctx, MG_ERR_NUMERIC, "mg_etkf: the k x k system was not positive definite");
+  if (*hs) return mg::fail(ctx, MG_ERR_NUMERIC, "mg_etkf: the k x k system was not positive definite");
   return MG_OK;
 }
 
@@ -273,7 +270,7 @@ int run_etkf_static(cudaStream_t s, bool mixed, double* X, int64_t n, int k, int
     return MG_ERR_CUDA;
   }
   // The sizes that the entry point documents: what fits does not depend on
-  // how the kernels divide the work (the FP64 path needs no X' buffer).
+  // how the kernels divide the work (they keep no Y', and in FP64 no X').
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((p + 255) / 256, 2 * num_sms));
   mg::Carver cv;
   cv.reserve<double>(n);
@@ -288,12 +285,9 @@ int run_etkf_static(cudaStream_t s, bool mixed, double* X, int64_t n, int k, int
   if (cv.off > kStaticScratchBytes) return MG_ERR_CAPACITY;
   cv = mg::Carver{static_cast<char*>(base), 0};
   EtkfBuffers w{};
-  w.nblk = std::min(nblk, mg::cross_blocks(p, num_sms));
+  w.nblk = std::min(nblk, mg::obs_blocks(p, num_sms));
   w.mean = mean_out ? mean_out : cv.take<double>(n);
   w.Xp = cv.take<float>(mixed ? (size_t)n * k : 1);
-  w.Y = cv.take<double>((size_t)(p + 1) * k);
-  w.dinn = cv.take<double>(p + 1);
-  w.rinv = cv.take<double>(p + 1);
   w.part = cv.take<double>((size_t)w.nblk * k * (k + 1));
   w.T = cv.take<double>((size_t)k * k);
   w.status = cv.take<int>(4);

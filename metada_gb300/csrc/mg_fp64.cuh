@@ -23,6 +23,13 @@ __device__ __forceinline__ double recip_fp64(double d) {
   return __fma_rn(r, __fma_rn(e, e, e), r);
 }
 
+// A usable pivot: positive, and below 3e38 (so finite).  By the leading word:
+// a comparison of doubles is an FP64 instruction.
+__device__ __forceinline__ bool pivot_ok(double d) {
+  const int hi = __double2hiint(d);
+  return hi > 0 && hi < __double2hiint(3.0e38);
+}
+
 // a / b given r = 1 / b correctly rounded: one correction of a r by its exact
 // remainder gives the correctly rounded quotient (Markstein, 1990) while no
 // term leaves the normal range.

@@ -84,15 +84,28 @@ cudaError_t launch_obs_prior(const double* HX, const double* yo, const double* r
 size_t select_grid_bytes(int64_t npt);
 
 // FP64 contractions on the tensor cores by exact splitting, k <= 112
-// (mg_fp64gemm.cu).  gram: nblk partials of [Y^T diag(rinv) Y (k x k),
-// Y^T diag(rinv) d (k)]; cross: nblk partials of U^T diag(rinv) V; reduce:
-// out[e] = sum over partials (out == part allowed); update: X_i <- mean +
+// (mg_fp64gemm.cu).  obs products: nblk partials of [Y'^T R^-1 Y' (k x k),
+// Y'^T R^-1 d (k)] and, with eps, Y'^T R^-1 eps (k x k), from H(X) of the raw
+// members; the CTAs' sums of squared innovations (dsq_part, may be null); and
+// the ensemble mean of X where mean is set (mean_rides_along).  reduce:
+// out[e] = sum over partials (out == part allowed).  update: X_i <- mean +
 // sum_j (X_j - mean) T_ji in place, member-major.
-int cross_blocks(int64_t p, int num_sms);
-cudaError_t launch_gram_fp64(const double* Y, const double* rinv, const double* dinn, int64_t p, int k, int nblk,
-                             double* part, cudaStream_t s);
-cudaError_t launch_cross_fp64(const double* U, const double* V, const double* rinv, int64_t p, int k, int nblk,
-                              double* part, cudaStream_t s);
+struct ObsProducts {
+  const double* HX;
+  const double* eps;  // or null
+  const double* yo;
+  const double* rvar;
+  int64_t p;
+  int k, nblk;
+  double* part;
+  double* dsq_part;
+  const double* X;
+  int64_t n, ld;
+  double* mean;  // or null
+};
+int obs_blocks(int64_t p, int num_sms);
+bool mean_rides_along(int64_t n);
+cudaError_t launch_obs_products(const ObsProducts& a, cudaStream_t s);
 cudaError_t launch_reduce_parts(const double* part, int nblk, int64_t len, double* out, cudaStream_t s);
 cudaError_t launch_update_fp64(double* X, int64_t ld, int64_t n, int k, const double* mean, const double* T,
                                int num_sms, cudaStream_t s);
@@ -109,7 +122,9 @@ cudaError_t launch_hunt_global(const double* Gb, int k, double diag, double out_
 // k x k systems by one factorisation (mg_solve.cu).  etkf: from nblk
 // partials of [G, b], T_ji = scale (wa_j + W_ji) with A = diag I + G,
 // W = sqrt(k-1) chol_L(A^-1); enkf: T = sqrt(rho) (I + A^-1 (b 1^T + F - G)).
-// *status is set to 1 (not cleared) when A is not positive definite.
+// etkf: *status <- 1 when A is not positive definite, else 0; enkf: set to 1
+// (not cleared).
+int etkf_chol_parts();  // partials that launch_etkf_chol takes
 cudaError_t launch_etkf_chol(const double* part, int nblk, int k, double diag, double scale, double* T, int* status,
                              cudaStream_t s);
 cudaError_t launch_enkf_chol(const double* G, const double* F, const double* b, int k, double rho, double* T,

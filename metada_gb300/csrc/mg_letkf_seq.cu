@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads) letkf_seq_kernel(SeqParams prm) {
         for (int j = k - 1; j >= 0; --j) {
           double* const rw = P + j * (j + 1) / 2;
           double d = rw[j];
-          if (!(d > 0.0) || !(d < 3.0e38)) {
+          if (!mg::pivot_ok(d)) {
             ok = false;
             d = 1.0;
           }

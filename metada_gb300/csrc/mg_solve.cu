@@ -8,12 +8,11 @@
 // columns are the identity's, and chol_L(A^-1) = U^-T D^-1/2 is their
 // transpose scaled (mg_letkf_chol.cu has the algebra): row i of T needs only
 // column i.  For the EnKF they are b 1^T + F - G, followed by D^-1 and U^-T.
-// One SM's FP64 unit is the limit (two multiply-adds per clock), so the
-// columns are spread over CTAs, eight each, and every CTA repeats the
-// factorisation; FP64 instructions are kept full (a warp walks a row of A
-// and its columns together, one reciprocal per step).
+// One system is a chain of k steps, and one SM runs two FP64 multiply-adds per
+// clock, so the columns are spread over CTAs, eight each, every CTA repeats
+// the factorisation, and a step is kept short (eliminate).
 // 64 x 64 grid, k = 32: 129 us by one CTA (inverse and two factorisations)
-// -> 36 us; EnKF, k = 64: 354 -> 102 us.
+// -> 30 us; EnKF, k = 64: 354 -> 118 us.
 #include <cmath>
 
 #include "mg_fp64.cuh"
@@ -25,45 +24,65 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kCols = 8;        // right-hand-side columns per CTA
 constexpr int kLdb = kCols + 1;  // and b
+constexpr int kMaxParts = 4;     // partials summed here (more are summed on many SMs first)
 
 // Eliminates columns k-1 .. 0 of the packed lower triangle A (rows of length
-// i + 1), leaving row j's multipliers u_l in A[j][l], l < j, and d, 1/d;
-// B (k x kLdb) <- U^-1 B.
+// i + 1) with the columns B (k x kLdb) alongside: A's rows become the
+// multipliers u_l (l < j) of column j, B <- U^-1 B; d and 1/d by column.
+// A warp walks a row of A and of B together.  The chain from pivot to pivot
+// (multiply-add, reciprocal, multipliers) is what bounds a step: the first
+// warp updates the next pivot's row before anything else and leaves its
+// multipliers and a copy of the row, while the others update the rest, so a
+// step has one barrier and only one warp runs the reciprocal (a warp's FP64
+// instruction holds its scheduler's unit 64 cycles even where every warp
+// computes the same).
+template <int KMAX>
 __device__ bool eliminate(double* A, double* B, double* raw, double* dval, double* dinv, int k) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool ok = true;
-  for (int j = k - 1; j >= 0; --j) {
+  // Row j is final: multipliers, copy, pivot (the first warp).
+  auto pivot_row = [&](int j) {
     double* rw = A + j * (j + 1) / 2;
     double d = rw[j];
-    if (!(d > 0.0) || !(d < 3.0e38)) {
+    if (!mg::pivot_ok(d)) {
       ok = false;
       d = 1.0;
     }
     const double r = mg::recip_fp64(d);
-    for (int l = tid; l < j; l += kThreads) {
-      const double a = rw[l];
-      raw[l] = a;
-      rw[l] = a * r;
+    double* copy = raw + (j & 1) * KMAX;
+    __syncwarp();
+    for (int x = lane; x < j; x += 32) {
+      const double a = rw[x];
+      copy[x] = a;
+      rw[x] = a * r;
     }
-    if (tid == 0) {
+    if (lane == 0) {
       dval[j] = d;
       dinv[j] = r;
     }
-    __syncthreads();
-    const double* bj = B + j * kLdb;
-    for (int i = warp; i < j; i += kWarps) {
-      const double u = rw[i];
-      double* ri = A + i * (i + 1) / 2;
-      double* bi = B + i * kLdb;
-      for (int x = lane; x < i + 1 + kLdb; x += 32) {
-        double* dst = x <= i ? ri + x : bi + (x - i - 1);
-        const double src = x <= i ? raw[x] : bj[x - i - 1];
-        *dst = __fma_rn(-u, src, *dst);
-      }
+  };
+  auto update_row = [&](int i, int j) {
+    const double u = A[j * (j + 1) / 2 + i];
+    const double *src = raw + (j & 1) * KMAX, *bj = B + j * kLdb;
+    double *ri = A + i * (i + 1) / 2, *bi = B + i * kLdb;
+    for (int x = lane; x < i + 1 + kLdb; x += 32) {
+      double* dst = x <= i ? ri + x : bi + (x - i - 1);
+      *dst = __fma_rn(-u, x <= i ? src[x] : bj[x - i - 1], *dst);
     }
+  };
+  if (warp == 0) pivot_row(k - 1);
+  __syncthreads();
+  for (int j = k - 1; j > 0; --j) {
+    if (warp == 0) {
+      update_row(j - 1, j);
+      __syncwarp();
+      pivot_row(j - 1);
+    }
+    for (int i = j - 1 - warp; i >= 0; i -= kWarps)
+      if (i < j - 1) update_row(i, j);
     __syncthreads();
   }
-  return ok;
+  return __syncthreads_and(ok);
 }
 
 __device__ __forceinline__ double sum_parts(const double* part, int nblk, int64_t len, int64_t e) {
@@ -72,18 +91,13 @@ __device__ __forceinline__ double sum_parts(const double* part, int nblk, int64_
   return t;
 }
 
-size_t solve_bytes(int k) { return sizeof(double) * ((size_t)k * (k + 1) / 2 + (size_t)k * kLdb + 3 * (size_t)k); }
-
 // part: nblk partials of [G (k x k), b (k)].  T[j*k + i] = scale (wa_j + W_ji).
+template <int KMAX>
 __global__ void __launch_bounds__(kThreads) etkf_chol_kernel(const double* __restrict__ part, int nblk, int k,
                                                              double diag, double scale, double* __restrict__ T,
                                                              int* status) {
-  extern __shared__ __align__(16) double sh[];
-  double* A = sh;
-  double* B = A + k * (k + 1) / 2;
-  double* raw = B + k * kLdb;
-  double* dval = raw + k;
-  double* dinv = dval + k;
+  extern __shared__ __align__(16) double A[];
+  __shared__ double B[KMAX * kLdb], raw[2 * KMAX], dval[KMAX], dinv[KMAX], cd[KMAX];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t len = (int64_t)k * k + k;
   const int c0 = blockIdx.x * kCols;
@@ -96,10 +110,10 @@ __global__ void __launch_bounds__(kThreads) etkf_chol_kernel(const double* __res
     B[e] = q < kCols ? (r == c0 + q ? 1.0 : 0.0) : sum_parts(part, nblk, len, (int64_t)k * k + r);
   }
   __syncthreads();
-  const bool ok = eliminate(A, B, raw, dval, dinv, k);
-  if (!ok && blockIdx.x == 0 && tid == 0) *status = 1;
+  const bool ok = eliminate<KMAX>(A, B, raw, dval, dinv, k);
+  if (blockIdx.x == 0 && tid == 0) *status = ok ? 0 : 1;
   const double cw = sqrt((double)(k - 1));
-  for (int r = tid; r < k; r += kThreads) raw[r] = cw * rsqrt(dval[r]);
+  for (int r = tid; r < k; r += kThreads) cd[r] = cw * rsqrt(dval[r]);
   __syncthreads();
   const int i = c0 + warp;  // one row of T per warp
   if (i >= k) return;
@@ -108,21 +122,18 @@ __global__ void __launch_bounds__(kThreads) etkf_chol_kernel(const double* __res
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) wa += __shfl_xor_sync(0xffffffffu, wa, off);
   for (int m = lane; m < k; m += 32)
-    T[i * k + m] = scale * (wa + (m <= i ? B[m * kLdb + warp] * raw[m] : 0.0));
+    T[i * k + m] = scale * (wa + (m <= i ? B[m * kLdb + warp] * cd[m] : 0.0));
 }
 
 // G (k x k), F (k x k), b (k).  T = sr (I + A^-1 (b 1^T + F - G)), A = G + (k-1) I.
+template <int KMAX>
 __global__ void __launch_bounds__(kThreads) enkf_chol_kernel(const double* __restrict__ G,
                                                              const double* __restrict__ F,
                                                              const double* __restrict__ b, int k, double sr,
                                                              double* __restrict__ T, float* __restrict__ T32,
                                                              int* status) {
-  extern __shared__ __align__(16) double sh[];
-  double* A = sh;
-  double* B = A + k * (k + 1) / 2;
-  double* raw = B + k * kLdb;
-  double* dval = raw + k;
-  double* dinv = dval + k;
+  extern __shared__ __align__(16) double A[];
+  __shared__ double B[KMAX * kLdb], raw[2 * KMAX], dval[KMAX], dinv[KMAX];
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * kCols;
   for (int e = tid; e < k * k; e += kThreads) {
@@ -134,7 +145,7 @@ __global__ void __launch_bounds__(kThreads) enkf_chol_kernel(const double* __res
     B[e] = (q < kCols && c < k) ? (b[r] + F[r * k + c]) - G[r * k + c] : 0.0;
   }
   __syncthreads();
-  const bool ok = eliminate(A, B, raw, dval, dinv, k);
+  const bool ok = eliminate<KMAX>(A, B, raw, dval, dinv, k);
   if (!ok && blockIdx.x == 0 && tid == 0) *status = 1;
   for (int e = tid; e < k * kLdb; e += kThreads) B[e] *= dinv[e / kLdb];
   __syncthreads();
@@ -154,28 +165,46 @@ __global__ void __launch_bounds__(kThreads) enkf_chol_kernel(const double* __res
   }
 }
 
-}  // namespace
-
-namespace mg {
-
-cudaError_t launch_etkf_chol(const double* part, int nblk, int k, double diag, double scale, double* T, int* status,
-                             cudaStream_t s) {
-  const size_t smem = solve_bytes(k);
-  const cudaError_t e = cudaFuncSetAttribute(etkf_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int KMAX>
+cudaError_t run_etkf(const double* part, int nblk, int k, double diag, double scale, double* T, int* status,
+                     cudaStream_t s) {
+  constexpr size_t smem = sizeof(double) * (KMAX * (KMAX + 1) / 2);
+  const cudaError_t e =
+      cudaFuncSetAttribute(etkf_chol_kernel<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  etkf_chol_kernel<<<(k + kCols - 1) / kCols, kThreads, smem, s>>>(part, nblk, k, diag, scale, T, status);
+  etkf_chol_kernel<KMAX><<<(k + kCols - 1) / kCols, kThreads, smem, s>>>(part, nblk, k, diag, scale, T, status);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
-cudaError_t launch_enkf_chol(const double* G, const double* F, const double* b, int k, double rho, double* T,
-                             float* T32, int* status, cudaStream_t s) {
-  const size_t smem = solve_bytes(k);
-  const cudaError_t e = cudaFuncSetAttribute(enkf_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int KMAX>
+cudaError_t run_enkf(const double* G, const double* F, const double* b, int k, double rho, double* T, float* T32,
+                     int* status, cudaStream_t s) {
+  constexpr size_t smem = sizeof(double) * (KMAX * (KMAX + 1) / 2);
+  const cudaError_t e =
+      cudaFuncSetAttribute(enkf_chol_kernel<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  enkf_chol_kernel<<<(k + kCols - 1) / kCols, kThreads, smem, s>>>(G, F, b, k, std::sqrt(rho), T, T32, status);
+  enkf_chol_kernel<KMAX><<<(k + kCols - 1) / kCols, kThreads, smem, s>>>(G, F, b, k, std::sqrt(rho), T, T32, status);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
+}
+
+}  // namespace
+
+namespace mg {
+
+int etkf_chol_parts() { return kMaxParts; }
+
+cudaError_t launch_etkf_chol(const double* part, int nblk, int k, double diag, double scale, double* T, int* status,
+                             cudaStream_t s) {
+  return k <= 32 ? run_etkf<32>(part, nblk, k, diag, scale, T, status, s)
+                 : run_etkf<112>(part, nblk, k, diag, scale, T, status, s);
+}
+
+cudaError_t launch_enkf_chol(const double* G, const double* F, const double* b, int k, double rho, double* T,
+                             float* T32, int* status, cudaStream_t s) {
+  return k <= 32 ? run_enkf<32>(G, F, b, k, rho, T, T32, status, s)
+                 : run_enkf<112>(G, F, b, k, rho, T, T32, status, s);
 }
 
 }  // namespace mg
