@@ -1,26 +1,37 @@
 // Batched LETKF local analyses on the tensor cores (mixed precision, Hunt
-// transform, k <= 96): the k x k Gram Y'^T R^-1 Y', the products of the
-// symmetric inverse square root and the update X' W all run as tcgen05.mma
-// kind::tf32 products with an error-compensated 3-pass split
-// (hi*hi + hi*lo + lo*hi, hi = x rounded to TF32, lo = x - hi), accumulated in
-// FP32 in tensor memory.  Replaces the grid loop of LETKF::Analyse
-// (LETKF.hpp:101) and the solve and update of updateGridPoint
+// transform, k <= 96): the k x k Gram Y'^T R^-1 Y' as tcgen05.mma kind::tf32
+// products, the products of the symmetric inverse square root and the update
+// X' W as kind::f16 products of FP16 pairs, all with an error-compensated
+// 3-pass split (hi*hi + hi*lo + lo*hi, 22 significant bits an operand) and
+// accumulated in FP32 in tensor memory.  Replaces the grid loop of
+// LETKF::Analyse (LETKF.hpp:101) and the solve and update of updateGridPoint
 // (LETKF.hpp:214-238) in the Hunt et al. (2007) form with Gaspari-Cohn
 // R-localisation.
 //
-// Two instantiations by member slots KP:
-//  * KP = 64 (k <= 64): 256 threads, two CTAs per SM (256 TMEM columns each);
+// What bounds it: one analysis is a chain of about 12 dependent products,
+// each a barrier, an MMA burst and a TMEM -> registers -> operand pass, so a
+// CTA alone leaves the tensor core and the shared-memory port idle most of
+// the time; the time goes down with the analyses resident per SM and with
+// the bytes an operand pass moves.  FP16 pairs take half the shared memory
+// and half the MMA time of TF32 pairs.  Three instantiations by member slots
+// KP, each as many CTAs per SM as its operands and its tensor memory allow:
+//  * KP = 64 (k <= 64): 256 threads, 3 CTAs per SM (128 TMEM columns each);
 //    Z and Y are stacked as the 128 rows of one operand, so [Z; Y] T is one
 //    M = 128 product.
-//  * KP = 96 (64 < k <= 96, the high-resolution configuration's k = 80): 384
-//    threads, one CTA per SM with all 512 TMEM columns and 216 KB of
-//    operands; Z, Y and T are separate 96-row operands and [Z; Y] T is two
-//    products.
+//  * KP = 80 (64 < k <= 80, the high-resolution configuration's k = 80): 384
+//    threads, 2 CTAs per SM (256 columns); Z, Y and T are separate operands
+//    and [Z; Y] T is two products.
+//  * KP = 96 (80 < k <= 96): as KP = 80 with 1 CTA per SM: 96-slot operands
+//    and Gram need more than 256 columns.
+// Whole cycles with TF32 pairs (2, 1 and 1 CTAs, k = 80 in 96 slots) -> this:
+// 360 x 180 x 10 points, 4 variables, k = 64, 500k obs, FP32 members: 118.7
+// -> 91.9 ms; 360 x 180 x 30 points, k = 80, clustered obs: 819 -> 496 ms.  Error against 64 bits
+// on smaller grids: 2.5e-7 -> 2.3e-7 and 4.5e-7 -> 4.3e-7.
 //
 // Per local analysis (one CTA, persistent, points pulled in the grid's
 // column order from a work counter):
 //  1. Gram: the candidate list is filtered and weighted, the kept rows
-//     sqrt(w) Y'_o are gathered 64 at a time into a K-major, 128-byte
+//     sqrt(w) Y'_o are gathered 32 at a time into a K-major, 128-byte
 //     swizzled operand (members x obs) with sqrt(w) d_o as an extra row, and
 //     [G | b] = B^T [B | sqrt(w) d] accumulates in TMEM (two rotating
 //     buffers; each chunk's rows are loaded while the previous one's MMAs run).
@@ -35,7 +46,8 @@
 //     stops once max |Z Y - I| < 0.05 (one more step squares that error).
 //     Z -> M^-1/2, and A^-1/2 = (Z - 1 1^T / k) / sqrt(s) on the complement
 //     of 1.
-//  4. First-order finish from the matrix itself: C = Z^T A Z, F = C - P,
+//  4. First-order finish from the matrix itself: C = Z^T (P A P) Z, F = C - P
+//     (Z and P A P over their powers of s; the wa and W below carry s),
 //     W = sqrt((k-1) c) Z (I - F/2), wa = c Z (P - F) Z^T b (c = rho for the
 //     reference's inflation placement, else 1).  max |F| is the per-analysis
 //     residual.  Analyses whose conditioning bound s / delta is above
@@ -53,6 +65,7 @@
 
 #include "mg_internal.h"
 #include "mg_letkf.cuh"
+#include "mg_f16op.cuh"
 #include "mg_tcgen05.cuh"
 #include "mg_tf32op.cuh"
 
@@ -60,7 +73,7 @@ namespace {
 
 using namespace mg::t5;
 
-constexpr int kChunk = 64;      // obs per Gram chunk: two 128-byte swizzle atoms of TF32
+constexpr int kChunk = 32;      // obs per Gram chunk: one 128-byte swizzle atom of TF32
 constexpr int kNBuf = 2;        // Gram chunk buffers
 constexpr int kSelRing = 512;   // selected-entry ring (a candidate block + carry-over < kChunk)
 constexpr int kMaxIt = 14;      // Newton-Schulz iterations before an analysis is handed back
@@ -83,66 +96,85 @@ constexpr float kCondResid = 0.1f;
 // max |Z Y - I| above which the iteration has left its basin (a convergent
 // iterate stays below 1); the analysis is handed back at once.
 constexpr float kDiverged = 4.0f;
+// Powers of two that operands are stored with (mg_f16op.cuh): Z, Y, T, P A P
+// and products of theirs stay below about 20 (kMaxCond bounds Z); X' rows are
+// taken in units of their variable's largest entry (below 2), so E = Z^T X'^T
+// stays below 2^8; F is accepted up to kResidMax.
+constexpr float kSc = 64.0f;                  // Z, Y, T, P A P, Q
+constexpr float kScX = 32.0f;                 // X', E
+constexpr float kScF = 1048576.0f;            // F
+constexpr float kUnZ = 1.0f / (kSc * kSc);    // product of two kSc operands
+constexpr float kUnE = 1.0f / (kSc * kScX);   // Z^T X'^T
+constexpr float kUnD = 1.0f / (kScF * kScX);  // F^T E
+constexpr float kUnZF = 1.0f / (kSc * kScF);  // Z F
 constexpr int kVarTile = 16;    // variables per update MMA (N): two 8-column TMEM loads
 constexpr int kPre = 4;         // variables whose X' rows and means are prefetched during the finish
 
-// Shared and tensor memory of one CTA, by member slots KP (a multiple of 32).
-// Every operand is K-major with the 128-byte swizzle: a slab holds 32 TF32
-// columns of all its rows (128 bytes per row), with a hi and a lo copy.
-//   KP = 64: STACK (Z in rows 0-63, Y in rows 64-127; 16 KB slabs) and T
-//   (64 rows, 8 KB slabs): 96 KB.
-//   KP = 96: Z, Y and T, each 96 rows in 12 KB slabs: 216 KB.  As a 128-row
-//   A operand, Z's and Y's last 32 rows read the following 4 KB (the lo copy
-//   or the next operand); those products land in TMEM lanes 96-127, never read.
-// Gram view of the same region: two chunk buffers of KP + 16 rows (KP
-// members, the innovation row, 15 unused), then the selected-entry ring.
+// Shared and tensor memory of one CTA, by member slots KP.  The operands of
+// the solve are K-major FP16 pairs with the 64-byte swizzle (mg_f16op.cuh): a
+// slab holds 32 columns of all its rows (64 bytes per row), with a hi and a
+// lo copy.
+//   KP = 64: STACK (Z in rows 0-63, Y in rows 64-127), T and P A P (64 rows
+//   each): 64 KB.  P A P kept as an operand frees the Gram's tensor memory,
+//   so the products take its place: 128 columns.
+//   KP = 80, 96: Z, Y and T, each KP rows; P A P stays in tensor memory as
+//   the Gram: 90 KB and 256 columns, or 108 KB and 512.
+// As a 128-row A operand, operands of fewer rows read the bytes that follow;
+// those products land in TMEM lanes that nothing reads.
+// Gram view of the same region (TF32 pairs with the 128-byte swizzle, whose
+// exponent range needs no scale for the obs rows): two chunk buffers of
+// KP + 16 rows (KP members, the innovation row, 15 unused), then the
+// selected-entry ring.
 template <int KP>
 struct Lay {
-  static_assert(KP == 64 || KP == 96, "member slots");
-  static constexpr int NG = KP / 32;          // 32-column groups = TMEM lane quadrants holding rows
+  static_assert(KP == 64 || KP == 80 || KP == 96, "member slots");
+  static constexpr int NG = (KP + 31) / 32;   // 32-column groups = TMEM lane quadrants holding rows
   static constexpr int kThreads = 128 * NG;   // four lane quadrants x NG column groups of warps
   static constexpr int kWarps = kThreads / 32;
   static constexpr bool kStack = KP == 64;    // [Z; Y] as one 128-row operand
-  static constexpr int kMinBlocks = kStack ? 2 : 1;
+  static constexpr int kMinBlocks = kStack ? 3 : (KP == 80 ? 2 : 1);
+  static constexpr int kSteps = KP / 16;      // K-steps of a product
   static constexpr uint32_t ZR = kStack ? 128u : (uint32_t)KP;  // rows per slab of Z and Y
-  static constexpr uint32_t TR = KP;                            // rows per slab of T
-  static constexpr uint32_t kSlabZ = ZR * 128u;
-  static constexpr uint32_t kSlabT = TR * 128u;
+  static constexpr uint32_t TR = KP;                            // rows per slab of T (and P A P)
+  static constexpr uint32_t kSlabZ = ZR * 64u;
+  static constexpr uint32_t kSlabT = TR * 64u;
   static constexpr uint32_t OFF_Z_HI = 0;
   static constexpr uint32_t OFF_Z_LO = NG * kSlabZ;
-  static constexpr uint32_t OFF_Y_HI = kStack ? OFF_Z_HI + KP * 128u : 2 * NG * kSlabZ;
-  static constexpr uint32_t OFF_Y_LO = kStack ? OFF_Z_LO + KP * 128u : 3 * NG * kSlabZ;
+  static constexpr uint32_t OFF_Y_HI = kStack ? OFF_Z_HI + KP * 64u : 2 * NG * kSlabZ;
+  static constexpr uint32_t OFF_Y_LO = kStack ? OFF_Z_LO + KP * 64u : 3 * NG * kSlabZ;
   static constexpr uint32_t OFF_T_HI = (kStack ? 2 : 4) * NG * kSlabZ;
   static constexpr uint32_t OFF_T_LO = OFF_T_HI + NG * kSlabT;
-  static constexpr uint32_t kRegion = OFF_T_LO + NG * kSlabT;
+  static constexpr uint32_t OFF_A_HI = OFF_T_LO + NG * kSlabT;  // P A P (KP = 64)
+  static constexpr uint32_t OFF_A_LO = OFF_A_HI + NG * kSlabT;
+  static constexpr uint32_t kRegion = kStack ? OFF_A_LO + NG * kSlabT : OFF_A_HI;
   static constexpr int kGramRows = KP + 16;
   static constexpr int kGramN = KP + 16;      // Gram MMA N: members, the innovation row, 15 unused
   static constexpr uint32_t kGramSlab = kGramRows * 128u;
-  static constexpr uint32_t kGramBuf = 4 * kGramSlab;  // hi (2 slabs), lo (2 slabs)
+  static constexpr uint32_t kGramBuf = 2 * kGramSlab;  // hi, lo
   static constexpr uint32_t OFF_SEL = kNBuf * kGramBuf + (128 - kGramRows) * 128u;
   static constexpr uint32_t kSelBytes = kSelRing * 12u;  // obs index, sqrt(w), sqrt(w) d
   // Tensor memory: product scratch at column 0 (and a second product at
-  // kTmB for KP = 96), the Gram at kTmGram.
-  static constexpr uint32_t kTmemCols = kStack ? 256u : 512u;
-  static constexpr uint32_t kTmB = 128;
+  // kTmB), the Gram at kTmGram.
+  static constexpr uint32_t kTmemCols = kStack ? 128u : (KP == 80 ? 256u : 512u);
+  static constexpr uint32_t kTmB = KP == 80 ? 80u : 128u;
   static constexpr uint32_t kTmE = KP;  // E = Z^T X'^T (16 columns) beside the products
-  static constexpr uint32_t kTmGram = kStack ? 128u : 256u;
-  static_assert(kGramSlab % 1024 == 0 && kSlabZ % 1024 == 0 && kSlabT % 1024 == 0,
-                "swizzle atoms are 1024-byte aligned");
+  static constexpr uint32_t kTmGram = kStack ? 0u : (KP == 80 ? 160u : 256u);
+  static_assert(kGramSlab % 1024 == 0 && kSlabZ % 512 == 0 && kSlabT % 512 == 0, "swizzle atoms are aligned");
   static_assert(OFF_SEL + kSelBytes <= kRegion, "Gram buffers, A-operand overhang and the ring");
-  static_assert(kStack || (kTmB + KP <= kTmGram && kTmGram + kGramN <= kTmemCols), "tensor memory");
+  static_assert(kTmGram + kGramN <= kTmemCols && (kStack || kTmB + KP <= kTmGram), "tensor memory");
   static_assert(kSelRing >= kThreads + kChunk, "ring holds a candidate block and the carry-over");
 };
 
 // Vectors after the operand region.
 template <int KP>
 struct Vecs {
-  static constexpr int NG = KP / 32;
+  static constexpr int NG = Lay<KP>::NG;
   float b[KP], r[KP], u[KP], v[KP], wa[KP];
   float part[2 * NG][KP];
   float red[32];
   float xsq[kVarTile], inc[kVarTile], fac[kVarTile], one[kVarTile];
   float ssa[NG][kVarTile];
+  float xu[kVarTile];  // unit of each variable's X' row
   double xm[kVarTile];
   double xmpre[kPre];
   float xpre[kPre][KP];
@@ -153,7 +185,9 @@ template <int KP>
 constexpr size_t smem_bytes() {
   return 1024 + Lay<KP>::kRegion + sizeof(Vecs<KP>);
 }
-static_assert(smem_bytes<96>() + 1024 <= 233472, "one KP = 96 CTA fits the SM's shared memory");
+static_assert(3 * (smem_bytes<64>() + 1280) <= 233472 && 2 * (smem_bytes<80>() + 1280) <= 233472,
+              "CTAs per SM by shared memory");
+static_assert(sizeof(Vecs<64>) >= 64 * 64, "the last rows that P A P reads as a 128-row operand");
 
 // Scaled Newton-Schulz step.  The spectrum of Z Y lies in [l, 1] (l = delta / s
 // at the start: P A P >= delta on the complement of 1, s >= lambda_max).  The
@@ -201,6 +235,10 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   constexpr int NG = L::NG;
   constexpr int kThreads = L::kThreads;
   constexpr uint32_t ZR = L::ZR, TR = L::TR;
+  using h16::get_col8;
+  using h16::get_row8;
+  using h16::put_col8;
+  using h16::put_row8;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* R = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Vecs<KP>& V = *reinterpret_cast<Vecs<KP>*>(R + L::kRegion);
@@ -210,6 +248,8 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   unsigned char* const YL = R + L::OFF_Y_LO;
   unsigned char* const TH = R + L::OFF_T_HI;
   unsigned char* const TL = R + L::OFF_T_LO;
+  unsigned char* const AH = L::kStack ? R + L::OFF_A_HI : YH;
+  unsigned char* const AL = L::kStack ? R + L::OFF_A_LO : YL;
   int* const sel_o = reinterpret_cast<int*>(R + L::OFF_SEL);
   float* const sel_sw = reinterpret_cast<float*>(R + L::OFF_SEL + 4 * kSelRing);
   float* const sel_sd = reinterpret_cast<float*>(R + L::OFF_SEL + 8 * kSelRing);
@@ -245,13 +285,21 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   tc_fence_after();
   const uint32_t tmem = tmem_s;
   const uint32_t tm_row = ((uint32_t)(32 * q) << 16);  // this warp's TMEM lanes
+  // Warp-collective TMEM load; a warp that a row guard split (KP = 80) is
+  // brought together first.
+  auto ld8 = [](uint32_t addr, uint32_t(&v)[8]) {
+    if (KP % 32) __syncwarp();
+    tmem_ld8(addr, v);
+  };
   const uint32_t sR = smem_u32(R);
   const uint32_t sZH = sR + L::OFF_Z_HI, sZL = sR + L::OFF_Z_LO;
   const uint32_t sYH = sR + L::OFF_Y_HI, sYL = sR + L::OFF_Y_LO;
   const uint32_t sTH = sR + L::OFF_T_HI, sTL = sR + L::OFF_T_LO;
-  const uint32_t idescK = idesc_tf32_f32(128, KP);
+  const uint32_t sAH = L::kStack ? sR + L::OFF_A_HI : sYH, sAL = L::kStack ? sR + L::OFF_A_LO : sYL;  // P A P
+  constexpr uint32_t kSlabA = L::kStack ? L::kSlabT : L::kSlabZ;
+  const uint32_t idescK = h16::idesc_f16_f32(128, KP);
   const uint32_t idescG = idesc_tf32_f32(128, L::kGramN);
-  const uint32_t idescU = idesc_tf32_f32(128, kVarTile);
+  const uint32_t idescU = h16::idesc_f16_f32(128, kVarTile);
 
   uint32_t mma_ph = 0;      // parity of the next mma_bar phase
   uint32_t gchunk = 0;      // Gram chunks issued by this CTA (buffer rotation)
@@ -287,27 +335,27 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // registers while the previous chunk is stored and its MMAs issued.
     int64_t cpos = e0;
     int nloc = 0, nch = 0, head = 0, nsel = 0;
-    const int slot = tid & (kChunk - 1), m0 = (tid / kChunk) * 16;  // gather: obs slot x 16 members
-    auto load_rows = [&](int pos, int cnt, float (&x)[16], float& sd) {
+    const int slot = tid & (kChunk - 1), m0 = (tid / kChunk) * 8;  // gather: obs slot x 8 members
+    auto load_rows = [&](int pos, int cnt, float (&x)[8], float& sd) {
       if (slot < cnt) {
         const int e = (pos + slot) & (kSelRing - 1);
         const int o = sel_o[e];
         const float sw = sel_sw[e];
         sd = sel_sd[e];
         const float* yr = Y + (int64_t)o * k;
-        if (vec4 && m0 + 16 <= k) {
+        if (vec4 && m0 + 8 <= k) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
+          for (int q4 = 0; q4 < 2; ++q4) {
             const float4 a4 = *reinterpret_cast<const float4*>(yr + m0 + 4 * q4);
             x[4 * q4 + 0] = a4.x * sw; x[4 * q4 + 1] = a4.y * sw; x[4 * q4 + 2] = a4.z * sw; x[4 * q4 + 3] = a4.w * sw;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) x[j] = (m0 + j < k) ? yr[m0 + j] * sw : 0.0f;
+          for (int j = 0; j < 8; ++j) x[j] = (m0 + j < k) ? yr[m0 + j] * sw : 0.0f;
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = 0.0f;
+        for (int j = 0; j < 8; ++j) x[j] = 0.0f;
         sd = 0.0f;
       }
     };
@@ -360,21 +408,23 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
       const bool done = cpos >= e1;
       const int nchunks = done ? (nsel + kChunk - 1) / kChunk : nsel / kChunk;
-      float x[16], sdv;
+      float x[8], sdv;
       if (nchunks > 0) load_rows(head, nsel < kChunk ? nsel : kChunk, x, sdv);
       for (int c = 0; c < nchunks; ++c) {
         const int b = (int)(gchunk % kNBuf);
         const uint32_t use = gchunk / kNBuf;
         if (use > 0 && !wait_all(&buf_bar[b], (use - 1) & 1u)) { alive = false; break; }
         unsigned char* bh = R + b * L::kGramBuf;
-        unsigned char* bl = bh + 2 * L::kGramSlab;
+        unsigned char* bl = bh + L::kGramSlab;
+        if (m0 < KP) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const uint32_t off = sw_off(m0 + j, slot, L::kGramRows);
-          float h, l;
-          split(x[j], h, l);
-          *reinterpret_cast<float*>(bh + off) = h;
-          *reinterpret_cast<float*>(bl + off) = l;
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t off = sw_off(m0 + j, slot, L::kGramRows);
+            float h, l;
+            split(x[j], h, l);
+            *reinterpret_cast<float*>(bh + off) = h;
+            *reinterpret_cast<float*>(bl + off) = l;
+          }
         }
         if (m0 == 0) {  // the innovation row
           const uint32_t off = sw_off(KP, slot, L::kGramRows);
@@ -391,8 +441,8 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         if (warp == 0) {
           tc_fence_after();
           const uint32_t a = sR + b * L::kGramBuf;
-          issue3(tmem + L::kTmGram, a, a + 2 * L::kGramSlab, L::kGramSlab, a, a + 2 * L::kGramSlab, L::kGramSlab, 2,
-                 idescG, nch > 0);
+          issue3(tmem + L::kTmGram, a, a + L::kGramSlab, L::kGramSlab, a, a + L::kGramSlab, L::kGramSlab, 1, idescG,
+                 nch > 0);
           mma_commit_elect(&buf_bar[b]);
         }
         ++gchunk;
@@ -426,13 +476,14 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // column group g; each walks its 32 columns 8 at a time.
     const bool rowwarp = q < NG;
     const int row = 32 * q + lane;
-    const int cb = 32 * g;
+    const bool rowin = row < KP;  // KP = 80: the last rows of the third quadrant hold nothing
+    const int cb = 32 * g, ce = (cb + 32 < KP) ? cb + 32 : KP;
     if (rowwarp) {
       float rs = 0.0f, as = 0.0f, fa = 0.0f;
 #pragma unroll 1
-      for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+      for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + tm_row + L::kTmGram + c0, v);
+        ld8(tmem + tm_row + L::kTmGram + c0, v);
         tmem_wait_ld();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -445,15 +496,17 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           }
         }
       }
-      V.part[g][row] = rs;
-      V.part[NG + g][row] = as;
+      if (rowin) {
+        V.part[g][row] = rs;
+        V.part[NG + g][row] = as;
+      }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) fa += __shfl_xor_sync(0xffffffffu, fa, off);
       if (lane == 0) V.red[3 * NG + q * NG + g] = fa;  // ||A||_F^2, by warp
       if (g == 0) {
         const uint32_t bv = tmem_ld1(tmem + tm_row + L::kTmGram + KP);
         tmem_wait_ld();
-        V.b[row] = (row < k) ? __uint_as_float(bv) : 0.0f;
+        if (rowin) V.b[row] = (row < k) ? __uint_as_float(bv) : 0.0f;
       }
     }
     __syncthreads();
@@ -468,7 +521,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         }
         r *= ik;
       }
-      V.r[i] = r;
+      if (i < KP) V.r[i] = r;
       float sr = r, mx = ab, s2 = r * r;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
@@ -494,9 +547,9 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // outside the member block).
     auto pap8 = [&](int c0, float (&x)[8]) {
       uint32_t v[8];
-      tmem_ld8(tmem + tm_row + L::kTmGram + c0, v);
+      ld8(tmem + tm_row + L::kTmGram + c0, v);
       tmem_wait_ld();
-      const float ri = V.r[row];
+      const float ri = rowin ? V.r[row] : 0.0f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int c = c0 + j;
@@ -535,24 +588,32 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     float nsa, nsb;
     ns_coeffs(lsp, nsa, nsb);
     // M = PAP / s + 1 1^T / k (identity on unused member slots); Z <- I,
-    // Y <- M (row-major), T <- T0 = a I - b M stored transposed.
+    // Y <- M (row-major), T <- T0 = a I - b M stored transposed; P A P / s
+    // kept for the finish where it has its own operand.
     if (rowwarp) {
 #pragma unroll 1
-      for (int c0 = cb; c0 < cb + 32; c0 += 8) {
-        float x[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = (row == c0 + j) ? 1.0f : 0.0f;
-        put_row8(ZH, ZL, row, c0, ZR, x);
+      for (int c0 = cb; c0 < ce; c0 += 8) {
+        float x[8], y[8];
         pap8(c0, x);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int c = c0 + j;
-          x[j] = (row < k && c < k) ? x[j] * is + ik : ((row == c) ? 1.0f : 0.0f);
+          x[j] *= is * kSc;
+          y[j] = (row == c0 + j) ? kSc : 0.0f;
         }
-        put_row8(YH, YL, row, c0, ZR, x);
+        if (rowin) {
+          put_row8(ZH, ZL, row, c0, ZR, y);
+          if (L::kStack) put_row8(AH, AL, row, c0, TR, x);
+        }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = ((row == c0 + j) ? nsa : 0.0f) - nsb * x[j];
-        put_col8(TH, TL, row, c0, TR, x);
+        for (int j = 0; j < 8; ++j) {
+          const int c = c0 + j;
+          x[j] = (row < k && c < k) ? x[j] + ik * kSc : y[j];
+          y[j] = nsa * y[j] - nsb * x[j];
+        }
+        if (rowin) {
+          put_row8(YH, YL, row, c0, ZR, x);
+          put_col8(TH, TL, row, c0, TR, y);
+        }
       }
     }
 
@@ -581,10 +642,10 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       if (warp == 0) {
         tc_fence_after();
         if constexpr (L::kStack) {
-          issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescK, false);
+          h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
         } else {
-          issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescK, false);
-          issue3(tmem + L::kTmB, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescK, false);
+          h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
+          h16::issue3(tmem + L::kTmB, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
         }
         mma_commit_elect(&mma_bar);
       }
@@ -596,51 +657,55 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       if (!last) {
         if constexpr (L::kStack) {  // all warps: rows 0-63 Z, 64-127 Y
 #pragma unroll 1
-          for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+          for (int c0 = cb; c0 < ce; c0 += 8) {
             uint32_t v[8];
-            tmem_ld8(tmem + tm_row + c0, v);
+            ld8(tmem + tm_row + c0, v);
             tmem_wait_ld();
             float x[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]);
+            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
             put_row8(ZH, ZL, 32 * q + lane, c0, ZR, x);
           }
         } else if (rowwarp) {  // Z from the first product, Y from the second
 #pragma unroll 1
-          for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+          for (int c0 = cb; c0 < ce; c0 += 8) {
             uint32_t v[8];
             float x[8];
-            tmem_ld8(tmem + tm_row + c0, v);
+            ld8(tmem + tm_row + c0, v);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]);
-            put_row8(ZH, ZL, row, c0, ZR, x);
-            tmem_ld8(tmem + tm_row + L::kTmB + c0, v);
+            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
+            if (rowin) put_row8(ZH, ZL, row, c0, ZR, x);
+            ld8(tmem + tm_row + L::kTmB + c0, v);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]);
-            put_row8(YH, YL, row, c0, ZR, x);
+            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
+            if (rowin) put_row8(YH, YL, row, c0, ZR, x);
           }
         }
       } else if (rowwarp) {
-        // Final Z -> (Z - 1 1^T / k) / sqrt(s) on the member block, 0 elsewhere,
-        // stored transposed (Z's operand holds Z^T); Y's operand <- P A P (from
-        // the Gram in TMEM) for the finish.
-        const float isq = rsqrtf(s);
+        // Final Z -> Z - 1 1^T / k on the member block, 0 elsewhere (A^-1/2
+        // times sqrt(s)), stored transposed (Z's operand holds Z^T); without
+        // an operand of its own, P A P / s (from the Gram in TMEM) goes to
+        // Y's for the finish.
 #pragma unroll 1
-        for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+        for (int c0 = cb; c0 < ce; c0 += 8) {
           uint32_t v[8];
-          tmem_ld8(tmem + tm_row + c0, v);
+          ld8(tmem + tm_row + c0, v);
           tmem_wait_ld();
           float x[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int c = c0 + j;
-            x[j] = (row < k && c < k) ? (__uint_as_float(v[j]) - ik) * isq : 0.0f;
+            x[j] = (row < k && c < k) ? __uint_as_float(v[j]) * (kUnZ * kSc) - ik * kSc : 0.0f;
           }
-          put_col8(ZH, ZL, row, c0, ZR, x);
-          pap8(c0, x);
-          put_row8(YH, YL, row, c0, ZR, x);
+          if (rowin) put_col8(ZH, ZL, row, c0, ZR, x);
+          if (!L::kStack) {
+            pap8(c0, x);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] *= is * kSc;
+            if (rowin) put_row8(AH, AL, row, c0, ZR, x);
+          }
         }
       }
       if (last) break;
@@ -648,7 +713,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       operands_ready();
       if (warp == 0) {
         tc_fence_after();
-        issue3(tmem, sZH, sZL, L::kSlabZ, sYH, sYL, L::kSlabZ, NG, idescK, false);
+        h16::issue3(tmem, sZH, sZL, L::kSlabZ, sYH, sYL, L::kSlabZ, L::kSteps, idescK);
         mma_commit_elect(&mma_bar);
       }
       if (tid == 0) s_flag[0] = 0u;
@@ -658,19 +723,19 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       if (rowwarp) {
         float emax = 0.0f;
 #pragma unroll 1
-        for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+        for (int c0 = cb; c0 < ce; c0 += 8) {
           uint32_t v[8];
-          tmem_ld8(tmem + tm_row + c0, v);
+          ld8(tmem + tm_row + c0, v);
           tmem_wait_ld();
           float t[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int c = c0 + j;
-            const float d = __uint_as_float(v[j]) - ((row == c) ? 1.0f : 0.0f);
-            emax = nan_max(emax, fabsf(d));
-            t[j] = ((row == c) ? nsa - nsb : 0.0f) - nsb * d;  // a I - b P, P = I + d
+            const float d = __uint_as_float(v[j]) * kUnZ - ((row == c) ? 1.0f : 0.0f);
+            if (rowin) emax = nan_max(emax, fabsf(d));
+            t[j] = kSc * (((row == c) ? nsa - nsb : 0.0f) - nsb * d);  // a I - b P, P = I + d
           }
-          put_col8(TH, TL, row, c0, TR, t);
+          if (rowin) put_col8(TH, TL, row, c0, TR, t);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
@@ -696,23 +761,47 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // iteration leaves as right factors, so the finish takes C = Z^T A Z:
     // Q = (P A P) Z (A operand: Y's rows = P A P; B operand: Z^T rows), then
     // C = Z^T Q; A^-1 = Z C^-1 Z^T, A^-1/2 ~ Z C^-1/2.
+    // X' row of variable slot vv (zero beyond k and for unused slots), in
+    // units of its largest entry, -> T row vv: one warp.  Returns the values.
+    auto put_x = [&](int vv, float (&x)[NG]) {
+      float mx = 0.0f;
+#pragma unroll
+      for (int gg = 0; gg < NG; ++gg) mx = fmaxf(mx, fabsf(x[gg]));
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const int ex = min(max((int)(__float_as_uint(mx) >> 23), 6), 253);
+      const float inv = kScX * __uint_as_float((uint32_t)(254 - ex) << 23);
+#pragma unroll
+      for (int gg = 0; gg < NG; ++gg) {
+        const int m = lane + 32 * gg;
+        uint32_t h, l;
+        h16::split2(x[gg] * inv, 0.0f, h, l);
+        if (m < KP) {
+          const uint32_t o = h16::off(vv, m, TR);
+          *reinterpret_cast<uint16_t*>(TH + o) = (uint16_t)h;
+          *reinterpret_cast<uint16_t*>(TL + o) = (uint16_t)l;
+        }
+      }
+      if (lane == 0) V.xu[vv] = __uint_as_float((uint32_t)ex << 23);
+    };
     if (fast) {  // X' rows -> T rows 0..15 (B operand of E; T is free here)
       cp_async_wait_all();
       __syncthreads();
-      for (int e = tid; e < kVarTile * KP; e += kThreads) {
-        const int vv = e / KP, m = e - vv * KP;
-        const uint32_t off = sw_off(vv, m, TR);
-        float h, l;
-        split((vv < npre) ? V.xpre[vv][m] : 0.0f, h, l);
-        *reinterpret_cast<float*>(TH + off) = h;
-        *reinterpret_cast<float*>(TL + off) = l;
+      for (int vv = warp; vv < kVarTile; vv += L::kWarps) {
+        float x[NG];
+#pragma unroll
+        for (int gg = 0; gg < NG; ++gg) {
+          const int m = lane + 32 * gg;
+          x[gg] = (vv < npre && m < KP) ? V.xpre[vv][m] : 0.0f;
+        }
+        put_x(vv, x);
       }
     }
     operands_ready();
     if (warp == 0) {
       tc_fence_after();
-      issue3(tmem, sYH, sYL, L::kSlabZ, sZH, sZL, L::kSlabZ, NG, idescK, false);
-      if (fast) issue3(tmem + L::kTmE, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescU, false);
+      h16::issue3(tmem, sAH, sAL, kSlabA, sZH, sZL, L::kSlabZ, L::kSteps, idescK);
+      if (fast) h16::issue3(tmem + L::kTmE, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescU);
       mma_commit_elect(&mma_bar);
     }
     if (tid < KP) {  // u = Z^T b (row tid of Z^T)
@@ -724,27 +813,27 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc += z[j] * V.b[c0 + j];
       }
-      V.u[tid] = acc;
+      V.u[tid] = acc * (1.0f / kSc);
     }
     if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
     mma_ph ^= 1u;
     if (rowwarp) {  // Q -> T transposed
 #pragma unroll 1
-      for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+      for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + tm_row + c0, v);
+        ld8(tmem + tm_row + c0, v);
         tmem_wait_ld();
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]);
-        put_col8(TH, TL, row, c0, TR, x);
+        for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
+        if (rowin) put_col8(TH, TL, row, c0, TR, x);
       }
     }
     // C = Z^T Q
     operands_ready();
     if (warp == 0) {
       tc_fence_after();
-      issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescK, false);
+      h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
       mma_commit_elect(&mma_bar);
       if (lane == 0) s_flag[1] = 0u;
     }
@@ -758,23 +847,23 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     if (rowwarp) {
       float fu = 0.0f, fm = 0.0f;
 #pragma unroll 1
-      for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+      for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + tm_row + c0, v);
+        ld8(tmem + tm_row + c0, v);
         tmem_wait_ld();
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int c = c0 + j;
           const float pij = (row < k && c < k) ? (((row == c) ? 1.0f : 0.0f) - ik) : 0.0f;
-          const float x = (row < k && c < k) ? __uint_as_float(v[j]) - pij : 0.0f;
-          f[j] = x;
+          const float x = (row < k && c < k) ? __uint_as_float(v[j]) * kUnZ - pij : 0.0f;
+          f[j] = x * kScF;
           fm = nan_max(fm, fabsf(x));
           fu += x * V.u[c];
         }
-        if (fast) {
+        if (rowin && fast) {
           put_col8(YH, YL, row, c0, ZR, f);
-        } else {
+        } else if (rowin) {
           put_col8(TH, TL, row, c0, TR, f);
           get_col8(ZH, ZL, row, c0, ZR, f);
           put_row8(YH, YL, row, c0, ZR, f);
@@ -784,15 +873,15 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         uint32_t v[8];
 #pragma unroll 1
         for (int c0 = 0; c0 < kVarTile; c0 += 8) {
-          tmem_ld8(tmem + tm_row + L::kTmE + c0, v);
+          ld8(tmem + tm_row + L::kTmE + c0, v);
           tmem_wait_ld();
           float e8[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e8[j] = __uint_as_float(v[j]);
-          put_col8(TH, TL, row, c0, TR, e8);
+          for (int j = 0; j < 8; ++j) e8[j] = __uint_as_float(v[j]) * (kUnE * kScX);
+          if (rowin) put_col8(TH, TL, row, c0, TR, e8);
         }
       }
-      V.part[g][row] = fu;
+      if (rowin) V.part[g][row] = fu;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, off));
       // NaN or Inf residuals map to the maximum (positive floats order as integers)
@@ -802,8 +891,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     operands_ready();
     if (warp == 0) {
       tc_fence_after();
-      if (fast) issue3(tmem, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescU, false);
-      else issue3(tmem, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescK, false);
+      h16::issue3(tmem, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, fast ? idescU : idescK);
       mma_commit_elect(&mma_bar);
     }
     const float resid = __uint_as_float(s_flag[1]);
@@ -824,7 +912,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc += z[j] * V.v[c0 + j];
       }
-      V.wa[tid] = sc * acc;
+      V.wa[tid] = sc * is * (1.0f / kSc) * acc;
     }
     if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
     mma_ph ^= 1u;
@@ -833,22 +921,23 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       hand_back();
       continue;
     }
-    if (!fast && rowwarp) {  // W rows -> U^T = W^T into Z's operand (A operand of the update)
+    if (!fast && rowwarp) {  // W rows (over cw / sqrt(s)) -> W^T into Z's operand (A operand of the update)
 #pragma unroll 1
-      for (int c0 = cb; c0 < cb + 32; c0 += 8) {
+      for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + tm_row + c0, v);
+        ld8(tmem + tm_row + c0, v);
         tmem_wait_ld();
         float w[8];
-        get_row8(YH, YL, row, c0, ZR, w);
+        get_row8(YH, YL, rowin ? row : 0, c0, ZR, w);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] = cw * (w[j] - 0.5f * __uint_as_float(v[j]));
-        put_col8(ZH, ZL, row, c0, ZR, w);
+        for (int j = 0; j < 8; ++j) w[j] -= (0.5f * kUnZF * kSc) * __uint_as_float(v[j]);
+        if (rowin) put_col8(ZH, ZL, row, c0, ZR, w);
       }
     }
 
     // ---------------- 5. update ----------------
     const float c1 = cw * rsqrtf(delta);  // W's eigenvalue on the mean direction
+    const float cws = cw * rsqrtf(s);
     cp_async_wait_all();
     __syncthreads();  // the prefetched rows visible to every thread
     if (fast) {
@@ -860,8 +949,8 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
 #pragma unroll
         for (int gg = 0; gg < NG; ++gg) {
           const int m = lane + 32 * gg;
-          const float x0 = V.xpre[vv][m];
-          dw += x0 * V.wa[m];
+          const float x0 = m < KP ? V.xpre[vv][m] : 0.0f;
+          dw += x0 * (m < KP ? V.wa[m] : 0.0f);
           sx += x0;
           sq += x0 * x0;
         }
@@ -882,12 +971,13 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       float dv[kPre];
       if (rowwarp && g == 0) {
         uint32_t dd[8], ee[8];
-        tmem_ld8(tmem + tm_row, dd);
-        tmem_ld8(tmem + tm_row + L::kTmE, ee);
+        ld8(tmem + tm_row, dd);
+        ld8(tmem + tm_row + L::kTmE, ee);
         tmem_wait_ld();
 #pragma unroll
         for (int vv = 0; vv < kPre; ++vv)
-          dv[vv] = cw * (__uint_as_float(ee[vv]) - 0.5f * __uint_as_float(dd[vv])) + V.one[vv];
+          dv[vv] = cws * V.xu[vv] * (__uint_as_float(ee[vv]) * kUnE - 0.5f * kUnD * __uint_as_float(dd[vv])) +
+                   V.one[vv];
         if (rtps) {
 #pragma unroll
           for (int vv = 0; vv < kPre; ++vv) {
@@ -929,20 +1019,17 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       for (int vv = warp; vv < kVarTile; vv += L::kWarps) {
         const bool pre = v0 == 0 && vv < npre;
         const float* xr = (vv < nv && !pre) ? Xp + (base + (int64_t)(v0 + vv) * prm.var_stride) * k : nullptr;
-        float dw = 0.0f, sx = 0.0f, sq = 0.0f;
+        float dw = 0.0f, sx = 0.0f, sq = 0.0f, x[NG];
 #pragma unroll
         for (int gg = 0; gg < NG; ++gg) {
           const int m = lane + 32 * gg;
-          const float x0 = pre ? V.xpre[vv][m] : ((xr && m < k) ? xr[m] : 0.0f);
-          const uint32_t o0 = sw_off(vv, m, TR);
-          float h, l;
-          split(x0, h, l);
-          *reinterpret_cast<float*>(TH + o0) = h;
-          *reinterpret_cast<float*>(TL + o0) = l;
-          dw += x0 * V.wa[m];
+          const float x0 = m < KP ? (pre ? V.xpre[vv][m] : ((xr && m < k) ? xr[m] : 0.0f)) : 0.0f;
+          x[gg] = x0;
+          dw += x0 * (m < KP ? V.wa[m] : 0.0f);
           sx += x0;
           sq += x0 * x0;
         }
+        put_x(vv, x);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
           dw += __shfl_xor_sync(0xffffffffu, dw, off);
@@ -959,7 +1046,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       operands_ready();
       if (warp == 0) {
         tc_fence_after();
-        issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, NG, idescU, false);
+        h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescU);
         mma_commit_elect(&mma_bar);
       }
       if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
@@ -967,13 +1054,13 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       float dv[kVarTile];
       if (rowwarp && g == 0) {
         uint32_t v[8], v2[8];
-        tmem_ld8(tmem + tm_row, v);
-        tmem_ld8(tmem + tm_row + 8, v2);
+        ld8(tmem + tm_row, v);
+        ld8(tmem + tm_row + 8, v2);
         tmem_wait_ld();
 #pragma unroll
         for (int vv = 0; vv < 8; ++vv) {
-          dv[vv] = __uint_as_float(v[vv]) + V.one[vv];
-          dv[8 + vv] = __uint_as_float(v2[vv]) + V.one[8 + vv];
+          dv[vv] = cws * kUnE * V.xu[vv] * __uint_as_float(v[vv]) + V.one[vv];
+          dv[8 + vv] = cws * kUnE * V.xu[8 + vv] * __uint_as_float(v2[vv]) + V.one[8 + vv];
         }
         if (rtps) {  // analysis spread per variable (members = rows 0 .. KP-1)
 #pragma unroll
@@ -1038,8 +1125,8 @@ int launch_tc(const mg::LetkfParams& prm, int num_sms, void* stream, int* ctas) 
   auto kern = letkf_tc_kernel<KP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
-  // The whole unified L1/shared array as shared memory (two KP = 64 CTAs or
-  // one KP = 96 CTA per SM).
+  // The whole unified L1/shared array as shared memory (three KP = 64 CTAs,
+  // two of KP = 80 or one of KP = 96 per SM).
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return (int)e;
@@ -1081,7 +1168,11 @@ bool letkf_tc_supported(const LetkfParams& prm) {
 }
 
 int letkf_tc_launch(const LetkfParams& prm, int num_sms, void* stream, int* ctas) {
-  return prm.k <= 64 ? launch_tc<64>(prm, num_sms, stream, ctas) : launch_tc<96>(prm, num_sms, stream, ctas);
+  // The smallest member slots that hold k: fewer slots are less work and more
+  // CTAs per SM (k = 80: 496 ms in 80 slots, 819 in 96).
+  if (prm.k <= 64) return launch_tc<64>(prm, num_sms, stream, ctas);
+  if (prm.k <= 80) return launch_tc<80>(prm, num_sms, stream, ctas);
+  return launch_tc<96>(prm, num_sms, stream, ctas);
 }
 
 }  // namespace mg
