@@ -33,6 +33,43 @@ void* workspace(mg_context* ctx, size_t bytes) {
   return ctx->ws;
 }
 
+// What a context keeps for its next text call; larger blocks are freed at the
+// end of the call (an allocation is a few hundred us, such a text takes tens
+// of ms).
+constexpr size_t kIoKeep = (size_t)256 << 20;
+
+void* io_workspace(mg_context* ctx, size_t bytes) {
+  if (ctx->io_done) cudaStreamWaitEvent(ctx->stream, ctx->io_done, 0);
+  if (bytes <= ctx->io_ws_bytes) return ctx->io_ws;
+  if (ctx->io_ws) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->io_ws);
+    ctx->io_ws = nullptr;
+    ctx->io_ws_bytes = 0;
+  }
+  const size_t want = bytes + bytes / 8 + (1u << 20);
+  if ((!ctx->io_done && cudaEventCreateWithFlags(&ctx->io_done, cudaEventDisableTiming) != cudaSuccess) ||
+      cudaMalloc(&ctx->io_ws, want) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->last_error = "device workspace allocation of " + std::to_string(want) + " bytes failed";
+    return nullptr;
+  }
+  ctx->io_ws_bytes = want;
+  return ctx->io_ws;
+}
+
+void io_release(mg_context* ctx) {
+  if (!ctx->io_ws) return;
+  if (ctx->io_ws_bytes <= kIoKeep) {
+    cudaEventRecord(ctx->io_done, ctx->stream);
+    return;
+  }
+  cudaStreamSynchronize(ctx->stream);
+  cudaFree(ctx->io_ws);
+  ctx->io_ws = nullptr;
+  ctx->io_ws_bytes = 0;
+}
+
 void* host_stage(mg_context* ctx, size_t bytes) {
   if (bytes <= ctx->host_stage_bytes) return ctx->host_stage;
   if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
@@ -97,6 +134,11 @@ void mg_destroy(mg_context* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->ws);
   }
+  if (ctx->io_ws) {
+    cudaEventSynchronize(ctx->io_done);
+    cudaFree(ctx->io_ws);
+  }
+  if (ctx->io_done) cudaEventDestroy(ctx->io_done);
   if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
   for (auto& e : ctx->ev)
     if (e) cudaEventDestroy(e);

@@ -16,6 +16,9 @@ struct mg_context {
   cudaStream_t stream = nullptr;
   void* ws = nullptr;  // device workspace, grown on demand
   size_t ws_bytes = 0;
+  void* io_ws = nullptr;  // second workspace of the text I/O (the first holds the text)
+  size_t io_ws_bytes = 0;
+  cudaEvent_t io_done = nullptr;  // its last use
   void* host_stage = nullptr;  // pinned host staging for small read-backs
   size_t host_stage_bytes = 0;
   std::string last_error;
@@ -34,6 +37,15 @@ extern thread_local int64_t g_launches;
 int fail(mg_context* ctx, int code, const std::string& msg);
 // Device workspace of at least `bytes`; nullptr (with last_error set) on failure.
 void* workspace(mg_context* ctx, size_t bytes);
+// The text I/O's second workspace: work enqueued on the context's stream from
+// here on waits for its last use, on whatever stream that was.  IoUse marks
+// that use's end; a block above the size that is kept is freed there.
+void* io_workspace(mg_context* ctx, size_t bytes);
+void io_release(mg_context* ctx);
+struct IoUse {
+  mg_context* ctx;
+  ~IoUse() { io_release(ctx); }
+};
 // Pinned host staging of at least `bytes`.
 void* host_stage(mg_context* ctx, size_t bytes);
 

@@ -393,6 +393,9 @@ __global__ void values_write_kernel(const char* __restrict__ t, int64_t n, const
 // to the sequential loop (lane 0).
 constexpr int kWin = 16;
 constexpr int kRound = 32 * kWin;
+// Bytes kept per formatted value (13 up to 99999.999999, 317 at most); a
+// longer text gets a block of its own.
+constexpr int64_t kTextRoom = 24;
 constexpr int64_t kWarpLineBytes = 256;  // mean line length from which a warp reads each line
 
 // Bit j set: a token (a non-blank byte after a blank or at the line start)
@@ -581,8 +584,10 @@ __global__ void fmt_write_kernel(const double* __restrict__ v, int64_t count, in
   }
 }
 
-template <typename F>
-int with_lines(mg_context* ctx, const char* text, int64_t nbytes, F&& body) {
+// Uploads and indexes the text, then body(text, lines, line starts);
+// take(carver, lines) carves the body's own buffers.
+template <typename T, typename F>
+int with_lines(mg_context* ctx, const char* text, int64_t nbytes, T&& take, F&& body) {
   cudaStream_t s = ctx->stream;
   const int64_t nch = (nbytes + kChunk - 1) / kChunk;
   mg::Carver cv;
@@ -601,35 +606,52 @@ int with_lines(mg_context* ctx, const char* text, int64_t nbytes, F&& body) {
   line_count_kernel<<<(unsigned)nch, kThreads, 0, s>>>(t, nbytes, ccount);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(mg::exclusive_scan(ccount, coff, nch, tmp, mg::scan_temp_bytes(nch), s));
-  int64_t L = 0;
-  MG_TRY_CUDA(cudaMemcpyAsync(&L, coff + nch, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  int64_t* stage = static_cast<int64_t*>(mg::host_stage(ctx, 2 * sizeof(int64_t)));  // pinned
+  if (!stage) return MG_ERR_NOMEM;
+  MG_TRY_CUDA(cudaMemcpyAsync(stage, coff + nch, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   MG_TRY_CUDA(cudaStreamSynchronize(s));
-  // The per-line buffers live in a second allocation: the workspace above
-  // holds the text.
+  const int64_t L = stage[0];
+  // The per-line buffers live in a second workspace, kept with the context:
+  // the one above holds the text.  (Allocating them on each call from the
+  // stream-ordered pool, which gives its memory back at every
+  // synchronisation, and pageable read-backs took about half of a call.)
+  mg::Carver io;
+  mg::IoUse use{ctx};
   int64_t* starts = nullptr;
-  MG_TRY_CUDA(cudaMallocAsync(&starts, sizeof(int64_t) * (L + 1), s));
+  for (int pass = 0; pass < 2; ++pass) {
+    starts = io.take<int64_t>(L + 1);
+    take(io, L);
+    if (pass == 1) break;
+    void* iws = mg::io_workspace(ctx, io.off);
+    if (!iws) return MG_ERR_NOMEM;
+    io = mg::Carver{static_cast<char*>(iws), 0};
+  }
   line_fill_kernel<<<(unsigned)nch, kThreads, 0, s>>>(t, nbytes, coff, starts);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
-  const int rc = body(t, L, starts);
-  cudaFreeAsync(starts, s);
-  return rc;
+  return body(t, L, starts);
 }
 
-// The lines a host istringstream must read (numbers outside the fast path);
-// nflag is the device count of them, so the flags are copied only when some
-// are set.
-std::vector<int64_t> host_lines(mg_context* ctx, const int32_t* flags, int64_t L, int32_t want, const int32_t* nflag,
-                                int* rc) {
+// Reads back, in one synchronisation, how many items the host has to convert
+// and the total of the scanned lengths.
+int read_counts(mg_context* ctx, const int32_t* nflag, const int64_t* total_d, int32_t* nf, int64_t* total) {
+  int64_t* stage = static_cast<int64_t*>(mg::host_stage(ctx, 2 * sizeof(int64_t)));
+  if (!stage) return MG_ERR_NOMEM;
+  stage[0] = 0;
+  MG_TRY_CUDA(cudaMemcpyAsync(stage, nflag, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  MG_TRY_CUDA(cudaMemcpyAsync(stage + 1, total_d, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  MG_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+  memcpy(nf, stage, sizeof(int32_t));
+  *total = stage[1];
+  return MG_OK;
+}
+
+// The items (lines or values) a host istringstream must read, numbers outside
+// the fast path; nf is how many the device counted, so the flags are copied
+// only when some are set.
+std::vector<int64_t> host_lines(mg_context* ctx, const int32_t* flags, int64_t L, int32_t want, int32_t nf, int* rc) {
   *rc = MG_OK;
   ctx->io_host_items = 0;
-  if (L == 0) return {};
-  int32_t nf = 0;
-  if (cudaMemcpyAsync(&nf, nflag, sizeof(nf), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-      cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-    *rc = mg::fail(ctx, MG_ERR_CUDA, "text I/O: device copy failed");
-    return {};
-  }
   if (nf == 0) return {};
   std::vector<int32_t> h(L);
   if (cudaMemcpyAsync(h.data(), flags, sizeof(int32_t) * L, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
@@ -662,31 +684,23 @@ int mg_parse_grid_obs(mg_context* ctx, const char* text, int64_t nbytes, double 
   *count = 0;
   if (nbytes == 0) return MG_OK;
   cudaStream_t s = ctx->stream;
-  return with_lines(ctx, text, nbytes, [&](const char* t, int64_t L, int64_t* starts) -> int {
-    ObsLines ol{};
-    unsigned long long* marks = nullptr;  // first header, first separator after it
-    int32_t* nhost = nullptr;
-    int64_t *keep = nullptr, *pos = nullptr;
-    void* tmp = nullptr;
+  ObsLines ol{};
+  unsigned long long* marks = nullptr;  // first header, first separator after it
+  int32_t* nhost = nullptr;
+  int64_t *keep = nullptr, *pos = nullptr;
+  void* tmp = nullptr;
+  auto take = [&](mg::Carver& io, int64_t L) {
+    ol.type = io.take<int32_t>(L);
+    ol.ival = io.take<int32_t>(4 * L);
+    ol.dval = io.take<double>(4 * L);
+    marks = io.take<unsigned long long>(2);
+    nhost = io.take<int32_t>(1);
+    keep = io.take<int64_t>(L + 1);
+    pos = io.take<int64_t>(L + 1);
+    tmp = io.take<char>(mg::scan_temp_bytes(L));
+  };
+  return with_lines(ctx, text, nbytes, take, [&](const char* t, int64_t L, int64_t* starts) -> int {
     const size_t tmpb = mg::scan_temp_bytes(L);
-    MG_TRY_CUDA(cudaMallocAsync(&ol.type, sizeof(int32_t) * L, s));
-    MG_TRY_CUDA(cudaMallocAsync(&ol.ival, sizeof(int32_t) * 4 * L, s));
-    MG_TRY_CUDA(cudaMallocAsync(&ol.dval, sizeof(double) * 4 * L, s));
-    MG_TRY_CUDA(cudaMallocAsync(&marks, sizeof(unsigned long long) * 2, s));
-    MG_TRY_CUDA(cudaMallocAsync(&nhost, sizeof(int32_t), s));
-    MG_TRY_CUDA(cudaMallocAsync(&keep, sizeof(int64_t) * (L + 1), s));
-    MG_TRY_CUDA(cudaMallocAsync(&pos, sizeof(int64_t) * (L + 1), s));
-    MG_TRY_CUDA(cudaMallocAsync(&tmp, tmpb, s));
-    auto release = [&]() {
-      cudaFreeAsync(ol.type, s);
-      cudaFreeAsync(ol.ival, s);
-      cudaFreeAsync(ol.dval, s);
-      cudaFreeAsync(marks, s);
-      cudaFreeAsync(nhost, s);
-      cudaFreeAsync(keep, s);
-      cudaFreeAsync(pos, s);
-      cudaFreeAsync(tmp, s);
-    };
     MG_TRY_CUDA(cudaMemsetAsync(marks, 0xff, sizeof(unsigned long long) * 2, s));
     MG_TRY_CUDA(cudaMemsetAsync(nhost, 0, sizeof(int32_t), s));
     const unsigned g = (unsigned)((L + kThreads - 1) / kThreads);
@@ -695,11 +709,20 @@ int mg_parse_grid_obs(mg_context* ctx, const char* text, int64_t nbytes, double 
     obs_sep_kernel<<<g, kThreads, 0, s>>>(ol.type, L, marks, marks + 1);
     MG_COUNT_LAUNCH();
     MG_TRY_CUDA(cudaGetLastError());
+    auto scan_kept = [&]() -> int {
+      obs_keep_kernel<<<g, kThreads, 0, s>>>(ol, L, marks + 1, missing_value, keep);
+      MG_COUNT_LAUNCH();
+      MG_TRY_CUDA(mg::exclusive_scan(keep, pos, L, tmp, tmpb, s));
+      return MG_OK;
+    };
+    int32_t nf = 0;
+    int64_t total = 0;
+    int rc = scan_kept();
+    if (rc != MG_OK || (rc = read_counts(ctx, nhost, pos + L, &nf, &total)) != MG_OK) return rc;
     // Lines with numbers outside the fast path: the reference's own
     // extraction on the host.
-    int rc = MG_OK;
-    const std::vector<int64_t> hl = host_lines(ctx, ol.type, L, kHost, nhost, &rc);
-    if (rc != MG_OK) return release(), rc;
+    const std::vector<int64_t> hl = host_lines(ctx, ol.type, L, kHost, nf, &rc);
+    if (rc != MG_OK) return rc;
     if (!hl.empty()) {
       std::vector<int64_t> hs(L);
       MG_TRY_CUDA(cudaMemcpyAsync(hs.data(), starts, sizeof(int64_t) * L, cudaMemcpyDeviceToHost, s));
@@ -719,24 +742,16 @@ int mg_parse_grid_obs(mg_context* ctx, const char* text, int64_t nbytes, double 
         MG_TRY_CUDA(cudaMemcpyAsync(ol.type + l, &ty, sizeof(ty), cudaMemcpyHostToDevice, s));
         MG_TRY_CUDA(cudaStreamSynchronize(s));
       }
+      if ((rc = scan_kept()) != MG_OK || (rc = read_counts(ctx, nhost, pos + L, &nf, &total)) != MG_OK) return rc;
     }
-    obs_keep_kernel<<<g, kThreads, 0, s>>>(ol, L, marks + 1, missing_value, keep);
-    MG_COUNT_LAUNCH();
-    MG_TRY_CUDA(mg::exclusive_scan(keep, pos, L, tmp, tmpb, s));
-    int64_t total = 0;
-    MG_TRY_CUDA(cudaMemcpyAsync(&total, pos + L, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    MG_TRY_CUDA(cudaStreamSynchronize(s));
     *count = total;
-    if (total > cap || (total > 0 && (!xyz || !vals))) {
-      release();
+    if (total > cap || (total > 0 && (!xyz || !vals)))
       return mg::fail(ctx, MG_ERR_CAPACITY, "mg_parse_grid_obs: output arrays too small");
-    }
     if (total > 0) {
       obs_write_kernel<<<g, kThreads, 0, s>>>(ol, L, keep, pos, xyz, vals);
       MG_COUNT_LAUNCH();
     }
     MG_TRY_CUDA(cudaGetLastError());
-    release();
     return MG_OK;
   });
 }
@@ -747,23 +762,18 @@ int mg_parse_values(mg_context* ctx, const char* text, int64_t nbytes, double* o
   *count = 0;
   if (nbytes == 0) return MG_OK;
   cudaStream_t s = ctx->stream;
-  return with_lines(ctx, text, nbytes, [&](const char* t, int64_t L, int64_t* starts) -> int {
-    int64_t *counts = nullptr, *offs = nullptr;
-    int32_t *mode = nullptr, *nhost = nullptr;
-    void* tmp = nullptr;
+  int64_t *counts = nullptr, *offs = nullptr;
+  int32_t *mode = nullptr, *nhost = nullptr;
+  void* tmp = nullptr;
+  auto take = [&](mg::Carver& io, int64_t L) {
+    counts = io.take<int64_t>(L + 1);
+    offs = io.take<int64_t>(L + 1);
+    mode = io.take<int32_t>(L);
+    nhost = io.take<int32_t>(1);
+    tmp = io.take<char>(mg::scan_temp_bytes(L));
+  };
+  return with_lines(ctx, text, nbytes, take, [&](const char* t, int64_t L, int64_t* starts) -> int {
     const size_t tmpb = mg::scan_temp_bytes(L);
-    MG_TRY_CUDA(cudaMallocAsync(&counts, sizeof(int64_t) * (L + 1), s));
-    MG_TRY_CUDA(cudaMallocAsync(&offs, sizeof(int64_t) * (L + 1), s));
-    MG_TRY_CUDA(cudaMallocAsync(&mode, sizeof(int32_t) * L, s));
-    MG_TRY_CUDA(cudaMallocAsync(&nhost, sizeof(int32_t), s));
-    MG_TRY_CUDA(cudaMallocAsync(&tmp, tmpb, s));
-    auto release = [&]() {
-      cudaFreeAsync(counts, s);
-      cudaFreeAsync(offs, s);
-      cudaFreeAsync(mode, s);
-      cudaFreeAsync(nhost, s);
-      cudaFreeAsync(tmp, s);
-    };
     MG_TRY_CUDA(cudaMemsetAsync(nhost, 0, sizeof(int32_t), s));
     // Long lines (a state row per line): a warp per line; short ones: a thread.
     const bool by_warp = nbytes >= kWarpLineBytes * L;
@@ -776,8 +786,12 @@ int mg_parse_values(mg_context* ctx, const char* text, int64_t nbytes, double* o
     MG_COUNT_LAUNCH();
     MG_TRY_CUDA(cudaGetLastError());
     int rc = MG_OK;
-    const std::vector<int64_t> hl = host_lines(ctx, mode, L, kValHost, nhost, &rc);
-    if (rc != MG_OK) return release(), rc;
+    int32_t nf = 0;
+    int64_t total = 0;
+    MG_TRY_CUDA(mg::exclusive_scan(counts, offs, L, tmp, tmpb, s));
+    if ((rc = read_counts(ctx, nhost, offs + L, &nf, &total)) != MG_OK) return rc;
+    const std::vector<int64_t> hl = host_lines(ctx, mode, L, kValHost, nf, &rc);
+    if (rc != MG_OK) return rc;
     std::vector<int64_t> hs;
     std::vector<std::vector<double>> hv(hl.size());
     if (!hl.empty()) {
@@ -792,16 +806,12 @@ int mg_parse_values(mg_context* ctx, const char* text, int64_t nbytes, double* o
         MG_TRY_CUDA(cudaMemcpyAsync(counts + hl[q], &c, sizeof(c), cudaMemcpyHostToDevice, s));
         MG_TRY_CUDA(cudaStreamSynchronize(s));
       }
+      MG_TRY_CUDA(mg::exclusive_scan(counts, offs, L, tmp, tmpb, s));
+      if ((rc = read_counts(ctx, nhost, offs + L, &nf, &total)) != MG_OK) return rc;
     }
-    MG_TRY_CUDA(mg::exclusive_scan(counts, offs, L, tmp, tmpb, s));
-    int64_t total = 0;
-    MG_TRY_CUDA(cudaMemcpyAsync(&total, offs + L, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    MG_TRY_CUDA(cudaStreamSynchronize(s));
     *count = total;
-    if (total > cap || (total > 0 && !out)) {
-      release();
+    if (total > cap || (total > 0 && !out))
       return mg::fail(ctx, MG_ERR_CAPACITY, "mg_parse_values: output array too small");
-    }
     if (total > 0) {
       if (by_warp)
         values_write_warp_kernel<<<gw, kThreads, 0, s>>>(t, nbytes, starts, L, offs, mode, out);
@@ -818,7 +828,6 @@ int mg_parse_values(mg_context* ctx, const char* text, int64_t nbytes, double* o
       }
       MG_TRY_CUDA(cudaStreamSynchronize(s));
     }
-    release();
     return MG_OK;
   });
 }
@@ -836,21 +845,24 @@ int mg_format_state(mg_context* ctx, const double* values, int32_t nx, int32_t n
   cudaStream_t s = ctx->stream;
   const int64_t count = (int64_t)nx * ny;
   const size_t tmpb = mg::scan_temp_bytes(count);
+  mg::Carver io;
+  mg::IoUse use{ctx};
   int64_t *len = nullptr, *off = nullptr;
   int32_t *host = nullptr, *nhost = nullptr;
   void* tmp = nullptr;
-  MG_TRY_CUDA(cudaMallocAsync(&len, sizeof(int64_t) * (count + 1), s));
-  MG_TRY_CUDA(cudaMallocAsync(&off, sizeof(int64_t) * (count + 1), s));
-  MG_TRY_CUDA(cudaMallocAsync(&host, sizeof(int32_t) * count, s));
-  MG_TRY_CUDA(cudaMallocAsync(&nhost, sizeof(int32_t), s));
-  MG_TRY_CUDA(cudaMallocAsync(&tmp, tmpb, s));
-  auto release = [&]() {
-    cudaFreeAsync(len, s);
-    cudaFreeAsync(off, s);
-    cudaFreeAsync(host, s);
-    cudaFreeAsync(nhost, s);
-    cudaFreeAsync(tmp, s);
-  };
+  char* dout = nullptr;
+  for (int pass = 0; pass < 2; ++pass) {
+    len = io.take<int64_t>(count + 1);
+    off = io.take<int64_t>(count + 1);
+    host = io.take<int32_t>(count);
+    nhost = io.take<int32_t>(1);
+    tmp = io.take<char>(tmpb);
+    dout = io.take<char>((size_t)count * kTextRoom);
+    if (pass == 1) break;
+    void* iws = mg::io_workspace(ctx, io.off);
+    if (!iws) return MG_ERR_NOMEM;
+    io = mg::Carver{static_cast<char*>(iws), 0};
+  }
   MG_TRY_CUDA(cudaMemsetAsync(nhost, 0, sizeof(int32_t), s));
   const unsigned g = (unsigned)((count + kThreads - 1) / kThreads);
   fmt_len_kernel<<<g, kThreads, 0, s>>>(values, count, nx, len, host, nhost);
@@ -858,8 +870,12 @@ int mg_format_state(mg_context* ctx, const double* values, int32_t nx, int32_t n
   MG_TRY_CUDA(cudaGetLastError());
   // Values the device does not format: their text length comes from the host.
   int rc = MG_OK;
-  const std::vector<int64_t> hl = host_lines(ctx, host, count, 1, nhost, &rc);
-  if (rc != MG_OK) return release(), rc;
+  int32_t nf = 0;
+  int64_t total = 0;
+  MG_TRY_CUDA(mg::exclusive_scan(len, off, count, tmp, tmpb, s));
+  if ((rc = read_counts(ctx, nhost, off + count, &nf, &total)) != MG_OK) return rc;
+  const std::vector<int64_t> hl = host_lines(ctx, host, count, 1, nf, &rc);
+  if (rc != MG_OK) return rc;
   std::vector<std::string> htxt(hl.size());
   for (size_t q = 0; q < hl.size(); ++q) {
     double v = 0.0;
@@ -875,17 +891,19 @@ int mg_format_state(mg_context* ctx, const double* values, int32_t nx, int32_t n
     MG_TRY_CUDA(cudaMemcpyAsync(len + hl[q], &l, sizeof(l), cudaMemcpyHostToDevice, s));
     MG_TRY_CUDA(cudaStreamSynchronize(s));
   }
-  MG_TRY_CUDA(mg::exclusive_scan(len, off, count, tmp, tmpb, s));
-  int64_t total = 0;
-  MG_TRY_CUDA(cudaMemcpyAsync(&total, off + count, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  MG_TRY_CUDA(cudaStreamSynchronize(s));
+  if (!hl.empty()) {
+    MG_TRY_CUDA(mg::exclusive_scan(len, off, count, tmp, tmpb, s));
+    if ((rc = read_counts(ctx, nhost, off + count, &nf, &total)) != MG_OK) return rc;
+  }
   *nbytes = total;
   if (total > cap || !out) {
-    release();
     return out ? mg::fail(ctx, MG_ERR_CAPACITY, "mg_format_state: output buffer too small") : MG_ERR_CAPACITY;
   }
-  char* dout = nullptr;
-  MG_TRY_CUDA(cudaMallocAsync(&dout, (size_t)total, s));
+  char* big = nullptr;
+  if (total > count * kTextRoom) {
+    MG_TRY_CUDA(cudaMallocAsync(&big, (size_t)total, s));
+    dout = big;
+  }
   fmt_write_kernel<<<g, kThreads, 0, s>>>(values, count, nx, off, host, dout);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
@@ -896,8 +914,7 @@ int mg_format_state(mg_context* ctx, const double* values, int32_t nx, int32_t n
     MG_TRY_CUDA(cudaMemcpy(&o, off + hl[q], sizeof(o), cudaMemcpyDeviceToHost));
     std::memcpy(out + o, htxt[q].data(), htxt[q].size());
   }
-  cudaFreeAsync(dout, s);
-  release();
+  if (big) cudaFreeAsync(big, s);
   return MG_OK;
 }
 
