@@ -48,6 +48,22 @@ static __device__ __forceinline__ void put_row8(unsigned char* hi, unsigned char
   *reinterpret_cast<uint4*>(lo + o) = vl;
 }
 
+// The same values to two operands.
+static __device__ __forceinline__ void put_row8x2(unsigned char* hi, unsigned char* lo, uint32_t rows,
+                                                  unsigned char* hi2, unsigned char* lo2, uint32_t rows2, int r, int c0,
+                                                  const float (&x)[8]) {
+  uint4 vh, vl;
+  split2(x[0], x[1], vh.x, vl.x);
+  split2(x[2], x[3], vh.y, vl.y);
+  split2(x[4], x[5], vh.z, vl.z);
+  split2(x[6], x[7], vh.w, vl.w);
+  const uint32_t o = off(r, c0, rows), o2 = off(r, c0, rows2);
+  *reinterpret_cast<uint4*>(hi + o) = vh;
+  *reinterpret_cast<uint4*>(lo + o) = vl;
+  *reinterpret_cast<uint4*>(hi2 + o2) = vh;
+  *reinterpret_cast<uint4*>(lo2 + o2) = vl;
+}
+
 static __device__ __forceinline__ void get_row8(const unsigned char* hi, const unsigned char* lo, int r, int c0,
                                                 uint32_t rows, float (&x)[8]) {
   const uint32_t o = off(r, c0, rows);
@@ -109,30 +125,32 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-static __device__ __forceinline__ void mma_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+static __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// D (TMEM) = A B over nk K-steps of 16, 3 passes each.  A: 128 rows from
-// a_hi / a_lo (slab stride a_slab); B: N rows from b_hi / b_lo.  Called by
-// all of warp 0 with the same arguments; out of line: one copy of the issue
-// loop for every product of the kernel.
-static __device__ __noinline__ void issue3(uint32_t dtm, uint32_t a_hi, uint32_t a_lo, uint32_t a_slab, uint32_t b_hi,
-                                           uint32_t b_lo, uint32_t b_slab, int nk, uint32_t idesc) {
+// D (TMEM) = A B over NK K-steps of 16, 3 passes each.  A: 128 rows from
+// a_hi / a_lo (slab stride A_SLAB); B: N rows from b_hi / b_lo.  Called by one
+// thread.  Unrolled and inline: the descriptors are constants off the
+// operands' addresses; as a loop in a function of its own, the issue took
+// 1300 cycles of a step in which the tensor core needs about 500.
+template <int NK, uint32_t A_SLAB, uint32_t B_SLAB>
+static __device__ __forceinline__ void issue3(uint32_t dtm, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
+                                              uint32_t idesc) {
   const uint64_t ah = smem_desc_sw64(a_hi), al = smem_desc_sw64(a_lo);
   const uint64_t bh = smem_desc_sw64(b_hi), bl = smem_desc_sw64(b_lo);
-  for (int s = 0; s < nk; ++s) {
-    const uint64_t ao = (uint64_t)(((s >> 1) * a_slab + (s & 1) * 32) >> 4);
-    const uint64_t bo = (uint64_t)(((s >> 1) * b_slab + (s & 1) * 32) >> 4);
-    mma_elect(dtm, ah + ao, bh + bo, idesc, s > 0 ? 1u : 0u);
-    mma_elect(dtm, ah + ao, bl + bo, idesc, 1u);
-    mma_elect(dtm, al + ao, bh + bo, idesc, 1u);
+#pragma unroll
+  for (int s = 0; s < NK; ++s) {
+    const uint64_t ao = (uint64_t)(((s >> 1) * A_SLAB + (s & 1) * 32) >> 4);
+    const uint64_t bo = (uint64_t)(((s >> 1) * B_SLAB + (s & 1) * 32) >> 4);
+    mma(dtm, ah + ao, bh + bo, idesc, s > 0 ? 1u : 0u);
+    mma(dtm, ah + ao, bl + bo, idesc, 1u);
+    mma(dtm, al + ao, bh + bo, idesc, 1u);
   }
 }
 

@@ -23,10 +23,16 @@
 //    and [Z; Y] T is two products.
 //  * KP = 96 (80 < k <= 96): as KP = 80 with 1 CTA per SM: 96-slot operands
 //    and Gram need more than 256 columns.
-// Whole cycles with TF32 pairs (2, 1 and 1 CTAs, k = 80 in 96 slots) -> this:
-// 360 x 180 x 10 points, 4 variables, k = 64, 500k obs, FP32 members: 118.7
-// -> 91.9 ms; 360 x 180 x 30 points, k = 80, clustered obs: 819 -> 496 ms.  Error against 64 bits
-// on smaller grids: 2.5e-7 -> 2.3e-7 and 4.5e-7 -> 4.3e-7.
+// The chain is kept short: one CTA barrier per product (a wait that gave up is
+// decided on at the next one), the MMAs of a product issued as straight code
+// by one thread (as a loop with a lane election each, issuing took 1300
+// cycles a product), T stored by rows, the next analysis pulled and the next
+// rows of Y' loaded while others are worked on.
+// Whole cycles with TF32 pairs (2, 1 and 1 CTAs, k = 80 in 96 slots) -> FP16
+// pairs -> the shorter chain: 360 x 180 x 10 points, 4 variables, k = 64, 500k
+// obs, FP32 members: 118.7 -> 91.9 -> 79.8 ms; 360 x 180 x 30 points, k = 80,
+// clustered obs: 819 -> 496 -> 406 ms.  Error against 64 bits on smaller
+// grids: 2.5e-7 -> 2.3e-7 and 4.5e-7 -> 4.3e-7.
 //
 // Per local analysis (one CTA, persistent, points pulled in the grid's
 // column order from a work counter):
@@ -229,6 +235,38 @@ __device__ __noinline__ bool vertical_keep_fp64(int lev, double obs_lev, double 
   return fabs((double)lev - obs_lev) <= vsupport;
 }
 
+// One analysis of the grid, and where its candidates lie.
+struct Item {
+  int64_t base, e0, e1;
+  int col, lev;  // lev < 0: none left
+};
+
+// The next analysis, by one thread: a chain of four dependent global loads.
+__device__ __noinline__ void pull(const mg::LetkfParams& prm, Item& it) {
+  const unsigned long long n = atomicAdd(prm.next, 1ull);
+  if (n >= (unsigned long long)prm.npoints) {
+    it.lev = -1;
+    return;
+  }
+  const uint32_t item = (uint32_t)n, nlev = (uint32_t)prm.nlev;  // npoints fits an int32 (redo_out)
+  const int lev = (int)(item % nlev);
+  const int64_t col = prm.order[item / nlev];
+  it.col = (int)col;
+  it.lev = lev;
+  it.base = prm.col_base[col] + (int64_t)lev * prm.lev_stride;
+  int64_t e0 = prm.loc_off[col], e1 = prm.loc_off[col + 1];
+  if (prm.lev_boff) {  // only the level buckets that can reach this level
+    const int32_t* bo = prm.lev_boff + col * (int64_t)(prm.nlev + 1);
+    const double fl = floor((double)lev - prm.vsupport), fh = floor((double)lev + prm.vsupport);
+    const int lo = (fl <= 0.0) ? 0 : (int)fl;
+    const int hi = (fh >= (double)(prm.nlev - 1)) ? prm.nlev - 1 : (int)fh;
+    e1 = e0 + bo[hi + 1];
+    e0 = e0 + bo[lo];
+  }
+  it.e0 = e0;
+  it.e1 = e1;
+}
+
 template <int KP>
 __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_tc_kernel(mg::LetkfParams prm) {
   using L = Lay<KP>;
@@ -239,6 +277,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   using h16::get_row8;
   using h16::put_col8;
   using h16::put_row8;
+  using h16::put_row8x2;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* R = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Vecs<KP>& V = *reinterpret_cast<Vecs<KP>*>(R + L::kRegion);
@@ -256,10 +295,11 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   __shared__ uint64_t mma_bar;
   __shared__ uint64_t buf_bar[kNBuf];
   __shared__ uint32_t tmem_s;
-  __shared__ long long s_item;
-  __shared__ unsigned s_flag[4];
+  __shared__ Item s_it;
+  __shared__ unsigned s_flag[2];  // of the iteration's parity; the finish uses the first
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform to the compiler
   const int q = warp & 3, g = warp >> 2;  // TMEM lane quadrant, 32-column group
   const int k = prm.k;
   const float ik = 1.0f / (float)k;
@@ -305,57 +345,62 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
   uint32_t gchunk = 0;      // Gram chunks issued by this CTA (buffer rotation)
   bool alive = true;
 
+  const int32_t* __restrict__ lidx = prm.lev_boff ? prm.bidx : prm.loc_idx;
+  const double* __restrict__ ldist = prm.lev_boff ? prm.bdist : prm.loc_dist;
+  bool pulled = false;  // s_it holds this analysis
+
   for (;;) {
     cp_async_wait_all();  // a handed-back analysis may leave its prefetch in flight
-    if (tid == 0) s_item = (long long)atomicAdd(prm.next, 1ull);
-    __syncthreads();
-    const long long item = s_item;
-    __syncthreads();
-    if (item >= prm.npoints) break;
-    const int lev = (int)(item % prm.nlev);
-    const int64_t col = prm.order[item / prm.nlev];
-    const int64_t base = prm.col_base[col] + (int64_t)lev * prm.lev_stride;
-    int64_t e0 = prm.loc_off[col], e1 = prm.loc_off[col + 1];
-    const int32_t* lidx = prm.loc_idx;
-    const double* ldist = prm.loc_dist;
-    if (prm.lev_boff) {  // only the level buckets that can reach this level
-      const int32_t* bo = prm.lev_boff + col * (int64_t)(prm.nlev + 1);
-      const double fl = floor((double)lev - prm.vsupport), fh = floor((double)lev + prm.vsupport);
-      const int lo = (fl <= 0.0) ? 0 : (int)fl;
-      const int hi = (fh >= (double)(prm.nlev - 1)) ? prm.nlev - 1 : (int)fh;
-      e1 = e0 + bo[hi + 1];
-      e0 = e0 + bo[lo];
-      lidx = prm.bidx;
-      ldist = prm.bdist;
+    if (!pulled) {
+      if (tid == 0) pull(prm, s_it);
+      __syncthreads();
     }
+    pulled = false;
+    const int lev = s_it.lev, col = s_it.col;
+    if (lev < 0) break;
+    const int64_t base = s_it.base, e0 = s_it.e0, e1 = s_it.e1;
 
     // ---------------- 1. selection and Gram ----------------
     // Rounds: compact candidates into the ring (up to kSelRing - kThreads
     // entries), then emit its chunks; each chunk's rows are loaded into
     // registers while the previous chunk is stored and its MMAs issued.
     int64_t cpos = e0;
+    bool ok = true;  // this thread's waits since the last decision
+    // A block's indices and distances are loaded one block ahead.
+    int o_n = 0;
+    double d_n = 0.0;
+    auto fetch = [&](int64_t c) {
+      if (c + tid < e1) {
+        o_n = lidx[c + tid];
+        if (ldist) d_n = ldist[c + tid];
+      }
+    };
+    fetch(cpos);
     int nloc = 0, nch = 0, head = 0, nsel = 0;
     const int slot = tid & (kChunk - 1), m0 = (tid / kChunk) * 8;  // gather: obs slot x 8 members
-    auto load_rows = [&](int pos, int cnt, float (&x)[8], float& sd) {
+    // Raw values: they are scaled when they are stored, so the loads stay in
+    // flight until then.
+    auto load_rows = [&](int pos, int cnt, float (&x)[8], float& sw, float& sd) {
       if (slot < cnt) {
         const int e = (pos + slot) & (kSelRing - 1);
         const int o = sel_o[e];
-        const float sw = sel_sw[e];
+        sw = sel_sw[e];
         sd = sel_sd[e];
         const float* yr = Y + (int64_t)o * k;
         if (vec4 && m0 + 8 <= k) {
 #pragma unroll
           for (int q4 = 0; q4 < 2; ++q4) {
             const float4 a4 = *reinterpret_cast<const float4*>(yr + m0 + 4 * q4);
-            x[4 * q4 + 0] = a4.x * sw; x[4 * q4 + 1] = a4.y * sw; x[4 * q4 + 2] = a4.z * sw; x[4 * q4 + 3] = a4.w * sw;
+            x[4 * q4 + 0] = a4.x; x[4 * q4 + 1] = a4.y; x[4 * q4 + 2] = a4.z; x[4 * q4 + 3] = a4.w;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] = (m0 + j < k) ? yr[m0 + j] * sw : 0.0f;
+          for (int j = 0; j < 8; ++j) x[j] = (m0 + j < k) ? yr[m0 + j] : 0.0f;
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = 0.0f;
+        sw = 0.0f;
         sd = 0.0f;
       }
     };
@@ -364,9 +409,10 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         bool keep = false;
         int o = 0;
         float sw = 0.0f, sd = 0.0f;
+        const double d = d_n;
+        o = o_n;
+        fetch(cpos + kThreads);
         if (cpos + tid < e1) {
-          const int64_t e = cpos + tid;
-          o = lidx[e];
           const float4 pk = prm.opack[o];  // (level, 1/sigma^2, innovation, 0) as FP32
           float w = 1.0f;
           keep = true;
@@ -377,7 +423,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
             if (keep && !r_identity) w *= mg::gaspari_cohn<float>(dl / vc);
           }
           if (keep && !r_identity) {
-            if (ldist) w *= mg::gaspari_cohn<float>((float)ldist[e] / hc);
+            if (ldist) w *= mg::gaspari_cohn<float>((float)d / hc);
             w *= pk.y;
             if (!(w > 0.0f)) keep = false;
           }
@@ -408,12 +454,12 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
       const bool done = cpos >= e1;
       const int nchunks = done ? (nsel + kChunk - 1) / kChunk : nsel / kChunk;
-      float x[8], sdv;
-      if (nchunks > 0) load_rows(head, nsel < kChunk ? nsel : kChunk, x, sdv);
+      float x[8], swv, sdv;
+      if (nchunks > 0) load_rows(head, nsel < kChunk ? nsel : kChunk, x, swv, sdv);
       for (int c = 0; c < nchunks; ++c) {
         const int b = (int)(gchunk % kNBuf);
         const uint32_t use = gchunk / kNBuf;
-        if (use > 0 && !wait_all(&buf_bar[b], (use - 1) & 1u)) { alive = false; break; }
+        if (use > 0 && !wait_one(&buf_bar[b], (use - 1) & 1u)) ok = false;
         unsigned char* bh = R + b * L::kGramBuf;
         unsigned char* bl = bh + L::kGramSlab;
         if (m0 < KP) {
@@ -421,7 +467,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           for (int j = 0; j < 8; ++j) {
             const uint32_t off = sw_off(m0 + j, slot, L::kGramRows);
             float h, l;
-            split(x[j], h, l);
+            split(x[j] * swv, h, l);
             *reinterpret_cast<float*>(bh + off) = h;
             *reinterpret_cast<float*>(bl + off) = l;
           }
@@ -435,15 +481,17 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         }
         if (c + 1 < nchunks) {  // next chunk's rows in flight during the barrier and the MMAs
           const int rem = nsel - (c + 1) * kChunk;
-          load_rows(head + (c + 1) * kChunk, rem < kChunk ? rem : kChunk, x, sdv);
+          load_rows(head + (c + 1) * kChunk, rem < kChunk ? rem : kChunk, x, swv, sdv);
         }
-        operands_ready();
+        if (!operands_ready(ok)) { alive = false; break; }
         if (warp == 0) {
           tc_fence_after();
           const uint32_t a = sR + b * L::kGramBuf;
-          issue3(tmem + L::kTmGram, a, a + L::kGramSlab, L::kGramSlab, a, a + L::kGramSlab, L::kGramSlab, 1, idescG,
-                 nch > 0);
-          mma_commit_elect(&buf_bar[b]);
+          if (elect_one()) {
+            issue3(tmem + L::kTmGram, a, a + L::kGramSlab, a, a + L::kGramSlab, idescG, nch > 0);
+            mma_commit(&buf_bar[b]);
+          }
+          __syncwarp();
         }
         ++gchunk;
         ++nch;
@@ -467,9 +515,15 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       __syncthreads();
       continue;
     }
-    if (warp == 0) mma_commit_elect(&mma_bar);
-    if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+    if (warp == 0) {
+      if (elect_one()) mma_commit(&mma_bar);
+      __syncwarp();
+    }
+    if (!wait_all(&mma_bar, mma_ph, ok)) { alive = false; break; }
     mma_ph ^= 1u;
+    // The next analysis, by a warp that holds no rows in this phase.
+    if (tid == kThreads - 1) pull(prm, s_it);
+    pulled = true;
 
     // ---------------- 2. A, b, deflation and scaling ----------------
     // Warps of quadrants 0 .. NG-1 hold rows 0 .. KP-1 (their TMEM lanes),
@@ -587,9 +641,12 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     }
     float nsa, nsb;
     ns_coeffs(lsp, nsa, nsb);
-    // M = PAP / s + 1 1^T / k (identity on unused member slots); Z <- I,
-    // Y <- M (row-major), T <- T0 = a I - b M stored transposed; P A P / s
-    // kept for the finish where it has its own operand.
+    // M = PAP / s + 1 1^T / k (identity on unused member slots); Y <- M, T
+    // <- T0 = a I - b M, and Z <- T0: the first step's Z (Z = I before it), so
+    // that step computes Y T only.  P A P / s is kept for the finish where it
+    // has its own operand.  T is symmetric up to rounding and stored as
+    // computed (a transposed store took 16 two-byte stores for two of 16
+    // bytes; on a CPU model of this arithmetic either gives the same errors).
     if (rowwarp) {
 #pragma unroll 1
       for (int c0 = cb; c0 < ce; c0 += 8) {
@@ -600,10 +657,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           x[j] *= is * kSc;
           y[j] = (row == c0 + j) ? kSc : 0.0f;
         }
-        if (rowin) {
-          put_row8(ZH, ZL, row, c0, ZR, y);
-          if (L::kStack) put_row8(AH, AL, row, c0, TR, x);
-        }
+        if (L::kStack && rowin) put_row8(AH, AL, row, c0, TR, x);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int c = c0 + j;
@@ -612,7 +666,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         }
         if (rowin) {
           put_row8(YH, YL, row, c0, ZR, x);
-          put_col8(TH, TL, row, c0, TR, y);
+          put_row8x2(TH, TL, TR, ZH, ZL, ZR, row, c0, y);
         }
       }
     }
@@ -637,25 +691,40 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     bool conv = false;
     bool diverged = false;
     for (;;) {
-      // [Z; Y] <- [Z; Y] T
-      operands_ready();
+      // [Z; Y] <- [Z; Y] T (the first step: Y only)
+      if (!operands_ready(ok)) { alive = false; break; }
+      if (its > 0) {
+        const unsigned fl = s_flag[its & 1];
+        stop = fl == 0u;
+        if (fl & 2u) {
+          diverged = true;
+          break;
+        }
+      }
       if (warp == 0) {
         tc_fence_after();
-        if constexpr (L::kStack) {
-          h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
-        } else {
-          h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
-          h16::issue3(tmem + L::kTmB, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
+        if (elect_one()) {
+          if constexpr (L::kStack) {
+            h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
+          } else {
+            if (its > 0) h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
+            h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem + L::kTmB, sYH, sYL, sTH, sTL, idescK);
+          }
+          mma_commit(&mma_bar);
         }
-        mma_commit_elect(&mma_bar);
+        __syncwarp();
       }
+      const bool zstep = its > 0;
       ++its;
       const bool last = stop || its >= kMaxIt;
       conv = stop;
-      if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+      // This iteration's flags (the last ones were read before the barrier
+      // that follows).
+      if (tid == 0) s_flag[its & 1] = 0u;
+      if (!wait_one(&mma_bar, mma_ph)) ok = false;
       mma_ph ^= 1u;
       if (!last) {
-        if constexpr (L::kStack) {  // all warps: rows 0-63 Z, 64-127 Y
+        if (L::kStack && (zstep || !rowwarp)) {  // all warps: rows 0-63 Z, 64-127 Y
 #pragma unroll 1
           for (int c0 = cb; c0 < ce; c0 += 8) {
             uint32_t v[8];
@@ -666,16 +735,18 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
             for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
             put_row8(ZH, ZL, 32 * q + lane, c0, ZR, x);
           }
-        } else if (rowwarp) {  // Z from the first product, Y from the second
+        } else if (!L::kStack && rowwarp) {  // Z from the first product, Y from the second
 #pragma unroll 1
           for (int c0 = cb; c0 < ce; c0 += 8) {
             uint32_t v[8];
             float x[8];
-            ld8(tmem + tm_row + c0, v);
-            tmem_wait_ld();
+            if (zstep) {
+              ld8(tmem + tm_row + c0, v);
+              tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
-            if (rowin) put_row8(ZH, ZL, row, c0, ZR, x);
+              for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
+              if (rowin) put_row8(ZH, ZL, row, c0, ZR, x);
+            }
             ld8(tmem + tm_row + L::kTmB + c0, v);
             tmem_wait_ld();
 #pragma unroll
@@ -709,45 +780,40 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         }
       }
       if (last) break;
-      // P = Z Y (Y as stored), T = a I - b P (scaled step) -> T transposed.
-      operands_ready();
+      // P = Z Y (Y as stored), T = a I - b P (scaled step).
+      if (!operands_ready(ok)) { alive = false; break; }
       if (warp == 0) {
         tc_fence_after();
-        h16::issue3(tmem, sZH, sZL, L::kSlabZ, sYH, sYL, L::kSlabZ, L::kSteps, idescK);
-        mma_commit_elect(&mma_bar);
+        if (elect_one()) {
+          h16::issue3<L::kSteps, L::kSlabZ, L::kSlabZ>(tmem, sZH, sZL, sYH, sYL, idescK);
+          mma_commit(&mma_bar);
+        }
+        __syncwarp();
       }
-      if (tid == 0) s_flag[0] = 0u;
       ns_coeffs(lsp, nsa, nsb);
-      if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+      const float td = kSc * (nsa - nsb), tb = -kSc * nsb;
+      if (!wait_one(&mma_bar, mma_ph)) ok = false;
       mma_ph ^= 1u;
       if (rowwarp) {
-        float emax = 0.0f;
+        unsigned emax = 0u;  // max |d| by bits: a NaN is above every number
 #pragma unroll 1
         for (int c0 = cb; c0 < ce; c0 += 8) {
           uint32_t v[8];
           ld8(tmem + tm_row + c0, v);
           tmem_wait_ld();
           float t[8];
+          const int dj = row - c0;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const int c = c0 + j;
-            const float d = __uint_as_float(v[j]) * kUnZ - ((row == c) ? 1.0f : 0.0f);
-            if (rowin) emax = nan_max(emax, fabsf(d));
-            t[j] = kSc * (((row == c) ? nsa - nsb : 0.0f) - nsb * d);  // a I - b P, P = I + d
+            const float d = __uint_as_float(v[j]) * kUnZ - ((dj == j) ? 1.0f : 0.0f);
+            emax = max(emax, __float_as_uint(d) & 0x7fffffffu);
+            t[j] = tb * d + ((dj == j) ? td : 0.0f);  // a I - b P, P = I + d
           }
-          if (rowin) put_col8(TH, TL, row, c0, TR, t);
+          if (rowin) put_row8(TH, TL, row, c0, TR, t);
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
-        if (lane == 0 && !(emax < kStop)) atomicOr(&s_flag[0], 1u);
-        if (lane == 0 && !(emax < kDiverged)) atomicOr(&s_flag[0], 2u);
-      }
-      __syncthreads();
-      const unsigned fl = s_flag[0];
-      stop = fl == 0u;
-      if (fl & 2u) {
-        diverged = true;
-        break;
+        emax = __reduce_max_sync(0xffffffffu, rowin ? emax : 0u);
+        if (lane == 0 && emax >= __float_as_uint(kStop))
+          atomicOr(&s_flag[its & 1], emax >= __float_as_uint(kDiverged) ? 3u : 1u);
       }
     }
     if (!alive) break;
@@ -797,12 +863,15 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         put_x(vv, x);
       }
     }
-    operands_ready();
+    if (!operands_ready(ok)) { alive = false; break; }
     if (warp == 0) {
       tc_fence_after();
-      h16::issue3(tmem, sAH, sAL, kSlabA, sZH, sZL, L::kSlabZ, L::kSteps, idescK);
-      if (fast) h16::issue3(tmem + L::kTmE, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescU);
-      mma_commit_elect(&mma_bar);
+      if (elect_one()) {
+        h16::issue3<L::kSteps, kSlabA, L::kSlabZ>(tmem, sAH, sAL, sZH, sZL, idescK);
+        if (fast) h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem + L::kTmE, sZH, sZL, sTH, sTL, idescU);
+        mma_commit(&mma_bar);
+      }
+      __syncwarp();
     }
     if (tid < KP) {  // u = Z^T b (row tid of Z^T)
       float acc = 0.0f;
@@ -815,7 +884,8 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
       V.u[tid] = acc * (1.0f / kSc);
     }
-    if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+    if (tid == 0) s_flag[0] = 0u;
+    if (!wait_one(&mma_bar, mma_ph)) ok = false;
     mma_ph ^= 1u;
     if (rowwarp) {  // Q -> T transposed
 #pragma unroll 1
@@ -830,14 +900,16 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
     }
     // C = Z^T Q
-    operands_ready();
+    if (!operands_ready(ok)) { alive = false; break; }
     if (warp == 0) {
       tc_fence_after();
-      h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescK);
-      mma_commit_elect(&mma_bar);
-      if (lane == 0) s_flag[1] = 0u;
+      if (elect_one()) {
+        h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
+        mma_commit(&mma_bar);
+      }
+      __syncwarp();
     }
-    if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+    if (!wait_one(&mma_bar, mma_ph)) ok = false;
     mma_ph ^= 1u;
     // F = C - P (residual, partial F u) -> T transposed (B operand of Z F);
     // Z rows, read from the columns of Z^T, -> Y's operand row-major (A
@@ -885,16 +957,19 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, off));
       // NaN or Inf residuals map to the maximum (positive floats order as integers)
-      if (lane == 0) atomicMax(&s_flag[1], (fm == fm && fm < 3.0e38f) ? __float_as_uint(fm) : 0x7f800000u);
+      if (lane == 0) atomicMax(&s_flag[0], (fm == fm && fm < 3.0e38f) ? __float_as_uint(fm) : 0x7f800000u);
     }
     // W = cw Z (I - F/2): D = Z F (short finish: D = F^T E, 16 columns)
-    operands_ready();
+    if (!operands_ready(ok)) { alive = false; break; }
     if (warp == 0) {
       tc_fence_after();
-      h16::issue3(tmem, sYH, sYL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, fast ? idescU : idescK);
-      mma_commit_elect(&mma_bar);
+      if (elect_one()) {
+        h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sYH, sYL, sTH, sTL, fast ? idescU : idescK);
+        mma_commit(&mma_bar);
+      }
+      __syncwarp();
     }
-    const float resid = __uint_as_float(s_flag[1]);
+    const float resid = __uint_as_float(s_flag[0]);
     if (tid < KP) {
       float fu = 0.0f;
 #pragma unroll
@@ -914,7 +989,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
       V.wa[tid] = sc * is * (1.0f / kSc) * acc;
     }
-    if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+    if (!wait_all(&mma_bar, mma_ph, ok)) { alive = false; break; }
     mma_ph ^= 1u;
     const bool redo = !conv || !(resid <= fminf(kResidMax, kCondResid * l0));
     if (redo) {
@@ -1043,13 +1118,16 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           V.xm[vv] = pre ? V.xmpre[vv] : ((vv < nv) ? prm.xmean[base + (int64_t)(v0 + vv) * prm.var_stride] : 0.0);
         }
       }
-      operands_ready();
+      operands_ready(true);
       if (warp == 0) {
         tc_fence_after();
-        h16::issue3(tmem, sZH, sZL, L::kSlabZ, sTH, sTL, L::kSlabT, L::kSteps, idescU);
-        mma_commit_elect(&mma_bar);
+        if (elect_one()) {
+          h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescU);
+          mma_commit(&mma_bar);
+        }
+        __syncwarp();
       }
-      if (!wait_all(&mma_bar, mma_ph)) { alive = false; break; }
+      if (!wait_all(&mma_bar, mma_ph, true)) { alive = false; break; }
       mma_ph ^= 1u;
       float dv[kVarTile];
       if (rowwarp && g == 0) {
@@ -1099,7 +1177,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       atomicAdd(prm.total_sweeps, (unsigned long long)its);
       atomicMax(prm.max_local, nloc);
       atomicMax(prm.max_sweeps, its);
-      atomicMax(prm.max_resid_bits, s_flag[1]);
+      atomicMax(prm.max_resid_bits, s_flag[0]);
     }
   }
 
@@ -1169,7 +1247,7 @@ bool letkf_tc_supported(const LetkfParams& prm) {
 
 int letkf_tc_launch(const LetkfParams& prm, int num_sms, void* stream, int* ctas) {
   // The smallest member slots that hold k: fewer slots are less work and more
-  // CTAs per SM (k = 80: 496 ms in 80 slots, 819 in 96).
+  // CTAs per SM (k = 80, FP16 pairs: 496 ms in 80 slots; TF32 pairs in 96: 819).
   if (prm.k <= 64) return launch_tc<64>(prm, num_sms, stream, ctas);
   if (prm.k <= 80) return launch_tc<80>(prm, num_sms, stream, ctas);
   return launch_tc<96>(prm, num_sms, stream, ctas);

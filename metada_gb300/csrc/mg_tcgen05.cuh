@@ -55,13 +55,18 @@ __device__ __forceinline__ bool mbar_test(uint32_t addr, uint32_t parity) {
 // Wait for the given phase parity, bounded by elapsed time (kWaitNs, checked
 // every 64 polls; try_wait itself may suspend for a hardware-defined time, so
 // a poll count would not bound the wall time) and, for mbar_wait_ab, by
-// another role raising *abort.  False if it gave up.
+// another role raising *abort.  False if it gave up.  The clock is first read
+// after 64 polls: the usual wait ends before.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (unsigned it = 1;; ++it) {
     if (mbar_test(addr, parity)) return true;
-    if ((it & 63u) == 0u && global_ns() - t0 > kWaitNs) return false;
+    if ((it & 63u) == 0u) {
+      const uint64_t t = global_ns();
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > kWaitNs) return false;
+    }
   }
 }
 
@@ -112,16 +117,24 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// kind::tf32 issued from a converged warp: every lane passes the same
-// operands and elect.sync picks the one lane that issues (the lowest, lane 0
-// of a full warp, so a later commit from that lane tracks it).
-__device__ __forceinline__ void mma_tf32_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
+// True in one lane of a converged warp (always the same one): the lane that
+// issues a warp's MMAs and their commit.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
+}
+
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
@@ -130,15 +143,6 @@ __device__ __forceinline__ void mma_tf32_elect(uint32_t tmem_d, uint64_t adesc, 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
-}
-
-// Commit from the lane that elect.sync picks in a converged warp.
-__device__ __forceinline__ void mma_commit_elect(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
-      : "memory");
 }
 
 // Tensor memory: allocation (one warp, the column count a power of two >= 32),

@@ -27,38 +27,44 @@ static __device__ __forceinline__ void split(float x, float& h, float& l) {
   l = x - h;
 }
 
-// D (TMEM) += A B over nslab slabs of 32 K-columns, 3 passes per K-step of 8.
-// A: 128 rows from a_hi/a_lo (slab stride a_slab); B: N rows from b_hi/b_lo.
-// Called by all of warp 0 with the same arguments (lane 0 issues); out of
-// line: one copy of the issue loop for every product of the kernel.
-static __device__ __noinline__ void issue3(uint32_t dtm, uint32_t a_hi, uint32_t a_lo, uint32_t a_slab, uint32_t b_hi,
-                                       uint32_t b_lo, uint32_t b_slab, int nslab, uint32_t idesc, bool accumulate) {
+// D (TMEM) (+)= A B over one slab of 32 K-columns, 3 passes per K-step of 8.
+// A: 128 rows from a_hi/a_lo; B: N rows from b_hi/b_lo.  Called by one thread.
+static __device__ __forceinline__ void issue3(uint32_t dtm, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
+                                              uint32_t idesc, bool accumulate) {
   // Descriptors of the first K-step; later steps add (byte offset >> 4) to
   // the 14-bit start-address field (shared addresses stay below 256 KB).
   const uint64_t ah = smem_desc_sw128(a_hi), al = smem_desc_sw128(a_lo);
   const uint64_t bh = smem_desc_sw128(b_hi), bl = smem_desc_sw128(b_lo);
-  for (int s = 0; s < nslab; ++s) {
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const uint64_t ao = (uint64_t)((s * a_slab + kk * 32) >> 4), bo = (uint64_t)((s * b_slab + kk * 32) >> 4);
-      mma_tf32_elect(dtm, ah + ao, bh + bo, idesc, (accumulate || s > 0 || kk > 0) ? 1u : 0u);
-      mma_tf32_elect(dtm, ah + ao, bl + bo, idesc, 1u);
-      mma_tf32_elect(dtm, al + ao, bh + bo, idesc, 1u);
-    }
+  for (int kk = 0; kk < 4; ++kk) {
+    const uint64_t o = (uint64_t)(kk * 32 >> 4);
+    mma_tf32(dtm, ah + o, bh + o, idesc, (accumulate || kk > 0) ? 1u : 0u);
+    mma_tf32(dtm, ah + o, bl + o, idesc, 1u);
+    mma_tf32(dtm, al + o, bh + o, idesc, 1u);
   }
 }
 
 // Operands written by the generic proxy become visible to the tensor core,
-// earlier TMEM reads are ordered before what follows the barrier.
-static __device__ __forceinline__ void operands_ready() {
+// earlier TMEM reads are ordered before what follows the barrier.  One
+// CTA-wide decision on the waits of the step before: false if any thread's
+// gave up.
+static __device__ __forceinline__ bool operands_ready(bool ok) {
   fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();
+  return __syncthreads_or(ok ? 0 : 1) == 0;
 }
 
-// Every thread waits (bounded) for the phase; one CTA-wide decision.
-static __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity) {
+// This thread waits (bounded) for the phase; what it reads or writes next is
+// in bounds either way, and operands_ready takes the CTA's decision.
+static __device__ __forceinline__ bool wait_one(uint64_t* bar, uint32_t parity) {
   const bool ok = mbar_wait(bar, parity);
+  tc_fence_after();
+  return ok;
+}
+
+// As wait_one, with the CTA's decision at once.
+static __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, bool ok) {
+  if (!mbar_wait(bar, parity)) ok = false;
   const int bad = __syncthreads_or(ok ? 0 : 1);
   tc_fence_after();
   return bad == 0;
