@@ -28,10 +28,12 @@
 // by one thread (as a loop with a lane election each, issuing took 1300
 // cycles a product), T stored by rows, the next analysis pulled and the next
 // rows of Y' loaded while others are worked on.
+// The finish's products are taken transposed, so that each operand is stored
+// by rows (16-byte stores), and the mean's increment rides along as a column.
 // Whole cycles with TF32 pairs (2, 1 and 1 CTAs, k = 80 in 96 slots) -> FP16
-// pairs -> the shorter chain: 360 x 180 x 10 points, 4 variables, k = 64, 500k
-// obs, FP32 members: 118.7 -> 91.9 -> 79.8 ms; 360 x 180 x 30 points, k = 80,
-// clustered obs: 819 -> 496 -> 406 ms.  Error against 64 bits on smaller
+// pairs -> the shorter chain -> this finish: 360 x 180 x 10 points, 4 variables, k = 64, 500k
+// obs, FP32 members: 118.7 -> 91.9 -> 79.8 -> 73.1 ms; 360 x 180 x 30 points, k = 80,
+// clustered obs: 819 -> 496 -> 406 -> 372 ms.  Error against 64 bits on smaller
 // grids: 2.5e-7 -> 2.3e-7 and 4.5e-7 -> 4.3e-7.
 //
 // Per local analysis (one CTA, persistent, points pulled in the grid's
@@ -63,8 +65,9 @@
 //  5. Update: D = W^T X'^T (members x variables) on the tensor core, then
 //     x_a = x_mean + X' wa + D (+ RTPS relaxation), written in FP64 (or FP32
 //     storage).  Points with at most kPre variables take the short finish:
-//     E = Z^T X'^T is issued beside the finish's first product and
-//     W^T X'^T = cw (E - F^T E / 2), so W is never formed.
+//     E = Z^T [X'^T b] is issued beside the finish's first product,
+//     W^T X'^T = cw (E - F^T E / 2) and X' wa = c E^T (I - F) Z^T b, so
+//     neither W nor wa is formed.
 // Every mbarrier wait is bounded in time; a wait that gives up makes the CTA
 // set the status word, drain its own MMAs (bounded) and free its TMEM.
 #include <cuda_runtime.h>
@@ -179,8 +182,8 @@ struct Vecs {
   float part[2 * NG][KP];
   float red[32];
   float xsq[kVarTile], inc[kVarTile], fac[kVarTile], one[kVarTile];
-  float ssa[NG][kVarTile];
-  float xu[kVarTile];  // unit of each variable's X' row
+  float ssa[NG][kVarTile], sdw[NG][kPre];
+  float xu[kVarTile];  // unit of each variable's X' row (slot kPre in the finish: of b)
   double xm[kVarTile];
   double xmpre[kPre];
   float xpre[kPre][KP];
@@ -193,7 +196,7 @@ constexpr size_t smem_bytes() {
 }
 static_assert(3 * (smem_bytes<64>() + 1280) <= 233472 && 2 * (smem_bytes<80>() + 1280) <= 233472,
               "CTAs per SM by shared memory");
-static_assert(sizeof(Vecs<64>) >= 64 * 64, "the last rows that P A P reads as a 128-row operand");
+static_assert(sizeof(Vecs<80>) >= 48 * 64 && sizeof(Vecs<96>) >= 32 * 64, "the last rows that T reads as a 128-row operand");
 
 // Scaled Newton-Schulz step.  The spectrum of Z Y lies in [l, 1] (l = delta / s
 // at the start: P A P >= delta on the complement of 1, s >= lambda_max).  The
@@ -215,9 +218,6 @@ __device__ __forceinline__ void ns_coeffs(float& l, float& a, float& b) {
   const float ml = fminf(mu * l, 1.0f);
   l = ml * (3.0f - ml) * (3.0f - ml) * 0.25f;
 }
-
-// Maximum that a NaN poisons (fmaxf would drop it): NaN -> +inf.
-__device__ __forceinline__ float nan_max(float m, float x) { return (x != x) ? __int_as_float(0x7f800000) : fmaxf(m, x); }
 
 // Asynchronous global -> shared copies (no registers held while in flight).
 __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
@@ -685,6 +685,29 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // never formed (one dependent product and two epilogues fewer).
     const bool fast = prm.n_var <= kPre;
 
+    // X' row of variable slot vv (zero beyond k and for unused slots), in
+    // units of its largest entry, -> T row vv: one warp.
+    auto put_x = [&](int vv, float (&x)[NG]) {
+      float mx = 0.0f;
+#pragma unroll
+      for (int gg = 0; gg < NG; ++gg) mx = fmaxf(mx, fabsf(x[gg]));
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const int ex = min(max((int)(__float_as_uint(mx) >> 23), 6), 253);
+      const float inv = kScX * __uint_as_float((uint32_t)(254 - ex) << 23);
+#pragma unroll
+      for (int gg = 0; gg < NG; ++gg) {
+        const int m = lane + 32 * gg;
+        uint32_t h, l;
+        h16::split2(x[gg] * inv, 0.0f, h, l);
+        if (m < KP) {
+          const uint32_t o = h16::off(vv, m, TR);
+          *reinterpret_cast<uint16_t*>(TH + o) = (uint16_t)h;
+          *reinterpret_cast<uint16_t*>(TL + o) = (uint16_t)l;
+        }
+      }
+      if (lane == 0) V.xu[vv] = __uint_as_float((uint32_t)ex << 23);
+    };
     // ---------------- 3. coupled Newton-Schulz ----------------
     int its = 0;
     bool stop = false;  // decided from max |Z Y - I| of the current iterate
@@ -704,7 +727,9 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       if (warp == 0) {
         tc_fence_after();
         if (elect_one()) {
-          if constexpr (L::kStack) {
+          if (stop || its + 1 >= kMaxIt) {  // the last step: Z^T = T^T Z^T, by rows as the finish reads it
+            h16::issue3<L::kSteps, L::kSlabT, L::kSlabZ>(tmem, sTH, sTL, sZH, sZL, idescK);
+          } else if constexpr (L::kStack) {
             h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
           } else {
             if (its > 0) h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
@@ -755,10 +780,9 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           }
         }
       } else if (rowwarp) {
-        // Final Z -> Z - 1 1^T / k on the member block, 0 elsewhere (A^-1/2
-        // times sqrt(s)), stored transposed (Z's operand holds Z^T); without
-        // an operand of its own, P A P / s (from the Gram in TMEM) goes to
-        // Y's for the finish.
+        // Final Z^T -> Z^T - 1 1^T / k on the member block, 0 elsewhere (A^-1/2
+        // times sqrt(s)); without an operand of its own, P A P / s (from the
+        // Gram in TMEM) goes to Y's for the finish.
 #pragma unroll 1
         for (int c0 = cb; c0 < ce; c0 += 8) {
           uint32_t v[8];
@@ -770,7 +794,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
             const int c = c0 + j;
             x[j] = (row < k && c < k) ? __uint_as_float(v[j]) * (kUnZ * kSc) - ik * kSc : 0.0f;
           }
-          if (rowin) put_col8(ZH, ZL, row, c0, ZR, x);
+          if (rowin) put_row8(ZH, ZL, row, c0, ZR, x);
           if (!L::kStack) {
             pap8(c0, x);
 #pragma unroll
@@ -778,9 +802,24 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
             if (rowin) put_row8(AH, AL, row, c0, ZR, x);
           }
         }
+      } else {
+        // Warps without rows: X' of the first variables and b -> T rows 0 ..
+        // kPre (B operand of E; T is free here).
+        for (int vv = (q - NG) * NG + g; vv <= kPre; vv += (4 - NG) * NG) {
+          if (vv < kPre && vv >= npre) continue;
+          const float* xr = vv < kPre ? V.xpre[vv] : V.b;
+          float x[NG];
+#pragma unroll
+          for (int gg = 0; gg < NG; ++gg) {
+            const int m = lane + 32 * gg;
+            x[gg] = m < KP ? xr[m] : 0.0f;
+          }
+          put_x(vv, x);
+        }
       }
       if (last) break;
       // P = Z Y (Y as stored), T = a I - b P (scaled step).
+      cp_async_wait_all();  // the prefetched X' rows, visible to every thread from the barrier on
       if (!operands_ready(ok)) { alive = false; break; }
       if (warp == 0) {
         tc_fence_after();
@@ -825,69 +864,24 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // ---------------- 4. finish ----------------
     // The iterate is Z = p(M) up to rounding errors that the coupled
     // iteration leaves as right factors, so the finish takes C = Z^T A Z:
-    // Q = (P A P) Z (A operand: Y's rows = P A P; B operand: Z^T rows), then
-    // C = Z^T Q; A^-1 = Z C^-1 Z^T, A^-1/2 ~ Z C^-1/2.
-    // X' row of variable slot vv (zero beyond k and for unused slots), in
-    // units of its largest entry, -> T row vv: one warp.  Returns the values.
-    auto put_x = [&](int vv, float (&x)[NG]) {
-      float mx = 0.0f;
-#pragma unroll
-      for (int gg = 0; gg < NG; ++gg) mx = fmaxf(mx, fabsf(x[gg]));
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const int ex = min(max((int)(__float_as_uint(mx) >> 23), 6), 253);
-      const float inv = kScX * __uint_as_float((uint32_t)(254 - ex) << 23);
-#pragma unroll
-      for (int gg = 0; gg < NG; ++gg) {
-        const int m = lane + 32 * gg;
-        uint32_t h, l;
-        h16::split2(x[gg] * inv, 0.0f, h, l);
-        if (m < KP) {
-          const uint32_t o = h16::off(vv, m, TR);
-          *reinterpret_cast<uint16_t*>(TH + o) = (uint16_t)h;
-          *reinterpret_cast<uint16_t*>(TL + o) = (uint16_t)l;
-        }
-      }
-      if (lane == 0) V.xu[vv] = __uint_as_float((uint32_t)ex << 23);
-    };
-    if (fast) {  // X' rows -> T rows 0..15 (B operand of E; T is free here)
-      cp_async_wait_all();
-      __syncthreads();
-      for (int vv = warp; vv < kVarTile; vv += L::kWarps) {
-        float x[NG];
-#pragma unroll
-        for (int gg = 0; gg < NG; ++gg) {
-          const int m = lane + 32 * gg;
-          x[gg] = (vv < npre && m < KP) ? V.xpre[vv][m] : 0.0f;
-        }
-        put_x(vv, x);
-      }
-    }
+    // Q^T = Z^T (P A P) (A operand: Z^T rows; B operand: P A P), C^T = Q^T Z;
+    // A^-1 = Z C^-1 Z^T, A^-1/2 ~ Z C^-1/2.  The transposed products leave
+    // every operand of the next one in the rows that the threads hold (16-byte
+    // stores).  E = Z^T [X'^T b] beside Q^T; u = Z^T b is its column kPre.
     if (!operands_ready(ok)) { alive = false; break; }
     if (warp == 0) {
       tc_fence_after();
       if (elect_one()) {
-        h16::issue3<L::kSteps, kSlabA, L::kSlabZ>(tmem, sAH, sAL, sZH, sZL, idescK);
-        if (fast) h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem + L::kTmE, sZH, sZL, sTH, sTL, idescU);
+        h16::issue3<L::kSteps, L::kSlabZ, kSlabA>(tmem, sZH, sZL, sAH, sAL, idescK);
+        h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem + L::kTmE, sZH, sZL, sTH, sTL, idescU);
         mma_commit(&mma_bar);
       }
       __syncwarp();
     }
-    if (tid < KP) {  // u = Z^T b (row tid of Z^T)
-      float acc = 0.0f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < KP; c0 += 8) {
-        float z[8];
-        get_row8(ZH, ZL, tid, c0, ZR, z);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc += z[j] * V.b[c0 + j];
-      }
-      V.u[tid] = acc * (1.0f / kSc);
-    }
     if (tid == 0) s_flag[0] = 0u;
     if (!wait_one(&mma_bar, mma_ph)) ok = false;
     mma_ph ^= 1u;
-    if (rowwarp) {  // Q -> T transposed
+    if (rowwarp) {  // Q^T -> T
 #pragma unroll 1
       for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
@@ -896,68 +890,70 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         float x[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[j]) * (kUnZ * kSc);
-        if (rowin) put_col8(TH, TL, row, c0, TR, x);
+        if (rowin) put_row8(TH, TL, row, c0, TR, x);
+      }
+      if (!fast && g == 0) {
+        const uint32_t uv = tmem_ld1(tmem + tm_row + L::kTmE + kPre);
+        tmem_wait_ld();
+        if (rowin) V.u[row] = kUnE * V.xu[kPre] * __uint_as_float(uv);
       }
     }
-    // C = Z^T Q
+    // C^T = Q^T Z
     if (!operands_ready(ok)) { alive = false; break; }
     if (warp == 0) {
       tc_fence_after();
       if (elect_one()) {
-        h16::issue3<L::kSteps, L::kSlabZ, L::kSlabT>(tmem, sZH, sZL, sTH, sTL, idescK);
+        h16::issue3<L::kSteps, L::kSlabT, L::kSlabZ>(tmem, sTH, sTL, sZH, sZL, idescK);
         mma_commit(&mma_bar);
       }
       __syncwarp();
     }
     if (!wait_one(&mma_bar, mma_ph)) ok = false;
     mma_ph ^= 1u;
-    // F = C - P (residual, partial F u) -> T transposed (B operand of Z F);
-    // Z rows, read from the columns of Z^T, -> Y's operand row-major (A
-    // operand of Z F; P A P there is not read any more).  Short finish:
-    // F^T -> Y's operand (A operand of F^T E) and E -> T rows 0..15 (its B
-    // operand).
+    // F = C - P, symmetric up to rounding (residual).  Short finish: F^T ->
+    // Y's operand (A operand of F^T E) and E -> T rows 0 .. 7 (its B operand).
+    // Else F^T -> T (B operand of Z F), partial F u, and the rows of Z, read
+    // from the columns of Z^T, -> Y's operand (A operand of Z F).
     if (rowwarp) {
-      float fu = 0.0f, fm = 0.0f;
+      float fu = 0.0f;
+      unsigned fm = 0u;  // max |F| by bits: a NaN is above every number
 #pragma unroll 1
       for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
         ld8(tmem + tm_row + c0, v);
         tmem_wait_ld();
         float f[8];
+        const int dj = row - c0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int c = c0 + j;
-          const float pij = (row < k && c < k) ? (((row == c) ? 1.0f : 0.0f) - ik) : 0.0f;
-          const float x = (row < k && c < k) ? __uint_as_float(v[j]) * kUnZ - pij : 0.0f;
+          const float x =
+              (row < k && c < k) ? __uint_as_float(v[j]) * kUnZ - (((dj == j) ? 1.0f : 0.0f) - ik) : 0.0f;
           f[j] = x * kScF;
-          fm = nan_max(fm, fabsf(x));
-          fu += x * V.u[c];
+          fm = max(fm, __float_as_uint(x) & 0x7fffffffu);
+          if (!fast) fu += x * V.u[c];
         }
         if (rowin && fast) {
-          put_col8(YH, YL, row, c0, ZR, f);
+          put_row8(YH, YL, row, c0, ZR, f);
         } else if (rowin) {
-          put_col8(TH, TL, row, c0, TR, f);
+          put_row8(TH, TL, row, c0, TR, f);
           get_col8(ZH, ZL, row, c0, ZR, f);
           put_row8(YH, YL, row, c0, ZR, f);
         }
       }
       if (fast && g == 0) {
         uint32_t v[8];
-#pragma unroll 1
-        for (int c0 = 0; c0 < kVarTile; c0 += 8) {
-          ld8(tmem + tm_row + L::kTmE + c0, v);
-          tmem_wait_ld();
-          float e8[8];
+        ld8(tmem + tm_row + L::kTmE, v);
+        tmem_wait_ld();
+        float e8[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e8[j] = __uint_as_float(v[j]) * (kUnE * kScX);
-          if (rowin) put_col8(TH, TL, row, c0, TR, e8);
-        }
+        for (int j = 0; j < 8; ++j) e8[j] = __uint_as_float(v[j]) * (kUnE * kScX);
+        if (rowin) put_col8(TH, TL, row, 0, TR, e8);
       }
-      if (rowin) V.part[g][row] = fu;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, off));
+      if (!fast && rowin) V.part[g][row] = fu;
+      fm = __reduce_max_sync(0xffffffffu, rowin ? fm : 0u);
       // NaN or Inf residuals map to the maximum (positive floats order as integers)
-      if (lane == 0) atomicMax(&s_flag[0], (fm == fm && fm < 3.0e38f) ? __float_as_uint(fm) : 0x7f800000u);
+      if (lane == 0) atomicMax(&s_flag[0], min(fm, 0x7f800000u));
     }
     // W = cw Z (I - F/2): D = Z F (short finish: D = F^T E, 16 columns)
     if (!operands_ready(ok)) { alive = false; break; }
@@ -970,24 +966,47 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       __syncwarp();
     }
     const float resid = __uint_as_float(s_flag[0]);
-    if (tid < KP) {
-      float fu = 0.0f;
+    const float c1 = cw * rsqrtf(delta);  // W's eigenvalue on the mean direction
+    const float cws = cw * rsqrtf(s);
+    if (fast) {  // the mean of X' and sum of X'^2 (one warp per variable)
+      for (int vv = warp; vv < prm.n_var; vv += L::kWarps) {
+        float sx = 0.0f, sq = 0.0f;
 #pragma unroll
-      for (int gg = 0; gg < NG; ++gg) fu += V.part[gg][tid];
-      V.v[tid] = (tid < k) ? V.u[tid] - fu : 0.0f;
-    }
-    __syncthreads();
-    if (tid < KP) {  // wa = c Z v (row tid of Z: in Y's operand, or column tid of Z^T)
-      float acc = 0.0f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < KP; c0 += 8) {
-        float z[8];
-        if (fast) get_col8(ZH, ZL, tid, c0, ZR, z);
-        else get_row8(YH, YL, tid, c0, ZR, z);
+        for (int gg = 0; gg < NG; ++gg) {
+          const int m = lane + 32 * gg;
+          const float x0 = m < KP ? V.xpre[vv][m] : 0.0f;
+          sx += x0;
+          sq += x0 * x0;
+        }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc += z[j] * V.v[c0 + j];
+        for (int off = 16; off > 0; off >>= 1) {
+          sx += __shfl_xor_sync(0xffffffffu, sx, off);
+          if (rtps) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        }
+        if (lane == 0) {
+          V.one[vv] = c1 * sx * ik;
+          V.xsq[vv] = sq;
+        }
       }
-      V.wa[tid] = sc * is * (1.0f / kSc) * acc;
+    } else {
+      if (tid < KP) {
+        float fu = 0.0f;
+#pragma unroll
+        for (int gg = 0; gg < NG; ++gg) fu += V.part[gg][tid];
+        V.v[tid] = (tid < k) ? V.u[tid] - fu : 0.0f;
+      }
+      __syncthreads();
+      if (tid < KP) {  // wa = c Z v (row tid of Z, in Y's operand)
+        float acc = 0.0f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < KP; c0 += 8) {
+          float z[8];
+          get_row8(YH, YL, tid, c0, ZR, z);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc += z[j] * V.v[c0 + j];
+        }
+        V.wa[tid] = sc * is * (1.0f / kSc) * acc;
+      }
     }
     if (!wait_all(&mma_bar, mma_ph, ok)) { alive = false; break; }
     mma_ph ^= 1u;
@@ -1011,77 +1030,55 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     }
 
     // ---------------- 5. update ----------------
-    const float c1 = cw * rsqrtf(delta);  // W's eigenvalue on the mean direction
-    const float cws = cw * rsqrtf(s);
-    cp_async_wait_all();
-    __syncthreads();  // the prefetched rows visible to every thread
     if (fast) {
-      // X' W = cw (E - D / 2), D = F^T E, from TMEM; X' wa, the mean of X'
-      // and sum of X'^2 from the prefetched rows (one warp per variable).
+      // X' W = cw (E - D / 2), D = F^T E, from TMEM; with v = u - F u (column
+      // kPre of both) the mean's increment X' wa is c E^T v, a sum over the
+      // rows like RTPS's spread.
       const int nv = prm.n_var;
-      for (int vv = warp; vv < nv; vv += L::kWarps) {
-        float dw = 0.0f, sx = 0.0f, sq = 0.0f;
-#pragma unroll
-        for (int gg = 0; gg < NG; ++gg) {
-          const int m = lane + 32 * gg;
-          const float x0 = m < KP ? V.xpre[vv][m] : 0.0f;
-          dw += x0 * (m < KP ? V.wa[m] : 0.0f);
-          sx += x0;
-          sq += x0 * x0;
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          dw += __shfl_xor_sync(0xffffffffu, dw, off);
-          sx += __shfl_xor_sync(0xffffffffu, sx, off);
-          sq += __shfl_xor_sync(0xffffffffu, sq, off);
-        }
-        if (lane == 0) {
-          V.one[vv] = c1 * sx * ik;
-          V.inc[vv] = dw;
-          V.xsq[vv] = sq;
-          V.xm[vv] = V.xmpre[vv];
-        }
-      }
-      __syncthreads();
       float dv[kPre];
       if (rowwarp && g == 0) {
         uint32_t dd[8], ee[8];
         ld8(tmem + tm_row, dd);
         ld8(tmem + tm_row + L::kTmE, ee);
         tmem_wait_ld();
+        const float vr = V.xu[kPre] * (__uint_as_float(ee[kPre]) * kUnE - kUnD * __uint_as_float(dd[kPre]));
 #pragma unroll
-        for (int vv = 0; vv < kPre; ++vv)
-          dv[vv] = cws * V.xu[vv] * (__uint_as_float(ee[vv]) * kUnE - 0.5f * kUnD * __uint_as_float(dd[vv])) +
-                   V.one[vv];
-        if (rtps) {
+        for (int vv = 0; vv < kPre; ++vv) {
+          const bool in = row < k && vv < nv;
+          const float e = __uint_as_float(ee[vv]) * kUnE;
+          dv[vv] = in ? cws * V.xu[vv] * (e - 0.5f * kUnD * __uint_as_float(dd[vv])) + V.one[vv] : 0.0f;
+          float dw = in ? e * vr : 0.0f, s2 = dv[vv] * dv[vv];
 #pragma unroll
-          for (int vv = 0; vv < kPre; ++vv) {
-            float s2 = (row < k && vv < nv) ? dv[vv] * dv[vv] : 0.0f;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-            if (lane == 0) V.ssa[q][vv] = s2;
+          for (int off = 16; off > 0; off >>= 1) {
+            dw += __shfl_xor_sync(0xffffffffu, dw, off);
+            if (rtps) s2 += __shfl_xor_sync(0xffffffffu, s2, off);
+          }
+          if (lane == 0) {
+            V.sdw[q][vv] = dw;
+            V.ssa[q][vv] = s2;
           }
         }
       }
-      if (rtps) {
-        __syncthreads();
-        if (tid < nv) {
-          float s2 = 0.0f;
-#pragma unroll
-          for (int qq = 0; qq < NG; ++qq) s2 += V.ssa[qq][tid];
-          const float sb = sqrtf(V.xsq[tid] / (float)(k - 1));
-          const float sa = sqrtf(s2 / (float)(k - 1));
-          V.fac[tid] = (sa > 0.0f) ? (float)prm.rho * (sb - sa) / sa : 0.0f;  // factor - 1
-        }
-        __syncthreads();
-      }
+      __syncthreads();
       if (rowwarp && g == 0 && row < k) {
 #pragma unroll
         for (int vv = 0; vv < kPre; ++vv) {
           if (vv < nv) {
-            const float a2 = rtps ? dv[vv] * (1.0f + V.fac[vv]) : dv[vv];
+            float dw = 0.0f, s2 = 0.0f;
+#pragma unroll
+            for (int qq = 0; qq < NG; ++qq) {
+              dw += V.sdw[qq][vv];
+              s2 += V.ssa[qq][vv];
+            }
+            float a2 = dv[vv];
+            if (rtps) {
+              const float sb = sqrtf(V.xsq[vv] / (float)(k - 1));
+              const float sa = sqrtf(s2 / (float)(k - 1));
+              a2 *= 1.0f + ((sa > 0.0f) ? (float)prm.rho * (sb - sa) / sa : 0.0f);
+            }
+            const float inc = sc * is * V.xu[vv] * dw;
             mg::letkf_store(prm, (base + (int64_t)vv * prm.var_stride) * k + row,
-                            (V.xm[vv] + (double)V.inc[vv]) + (double)a2);
+                            (V.xmpre[vv] + (double)inc) + (double)a2);
           }
         }
       }
