@@ -30,18 +30,21 @@
 // rows of Y' loaded while others are worked on.
 // The finish's products are taken transposed, so that each operand is stored
 // by rows (16-byte stores), and the mean's increment rides along as a column.
+// The Gram's compensated product takes one MMA pass (k <= 64) or two instead
+// of three: its third term is the transpose of the second.
 // Whole cycles with TF32 pairs (2, 1 and 1 CTAs, k = 80 in 96 slots) -> FP16
-// pairs -> the shorter chain -> this finish: 360 x 180 x 10 points, 4 variables, k = 64, 500k
-// obs, FP32 members: 118.7 -> 91.9 -> 79.8 -> 73.1 ms; 360 x 180 x 30 points, k = 80,
-// clustered obs: 819 -> 496 -> 406 -> 372 ms.  Error against 64 bits on smaller
-// grids: 2.5e-7 -> 2.3e-7 and 4.5e-7 -> 4.3e-7.
+// pairs -> the shorter chain -> this finish -> this Gram: 360 x 180 x 10
+// points, 4 variables, k = 64, 500k obs, FP32 members: 118.7 -> 91.9 -> 79.8
+// -> 73.1 -> 71.5 ms; 360 x 180 x 30 points, k = 80, clustered obs: 819 -> 496
+// -> 406 -> 372 -> 370 ms.  Error against 64 bits on a smaller grid: 2.5e-7 ->
+// 2.1e-7.
 //
 // Per local analysis (one CTA, persistent, points pulled in the grid's
 // column order from a work counter):
 //  1. Gram: the candidate list is filtered and weighted, the kept rows
 //     sqrt(w) Y'_o are gathered 32 at a time into a K-major, 128-byte
 //     swizzled operand (members x obs) with sqrt(w) d_o as an extra row, and
-//     [G | b] = B^T [B | sqrt(w) d] accumulates in TMEM (two rotating
+//     [b | G] = B^T [sqrt(w) d | B] accumulates in TMEM (three rotating
 //     buffers; each chunk's rows are loaded while the previous one's MMAs run).
 //  2. A = (k-1)/rho I + G.  The ensemble-mean direction 1 is an exact
 //     eigenvector of A (Y' 1 = 0, eigenvalue delta) that never reaches the
@@ -83,7 +86,7 @@ namespace {
 using namespace mg::t5;
 
 constexpr int kChunk = 32;      // obs per Gram chunk: one 128-byte swizzle atom of TF32
-constexpr int kNBuf = 2;        // Gram chunk buffers
+constexpr int kNBuf = 3;        // Gram chunk buffers
 constexpr int kSelRing = 512;   // selected-entry ring (a candidate block + carry-over < kChunk)
 constexpr int kMaxIt = 14;      // Newton-Schulz iterations before an analysis is handed back
 constexpr float kStop = 0.05f;  // max |Z Y - I| that ends the iteration (after one more step)
@@ -130,10 +133,16 @@ constexpr int kPre = 4;         // variables whose X' rows and means are prefetc
 //   the Gram: 90 KB and 256 columns, or 108 KB and 512.
 // As a 128-row A operand, operands of fewer rows read the bytes that follow;
 // those products land in TMEM lanes that nothing reads.
-// Gram view of the same region (TF32 pairs with the 128-byte swizzle, whose
-// exponent range needs no scale for the obs rows): two chunk buffers of
-// KP + 16 rows (KP members, the innovation row, 15 unused), then the
-// selected-entry ring.
+// Gram view of the same region (TF32 with the 128-byte swizzle, whose exponent
+// range needs no scale for the obs rows): three chunk buffers, each of 16
+// rows (the innovation's hi and lo, 14 unused), the members' hi rows and their
+// lo rows, then the selected-entry ring.  B = the first KP + 16 rows, so one
+// MMA gives [hi.d_hi, hi.d_lo | hi hi^T] from the hi rows as A and
+// [lo.d_hi, . | lo hi^T] from the lo rows; the third term of the compensated
+// product, hi lo^T, is the transpose of the second and is added when the Gram
+// is read.  KP = 64: hi and lo rows are the two halves of one 128-row A, a
+// third of the MMAs that three passes take; else they are two MMAs into two
+// column ranges.
 template <int KP>
 struct Lay {
   static_assert(KP == 64 || KP == 80 || KP == 96, "member slots");
@@ -156,11 +165,10 @@ struct Lay {
   static constexpr uint32_t OFF_A_HI = OFF_T_LO + NG * kSlabT;  // P A P (KP = 64)
   static constexpr uint32_t OFF_A_LO = OFF_A_HI + NG * kSlabT;
   static constexpr uint32_t kRegion = kStack ? OFF_A_LO + NG * kSlabT : OFF_A_HI;
-  static constexpr int kGramRows = KP + 16;
-  static constexpr int kGramN = KP + 16;      // Gram MMA N: members, the innovation row, 15 unused
-  static constexpr uint32_t kGramSlab = kGramRows * 128u;
-  static constexpr uint32_t kGramBuf = 2 * kGramSlab;  // hi, lo
-  static constexpr uint32_t OFF_SEL = kNBuf * kGramBuf + (128 - kGramRows) * 128u;
+  static constexpr int kGramRows = 16 + 2 * KP;
+  static constexpr int kGramN = KP + 16;      // Gram MMA N: 16 innovation columns, members
+  static constexpr uint32_t kGramBuf = kGramRows * 128u;
+  static constexpr uint32_t OFF_SEL = kNBuf * kGramBuf;
   static constexpr uint32_t kSelBytes = kSelRing * 12u;  // obs index, sqrt(w), sqrt(w) d
   // Tensor memory: product scratch at column 0 (and a second product at
   // kTmB), the Gram at kTmGram.
@@ -168,8 +176,12 @@ struct Lay {
   static constexpr uint32_t kTmB = KP == 80 ? 80u : 128u;
   static constexpr uint32_t kTmE = KP;  // E = Z^T X'^T (16 columns) beside the products
   static constexpr uint32_t kTmGram = kStack ? 0u : (KP == 80 ? 160u : 256u);
-  static_assert(kGramSlab % 1024 == 0 && kSlabZ % 512 == 0 && kSlabT % 512 == 0, "swizzle atoms are aligned");
-  static_assert(OFF_SEL + kSelBytes <= kRegion, "Gram buffers, A-operand overhang and the ring");
+  static constexpr uint32_t kTmG = kTmGram + 16;  // its member columns
+  static constexpr int kLd = KP + 1;              // lo hi^T on its way to be transposed, FP32 in shared memory
+  static_assert(KP * kLd * 4 <= kRegion, "transposition buffer");
+  static_assert(kGramBuf % 1024 == 0 && kSlabZ % 512 == 0 && kSlabT % 512 == 0, "swizzle atoms are aligned");
+  static_assert(OFF_SEL + kSelBytes <= kRegion && (kStack || OFF_SEL + (128 - KP) * 128 <= kRegion),
+                "Gram buffers, the ring, and what the last lo rows read as a 128-row A");
   static_assert(kTmGram + kGramN <= kTmemCols && (kStack || kTmB + KP <= kTmGram), "tensor memory");
   static_assert(kSelRing >= kThreads + kChunk, "ring holds a candidate block and the carry-over");
 };
@@ -186,8 +198,9 @@ struct Vecs {
   float xu[kVarTile];  // unit of each variable's X' row (slot kPre in the finish: of b)
   double xm[kVarTile];
   double xmpre[kPre];
+  float xmh[kPre], xml[kPre];  // xmpre as a sum of two floats
   float xpre[kPre][KP];
-  int wcnt[Lay<KP>::kWarps];
+  int wcnt[2][Lay<KP>::kWarps];
 };
 
 template <int KP>
@@ -217,6 +230,17 @@ __device__ __forceinline__ void ns_coeffs(float& l, float& a, float& b) {
   b = 0.5f * mu * smu;
   const float ml = fminf(mu * l, 1.0f);
   l = ml * (3.0f - ml) * (3.0f - ml) * 0.25f;
+}
+
+// hi + lo + a + b rounded to FP32 from exact partial sums (Knuth's TwoSum): what
+// the sum in FP64 gives for FP32 storage, without four instructions of the
+// FP64 pipe, each of which holds a scheduler for 64 cycles.
+__device__ __forceinline__ float add3(float hi, float lo, float a, float b) {
+  const float s1 = __fadd_rn(hi, a), t1 = __fsub_rn(s1, hi);
+  const float r1 = __fadd_rn(__fsub_rn(hi, __fsub_rn(s1, t1)), __fsub_rn(a, t1));
+  const float s2 = __fadd_rn(s1, b), t2 = __fsub_rn(s2, s1);
+  const float r2 = __fadd_rn(__fsub_rn(s1, __fsub_rn(s2, t2)), __fsub_rn(b, t2));
+  return __fadd_rn(s2, __fadd_rn(__fadd_rn(r1, r2), lo));
 }
 
 // Asynchronous global -> shared copies (no registers held while in flight).
@@ -376,7 +400,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       }
     };
     fetch(cpos);
-    int nloc = 0, nch = 0, head = 0, nsel = 0;
+    int nloc = 0, nch = 0, head = 0, nsel = 0, par = 0;
     const int slot = tid & (kChunk - 1), m0 = (tid / kChunk) * 8;  // gather: obs slot x 8 members
     // Raw values: they are scaled when they are stored, so the loads stay in
     // flight until then.
@@ -433,13 +457,13 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) V.wcnt[warp] = __popc(bal);
+        if (lane == 0) V.wcnt[par][warp] = __popc(bal);
         __syncthreads();
         int wb = 0, cnt = 0;
 #pragma unroll
         for (int w = 0; w < L::kWarps; ++w) {
-          if (w < warp) wb += V.wcnt[w];
-          cnt += V.wcnt[w];
+          if (w < warp) wb += V.wcnt[par][w];
+          cnt += V.wcnt[par][w];
         }
         if (keep) {
           const int pos = (head + nsel + wb + __popc(bal & ((1u << lane) - 1u))) & (kSelRing - 1);
@@ -447,11 +471,12 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           sel_sw[pos] = sw;
           sel_sd[pos] = sd;
         }
-        __syncthreads();
+        par ^= 1;  // the counts are read before the next but one block writes its own
         nsel += cnt;
         nloc += cnt;
         cpos += kThreads;
       }
+      __syncthreads();  // the ring's entries
       const bool done = cpos >= e1;
       const int nchunks = done ? (nsel + kChunk - 1) / kChunk : nsel / kChunk;
       float x[8], swv, sdv;
@@ -461,23 +486,21 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         const uint32_t use = gchunk / kNBuf;
         if (use > 0 && !wait_one(&buf_bar[b], (use - 1) & 1u)) ok = false;
         unsigned char* bh = R + b * L::kGramBuf;
-        unsigned char* bl = bh + L::kGramSlab;
         if (m0 < KP) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const uint32_t off = sw_off(m0 + j, slot, L::kGramRows);
+            const uint32_t off = sw_off(16 + m0 + j, slot, L::kGramRows);
             float h, l;
             split(x[j] * swv, h, l);
             *reinterpret_cast<float*>(bh + off) = h;
-            *reinterpret_cast<float*>(bl + off) = l;
+            *reinterpret_cast<float*>(bh + off + KP * 128) = l;
           }
         }
-        if (m0 == 0) {  // the innovation row
-          const uint32_t off = sw_off(KP, slot, L::kGramRows);
+        if (m0 == 0) {  // the innovation rows
           float h, l;
           split(sdv, h, l);
-          *reinterpret_cast<float*>(bh + off) = h;
-          *reinterpret_cast<float*>(bl + off) = l;
+          *reinterpret_cast<float*>(bh + sw_off(0, slot, L::kGramRows)) = h;
+          *reinterpret_cast<float*>(bh + sw_off(1, slot, L::kGramRows)) = l;
         }
         if (c + 1 < nchunks) {  // next chunk's rows in flight during the barrier and the MMAs
           const int rem = nsel - (c + 1) * kChunk;
@@ -488,7 +511,8 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
           tc_fence_after();
           const uint32_t a = sR + b * L::kGramBuf;
           if (elect_one()) {
-            issue3(tmem + L::kTmGram, a, a + L::kGramSlab, a, a + L::kGramSlab, idescG, nch > 0);
+            issue_slab(tmem + L::kTmGram, a + 16 * 128, a, idescG, nch > 0);
+            if (!L::kStack) issue_slab(tmem, a + (16 + KP) * 128, a, idescG, nch > 0);
             mma_commit(&buf_bar[b]);
           }
           __syncwarp();
@@ -532,36 +556,65 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     const int row = 32 * q + lane;
     const bool rowin = row < KP;  // KP = 80: the last rows of the third quadrant hold nothing
     const int cb = 32 * g, ce = (cb + 32 < KP) ? cb + 32 : KP;
-    if (rowwarp) {
-      float rs = 0.0f, as = 0.0f, fa = 0.0f;
+    // lo hi^T -> shared memory, with lo.d_hi as its last column.
+    float* const S = reinterpret_cast<float*>(R);
+    if (L::kStack ? !rowwarp : rowwarp) {
+      const int i = L::kStack ? row - 64 : row;
 #pragma unroll 1
       for (int c0 = cb; c0 < ce; c0 += 8) {
         uint32_t v[8];
-        ld8(tmem + tm_row + L::kTmGram + c0, v);
+        ld8(tmem + tm_row + 16 + c0, v);
         tmem_wait_ld();
+        if (L::kStack || rowin) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) S[i * L::kLd + c0 + j] = __uint_as_float(v[j]);
+        }
+      }
+      if (g == 0) {
+        const uint32_t bv = tmem_ld1(tmem + tm_row);
+        tmem_wait_ld();
+        if (L::kStack || rowin) S[i * L::kLd + KP] = __uint_as_float(bv);
+      }
+    }
+    __syncthreads();
+    if (rowwarp) {
+      float rs = 0.0f, as = 0.0f, fa = 0.0f;
+      const int ri = rowin ? row : 0;
+      const float dr = (row < k) ? delta : 0.0f;
+#pragma unroll 1
+      for (int c0 = cb; c0 < ce; c0 += 8) {
+        uint32_t v[8];
+        ld8(tmem + tm_row + L::kTmG + c0, v);
+        tmem_wait_ld();
+        const int dj = row - c0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int c = c0 + j;
-          const float x = __uint_as_float(v[j]) + ((c == row) ? delta : 0.0f);
-          if (row < k && c < k) {
-            rs += x;
-            as += fabsf(x);
-            fa += x * x;
-          }
+          const float gv = __uint_as_float(v[j]) + (S[ri * L::kLd + c] + S[c * L::kLd + ri]);
+          v[j] = __float_as_uint(gv);  // zero outside the member block (zero rows)
+          const float x = gv + ((dj == j) ? dr : 0.0f);
+          rs += x;
+          as += fabsf(x);
+          fa += x * x;
         }
+        if (KP % 32) __syncwarp();
+        tmem_st8(tmem + tm_row + L::kTmG + c0, v);
       }
       if (rowin) {
         V.part[g][row] = rs;
         V.part[NG + g][row] = as;
       }
+      if (!rowin) fa = 0.0f;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) fa += __shfl_xor_sync(0xffffffffu, fa, off);
       if (lane == 0) V.red[3 * NG + q * NG + g] = fa;  // ||A||_F^2, by warp
       if (g == 0) {
-        const uint32_t bv = tmem_ld1(tmem + tm_row + L::kTmGram + KP);
+        const uint32_t b0 = tmem_ld1(tmem + tm_row + L::kTmGram), b1 = tmem_ld1(tmem + tm_row + L::kTmGram + 1);
         tmem_wait_ld();
-        if (rowin) V.b[row] = (row < k) ? __uint_as_float(bv) : 0.0f;
+        if (rowin)
+          V.b[row] = (row < k) ? __uint_as_float(b0) + (__uint_as_float(b1) + S[row * L::kLd + KP]) : 0.0f;
       }
+      tmem_wait_st();
     }
     __syncthreads();
     if (warp < NG) {  // row means r, grand mean c, infinity norm
@@ -601,7 +654,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     // outside the member block).
     auto pap8 = [&](int c0, float (&x)[8]) {
       uint32_t v[8];
-      ld8(tmem + tm_row + L::kTmGram + c0, v);
+      ld8(tmem + tm_row + L::kTmG + c0, v);
       tmem_wait_ld();
       const float ri = rowin ? V.r[row] : 0.0f;
 #pragma unroll
@@ -986,6 +1039,10 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         if (lane == 0) {
           V.one[vv] = c1 * sx * ik;
           V.xsq[vv] = sq;
+          if (prm.Xa32) {
+            V.xmh[vv] = (float)V.xmpre[vv];
+            V.xml[vv] = (float)(V.xmpre[vv] - (double)V.xmh[vv]);
+          }
         }
       }
     } else {
@@ -1035,19 +1092,28 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
       // kPre of both) the mean's increment X' wa is c E^T v, a sum over the
       // rows like RTPS's spread.
       const int nv = prm.n_var;
-      float dv[kPre];
-      if (rowwarp && g == 0) {
-        uint32_t dd[8], ee[8];
-        ld8(tmem + tm_row, dd);
-        ld8(tmem + tm_row + L::kTmE, ee);
-        tmem_wait_ld();
-        const float vr = V.xu[kPre] * (__uint_as_float(ee[kPre]) * kUnE - kUnD * __uint_as_float(dd[kPre]));
+      // Column group g takes the variables g, g + NG, ..
+      constexpr int kMine = (kPre + NG - 1) / NG;
+      float dv[kMine];
+      if (rowwarp) {
+        const uint32_t tr = tmem + tm_row;
+        uint32_t ev = tmem_ld1(tr + L::kTmE + kPre), uv = tmem_ld1(tr + kPre);
+        uint32_t e_[kMine], d_[kMine];
 #pragma unroll
-        for (int vv = 0; vv < kPre; ++vv) {
-          const bool in = row < k && vv < nv;
-          const float e = __uint_as_float(ee[vv]) * kUnE;
-          dv[vv] = in ? cws * V.xu[vv] * (e - 0.5f * kUnD * __uint_as_float(dd[vv])) + V.one[vv] : 0.0f;
-          float dw = in ? e * vr : 0.0f, s2 = dv[vv] * dv[vv];
+        for (int i = 0; i < kMine; ++i) {
+          e_[i] = tmem_ld1(tr + L::kTmE + g + i * NG);
+          d_[i] = tmem_ld1(tr + g + i * NG);
+        }
+        tmem_wait_ld();
+        const float vr = V.xu[kPre] * (__uint_as_float(ev) * kUnE - kUnD * __uint_as_float(uv));
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          const int vv = g + i * NG;
+          if (vv >= nv) break;
+          const bool in = row < k;
+          const float e = __uint_as_float(e_[i]) * kUnE;
+          dv[i] = in ? cws * V.xu[vv] * (e - 0.5f * kUnD * __uint_as_float(d_[i])) + V.one[vv] : 0.0f;
+          float dw = in ? e * vr : 0.0f, s2 = dv[i] * dv[i];
 #pragma unroll
           for (int off = 16; off > 0; off >>= 1) {
             dw += __shfl_xor_sync(0xffffffffu, dw, off);
@@ -1060,26 +1126,27 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
         }
       }
       __syncthreads();
-      if (rowwarp && g == 0 && row < k) {
+      if (rowwarp && row < k) {
 #pragma unroll
-        for (int vv = 0; vv < kPre; ++vv) {
-          if (vv < nv) {
-            float dw = 0.0f, s2 = 0.0f;
+        for (int i = 0; i < kMine; ++i) {
+          const int vv = g + i * NG;
+          if (vv >= nv) break;
+          float dw = 0.0f, s2 = 0.0f;
 #pragma unroll
-            for (int qq = 0; qq < NG; ++qq) {
-              dw += V.sdw[qq][vv];
-              s2 += V.ssa[qq][vv];
-            }
-            float a2 = dv[vv];
-            if (rtps) {
-              const float sb = sqrtf(V.xsq[vv] / (float)(k - 1));
-              const float sa = sqrtf(s2 / (float)(k - 1));
-              a2 *= 1.0f + ((sa > 0.0f) ? (float)prm.rho * (sb - sa) / sa : 0.0f);
-            }
-            const float inc = sc * is * V.xu[vv] * dw;
-            mg::letkf_store(prm, (base + (int64_t)vv * prm.var_stride) * k + row,
-                            (V.xmpre[vv] + (double)inc) + (double)a2);
+          for (int qq = 0; qq < NG; ++qq) {
+            dw += V.sdw[qq][vv];
+            s2 += V.ssa[qq][vv];
           }
+          float a2 = dv[i];
+          if (rtps) {
+            const float sb = sqrtf(V.xsq[vv] / (float)(k - 1));
+            const float sa = sqrtf(s2 / (float)(k - 1));
+            a2 *= 1.0f + ((sa > 0.0f) ? (float)prm.rho * (sb - sa) / sa : 0.0f);
+          }
+          const float inc = sc * is * V.xu[vv] * dw;
+          const int64_t o = (base + (int64_t)vv * prm.var_stride) * k + row;
+          if (prm.Xa32) prm.Xa32[o] = add3(V.xmh[vv], V.xml[vv], inc, a2);
+          else prm.Xa[o] = (V.xmpre[vv] + (double)inc) + (double)a2;
         }
       }
       __syncthreads();

@@ -1,10 +1,9 @@
-// TF32 tensor-core operands in shared memory and the 3-pass product:
-// K-major operands with the 128-byte swizzle (a slab holds 32 TF32 columns
-// of all its rows, 128 bytes per row, 8-row groups 1024 bytes apart), each
-// value stored as a hi and a lo copy (hi = x rounded to TF32, lo = x - hi),
-// and D += A B^T issued as hi*hi + hi*lo + lo*hi per K-step of 8.  The
-// Gram of the tensor-core local analyses (mg_letkf_tc.cu), whose obs rows
-// need FP32's exponent range; FP16 pairs (mg_f16op.cuh) take half the space.
+// TF32 tensor-core operands in shared memory: K-major with the 128-byte
+// swizzle (a slab holds 32 TF32 columns of all its rows, 128 bytes per row,
+// 8-row groups 1024 bytes apart), each value kept as a hi and a lo part (hi =
+// x rounded to TF32, lo = x - hi).  The Gram of the tensor-core local analyses
+// (mg_letkf_tc.cu), whose obs rows need FP32's exponent range; FP16 pairs
+// (mg_f16op.cuh) take half the space.
 #pragma once
 
 #include <stdint.h>
@@ -27,20 +26,17 @@ static __device__ __forceinline__ void split(float x, float& h, float& l) {
   l = x - h;
 }
 
-// D (TMEM) (+)= A B over one slab of 32 K-columns, 3 passes per K-step of 8.
-// A: 128 rows from a_hi/a_lo; B: N rows from b_hi/b_lo.  Called by one thread.
-static __device__ __forceinline__ void issue3(uint32_t dtm, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
-                                              uint32_t idesc, bool accumulate) {
+// D (TMEM) (+)= A B^T over one slab of 32 K-columns (4 K-steps of 8).  A: 128
+// rows; B: N rows.  Called by one thread.
+static __device__ __forceinline__ void issue_slab(uint32_t dtm, uint32_t a, uint32_t b, uint32_t idesc,
+                                                  bool accumulate) {
   // Descriptors of the first K-step; later steps add (byte offset >> 4) to
   // the 14-bit start-address field (shared addresses stay below 256 KB).
-  const uint64_t ah = smem_desc_sw128(a_hi), al = smem_desc_sw128(a_lo);
-  const uint64_t bh = smem_desc_sw128(b_hi), bl = smem_desc_sw128(b_lo);
+  const uint64_t ad = smem_desc_sw128(a), bd = smem_desc_sw128(b);
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) {
     const uint64_t o = (uint64_t)(kk * 32 >> 4);
-    mma_tf32(dtm, ah + o, bh + o, idesc, (accumulate || kk > 0) ? 1u : 0u);
-    mma_tf32(dtm, ah + o, bl + o, idesc, 1u);
-    mma_tf32(dtm, al + o, bh + o, idesc, 1u);
+    mma_tf32(dtm, ad + o, bd + o, idesc, (accumulate || kk > 0) ? 1u : 0u);
   }
 }
 
