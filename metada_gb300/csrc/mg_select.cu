@@ -9,15 +9,23 @@
 // band bound plus a longitude bound from the haversine inequality
 // a >= cos(lat_c) cos(lat_o) sin^2(dlon/2)); the reachable cells of one
 // latitude band are one or two contiguous runs of the cell-sorted obs, which
-// the whole CTA sweeps after one warp has planned them (a lane per band).  The test on a candidate is the squared chord
-// |u_c - u_o|^2 between unit vectors (u_o stored with the hash), compared
-// with the chord of the radius: haversine <= r  <=>  chord^2 <= 4 sin^2(r/2R),
-// with an absolute error near 1e-16 against a band of 2e-9 relative in
-// chord^2 (radii of 50 km or more; smaller radii evaluate the reference
-// haversine instead).  Lists are sorted by obs index in shared memory.
+// the whole CTA sweeps as one sequence.  The test on a candidate is the squared
+// half chord |u_c - u_o|^2 / 4 between unit vectors (u_o stored with the hash),
+// compared with the radius's: haversine <= r  <=>  half chord^2 <=
+// sin^2(r/2R), with an absolute error near 1e-16 against a band of 2e-9
+// relative in chord^2 (radii of 50 km or more; smaller radii evaluate the
+// reference haversine instead).  Lists are sorted by obs index.
 // Pairs within 1e-9 relative of the radius are re-decided on the host with
 // the reference expression (glibc libm), so the selection is bit-exact
 // whatever the device's transcendental rounding.
+//
+// What bounds it is the FP64 pipe (an instruction of a warp holds its
+// scheduler for 64 cycles), so FP64 is kept for what needs it: the windows of
+// all columns come from one kernel that fills its lanes (made by one warp of
+// each column's CTA, twice, they were half of the search), a candidate is
+// tested in FP32 and in FP64 only within FP32's error of the radius, and the
+// distance takes about 24 instructions.  64800 columns, 500k obs, 50M list
+// entries: count 3.06 -> 0.37 ms, fill 5.91 -> 2.76 ms, windows 0.12 ms.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -194,160 +202,259 @@ __device__ __forceinline__ double3 unit_vec(double lat, double lon) {
   return make_double3(ca * co, ca * so, sa);
 }
 
-// Cell-sorted obs: index, latitude, longitude and unit vector.
+// Cell-sorted obs (half unit vector in FP32, obs index in w) and, in obs
+// order, the half unit vectors in FP64 (w unused: one 32-byte sector each).
+// Halved, the vectors' squared distance is the squared half chord.
 struct CellObs {
-  int32_t* obs;
-  double* lat;
-  double* lon;
-  double* ux;
-  double* uy;
-  double* uz;
+  float4* cell;
+  double2* half;  // two per obs
 };
 
-// Obs into their cells (positions from the cell starts), with unit vectors
-// both cell-sorted and in obs order (the latter for the list distances).
+// Obs into their cells (positions from the cell starts).
 __global__ void cell_scatter_kernel(const double* __restrict__ lat, const double* __restrict__ lon,
                                     int64_t p, const int64_t* __restrict__ start,
-                                    unsigned long long* __restrict__ cursor, CellObs co, double* __restrict__ oux,
-                                    double* __restrict__ ouy, double* __restrict__ ouz) {
+                                    unsigned long long* __restrict__ cursor, CellObs co) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p; o += stride) {
     const int c = cell_of(lat[o], lon[o]);
     const int64_t pos = start[c] + (int64_t)atomicAdd(&cursor[c], 1ull);
-    co.obs[pos] = (int32_t)o;
-    co.lat[pos] = lat[o];
-    co.lon[pos] = lon[o];
     const double3 u = unit_vec(lat[o], lon[o]);
-    co.ux[pos] = u.x;
-    co.uy[pos] = u.y;
-    co.uz[pos] = u.z;
-    oux[o] = u.x;
-    ouy[o] = u.y;
-    ouz[o] = u.z;
+    const double hx = 0.5 * u.x, hy = 0.5 * u.y, hz = 0.5 * u.z;
+    co.cell[pos] = make_float4((float)hx, (float)hy, (float)hz, __int_as_float((int)o));
+    co.half[2 * o] = make_double2(hx, hy);
+    co.half[2 * o + 1] = make_double2(hz, 0.0);
   }
 }
 
-// Search plan of one column in shared memory, made by warp 0: the chord
-// thresholds, the column's unit vector, and per reachable latitude band the
-// one or two contiguous runs of cell-sorted obs its longitude window covers
-// (slots 2 b and 2 b + 1, the second empty where one run suffices).  The
-// FP64 transcendentals run once per band on one lane, not on every thread
-// of the CTA (GB300's FP64 pipe does about 2 operations per clock per SM).
-constexpr int kMaxRuns = 2 * kNBand;
-
-struct ColPlan {
-  double la, lo, rlo, rhi, c2lo, c2hi, ux, uy, uz;
-  int chord, nrun;
+// What one search fixes for all columns.
+struct GeoRule {
+  double theta_deg, a_r;   // the radius as an angle, sin^2 of half of it
+  double rlo, rhi;         // the radius less and plus the border
+  double h2lo, h2hi;       // their squared half chords
+  float f_in, f_out;       // FP32: surely inside up to, surely outside above
+  int chord;               // the chord test decides (else the haversine)
+  int nslot;               // latitude bands a column can reach, at most
+  double cosb[91];         // cos of whole degrees
 };
 
-__device__ void plan_column(double la, double lo, double radius_km, const int64_t* __restrict__ start,
-                            ColPlan& pl, int64_t* run_lo, int64_t* run_hi) {
-  const int lane = threadIdx.x & 31;
-  const double theta = radius_km / kEarthKm;  // radians
-  const double theta_deg = theta * 180.0 / kPi;
-  int b0 = (int)floor(la + 90.0 - theta_deg - 1e-6);
-  int b1 = (int)floor(la + 90.0 + theta_deg + 1e-6);
+GeoRule geo_rule(double radius_km) {
+  GeoRule g;
+  const double theta = radius_km / kEarthKm;
+  g.theta_deg = theta * 180.0 / kPi;
+  const double sh = std::sin(0.5 * theta);
+  g.a_r = sh * sh;
+  g.rlo = radius_km * (1.0 - kBorderRel);
+  g.rhi = radius_km * (1.0 + kBorderRel);
+  const double slo = std::sin(0.5 * g.rlo / kEarthKm), shi = std::sin(0.5 * g.rhi / kEarthKm);
+  g.h2lo = slo * slo;
+  g.h2hi = shi * shi;
+  g.chord = radius_km >= 50.0;
+  // FP32 half chords: each coordinate (at most 1/2) is off by at most 2^-26,
+  // so a difference vector by at most sqrt(3) 2^-25 = 5.2e-8, and the
+  // subtraction, the squares and their sum add at most 4e-7 relative in the
+  // square; 1e-7 and 1e-6 cover both.
+  const double d = 1e-7, in = slo > d ? (slo - d) * (slo - d) * (1.0 - 1e-6) : -1.0;
+  g.f_in = g.chord ? (float)in : -1.0f;
+  g.f_out = (float)((shi + d) * (shi + d) * (1.0 + 1e-6));
+  g.nslot = std::min(kNBand, (int)std::floor(2.0 * g.theta_deg + 2e-6) + 2);
+  for (int e = 0; e <= 90; ++e) g.cosb[e] = std::cos(e * kPi / 180.0);
+  return g;
+}
+
+// Search plans: per column the half unit vector, the first reachable latitude
+// band, and per band the longitude window as its first and last cell (first >
+// last: it wraps; kNoWindow: none).
+struct GeoPlan {
+  double* hx;
+  double* hy;
+  double* hz;
+  int32_t* b0;
+  uint32_t* win;  // nslot per column
+};
+constexpr uint32_t kNoWindow = 0xffffffffu;
+
+// Four threads per column, each every fourth band.
+__global__ void __launch_bounds__(256) geo_plan_kernel(const double* __restrict__ col_lat,
+                                                       const double* __restrict__ col_lon, int64_t ncol,
+                                                       const __grid_constant__ GeoRule g, GeoPlan pl) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t col = t >> 2;
+  const int q = (int)(t & 3);
+  if (col >= ncol) return;
+  const double la = col_lat[col], lo = col_lon[col];
+  int b0 = (int)floor(la + 90.0 - g.theta_deg - 1e-6);
+  int b1 = (int)floor(la + 90.0 + g.theta_deg + 1e-6);
   b0 = b0 < 0 ? 0 : b0;
   b1 = b1 >= kNBand ? kNBand - 1 : b1;
-  if (lane == 0) {
-    const double rlo = radius_km * (1.0 - kBorderRel), rhi = radius_km * (1.0 + kBorderRel);
-    const double slo = sin(0.5 * rlo / kEarthKm), shi = sin(0.5 * rhi / kEarthKm);
-    const double3 uc = unit_vec(la, lo);
-    pl.la = la;
-    pl.lo = lo;
-    pl.rlo = rlo;
-    pl.rhi = rhi;
-    pl.c2lo = 4.0 * slo * slo;
-    pl.c2hi = 4.0 * shi * shi;
-    pl.ux = uc.x;
-    pl.uy = uc.y;
-    pl.uz = uc.z;
-    pl.chord = radius_km >= 50.0;
-    pl.nrun = 2 * (b1 - b0 + 1);
+  double sa, cosc;
+  sincos(la * kPi / 180.0, &sa, &cosc);
+  if (q == 0) {
+    double so, cl;
+    sincos(lo * kPi / 180.0, &so, &cl);
+    pl.hx[col] = 0.5 * (cosc * cl);
+    pl.hy[col] = 0.5 * (cosc * so);
+    pl.hz[col] = 0.5 * sa;
+    pl.b0[col] = b0;
   }
-  const double sh = sin(0.5 * theta);
-  const double a_r = sh * sh;
-  const double cosc = cos(la * kPi / 180.0);
-  for (int band = b0 + lane; band <= b1; band += 32) {
-    const double e0 = (double)band - 90.0, e1 = e0 + 1.0;
-    const double emax = fmax(fabs(e0), fabs(e1));
-    const double cmin = cos(emax * kPi / 180.0);
-    const double denom = cosc * cmin;
-    int c0 = 0, c1 = kNLonCell - 1;
-    if (denom > a_r * (1.0 + 1e-6)) {
-      const double sarg = sqrt(a_r / denom) * (1.0 + 1e-9);
-      if (sarg < 1.0) {
-        const double dl = 2.0 * asin(sarg) * 180.0 / kPi + 1e-6;
-        if (2.0 * dl + 2.0 < 360.0) {
-          c0 = (int)floor(lo - dl);
-          c1 = (int)floor(lo + dl);
+  for (int i = q; i < g.nslot; i += 4) {
+    const int band = b0 + i;
+    uint32_t w = kNoWindow;
+    if (band <= b1) {
+      const int e0 = band - 90, em = e0 >= 0 ? e0 + 1 : -e0;  // the band's larger |latitude|
+      const double denom = cosc * g.cosb[em];
+      int c0 = 0, c1 = kNLonCell - 1;
+      if (denom > g.a_r * (1.0 + 1e-6)) {
+        const double sarg = sqrt(g.a_r / denom) * (1.0 + 1e-9);
+        if (sarg < 1.0) {
+          const double dl = 2.0 * asin(sarg) * 180.0 / kPi + 1e-6;
+          if (2.0 * dl + 2.0 < 360.0) {
+            c0 = (int)floor(lo - dl);
+            c1 = (int)floor(lo + dl);
+          }
         }
       }
+      // The cells c0..c1 (mod 360) as at most two contiguous runs of obs.
+      if (c1 - c0 + 1 >= kNLonCell) {
+        w = (uint32_t)(kNLonCell - 1) << 16;
+      } else {
+        const int a0 = ((c0 % kNLonCell) + kNLonCell) % kNLonCell;
+        const int a1 = ((c1 % kNLonCell) + kNLonCell) % kNLonCell;
+        w = (uint32_t)a0 | ((uint32_t)a1 << 16);
+      }
     }
-    // The cells c0..c1 (mod 360) as at most two contiguous runs of obs.
-    const int bb = band * kNLonCell, slot = 2 * (band - b0);
-    run_lo[slot + 1] = run_hi[slot + 1] = 0;
-    if (c1 - c0 + 1 >= kNLonCell) {
-      run_lo[slot] = start[bb];
-      run_hi[slot] = start[bb + kNLonCell];
-    } else {
-      const int a0 = ((c0 % kNLonCell) + kNLonCell) % kNLonCell;
-      const int a1 = ((c1 % kNLonCell) + kNLonCell) % kNLonCell;
+    pl.win[col * g.nslot + i] = w;
+  }
+}
+
+constexpr int kMaxRuns = 2 * kNBand;
+
+// One column's plan in shared memory: its candidates as one sequence of the
+// runs, pre[r] of them before run r.
+struct ColPlan {
+  double la, lo, hx, hy, hz;
+  float fx, fy, fz;
+  int nrun;
+  int64_t first[kMaxRuns];
+  int32_t pre[kMaxRuns + 1];
+};
+
+// By warp 0.
+__device__ void load_plan(int64_t col, double la, double lo, const GeoRule& g, const GeoPlan& gp,
+                          const int64_t* __restrict__ start, ColPlan& pl) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) {
+    pl.la = la;
+    pl.lo = lo;
+    pl.hx = gp.hx[col];
+    pl.hy = gp.hy[col];
+    pl.hz = gp.hz[col];
+    pl.fx = (float)pl.hx;
+    pl.fy = (float)pl.hy;
+    pl.fz = (float)pl.hz;
+    pl.nrun = 2 * g.nslot;
+    pl.pre[0] = 0;
+  }
+  const int b0 = gp.b0[col];
+  int total = 0;
+  for (int s0 = 0; s0 < g.nslot; s0 += 32) {
+    const int s = s0 + lane;
+    int64_t f0 = 0, f1 = 0;
+    int n0 = 0, n1 = 0;
+    const uint32_t w = s < g.nslot ? gp.win[col * g.nslot + s] : kNoWindow;
+    if (w != kNoWindow) {
+      const int bb = (b0 + s) * kNLonCell, a0 = (int)(w & 0xffffu), a1 = (int)(w >> 16);
+      f0 = start[bb + a0];
       if (a0 <= a1) {
-        run_lo[slot] = start[bb + a0];
-        run_hi[slot] = start[bb + a1 + 1];
+        n0 = (int)(start[bb + a1 + 1] - f0);
       } else {
-        run_lo[slot] = start[bb + a0];
-        run_hi[slot] = start[bb + kNLonCell];
-        run_lo[slot + 1] = start[bb];
-        run_hi[slot + 1] = start[bb + a1 + 1];
+        n0 = (int)(start[bb + kNLonCell] - f0);
+        f1 = start[bb];
+        n1 = (int)(start[bb + a1 + 1] - f1);
       }
     }
+    int inc = n0 + n1;  // inclusive scan over the lanes
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += v;
+    }
+    if (s < g.nslot) {
+      pl.first[2 * s] = f0;
+      pl.first[2 * s + 1] = f1;
+      pl.pre[2 * s + 1] = total + inc - n1;
+      pl.pre[2 * s + 2] = total + inc;
+    }
+    total += __shfl_sync(0xffffffffu, inc, 31);
   }
 }
 
-// Visits every candidate obs of a planned column with the whole CTA and
-// calls f(t, cls) for the candidates at cell-sorted position t with
-// cls = +1 (inside) or 0 (within 1e-9 relative of the radius).
+// The FP64 test of a candidate within FP32's error of the radius, and of every
+// candidate near a small radius (out of line: a predicated FP64 instruction
+// would hold the pipe for every candidate).  +1 inside, 0 within 1e-9 relative
+// of the radius, -1 outside.
+__device__ __noinline__ int test_fp64(const ColPlan& pl, const GeoRule& g, const CellObs& co,
+                                      const double* __restrict__ obs_lat, const double* __restrict__ obs_lon, int o) {
+  if (g.chord) {
+    const double2 xy = co.half[2 * (int64_t)o], zw = co.half[2 * (int64_t)o + 1];
+    const double dx = xy.x - pl.hx, dy = xy.y - pl.hy, dz = zw.x - pl.hz;
+    const double h2 = dx * dx + dy * dy + dz * dz;
+    return h2 <= g.h2lo ? 1 : (h2 <= g.h2hi ? 0 : -1);
+  }
+  const double d = haversine_dev(pl.la, pl.lo, obs_lat[o], obs_lon[o]);
+  return d <= g.rlo ? 1 : (d <= g.rhi ? 0 : -1);
+}
+
+// Visits every candidate obs of a planned column with the whole CTA and calls
+// f(o, cls) with cls = +1 (inside), 0 (border) or -1; every lane of a warp
+// takes part in each call (cls = -1 past the end).
 template <typename F>
-__device__ void visit_candidates(const ColPlan& pl, const int64_t* run_lo, const int64_t* run_hi,
-                                 const CellObs& co, F&& f) {
-  const int nrun = pl.nrun;
-  const bool chord = pl.chord;
-  const double ux = pl.ux, uy = pl.uy, uz = pl.uz, c2lo = pl.c2lo, c2hi = pl.c2hi;
-  for (int r = 0; r < nrun; ++r) {
-    const int64_t hi = run_hi[r];
-    for (int64_t t = run_lo[r] + threadIdx.x; t < hi; t += blockDim.x) {
-      if (chord) {
-        const double dx = co.ux[t] - ux, dy = co.uy[t] - uy, dz = co.uz[t] - uz;
-        const double c2 = dx * dx + dy * dy + dz * dz;
-        if (c2 <= c2lo) f(t, 1);
-        else if (c2 <= c2hi) f(t, 0);
-      } else {
-        const double d = haversine_dev(pl.la, pl.lo, co.lat[t], co.lon[t]);
-        if (d <= pl.rlo) f(t, 1);
-        else if (d <= pl.rhi) f(t, 0);
-      }
+__device__ __forceinline__ void visit_candidates(const ColPlan& pl, const GeoRule& g, const CellObs& co,
+                                                 const double* __restrict__ obs_lat,
+                                                 const double* __restrict__ obs_lon, F&& f) {
+  const int n = pl.pre[pl.nrun];
+  const float fx = pl.fx, fy = pl.fy, fz = pl.fz, f_in = g.f_in, f_out = g.f_out;
+  int r = 0;
+  for (int i0 = threadIdx.x & ~31; i0 < n; i0 += blockDim.x) {
+    const int i = i0 + (threadIdx.x & 31);
+    int o = -1, cls = -1;
+    if (i < n) {
+      while (i >= pl.pre[r + 1]) ++r;
+      const float4 u = co.cell[pl.first[r] + (i - pl.pre[r])];
+      const float dx = u.x - fx, dy = u.y - fy, dz = u.z - fz;
+      const float h2 = dx * dx + dy * dy + dz * dz;
+      o = __float_as_int(u.w);
+      if (h2 <= f_in) cls = 1;
+      else if (h2 <= f_out) cls = test_fp64(pl, g, co, obs_lat, obs_lon, o);
     }
+    f(o, cls);
   }
 }
 
-// asin(h) for a half chord 0 <= h <= 1.  Up to h = 0.05 (great-circle
-// distances up to about 640 km) by its Maclaurin series
+// 2R asin(h) of a squared half chord h2 <= 1.  Up to h = 0.05 (great-circle
+// distances up to about 640 km) asin by its Maclaurin series
 // asin h = sum_n (2n)! / (4^n (n!)^2 (2n + 1)) h^(2n+1), through n = 5: the
-// first omitted term, 231/13312 h^13, is below 1e-18 of h there, so the
-// result is the correctly rounded value to within a few units in the last
-// place, at six FP64 multiply-adds (FP64 runs at 1/64 of the FP32 rate);
-// larger h take the library asin.
-__device__ __forceinline__ double asin_half_chord(double h) {
-  if (h > 0.05) return asin(h < 1.0 ? h : 1.0);
-  const double h2 = h * h;
+// first omitted term, 231/13312 h^13, is below 1e-18 of h there; larger h take
+// the library asin.  h = sqrt(h2) from an FP32 reciprocal root y by one step
+// of third order (h2 y^2 = 1 - e: sqrt(h2) = h2 y (1 + e/2 + 3 e^2/8 + ..), e
+// below 2^-21) and one Newton step on the result.
+__device__ __forceinline__ double geo_distance(double h2) {
+  double h;
+  if (h2 > 1e-30) {
+    const double y = (double)rsqrtf((float)h2);
+    const double t = h2 * y;
+    const double e = fma(-t, y, 1.0);
+    const double s = fma(t * e, fma(e, 0.375, 0.5), t);
+    h = fma(fma(-s, s, h2), 0.5 * y, s);
+  } else {
+    h = sqrt(h2);
+  }
+  if (h > 0.05) return 2.0 * kEarthKm * asin(h < 1.0 ? h : 1.0);
   double q = 63.0 / 2816.0;
   q = fma(q, h2, 35.0 / 1152.0);
   q = fma(q, h2, 5.0 / 112.0);
   q = fma(q, h2, 3.0 / 40.0);
   q = fma(q, h2, 1.0 / 6.0);
-  return fma(h * h2, q, h);
+  return 2.0 * kEarthKm * fma(h * h2, q, h);
 }
 
 __device__ __forceinline__ bool key_rejected(const unsigned long long* rej, int nrej,
@@ -361,31 +468,32 @@ __device__ __forceinline__ bool key_rejected(const unsigned long long* rej, int 
 }
 
 __global__ void __launch_bounds__(256) geo_count_kernel(
-    const double* __restrict__ col_lat, const double* __restrict__ col_lon, int64_t ncol,
-    double radius_km, const int64_t* __restrict__ start, CellObs co, int64_t* __restrict__ counts,
-    BorderRec* __restrict__ border, unsigned long long* __restrict__ nborder) {
-  __shared__ unsigned long long scount;
+    const double* __restrict__ col_lat, const double* __restrict__ col_lon, const __grid_constant__ GeoRule g,
+    GeoPlan gp, const int64_t* __restrict__ start, CellObs co, const double* __restrict__ obs_lat,
+    const double* __restrict__ obs_lon, int64_t* __restrict__ counts, BorderRec* __restrict__ border,
+    unsigned long long* __restrict__ nborder) {
+  __shared__ int scount;
   __shared__ ColPlan pl;
-  __shared__ int64_t run_lo[kMaxRuns], run_hi[kMaxRuns];
   const int64_t col = blockIdx.x;
   if (threadIdx.x == 0) scount = 0;
   const double la = col_lat[col], lo = col_lon[col];
-  if (threadIdx.x < 32) plan_column(la, lo, radius_km, start, pl, run_lo, run_hi);
+  if (threadIdx.x < 32) load_plan(col, la, lo, g, gp, start, pl);
   __syncthreads();
-  unsigned long long mine = 0;
-  visit_candidates(pl, run_lo, run_hi, co, [&](int64_t t, int cls) {
-    ++mine;
+  int mine = 0;
+  visit_candidates(pl, g, co, obs_lat, obs_lon, [&](int o, int cls) {
+    if (cls >= 0) ++mine;
     if (cls == 0) {
       const unsigned long long slot = atomicAdd(nborder, 1ull);
       if (slot < (unsigned long long)kBorderCap)
-        border[slot] = BorderRec{col, (int64_t)co.obs[t], la, lo, co.lat[t], co.lon[t]};
+        border[slot] = BorderRec{col, (int64_t)o, la, lo, obs_lat[o], obs_lon[o]};
     }
   });
-  atomicAdd(&scount, mine);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&scount, mine);
   __syncthreads();
   if (threadIdx.x == 0) {
     counts[col] = (int64_t)scount;
-    atomicMax(nborder + 1, scount);  // the longest list sizes the fill pass's shared memory
+    atomicMax(nborder + 1, (unsigned long long)scount);  // the longest list sizes the fill pass's shared memory
   }
 }
 
@@ -396,17 +504,73 @@ __global__ void apply_rejections_kernel(const unsigned long long* __restrict__ r
                           (unsigned long long)-1ll);
 }
 
+// Bitonic sort of 256 E keys by the CTA (ascending): thread t holds elements
+// E t .. E t + E - 1, so strides below E stay in registers, strides below 32 E
+// are shuffles, and only the rest (6 of 55 steps for 1024 keys) go through
+// shared memory, `x` with 256 E entries.
+template <int E>
+__device__ __forceinline__ void sort_keys(int (&v)[E], int32_t* x) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int size = 2; size <= 256 * E; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride < E) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          if (!(i & stride)) {
+            const bool up = (((E * t + i) & size) == 0);
+            const int a = v[i], b = v[i | stride];
+            const int lo = min(a, b), hi = max(a, b);
+            v[i] = up ? lo : hi;
+            v[i | stride] = up ? hi : lo;
+          }
+        }
+      } else {
+        const int d = stride / E;  // the partner's distance in threads
+        int w[E];
+        if (d < 32) {
+#pragma unroll
+          for (int i = 0; i < E; ++i) w[i] = __shfl_xor_sync(0xffffffffu, v[i], d);
+        } else {
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < E; ++i) x[256 * i + t] = v[i];
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < E; ++i) w[i] = x[256 * i + (t ^ d)];
+        }
+        const bool keep_min = (((E * t) & size) == 0) == ((t & d) == 0);
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = keep_min ? min(v[i], w[i]) : max(v[i], w[i]);
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < E; ++i) x[E * t + i] = v[i];
+}
+
+template <int E>
+__device__ __noinline__ void sort_list(int32_t* slist, int cnt) {
+  int v[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {  // any assignment of the keys to the elements
+    const int e = threadIdx.x + 256 * i;
+    v[i] = e < cnt ? slist[e] : 0x7fffffff;
+  }
+  sort_keys<E>(v, slist);
+}
+
 __global__ void __launch_bounds__(256) geo_fill_kernel(
-    const double* __restrict__ col_lat, const double* __restrict__ col_lon, int64_t ncol,
-    double radius_km, const int64_t* __restrict__ start, CellObs co,
-    const int64_t* __restrict__ offsets, const unsigned long long* __restrict__ rej, int nrej,
-    const double* __restrict__ obs_lat, const double* __restrict__ obs_lon, const double* __restrict__ oux,
-    const double* __restrict__ ouy, const double* __restrict__ ouz, int32_t* __restrict__ idx,
-    double* __restrict__ dist, int* __restrict__ overflow, int list_cap) {
-  extern __shared__ int32_t slist[];  // list_cap entries, a power of two
+    const double* __restrict__ col_lat, const double* __restrict__ col_lon, const __grid_constant__ GeoRule g,
+    GeoPlan gp, const int64_t* __restrict__ start, CellObs co, const int64_t* __restrict__ offsets,
+    const unsigned long long* __restrict__ rej, int nrej, const double* __restrict__ obs_lat,
+    const double* __restrict__ obs_lon, int32_t* __restrict__ idx, double* __restrict__ dist,
+    int* __restrict__ overflow, int list_cap) {
+  extern __shared__ int32_t slist[];  // list_cap entries, a power of two from 256
   __shared__ int scount;
   __shared__ ColPlan pl;
-  __shared__ int64_t run_lo[kMaxRuns], run_hi[kMaxRuns];
   const int64_t col = blockIdx.x;
   const int64_t base = offsets[col];
   const int64_t n = offsets[col + 1] - base;
@@ -417,13 +581,17 @@ __global__ void __launch_bounds__(256) geo_fill_kernel(
   }
   if (threadIdx.x == 0) scount = 0;
   const double la = col_lat[col], lo = col_lon[col];
-  if (threadIdx.x < 32) plan_column(la, lo, radius_km, start, pl, run_lo, run_hi);
+  if (threadIdx.x < 32) load_plan(col, la, lo, g, gp, start, pl);
   __syncthreads();
-  visit_candidates(pl, run_lo, run_hi, co, [&](int64_t t, int cls) {
-    const int32_t o = co.obs[t];
-    if (cls == 0 && nrej > 0 && key_rejected(rej, nrej, ((unsigned long long)col << 32) | (unsigned)o)) return;
-    const int pos = atomicAdd(&scount, 1);
-    if (pos < list_cap) slist[pos] = o;
+  const int lane = threadIdx.x & 31;
+  visit_candidates(pl, g, co, obs_lat, obs_lon, [&](int o, int cls) {
+    bool in = cls >= 0;
+    if (cls == 0 && nrej > 0 && key_rejected(rej, nrej, ((unsigned long long)col << 32) | (unsigned)o)) in = false;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    int pos = 0;
+    if (lane == 0 && m) pos = atomicAdd(&scount, __popc(m));
+    pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1u));
+    if (in && pos < list_cap) slist[pos] = o;
   });
   __syncthreads();
   const int cnt = scount;
@@ -431,35 +599,42 @@ __global__ void __launch_bounds__(256) geo_fill_kernel(
     if (threadIdx.x == 0) atomicExch(overflow, 2);
     return;
   }
-  int m = 1;
-  while (m < cnt) m <<= 1;
-  for (int t = cnt + threadIdx.x; t < m; t += blockDim.x) slist[t] = 0x7fffffff;
-  __syncthreads();
-  // Bitonic sort by obs index (obs order, as LETKF.hpp:160-165).
-  for (int size = 2; size <= m; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < (m >> 1); t += blockDim.x) {
-        const int lo_i = 2 * t - (t & (stride - 1));
-        const int hi_i = lo_i + stride;
-        const bool up = ((lo_i & size) == 0);
-        const int a = slist[lo_i], b = slist[hi_i];
-        if ((a > b) == up) {
-          slist[lo_i] = b;
-          slist[hi_i] = a;
+  // Sorted by obs index (obs order, as LETKF.hpp:160-165): in registers up to
+  // 2048 entries, else in shared memory.
+  if (cnt <= 256) sort_list<1>(slist, cnt);
+  else if (cnt <= 512) sort_list<2>(slist, cnt);
+  else if (cnt <= 1024) sort_list<4>(slist, cnt);
+  else if (cnt <= 2048) sort_list<8>(slist, cnt);
+  else {
+    int m = 4096;
+    while (m < cnt) m <<= 1;
+    for (int t = cnt + threadIdx.x; t < m; t += blockDim.x) slist[t] = 0x7fffffff;
+    __syncthreads();
+    for (int size = 2; size <= m; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int t = threadIdx.x; t < (m >> 1); t += blockDim.x) {
+          const int lo_i = 2 * t - (t & (stride - 1));
+          const int hi_i = lo_i + stride;
+          const bool up = ((lo_i & size) == 0);
+          const int a = slist[lo_i], b = slist[hi_i];
+          if ((a > b) == up) {
+            slist[lo_i] = b;
+            slist[hi_i] = a;
+          }
         }
+        __syncthreads();
       }
-      __syncthreads();
     }
   }
-  const bool chord = pl.chord;
+  __syncthreads();
   for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
     const int o = slist[t];
     idx[base + t] = o;
     if (dist) {
-      if (chord) {  // d = 2R asin(chord / 2): well conditioned for chords up to the radius
-        const double dx = oux[o] - pl.ux, dy = ouy[o] - pl.uy, dz = ouz[o] - pl.uz;
-        const double h = 0.5 * sqrt(dx * dx + dy * dy + dz * dz);
-        dist[base + t] = 2.0 * kEarthKm * asin_half_chord(h);
+      if (g.chord) {  // well conditioned for chords up to the radius
+        const double2 xy = co.half[2 * (int64_t)o], zw = co.half[2 * (int64_t)o + 1];
+        const double dx = xy.x - pl.hx, dy = xy.y - pl.hy, dz = zw.x - pl.hz;
+        dist[base + t] = geo_distance(dx * dx + dy * dy + dz * dz);
       } else {
         dist[base + t] = haversine_dev(la, lo, obs_lat[o], obs_lon[o]);
       }
@@ -534,8 +709,12 @@ int mg_select_geo(mg_context* ctx, const double* col_lat, const double* col_lon,
   cv.reserve<unsigned long long>(kNCell + 1);  // cell counts, then cursor
   cv.reserve<unsigned long long>(kNCell + 1);
   cv.reserve<int64_t>(kNCell + 1);             // cell start
-  cv.reserve<int32_t>(p + 1);
-  for (int a = 0; a < 8; ++a) cv.reserve<double>(p + 1);  // lat, lon, unit vector; unit vector in obs order
+  const GeoRule rule = geo_rule(radius_km);
+  cv.reserve<float4>(p + 1);                   // cell-sorted obs
+  cv.reserve<double2>(2 * p + 2);              // half unit vectors in obs order
+  for (int a = 0; a < 3; ++a) cv.reserve<double>(ncol);  // search plans
+  cv.reserve<int32_t>(ncol);
+  cv.reserve<uint32_t>((size_t)ncol * rule.nslot);
   cv.reserve<int64_t>(ncol + 1);               // column counts
   cv.reserve<BorderRec>(kBorderCap);
   cv.reserve<unsigned long long>(kBorderCap);  // rejected keys
@@ -549,15 +728,14 @@ int mg_select_geo(mg_context* ctx, const double* col_lat, const double* col_lon,
   auto* ccursor = cv.take<unsigned long long>(kNCell + 1);
   auto* cstart = cv.take<int64_t>(kNCell + 1);
   CellObs co;
-  co.obs = cv.take<int32_t>(p + 1);
-  co.lat = cv.take<double>(p + 1);
-  co.lon = cv.take<double>(p + 1);
-  co.ux = cv.take<double>(p + 1);
-  co.uy = cv.take<double>(p + 1);
-  co.uz = cv.take<double>(p + 1);
-  double* oux = cv.take<double>(p + 1);
-  double* ouy = cv.take<double>(p + 1);
-  double* ouz = cv.take<double>(p + 1);
+  co.cell = cv.take<float4>(p + 1);
+  co.half = cv.take<double2>(2 * p + 2);
+  GeoPlan plan;
+  plan.hx = cv.take<double>(ncol);
+  plan.hy = cv.take<double>(ncol);
+  plan.hz = cv.take<double>(ncol);
+  plan.b0 = cv.take<int32_t>(ncol);
+  plan.win = cv.take<uint32_t>((size_t)ncol * rule.nslot);
   auto* counts = cv.take<int64_t>(ncol + 1);
   auto* border = cv.take<BorderRec>(kBorderCap);
   auto* rej = cv.take<unsigned long long>(kBorderCap);
@@ -579,15 +757,18 @@ int mg_select_geo(mg_context* ctx, const double* col_lat, const double* col_lon,
     MG_TRY_CUDA(cudaGetLastError());
     MG_TRY_CUDA(mg::exclusive_scan(reinterpret_cast<const int64_t*>(ccount), cstart, kNCell, tmp,
                                    tmpb, s));
-    cell_scatter_kernel<<<gb, 256, 0, s>>>(obs_lat, obs_lon, p, cstart, ccursor, co, oux, ouy, ouz);
+    cell_scatter_kernel<<<gb, 256, 0, s>>>(obs_lat, obs_lon, p, cstart, ccursor, co);
     MG_COUNT_LAUNCH();
     MG_TRY_CUDA(cudaGetLastError());
   } else {
     MG_TRY_CUDA(cudaMemsetAsync(cstart, 0, sizeof(int64_t) * (kNCell + 1), s));
   }
   // Pass 1: counts (near-threshold pairs counted and recorded).
-  geo_count_kernel<<<(unsigned)ncol, 256, 0, s>>>(col_lat, col_lon, ncol, radius_km, cstart, co, counts, border,
-                                                  nborder);
+  geo_plan_kernel<<<(unsigned)((4 * ncol + 255) / 256), 256, 0, s>>>(col_lat, col_lon, ncol, rule, plan);
+  MG_COUNT_LAUNCH();
+  MG_TRY_CUDA(cudaGetLastError());
+  geo_count_kernel<<<(unsigned)ncol, 256, 0, s>>>(col_lat, col_lon, rule, plan, cstart, co, obs_lat, obs_lon, counts,
+                                                  border, nborder);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   unsigned long long nbm[2] = {0, 0};
@@ -623,14 +804,13 @@ int mg_select_geo(mg_context* ctx, const double* col_lat, const double* col_lon,
     return mg::fail(ctx, MG_ERR_CAPACITY, "mg_select_geo: index buffer too small");
   if (*total == 0) return MG_OK;
   // Pass 2: fill, sort each list by obs index, distances.
-  int smem_entries = 32;
+  int smem_entries = 256;
   while ((unsigned long long)smem_entries < longest) smem_entries <<= 1;
   const size_t smem = sizeof(int32_t) * smem_entries;
   MG_TRY_CUDA(cudaFuncSetAttribute(geo_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
-  geo_fill_kernel<<<(unsigned)ncol, 256, smem, s>>>(col_lat, col_lon, ncol, radius_km, cstart, co, offsets, rej,
-                                                    nrej, obs_lat, obs_lon, oux, ouy, ouz, idx, dist_km, overflow,
-                                                    smem_entries);
+  geo_fill_kernel<<<(unsigned)ncol, 256, smem, s>>>(col_lat, col_lon, rule, plan, cstart, co, offsets, rej, nrej,
+                                                    obs_lat, obs_lon, idx, dist_km, overflow, smem_entries);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   int ovf = 0;
