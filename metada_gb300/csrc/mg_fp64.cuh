@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace mg {
 
@@ -37,5 +38,20 @@ __device__ __forceinline__ double div_refined(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-q, b, a), r, q);
 }
+
+// (double)x by integer operations: a conversion runs on the FP64 pipe and
+// holds its scheduler for 64 cycles.  Exact for zeros and normal numbers;
+// wide_special(x) tells the others (subnormals, infinities, NaN), which take
+// the conversion.
+__device__ __forceinline__ bool wide_special(float x) {
+  const uint32_t mag = __float_as_uint(x) & 0x7fffffffu;
+  return mag - 0x00800000u >= 0x7f000000u && mag != 0u;
+}
+__device__ __forceinline__ double wide(float x) {
+  const uint32_t u = __float_as_uint(x), mag = u & 0x7fffffffu;
+  const uint32_t hi = (mag ? (mag >> 3) + 0x38000000u : 0u) | (u & 0x80000000u);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+static __device__ __noinline__ double wide_cvt(float x) { return (double)x; }
 
 }  // namespace mg

@@ -86,6 +86,30 @@ struct LatLonGeom {
   int32_t valid;
 };
 
+// The corners of the two planes, widened.
+__device__ __forceinline__ void load8(double (&x)[8], const double* a, const double* b, const double* c,
+                                      const double* d, int i0, int i1) {
+  x[0] = a[i0]; x[1] = a[i1]; x[2] = b[i0]; x[3] = b[i1];
+  x[4] = c[i0]; x[5] = c[i1]; x[6] = d[i0]; x[7] = d[i1];
+}
+// FP32 members: 21 FP64 instructions a value remain of 29 when the widening
+// takes integer operations (64 members, 500k obs in random order: 2.95 -> 2.64 ms;
+// the rest is 32-byte sectors from DRAM, four a value).
+__device__ __forceinline__ void load8(double (&x)[8], const float* a, const float* b, const float* c, const float* d,
+                                      int i0, int i1) {
+  const float v[8] = {a[i0], a[i1], b[i0], b[i1], c[i0], c[i1], d[i0], d[i1]};
+  bool special = false;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    special |= mg::wide_special(v[q]);
+    x[q] = mg::wide(v[q]);
+  }
+  if (special) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) x[q] = mg::wide_cvt(v[q]);
+  }
+}
+
 template <typename TX>
 __global__ void __launch_bounds__(256) hx_latlon_kernel(const TX* __restrict__ X, int k, int64_t ld, int nlon,
                                                         int nlat, int nlev, const double* __restrict__ olat,
@@ -154,10 +178,10 @@ __global__ void __launch_bounds__(256) hx_latlon_kernel(const TX* __restrict__ X
         }
         const TX* lo = X + (int64_t)m * ld + g.lo;
         const TX* hi = X + (int64_t)m * ld + g.hi;
-        const double l00 = (double)lo[g.r0 + g.i0], l01 = (double)lo[g.r0 + g.i1];
-        const double l10 = (double)lo[g.r1 + g.i0], l11 = (double)lo[g.r1 + g.i1];
-        const double h00 = (double)hi[g.r0 + g.i0], h01 = (double)hi[g.r0 + g.i1];
-        const double h10 = (double)hi[g.r1 + g.i0], h11 = (double)hi[g.r1 + g.i1];
+        double x[8];
+        load8(x, lo + g.r0, lo + g.r1, hi + g.r0, hi + g.r1, g.i0, g.i1);
+        const double l00 = x[0], l01 = x[1], l10 = x[2], l11 = x[3];
+        const double h00 = x[4], h01 = x[5], h10 = x[6], h11 = x[7];
         const double b0 = __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(l00, g.ax), __dmul_rn(l01, g.fx)), g.ay),
                                     __dmul_rn(__dadd_rn(__dmul_rn(l10, g.ax), __dmul_rn(l11, g.fx)), g.fy));
         const double b1 = __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn(h00, g.ax), __dmul_rn(h01, g.fx)), g.ay),
