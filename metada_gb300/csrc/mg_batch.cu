@@ -71,6 +71,18 @@ struct WorkItem {
   int64_t a, b;  // range [a, b) (states, obs or chunk index)
 };
 
+// The mixed path's cases in up to three groups: the Gram classes below 128
+// members, and the class of 128 in two halves of about the same work, the
+// larger k in the last.  The solves of a group are one CTA per case and wait on
+// dependent steps (1.2 ms for 112 members, on as many SMs as there are cases),
+// so each group is a chain of its own and the others' streaming kernels fill
+// the SMs meanwhile.
+constexpr int kGroups = 3;
+struct CaseGroup {
+  int64_t obs_off = 0, obs_cnt = 0, upd_off = 0, upd_cnt = 0, gram_off = 0, gram_cnt = 0;  // Gram: class 128's
+  int ord_off = 0, ncases = 0, maxk = 0;
+};
+
 struct mg_etkf_batch {
   int ncases = 0;
   int flags = 0;
@@ -90,6 +102,9 @@ struct mg_etkf_batch {
   unsigned long long* times = nullptr;     // [0] start, [1 + c] case finish (ns)
   int* status = nullptr;
   const int* order = nullptr;  // case indices, largest k first (one CTA per case kernels)
+  CaseGroup grp[kGroups];
+  cudaStream_t side[kGroups - 1] = {};  // the later groups' chains
+  cudaEvent_t fork = nullptr, join[kGroups - 1] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -179,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) batch_prep_obs_mixed_kernel(const De
                                                                         unsigned long long* times) {
   const WorkItem it = items[blockIdx.x];
   const DevCase& c = cases[it.c];
-  if (blockIdx.x == 0 && threadIdx.x == 0) times[0] = globaltimer();
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(times, globaltimer());  // the groups' first
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = c.k;
   const int64_t ob = it.a + (int64_t)warp * kObsWarp;
@@ -706,6 +721,7 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
     return wx > wy;
   };
   for (auto& g : gr_items) std::stable_sort(g.begin(), g.end(), by_k);
+  std::vector<int> group(b->ncases, 0);
   if (mh) {
     // Mixed update items (all of one size) run shortest case first, a case's
     // items together, so that small cases finish early in the batch.
@@ -714,6 +730,23 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
       if (work(x.c) != work(y.c)) return work(x.c) < work(y.c);
       return x.c != y.c ? x.c < y.c : x.a < y.a;
     });
+    // Groups, and each group's items together.
+    std::vector<int> big;
+    double total = 0.0, taken = 0.0;
+    for (int i = 0; i < b->ncases; ++i) {
+      if (dc[i].kclass != 2) continue;
+      big.push_back(i);
+      total += work(i);
+    }
+    std::stable_sort(big.begin(), big.end(), [&](int x, int y) { return dc[x].k > dc[y].k; });
+    for (int i : big) {
+      group[i] = 2 * taken < total ? 2 : 1;
+      taken += work(i);
+    }
+    auto by_group = [&](const WorkItem& x, const WorkItem& y) { return group[x.c] < group[y.c]; };
+    std::stable_sort(ob_items.begin(), ob_items.end(), by_group);
+    std::stable_sort(up_items.begin(), up_items.end(), by_group);
+    std::stable_sort(gr_items[2].begin(), gr_items[2].end(), by_group);
   } else {
     std::stable_sort(up_items.begin(), up_items.end(), by_k);
   }
@@ -729,6 +762,27 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
   }
   b->update_off = (int64_t)all.size();
   all.insert(all.end(), up_items.begin(), up_items.end());
+  for (CaseGroup& g : b->grp) g = CaseGroup{};
+  if (mh) {
+    for (int i = 0; i < b->ncases; ++i) {
+      CaseGroup& g = b->grp[group[i]];
+      ++g.ncases;
+      g.maxk = std::max(g.maxk, dc[i].k);
+    }
+    for (const WorkItem& x : ob_items) ++b->grp[group[x.c]].obs_cnt;
+    for (const WorkItem& x : up_items) ++b->grp[group[x.c]].upd_cnt;
+    for (const WorkItem& x : gr_items[2]) ++b->grp[group[x.c]].gram_cnt;
+    int64_t ob = b->obs_off, up = b->update_off, gr = b->gram_off[2];
+    for (CaseGroup& g : b->grp) {
+      g.obs_off = ob;
+      g.upd_off = up;
+      g.gram_off = gr;
+      ob += g.obs_cnt;
+      up += g.upd_cnt;
+      gr += g.gram_cnt;
+    }
+    for (int q = kGroups - 2; q >= 0; --q) b->grp[q].ord_off = b->grp[q + 1].ord_off + b->grp[q + 1].ncases;
+  }
   b->n_state_items = (int64_t)st_items.size();
   b->n_obs_items = (int64_t)ob_items.size();
   b->n_update_items = (int64_t)up_items.size();
@@ -784,7 +838,9 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
   b->order = order;
   std::vector<int> ord(b->ncases);
   std::iota(ord.begin(), ord.end(), 0);
-  std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return dc[x].k > dc[y].k; });
+  std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
+    return group[x] != group[y] ? group[x] > group[y] : dc[x].k > dc[y].k;
+  });
   MG_TRY_CUDA(cudaMemcpy(b->dcases, dc.data(), sizeof(DevCase) * dc.size(), cudaMemcpyHostToDevice));
   MG_TRY_CUDA(cudaMemcpy(b->items, all.data(), sizeof(WorkItem) * all.size(), cudaMemcpyHostToDevice));
   MG_TRY_CUDA(cudaMemcpy(order, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
@@ -803,6 +859,58 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
 constexpr size_t rebuild_bytes(int kmax) { return sizeof(float) * ((size_t)kmax * (kmax + 1) + 2 * 32 * (size_t)kmax); }
 
 // Enqueues the batch (no allocation, no host synchronisation: capturable).
+// One group's chain of the mixed path.
+int enqueue_group(mg_context* ctx, mg_etkf_batch* b, int gi, cudaStream_t s) {
+  const CaseGroup& gr = b->grp[gi];
+  const int kp = gr.maxk + (gr.maxk & 1);
+  const int* order = b->order + gr.ord_off;
+  const unsigned nc = (unsigned)gr.ncases;
+  batch_prep_obs_mixed_kernel<<<(unsigned)gr.obs_cnt, kThreads, 0, s>>>(b->dcases, b->items + gr.obs_off, b->times);
+  MG_COUNT_LAUNCH();
+  if (gi == 0) {
+    if (b->gram_cnt[0]) {
+      batch_gram_kernel<float, 32><<<(unsigned)b->gram_cnt[0], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[0]);
+      MG_COUNT_LAUNCH();
+    }
+    if (b->gram_cnt[1]) {
+      batch_gram_kernel<float, 64><<<(unsigned)b->gram_cnt[1], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[1]);
+      MG_COUNT_LAUNCH();
+    }
+  } else {
+    batch_gram_kernel<float, 128><<<(unsigned)gr.gram_cnt, kThreads, 0, s>>>(b->dcases, b->items + gr.gram_off);
+    MG_COUNT_LAUNCH();
+  }
+  const size_t s1 = sizeof(float) * solve1_floats(kp);
+  if (gr.maxk > 64)  // more threads per rotation round for the large cases
+    batch_solve1_kernel<512><<<nc, 512, s1, s>>>(b->dcases, order, b->flags);
+  else
+    batch_solve1_kernel<kThreads><<<nc, kThreads, s1, s>>>(b->dcases, order, b->flags);
+  MG_COUNT_LAUNCH();
+  if (gi == 0) {
+    if (b->gram_cnt[0]) {
+      batch_rebuild_kernel<32><<<(unsigned)b->gram_cnt[0], kThreads, rebuild_bytes(32), s>>>(b->dcases,
+                                                                                          b->items + b->gram_off[0]);
+      MG_COUNT_LAUNCH();
+    }
+    if (b->gram_cnt[1]) {
+      batch_rebuild_kernel<64><<<(unsigned)b->gram_cnt[1], kThreads, rebuild_bytes(64), s>>>(b->dcases,
+                                                                                          b->items + b->gram_off[1]);
+      MG_COUNT_LAUNCH();
+    }
+  } else {
+    batch_rebuild_kernel<128><<<(unsigned)gr.gram_cnt, kThreads, rebuild_bytes(128), s>>>(b->dcases,
+                                                                                        b->items + gr.gram_off);
+    MG_COUNT_LAUNCH();
+  }
+  batch_solve2_kernel<<<nc, kThreads, sizeof(float) * solve2_floats(kp), s>>>(b->dcases, order, b->flags, b->status);
+  MG_COUNT_LAUNCH();
+  batch_update_mixed_kernel<<<(unsigned)gr.upd_cnt, kThreads, mg::upd_bytes(gr.maxk), s>>>(
+      b->dcases, b->items + gr.upd_off, gr.maxk, b->counters, b->times);
+  MG_COUNT_LAUNCH();
+  MG_TRY_CUDA(cudaGetLastError());
+  return MG_OK;
+}
+
 int enqueue(mg_context* ctx, mg_etkf_batch* b) {
   cudaStream_t s = ctx->stream;
   const bool f64 = b->precision == MG_PREC_FP64;
@@ -815,61 +923,30 @@ int enqueue(mg_context* ctx, mg_etkf_batch* b) {
       batch_prep_state_kernel<float><<<(unsigned)b->n_state_items, kStateTile, 0, s>>>(b->dcases, b->items + b->state_off, b->times);
     MG_COUNT_LAUNCH();
   }
-  const bool mh = mixed_hunt(b);
+  if (mixed_hunt(b)) {
+    MG_TRY_CUDA(cudaMemsetAsync(b->times, 0xff, sizeof(unsigned long long), s));
+    // The largest cases' chain is the longest: it goes first, on the stream of
+    // the highest priority.  The first group there is stays on this stream.
+    int home = 0;
+    while (!b->grp[home].ncases) ++home;
+    MG_TRY_CUDA(cudaEventRecord(b->fork, s));
+    int rc = MG_OK;
+    for (int q = kGroups - 1; q > home && rc == MG_OK; --q) {
+      if (!b->grp[q].ncases) continue;
+      MG_TRY_CUDA(cudaStreamWaitEvent(b->side[q - 1], b->fork, 0));
+      rc = enqueue_group(ctx, b, q, b->side[q - 1]);
+      MG_TRY_CUDA(cudaEventRecord(b->join[q - 1], b->side[q - 1]));
+    }
+    if (rc == MG_OK) rc = enqueue_group(ctx, b, home, s);
+    for (int q = kGroups - 1; q > home; --q)
+      if (b->grp[q].ncases) MG_TRY_CUDA(cudaStreamWaitEvent(s, b->join[q - 1], 0));
+    return rc;
+  }
   if (b->n_obs_items) {
-    if (mh)
-      batch_prep_obs_mixed_kernel<<<(unsigned)b->n_obs_items, kThreads, 0, s>>>(b->dcases, b->items + b->obs_off,
-                                                                                 b->times);
-    else
-      batch_prep_obs_kernel<<<(unsigned)b->n_obs_items, kObsTile * 32, 0, s>>>(b->dcases, b->items + b->obs_off);
+    batch_prep_obs_kernel<<<(unsigned)b->n_obs_items, kObsTile * 32, 0, s>>>(b->dcases, b->items + b->obs_off);
     MG_COUNT_LAUNCH();
   }
   const int kp = b->maxk + (b->maxk & 1);
-  if (mh) {
-    if (b->gram_cnt[0]) {
-      batch_gram_kernel<float, 32><<<(unsigned)b->gram_cnt[0], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[0]);
-      MG_COUNT_LAUNCH();
-    }
-    if (b->gram_cnt[1]) {
-      batch_gram_kernel<float, 64><<<(unsigned)b->gram_cnt[1], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[1]);
-      MG_COUNT_LAUNCH();
-    }
-    if (b->gram_cnt[2]) {
-      batch_gram_kernel<float, 128><<<(unsigned)b->gram_cnt[2], kThreads, 0, s>>>(b->dcases,
-                                                                                  b->items + b->gram_off[2]);
-      MG_COUNT_LAUNCH();
-    }
-    if (b->maxk > 64)  // more threads per rotation round for the large cases
-      batch_solve1_kernel<512><<<(unsigned)b->ncases, 512, sizeof(float) * solve1_floats(kp), s>>>(b->dcases, b->order,
-                                                                                              b->flags);
-    else
-      batch_solve1_kernel<kThreads><<<(unsigned)b->ncases, kThreads, sizeof(float) * solve1_floats(kp), s>>>(
-          b->dcases, b->order, b->flags);
-    MG_COUNT_LAUNCH();
-    if (b->gram_cnt[0]) {
-      batch_rebuild_kernel<32><<<(unsigned)b->gram_cnt[0], kThreads, rebuild_bytes(32), s>>>(b->dcases,
-                                                                                          b->items + b->gram_off[0]);
-      MG_COUNT_LAUNCH();
-    }
-    if (b->gram_cnt[1]) {
-      batch_rebuild_kernel<64><<<(unsigned)b->gram_cnt[1], kThreads, rebuild_bytes(64), s>>>(b->dcases,
-                                                                                          b->items + b->gram_off[1]);
-      MG_COUNT_LAUNCH();
-    }
-    if (b->gram_cnt[2]) {
-      batch_rebuild_kernel<128><<<(unsigned)b->gram_cnt[2], kThreads, rebuild_bytes(128), s>>>(
-          b->dcases, b->items + b->gram_off[2]);
-      MG_COUNT_LAUNCH();
-    }
-    batch_solve2_kernel<<<(unsigned)b->ncases, kThreads, sizeof(float) * solve2_floats(kp), s>>>(b->dcases, b->order, b->flags,
-                                                                                                b->status);
-    MG_COUNT_LAUNCH();
-    batch_update_mixed_kernel<<<(unsigned)b->n_update_items, kThreads, mg::upd_bytes(b->maxk), s>>>(
-        b->dcases, b->items + b->update_off, b->maxk, b->counters, b->times);
-    MG_COUNT_LAUNCH();
-    MG_TRY_CUDA(cudaGetLastError());
-    return MG_OK;
-  }
   if (b->gram_cnt[0]) {
     batch_gram_kernel<double, 32><<<(unsigned)b->gram_cnt[0], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[0]);
     MG_COUNT_LAUNCH();
@@ -951,8 +1028,24 @@ int mg_etkf_batch_create(mg_context* ctx, const mg_etkf_case* cases, int32_t nca
   b->host_cases.assign(cases, cases + ncases);
   int rc = build(ctx, b.get());
   if (rc != MG_OK) return rc;
+  if (mixed_hunt(b.get())) {
+    int low = 0, high = 0;
+    cudaError_t e = cudaDeviceGetStreamPriorityRange(&low, &high);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    for (int q = 0; q < kGroups - 1 && e == cudaSuccess; ++q) {
+      e = cudaStreamCreateWithPriority(&b->side[q], cudaStreamNonBlocking, std::max(high, low - 1 - q));
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) {
+      mg_etkf_batch_destroy(b.release());
+      return mg::fail(ctx, MG_ERR_CUDA, std::string("mg_etkf_batch_create: ") + cudaGetErrorString(e));
+    }
+  }
   rc = set_attributes(ctx, b.get());
-  if (rc != MG_OK) return rc;
+  if (rc != MG_OK) {
+    mg_etkf_batch_destroy(b.release());
+    return rc;
+  }
   *out = b.release();
   return MG_OK;
 }
@@ -962,6 +1055,11 @@ void mg_etkf_batch_destroy(mg_etkf_batch* b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   if (b->ws) cudaFree(b->ws);
+  if (b->fork) cudaEventDestroy(b->fork);
+  for (cudaEvent_t e : b->join)
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t t : b->side)
+    if (t) cudaStreamDestroy(t);
   delete b;
 }
 

@@ -74,4 +74,17 @@ __device__ __forceinline__ double pair_to_double(float s, float e) {
   return __longlong_as_double((long long)d);
 }
 
+// Two FP32 fused multiply-adds in one instruction (lanes independent, each
+// rounded as fmaf): d = a b + d.  Half the issue slots of the scalar form.
+__device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "mov.b64 z, {%0, %1};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}"
+      : "+f"(d.x), "+f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+
 }  // namespace mg
