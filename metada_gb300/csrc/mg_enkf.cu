@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kThreads) mean_spread_kernel(const double* __r
     m = __dmul_rn(m, inv_k);
     mean[s] = m;
     const int emax = (mx >> 20) + 1;  // the mean may round up a binade
-    if (k > kFixMembers || emax < 64 || emax >= 0x7ff) {
+    if (k > kFixMembers || emax < 64 || emax >= 0x7ff - 7) {  // below: the sum of 128 values stays finite
       sq += spread_fp64(X + s, k, ld, m);
       continue;
     }

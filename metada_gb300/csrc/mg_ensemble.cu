@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(T) to_point_major_f32_kernel(const float* __re
       const float d = __fsub_rn(x, h), b = __fadd_rn(d, h);
       const float e = __fadd_rn(__fsub_rn(x, b), __fsub_rn(__fsub_rn(b, d), h));  // x - h - d, exact
       const float r = __fadd_rn(d, __fsub_rn(e, l));
-      p[i] = fabsf(h) <= 3.0e38f ? r : x - h;  // an infinite mean has no low part
+      p[i] = fabsf(d) <= 3.402823466e38f ? r : d;  // no low part where the difference is not finite
     }
   }
 }

@@ -10,9 +10,7 @@
 // exact, and the slices with s + t <= 6 (28 of 49) leave out less than
 // 2^-54 of (largest |a|) (largest |b|) per term: FP64 rounding.  mma.sync
 // and not tcgen05: the digits of one tile are produced by the threads that
-// consume them and an accumulator set is 28 registers, the tile is bound by
-// the FP64 operations around the product (mean, scale, add), not by the MMA
-// rate (the design doc has the counts).
+// consume them and an accumulator set is 28 registers.
 #pragma once
 
 #include <cuda_fp16.h>

@@ -43,3 +43,14 @@ def test_spread_diagnostics(dev, k, n, kind):
     after = Xd.cpu().numpy()
     np.testing.assert_allclose(diag["background_spread"], _spread(X), rtol=1e-12)
     np.testing.assert_allclose(diag["analysis_spread"], _spread(after), rtol=1e-12)
+
+
+def test_spread_of_members_whose_sum_overflows(dev):
+    """Finite members with an infinite sum: an infinite mean and spread, as the FP64 sums give."""
+    k, n, p = 64, 40, 5
+    r = np.random.default_rng(1)
+    X = np.ldexp(1.0 + r.uniform(0, 1, (k, n)), 1019)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)  # noqa: E731
+    _, diag = K.enkf(t(X), t(r.normal(0, 1, (p, k))), t(r.normal(0, 1, p)), t(np.full(p, 4.0)),
+                     t(r.normal(0, 2, (p, k))), 1.0)
+    assert diag["background_spread"] == np.inf
