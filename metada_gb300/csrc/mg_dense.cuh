@@ -333,18 +333,21 @@ __device__ __forceinline__ float4 jacobi_rot(float app, float aqq, float apq, fl
 // Diagonalises A (kp x kp, kp even, lda; read and written in its upper
 // triangle only) to the off-diagonal threshold tol.  Vt (rows of ldv
 // floats, ldv % 4 == 0, ldv >= 4 ceil(kp / 4), 16-byte aligned) receives the
-// eigenvectors as rows: Vt[j * ldv + i] = V_ij.  rot holds kp/2 float4
-// (16-byte aligned).  Returns the sweeps run.
-template <int KMAX, int NT>
+// eigenvectors as rows: Vt[j * ldv + i] = V_ij (GO_ON: the rows that Vt holds
+// are rotated on).  rot holds kp/2 float4 (16-byte aligned).  Returns the
+// sweeps run.
+template <int KMAX, int NT, bool GO_ON = false>
 __device__ int cta_jacobi_tri(float* A, int lda, float* Vt, int ldv, int kp, float tol, int max_sweeps,
                               float4* rot) {
   constexpr int HM = KMAX / 2;
   constexpr int NB = (HM * (HM + 1) / 2 + NT - 1) / NT;     // upper-triangle blocks per thread
   constexpr int NVI = (HM * ((KMAX + 3) / 4) + NT - 1) / NT;  // (pair, 4-row chunk) items per thread
   const int tid = threadIdx.x, h = kp >> 1, m = kp - 1, nch = (kp + 3) >> 2;
-  for (int e = tid; e < kp * 4 * nch; e += NT) {
-    const int j = e / (4 * nch), i = e - j * (4 * nch);
-    Vt[j * ldv + i] = (i == j) ? 1.0f : 0.0f;
+  if constexpr (!GO_ON) {
+    for (int e = tid; e < kp * 4 * nch; e += NT) {
+      const int j = e / (4 * nch), i = e - j * (4 * nch);
+      Vt[j * ldv + i] = (i == j) ? 1.0f : 0.0f;
+    }
   }
   int blk[NB];  // b << 8 | c with b <= c, or -1
 #pragma unroll

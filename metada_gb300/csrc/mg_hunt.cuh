@@ -19,10 +19,18 @@
 // A^-1/2 = V Ws V^T with Ws = (I + H)(C + F)(I + H), left in two factors.
 // A CPU model of this arithmetic against 200-bit references: 6e-16 relative
 // at condition number 17, 2e-15 at 300, 6e-14 at 1e4, below LAPACK's FP64
-// eigen-solver in each case.  Step 2 shows whether E is small (kGate); a
-// matrix where it is not (or that is not SPD) is left to the caller's FP64
-// Jacobi.
+// eigen-solver in each case.  Step 2 shows whether E is small (kHuntGate).
+// Where it is not, many eigenvalues are small beside the largest, and the
+// FP32 rotations' rounding, eps32 lambda_max, shows between the small ones
+// (100 members that span 25 directions well observed: condition number 300).
+// A2 is graded by then, and Jacobi on a graded matrix is accurate relative to
+// sqrt(d_i d_j): a second pass rotates V on by an FP32 Jacobi of A2 and goes
+// back to step 2, where the caller can supply A once more (the global
+// analyses).  What is left (or not SPD) goes to the caller's FP64 Jacobi.
 #pragma once
+
+#include <cstddef>
+#include <type_traits>
 
 #include "mg_dense.cuh"
 #include "mg_fp64.cuh"
@@ -131,8 +139,11 @@ struct Hunt {
   }
 
   // A <- Ws with A^-1/2 = scale V Ws V^T.  False: left to the caller (A is
-  // destroyed).  All threads; ends synchronised.
-  __device__ bool transform(int k, double* scale, int* sweeps) {
+  // destroyed).  All threads; ends synchronised.  reload() fills A as on entry
+  // for the second pass; nullptr: no second pass.
+  template <typename Reload>
+  __device__ bool transform(int k, double* scale, int* sweeps, Reload reload) {
+    constexpr bool kTwice = !std::is_same<Reload, std::nullptr_t>::value;
     const int tid = threadIdx.x, ti = tid / 16, tj = tid % 16;
     const int kp = k + (k & 1);
     // ---- scale, FP32 copy, FP32 Jacobi ----
@@ -160,186 +171,205 @@ struct Hunt {
     __syncthreads();
     *sweeps = cta_jacobi_tri<KP, kHuntThreads>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
     __syncthreads();
-    // ---- V <- (3 I - V V^T) V / 2 (rows are eigenvectors), in FP32 ----
-    {
-      float* M = A32;
-      float acc[R][R];
+    double w[NL];
+    float t[NL];
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+      // ---- V <- (3 I - V V^T) V / 2 (rows are eigenvectors), in FP32 ----
+      {
+        float* M = A32;
+        float acc[R][R];
 #pragma unroll
-      for (int a = 0; a < R; ++a)
+        for (int a = 0; a < R; ++a)
 #pragma unroll
-        for (int b = 0; b < R; ++b) acc[a][b] = 0.0f;
-      for (int m = 0; m < KP; m += 4) {
+          for (int b = 0; b < R; ++b) acc[a][b] = 0.0f;
+        for (int m = 0; m < KP; m += 4) {
+          float4 x[R], y[R];
+#pragma unroll
+          for (int a = 0; a < R; ++a) {
+            const int i = ti + 16 * a, j = tj + 16 * a;
+            x[a] = (i < k && m < kp) ? *reinterpret_cast<const float4*>(V + i * LDV + m) : make_float4(0, 0, 0, 0);
+            y[a] = (j < k && m < kp) ? *reinterpret_cast<const float4*>(V + j * LDV + m) : make_float4(0, 0, 0, 0);
+          }
+#pragma unroll
+          for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b < R; ++b)
+              acc[a][b] += (x[a].x * y[b].x + x[a].y * y[b].y) + (x[a].z * y[b].z + x[a].w * y[b].w);
+        }
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+#pragma unroll
+          for (int b = 0; b < R; ++b) {
+            const int i = ti + 16 * a, j = tj + 16 * b;
+            M[i * LDA + j] = (i == j ? 1.5f : 0.0f) - 0.5f * acc[a][b];
+            acc[a][b] = 0.0f;
+          }
+        __syncthreads();
+        for (int m = 0; m < k; ++m) {
+          float x[R], y[R];
+#pragma unroll
+          for (int a = 0; a < R; ++a) {
+            x[a] = M[(ti + 16 * a) * LDA + m];
+            y[a] = V[m * LDV + tj + 16 * a];
+          }
+#pragma unroll
+          for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b < R; ++b) acc[a][b] += x[a] * y[b];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+#pragma unroll
+          for (int b = 0; b < R; ++b) {
+            const int i = ti + 16 * a, j = tj + 16 * b;
+            if (i < k) V[i * LDV + j] = j < k ? acc[a][b] : 0.0f;  // beyond k: zero, read in fours below
+          }
+        __syncthreads();
+      }
+      // ---- H = -D/2 + 3/8 D^2, D = V V^T - I in FP64 ----
+#pragma unroll
+      for (int u = 0; u < NL; ++u) w[u] = 0.0;
+      for (int m = 0; m < k; m += 4) {
         float4 x[R], y[R];
 #pragma unroll
         for (int a = 0; a < R; ++a) {
-          const int i = ti + 16 * a, j = tj + 16 * a;
-          x[a] = (i < k && m < kp) ? *reinterpret_cast<const float4*>(V + i * LDV + m) : make_float4(0, 0, 0, 0);
-          y[a] = (j < k && m < kp) ? *reinterpret_cast<const float4*>(V + j * LDV + m) : make_float4(0, 0, 0, 0);
+          x[a] = *reinterpret_cast<const float4*>(V + min(ti + 16 * a, k - 1) * LDV + m);
+          y[a] = *reinterpret_cast<const float4*>(V + min(tj + 16 * a, k - 1) * LDV + m);
         }
 #pragma unroll
-        for (int a = 0; a < R; ++a)
+        for (int q = 0; q < 4; ++q) {
+          double xd[R], yd[R];
 #pragma unroll
-          for (int b = 0; b < R; ++b)
-            acc[a][b] += (x[a].x * y[b].x + x[a].y * y[b].y) + (x[a].z * y[b].z + x[a].w * y[b].w);
+          for (int a = 0; a < R; ++a) {
+            xd[a] = widen(q == 0 ? x[a].x : (q == 1 ? x[a].y : (q == 2 ? x[a].z : x[a].w)));
+            yd[a] = widen(q == 0 ? y[a].x : (q == 1 ? y[a].y : (q == 2 ? y[a].z : y[a].w)));
+          }
+          int u = 0;
+#pragma unroll
+          for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b, ++u) w[u] = __fma_rn(xd[a], yd[b], w[u]);
+        }
       }
-#pragma unroll
-      for (int a = 0; a < R; ++a)
-#pragma unroll
-        for (int b = 0; b < R; ++b) {
-          const int i = ti + 16 * a, j = tj + 16 * b;
-          M[i * LDA + j] = (i == j ? 1.5f : 0.0f) - 0.5f * acc[a][b];
-          acc[a][b] = 0.0f;
-        }
+      lower(ti, tj, k, [&](int u, int i, int j) { H[tri(i, j)] = w[u] - (i == j ? 1.0 : 0.0); });
       __syncthreads();
-      for (int m = 0; m < k; ++m) {
-        float x[R], y[R];
+      {
+        float t[NL];
 #pragma unroll
-        for (int a = 0; a < R; ++a) {
-          x[a] = M[(ti + 16 * a) * LDA + m];
-          y[a] = V[m * LDV + tj + 16 * a];
+        for (int u = 0; u < NL; ++u) t[u] = 0.0f;
+        for (int m = 0; m < k; ++m) {
+          float xi[R], xj[R];
+#pragma unroll
+          for (int a = 0; a < R; ++a) {
+            xi[a] = leading(H + tri(min(ti + 16 * a, k - 1), m));
+            xj[a] = leading(H + tri(min(tj + 16 * a, k - 1), m));
+          }
+          int u = 0;
+#pragma unroll
+          for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b, ++u) t[u] += xi[a] * xj[b];
         }
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = 0; b < R; ++b) acc[a][b] += x[a] * y[b];
+        __syncthreads();
+        lower(ti, tj, k, [&](int u, int i, int j) {
+          H[tri(i, j)] = __fma_rn(-0.5, H[tri(i, j)], widen(0.375f * t[u]));
+        });
       }
+      // ---- B = V A V^T (rows of V), in blocks of 16 rows of A ----
+#pragma unroll
+      for (int u = 0; u < NL; ++u) w[u] = 0.0;
+      for (int mb = 0; mb < k; mb += 16) {
+        {
+          const int m = min(mb + ti, k - 1);
+          double p[R];
+#pragma unroll
+          for (int b = 0; b < R; ++b) p[b] = 0.0;
+          for (int l = 0; l < k; l += 4) {
+            float4 y[R];
+#pragma unroll
+            for (int b = 0; b < R; ++b) y[b] = *reinterpret_cast<const float4*>(V + min(tj + 16 * b, k - 1) * LDV + l);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              if (l + q >= k) break;
+              const double a = A[tri(m, l + q)];
+#pragma unroll
+              for (int b = 0; b < R; ++b)
+                p[b] = __fma_rn(a, widen(q == 0 ? y[b].x : (q == 1 ? y[b].y : (q == 2 ? y[b].z : y[b].w))), p[b]);
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < R; ++b) blk[ti * KP + tj + 16 * b] = p[b];
+        }
+        __syncthreads();
+        for (int m = 0; m < 16 && mb + m < k; ++m) {
+          double x[R], y[R];
+#pragma unroll
+          for (int a = 0; a < R; ++a) {
+            x[a] = widen(V[min(ti + 16 * a, k - 1) * LDV + mb + m]);
+            y[a] = blk[m * KP + tj + 16 * a];
+          }
+          int u = 0;
+#pragma unroll
+          for (int a = 0; a < R; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b, ++u) w[u] = __fma_rn(x[a], y[b], w[u]);
+        }
+        __syncthreads();
+      }
+      // ---- A2 = (I + H) B (I + H) = diag(d) + E ----
+      lower(ti, tj, k, [&](int u, int i, int j) {
+        A[tri(i, j)] = w[u];
+        if (i == j) d[i] = w[u];
+      });
+      if (tid == 0) flag[0] = flag[1] = 0;
       __syncthreads();
-#pragma unroll
-      for (int a = 0; a < R; ++a)
-#pragma unroll
-        for (int b = 0; b < R; ++b) {
-          const int i = ti + 16 * a, j = tj + 16 * b;
-          if (i < k) V[i * LDV + j] = j < k ? acc[a][b] : 0.0f;  // beyond k: zero, read in fours below
-        }
-      __syncthreads();
-    }
-    // ---- H = -D/2 + 3/8 D^2, D = V V^T - I in FP64 ----
-    double w[NL];
-#pragma unroll
-    for (int u = 0; u < NL; ++u) w[u] = 0.0;
-    for (int m = 0; m < k; m += 4) {
-      float4 x[R], y[R];
-#pragma unroll
-      for (int a = 0; a < R; ++a) {
-        x[a] = *reinterpret_cast<const float4*>(V + min(ti + 16 * a, k - 1) * LDV + m);
-        y[a] = *reinterpret_cast<const float4*>(V + min(tj + 16 * a, k - 1) * LDV + m);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        double xd[R], yd[R];
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-          xd[a] = widen(q == 0 ? x[a].x : (q == 1 ? x[a].y : (q == 2 ? x[a].z : x[a].w)));
-          yd[a] = widen(q == 0 ? y[a].x : (q == 1 ? y[a].y : (q == 2 ? y[a].z : y[a].w)));
-        }
-        int u = 0;
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = 0; b <= a; ++b, ++u) w[u] = __fma_rn(xd[a], yd[b], w[u]);
-      }
-    }
-    lower(ti, tj, k, [&](int u, int i, int j) { H[tri(i, j)] = w[u] - (i == j ? 1.0 : 0.0); });
-    __syncthreads();
-    {
-      float t[NL];
-#pragma unroll
-      for (int u = 0; u < NL; ++u) t[u] = 0.0f;
-      for (int m = 0; m < k; ++m) {
-        float xi[R], xj[R];
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-          xi[a] = leading(H + tri(min(ti + 16 * a, k - 1), m));
-          xj[a] = leading(H + tri(min(tj + 16 * a, k - 1), m));
-        }
-        int u = 0;
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = 0; b <= a; ++b, ++u) t[u] += xi[a] * xj[b];
-      }
+      sandwich(t, H, A, d, ti, tj, k);
+      lower(ti, tj, k, [&](int u, int i, int j) { w[u] += __fma_rn(H[tri(i, j)], d[i] + d[j], widen(t[u])); });
       __syncthreads();
       lower(ti, tj, k, [&](int u, int i, int j) {
-        H[tri(i, j)] = __fma_rn(-0.5, H[tri(i, j)], widen(0.375f * t[u]));
+        A[tri(i, j)] = w[u];
+        if (i == j) {
+          const double dd = w[u], sq = sqrt(dd);
+          d[i] = dd;
+          s[i] = sq;
+          c[i] = 1.0 / sq;
+          if (!(dd > 0.0)) flag[0] = 1;
+        }
       });
-    }
-    // ---- B = V A V^T (rows of V), in blocks of 16 rows of A ----
-#pragma unroll
-    for (int u = 0; u < NL; ++u) w[u] = 0.0;
-    for (int mb = 0; mb < k; mb += 16) {
-      {
-        const int m = min(mb + ti, k - 1);
-        double p[R];
-#pragma unroll
-        for (int b = 0; b < R; ++b) p[b] = 0.0;
-        for (int l = 0; l < k; l += 4) {
-          float4 y[R];
-#pragma unroll
-          for (int b = 0; b < R; ++b) y[b] = *reinterpret_cast<const float4*>(V + min(tj + 16 * b, k - 1) * LDV + l);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (l + q >= k) break;
-            const double a = A[tri(m, l + q)];
-#pragma unroll
-            for (int b = 0; b < R; ++b)
-              p[b] = __fma_rn(a, widen(q == 0 ? y[b].x : (q == 1 ? y[b].y : (q == 2 ? y[b].z : y[b].w))), p[b]);
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < R; ++b) blk[ti * KP + tj + 16 * b] = p[b];
-      }
       __syncthreads();
-      for (int m = 0; m < 16 && mb + m < k; ++m) {
-        double x[R], y[R];
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-          x[a] = widen(V[min(ti + 16 * a, k - 1) * LDV + mb + m]);
-          y[a] = blk[m * KP + tj + 16 * a];
+      // ---- F = F1 + G; w: F1, t: G ----
+      lower(ti, tj, k, [&](int u, int i, int j) {
+        t[u] = 0.0f;
+        if (i == j) {
+          w[u] = 0.0;
+          return;
         }
-        int u = 0;
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = 0; b <= a; ++b, ++u) w[u] = __fma_rn(x[a], y[b], w[u]);
-      }
+        const float e = leading(A + tri(i, j)) * leading(c + i) * leading(c + j);
+        if (!(fabsf(e) <= kHuntGate)) flag[1] = 1;
+        const double si = s[i], sj = s[j];
+        w[u] = -w[u] * recip_fp64(si * sj * (si + sj));
+      });
       __syncthreads();
+      if (flag[0]) return false;
+      if (!flag[1]) break;
+      if constexpr (kTwice) {
+        if (pass > 0) return false;
+        for (int e = tid; e < KP * LDA; e += kHuntThreads) A32[e] = 0.0f;
+        __syncthreads();
+        lower(ti, tj, k, [&](int, int i, int j) { A32[j * LDA + i] = (float)A[tri(i, j)]; });
+        if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
+        __syncthreads();
+        *sweeps += cta_jacobi_tri<KP, kHuntThreads, true>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
+        reload();
+        __syncthreads();
+        lower(ti, tj, k, [&](int, int i, int j) { A[tri(i, j)] *= down; });
+        __syncthreads();
+      } else {
+        return false;
+      }
     }
-    // ---- A2 = (I + H) B (I + H) = diag(d) + E ----
-    lower(ti, tj, k, [&](int u, int i, int j) {
-      A[tri(i, j)] = w[u];
-      if (i == j) d[i] = w[u];
-    });
-    if (tid == 0) flag[0] = 0;
-    __syncthreads();
-    float t[NL];
-    sandwich(t, H, A, d, ti, tj, k);
-    lower(ti, tj, k, [&](int u, int i, int j) { w[u] += __fma_rn(H[tri(i, j)], d[i] + d[j], widen(t[u])); });
-    __syncthreads();
-    lower(ti, tj, k, [&](int u, int i, int j) {
-      A[tri(i, j)] = w[u];
-      if (i == j) {
-        const double dd = w[u], sq = sqrt(dd);
-        d[i] = dd;
-        s[i] = sq;
-        c[i] = 1.0 / sq;
-        if (!(dd > 0.0)) flag[0] = 1;
-      }
-    });
-    __syncthreads();
-    // ---- F = F1 + G; w: F1, t: G ----
-    lower(ti, tj, k, [&](int u, int i, int j) {
-      t[u] = 0.0f;
-      if (i == j) {
-        w[u] = 0.0;
-        return;
-      }
-      const float e = leading(A + tri(i, j)) * leading(c + i) * leading(c + j);
-      if (!(fabsf(e) <= kHuntGate)) flag[0] = 1;
-      const double si = s[i], sj = s[j];
-      w[u] = -w[u] * recip_fp64(si * sj * (si + sj));
-    });
-    __syncthreads();
-    if (flag[0]) return false;
     float* T1 = reinterpret_cast<float*>(blk);
 #pragma unroll 1
     for (int it = 0; it < 2; ++it) {

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<KP>::CTAS) letkf_hunt_kernel(Let
     __syncthreads();
     double scale;
     int sweeps = 0;
-    if (!h.transform(k, &scale, &sweeps)) {
+    if (!h.transform(k, &scale, &sweeps, nullptr)) {
       if (tid == 0) prm.redo_out[atomicAdd(prm.n_redo, 1ull)] = (int32_t)(col * prm.nlev + lev);
       __syncthreads();
       continue;
@@ -388,14 +388,17 @@ __global__ void __launch_bounds__(kThreads) hunt_factor_kernel(const double* __r
   H h;
   h.carve(smem_raw, smem_raw + AB, smem_raw + AB + (H::WORK_BYTES + 15) / 16 * 16);
   const int tid = threadIdx.x;
-  for (int e = tid; e < k * k; e += kThreads) {
-    const int i = e / k, j = e - i * k;
-    if (j <= i) h.A[mg::tri(i, j)] = Gb[e] + (i == j ? diag : 0.0);
-  }
+  auto load = [&] {
+    for (int e = tid; e < k * k; e += kThreads) {
+      const int i = e / k, j = e - i * k;
+      if (j <= i) h.A[mg::tri(i, j)] = Gb[e] + (i == j ? diag : 0.0);
+    }
+  };
+  load();
   __syncthreads();
   double scale = 0.0;
   int sweeps = 0;
-  const bool ok = h.transform(k, &scale, &sweeps);
+  const bool ok = h.transform(k, &scale, &sweeps, load);
   if (tid == 0) info[0] = ok ? scale : 0.0;
   if (!ok) return;
   for (int e = tid; e < k * H::LDV; e += kThreads) Vout[e] = h.V[e];

@@ -109,3 +109,23 @@ def test_etkf_hunt(dev, k, sigma):
     want = ob.letkf_points(X, pts, 1, 0, HX, yo, rvar, off[:21], idx[: 20 * p], None, 1.07, 0)[:, 0, :].T
     kappa = _kappa((HX - HX.mean(1, keepdims=True)) / np.sqrt(rvar)[:, None], k, 1.07)
     assert rel_err(Xd.cpu().numpy()[:, pts], want) <= _tol(kappa)
+
+
+@pytest.mark.parametrize("k", [33, 64, 99, 112])
+@pytest.mark.parametrize("sigma", [0.5, 0.02, 1e-3])
+def test_etkf_hunt_graded(dev, k, sigma):
+    """Obs that span 20 directions well: most eigenvalues at the bottom, the rest far above (the second pass)."""
+    g = np.random.default_rng(k)
+    n, p = 300, 250
+    X = g.standard_normal((k, n)) + 4.0
+    HX = (g.standard_normal((p, 20)) * np.geomspace(1.0, 0.1, 20)) @ g.standard_normal((20, k)) + 4.0
+    yo, rvar = g.standard_normal(p) + 4.0, sigma * sigma * g.uniform(0.5, 2.0, p)
+    Xd = torch.from_numpy(X.copy()).to(dev)
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)  # noqa: E731
+    K.etkf(Xd, T(HX), T(yo), T(rvar), 1.0, flags=0)
+    off = np.arange(n + 1, dtype=np.int64) * p
+    idx = np.tile(np.arange(p, dtype=np.int32), n)
+    pts = g.choice(n, 20, replace=False)
+    want = ob.letkf_points(X, pts, 1, 0, HX, yo, rvar, off[:21], idx[: 20 * p], None, 1.0, 0)[:, 0, :].T
+    kappa = _kappa((HX - HX.mean(1, keepdims=True)) / np.sqrt(rvar)[:, None], k, 1.0)
+    assert rel_err(Xd.cpu().numpy()[:, pts], want) <= _tol(kappa)
