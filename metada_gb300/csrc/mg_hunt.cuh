@@ -169,7 +169,7 @@ struct Hunt {
     });
     if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
     __syncthreads();
-    *sweeps = cta_jacobi_tri<KP, kHuntThreads>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
+    *sweeps = cta_jacobi_ahead<KP, kHuntThreads>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
     __syncthreads();
     double w[NL];
     float t[NL];
@@ -361,7 +361,7 @@ struct Hunt {
         lower(ti, tj, k, [&](int, int i, int j) { A32[j * LDA + i] = (float)A[tri(i, j)]; });
         if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
         __syncthreads();
-        *sweeps += cta_jacobi_tri<KP, kHuntThreads, true>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
+        *sweeps += cta_jacobi_ahead<KP, kHuntThreads, true>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
         reload();
         __syncthreads();
         lower(ti, tj, k, [&](int, int i, int j) { A[tri(i, j)] *= down; });
