@@ -330,73 +330,6 @@ __device__ __forceinline__ float4 jacobi_rot(float app, float aqq, float apq, fl
   return make_float4(c, s, app - t * apq, aqq + t * apq);
 }
 
-// The blocks b <= c of pairs that thread tid of NT owns, b << 8 | c, or -1.
-template <int NB, int NT>
-__device__ __forceinline__ void jacobi_blocks(int (&blk)[NB], int h) {
-#pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    int e = threadIdx.x + u * NT, b = 0;
-    if (e >= h * (h + 1) / 2) {
-      blk[u] = -1;
-      continue;
-    }
-    while (e >= h - b) {
-      e -= h - b;
-      ++b;
-    }
-    blk[u] = (b << 8) | (b + e);
-  }
-}
-
-// A's blocks after round r's rotations.
-template <int NB>
-__device__ __forceinline__ void jacobi_turn(float* A, int lda, const int (&blk)[NB], const float4* rot, int r, int m) {
-#pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    if (blk[u] < 0) continue;
-    const int b = blk[u] >> 8, c = blk[u] & 0xff;
-    const float4 pb = rot[b];
-    if (b == c) {
-      if (pb.y == 0.0f) continue;
-      int p, q;
-      jacobi_pair(b, r, m, p, q);
-      A[p * lda + p] = pb.z;
-      A[q * lda + q] = pb.w;
-      A[min(p, q) * lda + max(p, q)] = 0.0f;
-      continue;
-    }
-    const float4 pc = rot[c];
-    if (pb.y == 0.0f && pc.y == 0.0f) continue;
-    int r0, r1, c0, c1;
-    jacobi_pair(b, r, m, r0, r1);
-    jacobi_pair(c, r, m, c0, c1);
-    const int i00 = min(r0, c0) * lda + max(r0, c0), i01 = min(r0, c1) * lda + max(r0, c1);
-    const int i10 = min(r1, c0) * lda + max(r1, c0), i11 = min(r1, c1) * lda + max(r1, c1);
-    const float a00 = A[i00], a01 = A[i01], a10 = A[i10], a11 = A[i11];
-    const float m00 = pb.x * a00 - pb.y * a10, m01 = pb.x * a01 - pb.y * a11;
-    const float m10 = pb.y * a00 + pb.x * a10, m11 = pb.y * a01 + pb.x * a11;
-    A[i00] = pc.x * m00 - pc.y * m01;
-    A[i01] = pc.y * m00 + pc.x * m01;
-    A[i10] = pc.x * m10 - pc.y * m11;
-    A[i11] = pc.y * m10 + pc.x * m11;
-  }
-}
-
-// Whether a pair of this thread is above the threshold.
-template <int NT>
-__device__ __forceinline__ int jacobi_open(const float* A, int lda, int kp, float tol) {
-  const int tid = threadIdx.x;
-  int open = 0;
-  for (int i = tid >> 5; i < kp - 1; i += NT / 32) {
-    const float aii = A[i * lda + i];
-    for (int j = i + 1 + (tid & 31); j < kp; j += 32) {
-      const float aij = A[i * lda + j];
-      open |= (aij != 0.0f && aij * aij > tol * tol * fabsf(aii * A[j * lda + j]));
-    }
-  }
-  return open;
-}
-
 // Diagonalises A (kp x kp, kp even, lda; read and written in its upper
 // triangle only) to the off-diagonal threshold tol.  Vt (rows of ldv
 // floats, ldv % 4 == 0, ldv >= 4 ceil(kp / 4), 16-byte aligned) receives the
@@ -413,8 +346,20 @@ __device__ int cta_jacobi_tri(float* A, int lda, float* Vt, int ldv, int kp, flo
     const int j = e / (4 * nch), i = e - j * (4 * nch);
     Vt[j * ldv + i] = (i == j) ? 1.0f : 0.0f;
   }
-  int blk[NB];
-  jacobi_blocks<NB, NT>(blk, h);
+  int blk[NB];  // b << 8 | c with b <= c, or -1
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    int e = tid + u * NT, b = 0;
+    if (e >= h * (h + 1) / 2) {
+      blk[u] = -1;
+      continue;
+    }
+    while (e >= h - b) {
+      e -= h - b;
+      ++b;
+    }
+    blk[u] = (b << 8) | (b + e);
+  }
   __syncthreads();
   int sweep = 0;
   while (sweep < max_sweeps) {
@@ -428,7 +373,35 @@ __device__ int cta_jacobi_tri(float* A, int lda, float* Vt, int ldv, int kp, flo
         rotated |= (R.y != 0.0f);
       }
       __syncthreads();
-      jacobi_turn(A, lda, blk, rot, r, m);
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        if (blk[u] < 0) continue;
+        const int b = blk[u] >> 8, c = blk[u] & 0xff;
+        const float4 pb = rot[b];
+        if (b == c) {
+          if (pb.y == 0.0f) continue;
+          int p, q;
+          jacobi_pair(b, r, m, p, q);
+          A[p * lda + p] = pb.z;
+          A[q * lda + q] = pb.w;
+          A[min(p, q) * lda + max(p, q)] = 0.0f;
+          continue;
+        }
+        const float4 pc = rot[c];
+        if (pb.y == 0.0f && pc.y == 0.0f) continue;
+        int r0, r1, c0, c1;
+        jacobi_pair(b, r, m, r0, r1);
+        jacobi_pair(c, r, m, c0, c1);
+        const int i00 = min(r0, c0) * lda + max(r0, c0), i01 = min(r0, c1) * lda + max(r0, c1);
+        const int i10 = min(r1, c0) * lda + max(r1, c0), i11 = min(r1, c1) * lda + max(r1, c1);
+        const float a00 = A[i00], a01 = A[i01], a10 = A[i10], a11 = A[i11];
+        const float m00 = pb.x * a00 - pb.y * a10, m01 = pb.x * a01 - pb.y * a11;
+        const float m10 = pb.y * a00 + pb.x * a10, m11 = pb.y * a01 + pb.x * a11;
+        A[i00] = pc.x * m00 - pc.y * m01;
+        A[i01] = pc.y * m00 + pc.x * m01;
+        A[i10] = pc.x * m10 - pc.y * m11;
+        A[i11] = pc.y * m10 + pc.x * m11;
+      }
 #pragma unroll
       for (int u = 0; u < NVI; ++u) {
         const int e = tid + u * NT;
@@ -453,25 +426,35 @@ __device__ int cta_jacobi_tri(float* A, int lda, float* Vt, int ldv, int kp, flo
     // A sweep that rotated may still have left every pair under the
     // threshold: test all pairs at once (one barrier) instead of running a
     // further sweep whose rounds would only confirm it.
-    const int open = jacobi_open<NT>(A, lda, kp, tol);
+    int open = 0;
+    for (int i = tid >> 5; i < kp - 1; i += NT / 32) {
+      const float aii = A[i * lda + i];
+      for (int j = i + 1 + (tid & 31); j < kp; j += 32) {
+        const float aij = A[i * lda + j];
+        open |= (aij != 0.0f && aij * aij > tol * tol * fabsf(aii * A[j * lda + j]));
+      }
+    }
     if (!__syncthreads_or(open)) break;
   }
   return sweep;
 }
 
-// The same rotations for one system on its own or a few per SM: while the
-// eigenvectors take round r's rotations, the first warps work out round
-// r + 1's, which only needs A, so that the chain of one rotation (reciprocals,
-// square roots) is off the round's path; the eigenvectors' threads have their
-// rotations in registers by then.  k = 64, a CTA of 256 threads: 1.19 -> 1.09
-// ms for a global analysis, 71.0 -> 66.1 ms for 18,000 local ones; not for the
-// uneven batch, where the items of 100 members need too many registers (6.22
-// -> 6.52 ms).  GO_ON: the rows that Vt holds are rotated on.
+// The same rotations in fewer instructions, which bound a system that shares
+// its SM with few others.  While the eigenvectors take round r's rotations, the
+// first warps work out round r + 1's, which only needs A: the chain of one
+// rotation (reciprocals, square roots) is off the round's path.  Its thread also
+// writes the pair's own three entries, so that the blocks left are those of two
+// pairs (two instead of three per thread at k = 64), and leaves the pair beside
+// (c, s), so that nobody else works out indices from the round number.  rot
+// holds two rounds: kp float4.  GO_ON: the rows that Vt holds are rotated on.
+// k = 64, FP64 analyses: 18,000 local ones 71.0 -> 57.2 ms, a global one of 200k
+// states 1.19 -> 1.00 ms.  The uneven batch's solves, which run beside other
+// kernels, keep the plain order (6.25 against 6.35 ms).
 template <int KMAX, int NT, bool GO_ON = false>
 __device__ int cta_jacobi_ahead(float* A, int lda, float* Vt, int ldv, int kp, float tol, int max_sweeps,
                                 float4* rot) {
   constexpr int HM = KMAX / 2;
-  constexpr int NB = (HM * (HM + 1) / 2 + NT - 1) / NT;
+  constexpr int NB = (HM * (HM - 1) / 2 + NT - 1) / NT;  // blocks of two pairs per thread
   constexpr int NR = (HM + 31) / 32 * 32, NVT = NT - NR;  // threads of the rotations, of the eigenvectors
   constexpr int NVI = (HM * ((KMAX + 3) / 4) + NVT - 1) / NVT;  // (pair, 4-row chunk) items per thread
   const int tid = threadIdx.x, h = kp >> 1, m = kp - 1, nch = (kp + 3) >> 2;
@@ -481,47 +464,72 @@ __device__ int cta_jacobi_ahead(float* A, int lda, float* Vt, int ldv, int kp, f
       Vt[j * ldv + i] = (i == j) ? 1.0f : 0.0f;
     }
   }
-  int blk[NB], vsl[NVI], vch[NVI];  // vsl: the item's pair, or -1
-  jacobi_blocks<NB, NT>(blk, h);
+  int blk[NB], vit[NVI];  // b << 8 | c with b < c, pair << 8 | first row; or -1
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    int e = tid + u * NT, b = 0;
+    blk[u] = -1;
+    if (e >= h * (h - 1) / 2) continue;
+    while (e >= h - 1 - b) {
+      e -= h - 1 - b;
+      ++b;
+    }
+    blk[u] = (b << 8) | (b + 1 + e);
+  }
 #pragma unroll
   for (int u = 0; u < NVI; ++u) {
     const int e = tid - NR + u * NVT, sl = e / nch;
-    vsl[u] = (tid >= NR && sl < h) ? sl : -1;
-    vch[u] = 4 * (e - sl * nch);
+    vit[u] = (tid >= NR && sl < h) ? (sl << 8) | 4 * (e - sl * nch) : -1;
   }
-  auto rotate = [&](int r) {  // round r's rotation of pair tid < h; true when it turns
+  auto rotate = [&](int r, float4* out) {  // round r's rotation of pair tid < h
     int p, q;
     jacobi_pair(tid, r, m, p, q);
-    const float4 R = jacobi_rot(A[p * lda + p], A[q * lda + q], A[min(p, q) * lda + max(p, q)], tol);
-    rot[tid] = R;
-    return R.y != 0.0f;
+    float* const apq = A + min(p, q) * lda + max(p, q);
+    const float4 R = jacobi_rot(A[p * lda + p], A[q * lda + q], *apq, tol);
+    out[tid] = make_float4(R.x, R.y, __int_as_float(p), __int_as_float(q));
+    if (R.y == 0.0f) return 0;
+    A[p * lda + p] = R.z;
+    A[q * lda + q] = R.w;
+    *apq = 0.0f;
+    return 1;
   };
   __syncthreads();
-  int sweep = 0, rotated = 0;
-  if (tid < h) rotated = rotate(0);
-  __syncthreads();
+  int sweep = 0;
   while (sweep < max_sweeps) {
-    int next = 0;  // whether the next sweep's first round turns
+    int rotated = 0;
+    if (tid < h) rotated = rotate(0, rot);
+    __syncthreads();
     for (int r = 0; r < m; ++r) {
-      float2 vcs[NVI];
+      const float4* cur = rot + (r & 1) * h;
 #pragma unroll
-      for (int u = 0; u < NVI; ++u)
-        vcs[u] = vsl[u] < 0 ? make_float2(1.0f, 0.0f) : *reinterpret_cast<const float2*>(rot + vsl[u]);
-      jacobi_turn(A, lda, blk, rot, r, m);
-      __syncthreads();
-      if (tid < h) {
-        const int t = rotate(r + 1 < m ? r + 1 : 0);
-        if (r + 1 < m) rotated |= t;
-        else next = t;
+      for (int u = 0; u < NB; ++u) {
+        if (blk[u] < 0) continue;
+        const float4 pb = cur[blk[u] >> 8], pc = cur[blk[u] & 0xff];
+        if (pb.y == 0.0f && pc.y == 0.0f) continue;
+        const int r0 = __float_as_int(pb.z), r1 = __float_as_int(pb.w);
+        const int c0 = __float_as_int(pc.z), c1 = __float_as_int(pc.w);
+        float* const p00 = A + min(r0, c0) * lda + max(r0, c0);
+        float* const p01 = A + min(r0, c1) * lda + max(r0, c1);
+        float* const p10 = A + min(r1, c0) * lda + max(r1, c0);
+        float* const p11 = A + min(r1, c1) * lda + max(r1, c1);
+        const float a00 = *p00, a01 = *p01, a10 = *p10, a11 = *p11;
+        const float m00 = pb.x * a00 - pb.y * a10, m01 = pb.x * a01 - pb.y * a11;
+        const float m10 = pb.y * a00 + pb.x * a10, m11 = pb.y * a01 + pb.x * a11;
+        *p00 = pc.x * m00 - pc.y * m01;
+        *p01 = pc.y * m00 + pc.x * m01;
+        *p10 = pc.x * m10 - pc.y * m11;
+        *p11 = pc.y * m10 + pc.x * m11;
       }
+      __syncthreads();
+      if (tid < h && r + 1 < m) rotated |= rotate(r + 1, rot + ((r + 1) & 1) * h);
 #pragma unroll
       for (int u = 0; u < NVI; ++u) {
-        const float c = vcs[u].x, sn = vcs[u].y;
+        if (vit[u] < 0) continue;
+        const float4 ps = cur[vit[u] >> 8];
+        const float c = ps.x, sn = ps.y;
         if (sn == 0.0f) continue;
-        int p, q;
-        jacobi_pair(vsl[u], r, m, p, q);
-        float4* vp = reinterpret_cast<float4*>(Vt + p * ldv + vch[u]);
-        float4* vq = reinterpret_cast<float4*>(Vt + q * ldv + vch[u]);
+        float4* vp = reinterpret_cast<float4*>(Vt + __float_as_int(ps.z) * ldv + (vit[u] & 0xff));
+        float4* vq = reinterpret_cast<float4*>(Vt + __float_as_int(ps.w) * ldv + (vit[u] & 0xff));
         const float4 a = *vp, bq = *vq;
         *vp = make_float4(c * a.x - sn * bq.x, c * a.y - sn * bq.y, c * a.z - sn * bq.z, c * a.w - sn * bq.w);
         *vq = make_float4(sn * a.x + c * bq.x, sn * a.y + c * bq.y, sn * a.z + c * bq.z, sn * a.w + c * bq.w);
@@ -530,8 +538,15 @@ __device__ int cta_jacobi_ahead(float* A, int lda, float* Vt, int ldv, int kp, f
     }
     ++sweep;
     if (!__syncthreads_or(rotated)) break;
-    if (!__syncthreads_or(jacobi_open<NT>(A, lda, kp, tol))) break;
-    rotated = next;
+    int open = 0;  // as in cta_jacobi_tri
+    for (int i = tid >> 5; i < kp - 1; i += NT / 32) {
+      const float aii = A[i * lda + i];
+      for (int j = i + 1 + (tid & 31); j < kp; j += 32) {
+        const float aij = A[i * lda + j];
+        open |= (aij != 0.0f && aij * aij > tol * tol * fabsf(aii * A[j * lda + j]));
+      }
+    }
+    if (!__syncthreads_or(open)) break;
   }
   return sweep;
 }

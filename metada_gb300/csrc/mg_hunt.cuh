@@ -73,7 +73,7 @@ struct Hunt {
   static constexpr size_t F_BYTES = (sizeof(float) * PACKED + 15) / 16 * 16;
   static constexpr size_t BLK_BYTES = sizeof(double) * 16 * KP;
   static constexpr size_t WORK_BYTES = B_BYTES + V_BYTES + F_BYTES + BLK_BYTES;  // after A
-  static constexpr size_t VEC_BYTES = sizeof(double) * 3 * KP + sizeof(float4) * (KP / 2) + 64;
+  static constexpr size_t VEC_BYTES = sizeof(double) * 3 * KP + sizeof(float4) * KP + 64;
 
   double* A;    // in: A (lower rows); out: Ws
   double* H;
@@ -94,7 +94,7 @@ struct Hunt {
     F = reinterpret_cast<float*>(work + B_BYTES + V_BYTES);
     blk = reinterpret_cast<double*>(work + B_BYTES + V_BYTES + F_BYTES);
     rot = reinterpret_cast<float4*>(vec);
-    d = reinterpret_cast<double*>(vec + sizeof(float4) * (KP / 2));
+    d = reinterpret_cast<double*>(vec + sizeof(float4) * KP);
     s = d + KP;
     c = s + KP;
     flag = reinterpret_cast<int*>(c + KP);

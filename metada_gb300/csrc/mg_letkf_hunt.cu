@@ -11,7 +11,7 @@
 // Jacobi kernel.  What bounds it: the FP32 Jacobi's shared-memory rounds and
 // the 2.3 k^3 FP64 multiply-adds of the correction, which CTAs of one SM
 // overlap (three at k <= 64).  60 x 30 x 10 points, k = 64, about 290 local
-// obs: 782 ms with the FP64 Jacobi (ten sweeps on the FP64 units) -> 65 ms.
+// obs: 782 ms with the FP64 Jacobi (ten sweeps on the FP64 units) -> 56 ms.
 #include <algorithm>
 
 #include "mg_hunt.cuh"
@@ -377,7 +377,7 @@ cudaError_t launch(const LetkfParams& prm, int num_sms, cudaStream_t s) {
 // ------------------------------------------------------------ global ETKF --
 // The same transform of one system: a CTA factors it and leaves V and Ws;
 // rows of T = (wa_j + W_ji) follow on as many CTAs as there are rows / 8.
-// k = 64: 5.69 ms by FP64 Jacobi -> 0.74 + 0.04 ms.
+// k = 64: 5.69 ms by FP64 Jacobi -> 0.55 + 0.04 ms.
 template <int KP>
 __global__ void __launch_bounds__(kThreads) hunt_factor_kernel(const double* __restrict__ Gb, int k, double diag,
                                                                float* __restrict__ Vout, double* __restrict__ Wout,
