@@ -245,16 +245,16 @@ def timed(fn, steps, world):
 
 
 def tc_issued_flop(st, k, n_var):
-    """Tensor-core FLOP the tensor-core kernel issues per launch: 3 passes per
-    product, M = 128 tiles; Gram chunks of 32 obs (N = 80), per Newton-Schulz
-    step two 64-wide products (the first step one), the finish three, the
-    update one per 16 variables (N = 16)."""
+    """Tensor-core FLOP the tensor-core kernel issues per launch at k <= 64 and
+    up to four variables, M = 128 tiles: one pass over the hi and lo rows per
+    Gram chunk of 32 obs (N = 80); three passes per product of FP16 pairs, two
+    64-wide ones per Newton-Schulz step (the first step one), two in the finish
+    and two of N = 16 (E and F^T E)."""
     active = st.n_points - st.n_empty
-    mma = lambda n, kdim: 3 * 2.0 * 128 * n * kdim  # noqa: E731
+    mma = lambda n, kdim: 2.0 * 128 * n * kdim  # noqa: E731
     chunks = st.total_local / 32.0 + 0.5 * active
     ns = 2 * st.total_sweeps - active
-    upd = -(-n_var // 16)
-    return chunks * mma(80, 32) + (ns + 3 * active) * mma(64, 64) + upd * active * mma(16, 64)
+    return chunks * mma(80, 32) + 3 * ((ns + 2 * active) * mma(64, 64) + 2 * active * mma(16, 64))
 
 
 def flops_per_step(st, k, n_var):
@@ -964,7 +964,7 @@ def highres_results() -> dict:
     return {"metric": "local analyses/s, high-resolution LETKF (FP32 members)", "value": st.n_points / (ms_cycle / 1e3),
             "unit": "analyses/s", "n_gpus": 1, "steps": 1, "warmup": 1, "ms_per_step": ms_cycle,
             "higher_is_better": True,
-            "dtype": ("f32 storage; 3-pass TF32 tensor-core Gram, Newton-Schulz solve and update (96-slot layout), "
+            "dtype": ("f32 storage; tensor-core Gram (TF32 pairs), Newton-Schulz solve and update (FP16 pairs, 80-slot layout), "
                       "handed-back points on the SIMT two-stage solve; FP64 means and innovations"
                       if st.tensor_path else
                       "f32 storage; FP32 anomalies and SIMT two-stage Jacobi solve; FP64 means and innovations"),
@@ -1098,12 +1098,12 @@ def main():
         peaks = json.loads(pf.read_text())
     achieved_tf = fl / (ms_an / 1e3) / 1e12
     if st.tensor_path:
-        # kind::tf32 runs at half the dense BF16 rate on this part; the BF16
-        # rate is the measured one (burst: the kernel is timed on its own).
+        # The solve's products are kind::f16 at the dense BF16 rate (measured,
+        # burst: the kernel is timed on its own), the Gram's kind::tf32 at half.
         bf16 = peaks.get("bf16_tflops")
-        peak_tf = (bf16 if bf16 else 1900.0) / 2.0
+        peak_tf = bf16 if bf16 else 1900.0
         roof = {"kernel": "letkf_tc_kernel", "bound": "tensor",
-                "peak_basis": ("measured" if bf16 else "fallback") + " dense BF16 / 2 (the TF32 rate)",
+                "peak_basis": ("measured" if bf16 else "fallback") + " dense BF16 (the FP16 rate)",
                 "traffic": TC_TRAFFIC_REDUCED_BYTES * st.n_points / TC_TRAFFIC_REDUCED_ANALYSES,
                 "traffic_from": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the reduced "
                                 "180x90x10x4 case (162,000 analyses), scaled by analyses",
