@@ -33,7 +33,9 @@ __device__ __forceinline__ bool pivot_ok(double d) {
 
 // a / b given r = 1 / b correctly rounded: one correction of a r by its exact
 // remainder gives the correctly rounded quotient (Markstein, 1990) while no
-// term leaves the normal range.
+// term leaves the normal range.  b and r have to be normal numbers (an infinite
+// or zero b gives NaN), and an infinite a gives NaN: a caller whose result may
+// then differ from the division's guards both.
 __device__ __forceinline__ double div_refined(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-q, b, a), r, q);

@@ -40,6 +40,16 @@ __device__ __forceinline__ double gc64(double z) {
          2.0 / (3.0 * z);
 }
 
+// Half of a localisation support as a divisor of div_refined, which needs the
+// divisor and its reciprocal normal (1 / inf is zero, and the quotient's
+// remainder 0 x inf).  Above 2^800, infinite supports included (no localisation
+// in that direction), the quotient of any finite distance rounds to weight 1;
+// 0 and NaN stay (no obs).
+__device__ __forceinline__ double half_support(double support) {
+  const double c = fabs(0.5 * support), big = 0x1p800, small = 0x1p-800;
+  return c > big ? big : (c < small && c > 0.0 ? small : c);
+}
+
 template <int KP>
 struct Cfg {
   using H = mg::Hunt<KP>;
@@ -92,7 +102,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<KP>::CTAS) letkf_hunt_kernel(Let
   const bool infl_compat = prm.flags & MG_INFL_COMPAT;
   const bool upd_compat = prm.flags & MG_UPDATE_COMPAT;
   const bool rtps = prm.flags & MG_RTPS;
-  const double hc = 0.5 * prm.hsupport, vc = 0.5 * prm.vsupport, vs = prm.vsupport;
+  const double hc = half_support(prm.hsupport), vc = half_support(prm.vsupport), vs = prm.vsupport;
   const double rhc = 1.0 / hc, rvc = 1.0 / vc;
   const double diag = (infl_compat || rtps) ? (double)(k - 1) : (double)(k - 1) / prm.rho;
   const double sc = infl_compat ? prm.rho : 1.0;
