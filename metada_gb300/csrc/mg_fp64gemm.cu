@@ -299,6 +299,14 @@ struct UpdCfg {
                                   sizeof(int) * (KP + NS + 4);
 };
 
+// Any of the eight values not zero, by integer operations.
+__device__ __forceinline__ bool any_nonzero(const double (&v)[8]) {
+  long long b = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) b |= __double_as_longlong(v[q]);
+  return (b << 1) != 0;
+}
+
 template <int KP>
 __global__ void __launch_bounds__(kThreads) update_kernel(double* X, int64_t ld, int64_t n, int k,
                                                           const double* __restrict__ mean,
@@ -311,10 +319,10 @@ __global__ void __launch_bounds__(kThreads) update_kernel(double* X, int64_t ld,
   double* sm = reinterpret_cast<double*>(dX + oz::kSlices * NS * LD);
   int* exT = reinterpret_cast<int*>(sm + NS);
   int* exX = exT + KP;
-  int* odd = exX + NS;  // [0]: this tile, [1]: T
+  int* odd = exX + NS;  // [0]: this tile, [1]: T, [2]: T's smallest row exponent
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < KP; i += kThreads) exT[i] = 1;
-  if (tid < 2) odd[tid] = 0;
+  if (tid < 3) odd[tid] = tid == 2 ? 0x7ff : 0;
   __syncthreads();
   for (int it = tid; it < KP * (KP / 8); it += kThreads) {
     const int i = it % KP, jg = it / KP;
@@ -330,8 +338,11 @@ __global__ void __launch_bounds__(kThreads) update_kernel(double* X, int64_t ld,
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = (i < k && jg * 8 + q < k) ? T[(jg * 8 + q) * k + i] : 0.0;
     if (exT[i] > oz::kMaxEf) odd[1] = 1;
+    if (i < k) atomicMin(&odd[2], exT[i]);
     oz::store_digits8(v, exT[i], dT + i * LD + jg * 8, KP * LD);
   }
+  __syncthreads();
+  const int tiny = oz::kUnitEf - odd[2];  // exponents up to it: products below unit()'s (states of 1e-260 and less)
   const bool pair_ok = ((ld & 1) | ((reinterpret_cast<uintptr_t>(X) >> 3) & 1)) == 0;
   const int64_t ntiles = (n + NS - 1) / NS;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -376,11 +387,11 @@ __global__ void __launch_bounds__(kThreads) update_kernel(double* X, int64_t ld,
       if (it >= C::ITEMS) continue;
       const int sl = it % NS, jg = it / NS;
       const int ef = exX[sl];
-      if (ef > oz::kMaxEf) odd[0] = 1;
+      if ((unsigned)(ef - tiny - 1) >= (unsigned)(oz::kMaxEf - tiny) && (ef > tiny || any_nonzero(v[x]))) odd[0] = 1;
       oz::store_digits8(v[x], ef, dX + sl * LD + jg * 8, NS * LD);
     }
     __syncthreads();
-    if (odd[0]) {  // magnitudes the integers cannot hold: the plain FP64 sum
+    if (odd[0]) {  // magnitudes that the integers or their unit cannot hold: the plain FP64 sum
       double out[C::OUT];
 #pragma unroll
       for (int u = 0; u < C::OUT; ++u) {

@@ -126,9 +126,11 @@ __device__ __forceinline__ long long combine(const float (&acc)[kSlices][4], int
 }
 
 // 2^(exa + exb - 56), the weight of combine()'s unit for operand exponents
-// fields ea, eb (2^ex = 2^(ef - 1022)); zero below the normal range.
+// fields ea, eb (2^ex = 2^(ef - 1022)); zero below the normal range, up to a
+// sum of kUnitEf (products below 2^-968: nothing beside a Gram's k - 1).
+constexpr int kUnitEf = 1077;
 __device__ __forceinline__ double unit(int ea, int eb) {
-  const int f = ea + eb - 1077;
+  const int f = ea + eb - kUnitEf;
   return f > 0 ? __hiloint2double(f << 20, 0) : 0.0;
 }
 // Exponent fields up to which unit() and the scaled sums stay finite.
