@@ -151,6 +151,15 @@ int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int3
                          const double* yo, int64_t p, double radius, double rho,
                          double* mean_out);
 
+/* Self-test of that kernel's bounded waits: the same call with the time that
+ * a point waits for an earlier one given (10 s there).  A run in which a wait
+ * gives up returns MG_ERR_TIMEOUT and leaves X and mean_out as they were.  No
+ * counterpart in the reference. */
+int mg_letkf_compat_grid_wait_selftest(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx,
+                                       int32_t ny, const int32_t* obs_xy, const uint8_t* valid,
+                                       const double* yo, int64_t p, double radius, double rho,
+                                       double* mean_out, int64_t wait_ns);
+
 /* Allocation-free variant of mg_etkf, for callers that cannot allocate device
  * memory when they run the analysis: real-time assimilation loops whose
  * device memory is fixed at start-up (an allocation in the cycle could fail

@@ -151,6 +151,8 @@ _SIGNATURES = {
                 c_int32, c_int32, c_void_p],
     "mg_letkf_compat_grid": [c_void_p, c_void_p, c_int32, c_int64, c_int32, c_int32, c_void_p, c_void_p,
                              c_void_p, c_int64, c_double, c_double, c_void_p],
+    "mg_letkf_compat_grid_wait_selftest": [c_void_p, c_void_p, c_int32, c_int64, c_int32, c_int32, c_void_p, c_void_p,
+                                           c_void_p, c_int64, c_double, c_double, c_void_p, c_int64],
     "mg_letkf_batched": [c_void_p, POINTER(LetkfDesc)],
     "mg_letkf_last_stats": [c_void_p, POINTER(LetkfStats)],
     "mg_kernel_launches": [c_void_p],

@@ -15,12 +15,15 @@ constexpr int kTile = 32;  // state indices per transpose tile
 template <typename TX>
 __global__ void __launch_bounds__(256) mean_pert_members_kernel(
     const TX* __restrict__ X, int64_t n, int k, int64_t ld, double inv_k,
-    double* __restrict__ mean, double* __restrict__ Xp64, float* __restrict__ Xp32, int64_t ldp) {
+    double* __restrict__ mean, double* __restrict__ Xp64, float* __restrict__ Xp32, int64_t ldp,
+    const int* __restrict__ skip) {
+  const bool keep = skip && *skip;  // read beside the members
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += stride) {
     double m = 0.0;
     for (int i = 0; i < k; ++i) m = __dadd_rn(m, (double)__ldg(X + (int64_t)i * ld + s));
     m = __dmul_rn(m, inv_k);
+    if (keep) return;
     if (mean) mean[s] = m;
     if (Xp64 || Xp32) {
       for (int i = 0; i < k; ++i) {
@@ -70,8 +73,9 @@ __global__ void __launch_bounds__(256) to_point_major_kernel(const double* __res
 __global__ void __launch_bounds__(256) point_major_to_members_kernel(const double* __restrict__ P,
                                                                      int64_t n, int k,
                                                                      double* __restrict__ X,
-                                                                     int64_t ld) {
+                                                                     int64_t ld, const int* __restrict__ skip) {
   extern __shared__ double tile[];  // [kTile][k + 1]
+  const bool keep = skip && *skip;  // read beside the rows
   const int64_t s0 = (int64_t)blockIdx.x * kTile;
   const int total = kTile * k;
   for (int e = threadIdx.x; e < total; e += blockDim.x) {
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(256) point_major_to_members_kernel(const doubl
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int i = warp; i < k; i += nw) {
     const int64_t s = s0 + lane;
-    if (s < n) X[(int64_t)i * ld + s] = tile[lane * (k + 1) + i];
+    if (s < n && !keep) X[(int64_t)i * ld + s] = tile[lane * (k + 1) + i];
   }
 }
 
@@ -186,9 +190,9 @@ inline int grid_for(int64_t n, int threads) {
 namespace mg {
 
 cudaError_t launch_mean_pert_members(const double* X, int64_t n, int k, int64_t ld, double* mean,
-                                     double* Xp64, float* Xp32, int64_t ldp, cudaStream_t s) {
+                                     double* Xp64, float* Xp32, int64_t ldp, cudaStream_t s, const int* skip) {
   mean_pert_members_kernel<double><<<grid_for(n, 256), 256, 0, s>>>(X, n, k, ld, 1.0 / (double)k, mean,
-                                                                   Xp64, Xp32, ldp);
+                                                                   Xp64, Xp32, ldp, skip);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -208,10 +212,10 @@ cudaError_t launch_to_point_major(const double* X, int64_t n, int k, int64_t ld,
 }
 
 cudaError_t launch_point_major_to_members(const double* P, int64_t n, int k, double* X, int64_t ld,
-                                          cudaStream_t s) {
+                                          cudaStream_t s, const int* skip) {
   const int64_t blocks = (n + kTile - 1) / kTile;
   const size_t smem = (size_t)kTile * (k + 1) * sizeof(double);
-  point_major_to_members_kernel<<<(unsigned)blocks, 256, smem, s>>>(P, n, k, X, ld);
+  point_major_to_members_kernel<<<(unsigned)blocks, 256, smem, s>>>(P, n, k, X, ld, skip);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -220,7 +224,7 @@ cudaError_t launch_point_major_to_members(const double* P, int64_t n, int k, dou
 // order), FP32 perturbations point-major, and the FP32 write-back.
 cudaError_t launch_mean_members_f32(const float* X, int64_t n, int k, int64_t ld, double* mean, cudaStream_t s) {
   mean_pert_members_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(X, n, k, ld, 1.0 / (double)k, mean, nullptr,
-                                                                  nullptr, 0);
+                                                                  nullptr, 0, nullptr);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

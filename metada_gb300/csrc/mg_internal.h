@@ -73,13 +73,15 @@ size_t scan_temp_bytes(int64_t n);
 cudaError_t exclusive_scan(const int64_t* counts, int64_t* offsets, int64_t n, void* tmp,
                            size_t tmp_bytes, cudaStream_t s);
 
-// Internal stages shared between entry points (device pointers).
+// Internal stages shared between entry points (device pointers).  skip: where
+// *skip is not zero, nothing is written.
 cudaError_t launch_mean_pert_members(const double* X, int64_t n, int k, int64_t ld, double* mean,
-                                     double* Xp64, float* Xp32, int64_t ldp, cudaStream_t s);
+                                     double* Xp64, float* Xp32, int64_t ldp, cudaStream_t s,
+                                     const int* skip = nullptr);
 cudaError_t launch_to_point_major(const double* X, int64_t n, int k, int64_t ld, double* mean,
                                   double* P64, float* P32, cudaStream_t s);
 cudaError_t launch_point_major_to_members(const double* P, int64_t n, int k, double* X,
-                                          int64_t ld, cudaStream_t s);
+                                          int64_t ld, cudaStream_t s, const int* skip = nullptr);
 // The same stages for members stored as FP32 (FP64 mean of the widened values).
 cudaError_t launch_mean_members_f32(const float* X, int64_t n, int k, int64_t ld, double* mean, cudaStream_t s);
 cudaError_t launch_to_point_major_f32(const float* X, int64_t n, int k, int64_t ld, double* mean, float* P32,

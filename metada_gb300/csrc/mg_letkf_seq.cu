@@ -30,7 +30,7 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kCh = 32;  // obs per chunk (four threads per obs in the row means)
-constexpr unsigned long long kWaitNs = 10ull * 1000 * 1000 * 1000;
+constexpr int64_t kWaitNs = 10ll * 1000 * 1000 * 1000;
 
 // Interpolation of one grid obs (IdentityObsOperator.hpp:594-676): four cells
 // and inverse-distance weights; cell[0] < 0 marks an invalid obs (H = 0).
@@ -52,6 +52,8 @@ struct SeqParams {
   int* done;
   unsigned* next;
   int* status;
+  int* gave_up;  // set where a wait did
+  unsigned long long wait_ns;
 };
 
 __global__ void obs_stencil_kernel(const int32_t* __restrict__ obs_xy, const uint8_t* __restrict__ valid, int64_t p,
@@ -107,13 +109,13 @@ __device__ __forceinline__ unsigned long long now_ns() {
 
 // Waits until the point is published; false when the time is up or another
 // CTA has given up.
-__device__ bool wait_done(const int* flag, const int* status) {
+__device__ bool wait_done(const int* flag, const int* gave_up, unsigned long long wait_ns) {
   if (ld_acquire(flag)) return true;
   const unsigned long long t0 = now_ns();
   for (;;) {
     for (int i = 0; i < 64; ++i)
       if (ld_acquire(flag)) return true;
-    if (ld_acquire(status) == 2 || now_ns() - t0 > kWaitNs) return false;
+    if (ld_acquire(gave_up) || now_ns() - t0 > wait_ns) return false;
   }
 }
 
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(kThreads) letkf_seq_kernel(SeqParams prm) {
         const int c = s.cell[tid & 3];
         const double* q = nullptr;
         if (s.cell[0] >= 0) {
-          if (c < g && !wait_done(prm.done + c, prm.status)) s_fail = 1;
+          if (c < g && !wait_done(prm.done + c, prm.gave_up, prm.wait_ns)) s_fail = 1;
           q = (c < g ? prm.Xa : prm.Xb) + (int64_t)c * k;
         }
         src[tid] = q;
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(kThreads) letkf_seq_kernel(SeqParams prm) {
       asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prm.done + g), "r"(1) : "memory");
     }
   }
-  if (s_fail && tid == 0) atomicExch(prm.status, 2);
+  if (s_fail && tid == 0) atomicExch(prm.gave_up, 1);
 }
 
 template <int KMAX>
@@ -340,11 +342,9 @@ cudaError_t launch_seq(const SeqParams& prm, int num_sms, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-}  // namespace
-
-extern "C" int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,
-                                    const int32_t* obs_xy, const uint8_t* valid, const double* yo, int64_t p,
-                                    double radius, double rho, double* mean_out) {
+int compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny, const int32_t* obs_xy,
+                const uint8_t* valid, const double* yo, int64_t p, double radius, double rho, double* mean_out,
+                int64_t wait_ns) {
   if (!ctx) return MG_ERR_ARG;
   MG_CHECK_ARG(X && k >= 2 && k <= 64 && nx > 0 && ny > 0 && ld >= (int64_t)nx * ny && p >= 0 &&
                    (p == 0 || (obs_xy && yo)) && rho > 0.0,
@@ -384,7 +384,7 @@ extern "C" int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64
     Xa = cv.take<double>((size_t)npt * k);
     st = cv.take<ObsStencil>((size_t)p + 1);
     done = cv.take<int>((size_t)npt);
-    flags = cv.take<int>(4);  // next, status
+    flags = cv.take<int>(4);  // next, status, gave up
     off = cv.take<int64_t>((size_t)npt + 1);
     idx = cv.take<int32_t>((size_t)cap);
     const int rc = mg_select_grid(ctx, nx, ny, obs_xy, p, radius, off, idx, cap, &total);
@@ -401,18 +401,41 @@ extern "C" int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64
   members_to_points_kernel<<<(unsigned)((npt + 31) / 32), 256, 0, s>>>(X, npt, k, ld, Xb);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
-  const SeqParams prm{Xb, Xa, k, (int)npt, st, yo, off, idx, rho, done, reinterpret_cast<unsigned*>(flags), flags + 1};
+  const SeqParams prm{Xb, Xa, k, (int)npt, st, yo, off, idx, rho, done, reinterpret_cast<unsigned*>(flags), flags + 1,
+                      flags + 2, (unsigned long long)wait_ns};
   if (k <= 16) MG_TRY_CUDA(launch_seq<16>(prm, ctx->num_sms, s));
   else if (k <= 32) MG_TRY_CUDA(launch_seq<32>(prm, ctx->num_sms, s));
   else MG_TRY_CUDA(launch_seq<64>(prm, ctx->num_sms, s));
-  MG_TRY_CUDA(mg::launch_point_major_to_members(Xa, npt, k, X, ld, s));
+  // A run that gave up has points without an analysis: the members and the mean stay as they are.
+  MG_TRY_CUDA(mg::launch_point_major_to_members(Xa, npt, k, X, ld, s, prm.gave_up));
   if (mean_out)
-    MG_TRY_CUDA(mg::launch_mean_pert_members(X, npt, k, ld, mean_out, nullptr, nullptr, 0, s));
-  int hs = 0;
-  MG_TRY_CUDA(cudaMemcpyAsync(&hs, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MG_TRY_CUDA(mg::launch_mean_pert_members(X, npt, k, ld, mean_out, nullptr, nullptr, 0, s, prm.gave_up));
+  int* hs = static_cast<int*>(mg::host_stage(ctx, 2 * sizeof(int)));  // pinned
+  if (!hs) return MG_ERR_NOMEM;
+  MG_TRY_CUDA(cudaMemcpyAsync(hs, flags + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   MG_TRY_CUDA(cudaStreamSynchronize(s));
-  if (hs == 2) return mg::fail(ctx, MG_ERR_TIMEOUT, "mg_letkf_compat_grid: a bounded wait for an earlier point gave up");
-  if (hs != 0)
+  if (hs[1]) return mg::fail(ctx, MG_ERR_TIMEOUT, "mg_letkf_compat_grid: a bounded wait for an earlier point gave up");
+  if (hs[0] != 0)
     return mg::fail(ctx, MG_ERR_NUMERIC, "mg_letkf_compat_grid: a local k x k system was not positive definite");
   return MG_OK;
 }
+
+}  // namespace
+
+extern "C" {
+
+int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,
+                         const int32_t* obs_xy, const uint8_t* valid, const double* yo, int64_t p, double radius,
+                         double rho, double* mean_out) {
+  return compat_grid(ctx, X, k, ld, nx, ny, obs_xy, valid, yo, p, radius, rho, mean_out, kWaitNs);
+}
+
+int mg_letkf_compat_grid_wait_selftest(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,
+                                       const int32_t* obs_xy, const uint8_t* valid, const double* yo, int64_t p,
+                                       double radius, double rho, double* mean_out, int64_t wait_ns) {
+  if (!ctx) return MG_ERR_ARG;
+  MG_CHECK_ARG(wait_ns >= 0, "mg_letkf_compat_grid_wait_selftest: wait_ns must not be negative");
+  return compat_grid(ctx, X, k, ld, nx, ny, obs_xy, valid, yo, p, radius, rho, mean_out, wait_ns);
+}
+
+}  // extern "C"
