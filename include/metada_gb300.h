@@ -151,10 +151,11 @@ int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int3
                          const double* yo, int64_t p, double radius, double rho,
                          double* mean_out);
 
-/* Self-test of that kernel's bounded waits: the same call with the time that
- * a point waits for an earlier one given (10 s there).  A run in which a wait
- * gives up returns MG_ERR_TIMEOUT and leaves X and mean_out as they were.  No
- * counterpart in the reference. */
+/* Self-test of that kernel's bounded waits: the same call with the time
+ * without a finished point after which a wait for an earlier one gives up
+ * (there 10 s and 10 us an obs).  A run in which a wait gives up returns
+ * MG_ERR_TIMEOUT and leaves X and mean_out as they were.  No counterpart in
+ * the reference. */
 int mg_letkf_compat_grid_wait_selftest(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx,
                                        int32_t ny, const int32_t* obs_xy, const uint8_t* valid,
                                        const double* yo, int64_t p, double radius, double rho,

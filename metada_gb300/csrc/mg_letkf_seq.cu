@@ -10,8 +10,10 @@
 // its cells that come before it.  CTAs take points from a counter in
 // row-major order, wait on the cells' done flags and publish their own; a
 // point's cells were taken earlier, by CTAs that are running or finished, so
-// the waits end whatever the number of CTAs (each is bounded in time as
-// well, and gives up with a status).
+// the waits end whatever the number of CTAs.  They are bounded as well: a wait
+// gives up, with a status, when no point at all has been published for a
+// time that covers the longest list (the last of the points in flight waits
+// for all the others, however long that takes).
 //
 // A point on the critical chain is latency: the Gram's entries are spread
 // over the CTA by output (packed lower triangle of A with Y'^T d as its last
@@ -30,7 +32,9 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kCh = 32;  // obs per chunk (four threads per obs in the row means)
-constexpr int64_t kWaitNs = 10ll * 1000 * 1000 * 1000;
+// Time without a published point after which a wait gives up: 10 s, and 10 us
+// an obs (a CTA takes 1.3 us at k = 64).
+constexpr int64_t kWaitNs = 10ll * 1000 * 1000 * 1000, kWaitNsPerObs = 10000;
 
 // Interpolation of one grid obs (IdentityObsOperator.hpp:594-676): four cells
 // and inverse-distance weights; cell[0] < 0 marks an invalid obs (H = 0).
@@ -108,14 +112,21 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 
 // Waits until the point is published; false when the time is up or another
-// CTA has given up.
-__device__ bool wait_done(const int* flag, const int* gave_up, unsigned long long wait_ns) {
+// CTA has given up.  A CTA that publishes a point takes the next, so the points'
+// counter moves with every published one.
+__device__ bool wait_done(const int* flag, const unsigned* next, const int* gave_up, unsigned long long wait_ns) {
   if (ld_acquire(flag)) return true;
-  const unsigned long long t0 = now_ns();
+  unsigned long long t0 = now_ns();
+  int seen = ld_acquire(reinterpret_cast<const int*>(next));
   for (;;) {
     for (int i = 0; i < 64; ++i)
       if (ld_acquire(flag)) return true;
     if (ld_acquire(gave_up) || now_ns() - t0 > wait_ns) return false;
+    const int n = ld_acquire(reinterpret_cast<const int*>(next));
+    if (n != seen) {
+      seen = n;
+      t0 = now_ns();
+    }
   }
 }
 
@@ -171,7 +182,7 @@ __global__ void __launch_bounds__(kThreads) letkf_seq_kernel(SeqParams prm) {
         const int c = s.cell[tid & 3];
         const double* q = nullptr;
         if (s.cell[0] >= 0) {
-          if (c < g && !wait_done(prm.done + c, prm.gave_up, prm.wait_ns)) s_fail = 1;
+          if (c < g && !wait_done(prm.done + c, prm.next, prm.gave_up, prm.wait_ns)) s_fail = 1;
           q = (c < g ? prm.Xa : prm.Xb) + (int64_t)c * k;
         }
         src[tid] = q;
@@ -427,7 +438,8 @@ extern "C" {
 int mg_letkf_compat_grid(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,
                          const int32_t* obs_xy, const uint8_t* valid, const double* yo, int64_t p, double radius,
                          double rho, double* mean_out) {
-  return compat_grid(ctx, X, k, ld, nx, ny, obs_xy, valid, yo, p, radius, rho, mean_out, kWaitNs);
+  return compat_grid(ctx, X, k, ld, nx, ny, obs_xy, valid, yo, p, radius, rho, mean_out,
+                     kWaitNs + kWaitNsPerObs * p);
 }
 
 int mg_letkf_compat_grid_wait_selftest(mg_context* ctx, double* X, int32_t k, int64_t ld, int32_t nx, int32_t ny,

@@ -46,3 +46,22 @@ def test_members_stay_when_a_wait_gives_up(dev, k):
     want, wmean = ob.letkf_compat_grid(X, nx, ny, xy, yo, radius, rho, None)
     assert rc == _lib.MG_OK
     assert rel_err(got, want) <= 1e-10 and rel_err(mean, wmean) <= 1e-10
+
+
+def test_a_long_chain_is_not_a_stuck_one(dev):
+    """Every point reads its neighbours and takes some 0.1 ms or more: a CTA that
+    starts with the last of the points in flight waits far beyond the limit, but
+    never for that long without another point being finished."""
+    nx, ny, k, p, radius, rho, limit_ns = 40, 16, 48, 2000, 60.0, 1.05, 10_000_000
+    X, xy, yo = _case(nx, ny, k, p, 3)
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    _run(dev, X, nx, ny, xy, yo, radius, rho, 10 ** 11)
+    t0.record()
+    rc, want, wmean = _run(dev, X, nx, ny, xy, yo, radius, rho, 10 ** 11)
+    t1.record()
+    torch.cuda.synchronize()
+    assert rc == _lib.MG_OK
+    assert t0.elapsed_time(t1) * 1e6 > 5 * limit_ns  # the whole chain: the last wait is most of it
+    rc, got, mean = _run(dev, X, nx, ny, xy, yo, radius, rho, limit_ns)
+    assert rc == _lib.MG_OK
+    assert np.array_equal(got, want) and np.array_equal(mean, wmean)
