@@ -547,6 +547,7 @@ __global__ void __launch_bounds__(Lay<KP>::kThreads, Lay<KP>::kMinBlocks) letkf_
     mma_ph ^= 1u;
     // The next analysis, by a warp that holds no rows in this phase.
     if (tid == kThreads - 1) pull(prm, s_it);
+    __syncwarp();  // tensor-memory loads of the whole warp follow
     pulled = true;
 
     // ---------------- 2. A, b, deflation and scaling ----------------

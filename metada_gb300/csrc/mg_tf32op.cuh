@@ -51,9 +51,11 @@ static __device__ __forceinline__ bool operands_ready(bool ok) {
 }
 
 // This thread waits (bounded) for the phase; what it reads or writes next is
-// in bounds either way, and operands_ready takes the CTA's decision.
+// in bounds either way, and operands_ready takes the CTA's decision.  The poll
+// runs per lane: the warp comes together before its tensor-memory loads.
 static __device__ __forceinline__ bool wait_one(uint64_t* bar, uint32_t parity) {
   const bool ok = mbar_wait(bar, parity);
+  __syncwarp();
   tc_fence_after();
   return ok;
 }
