@@ -46,7 +46,8 @@ struct mg_mlp {
   float* dA = nullptr;  // nh-wide scratch
   float* dB = nullptr;
   float* loss = nullptr;
-  float* part = nullptr;  // partial weight gradients of the split batch, all layers
+  float* part = nullptr;  // partial weight gradients of the split batch (up to part_cap rows), all layers
+  int64_t part_cap = 0;
   // BF16 activations of the tensor-core inference path, up to tc_cap rows,
   // and its error flag (a bounded wait that gave up).
   int64_t tc_cap = 0;
@@ -468,28 +469,50 @@ inline unsigned grid_for(int64_t n, int threads = kThreads) {
   return (unsigned)b;
 }
 
+// Activations for batches up to B rows.  Where an allocation fails, the handle
+// holds none and no capacity.
 int ensure_capacity(mg_context* ctx, mg_mlp* m, int64_t B) {
   if (B <= m->cap) return MG_OK;
-  float* bufs[] = {m->Z1, m->H1, m->Z2, m->H2, m->Y, m->dY, m->dA, m->dB, m->part};
-  for (float* p : bufs)
-    if (p) cudaFree(p);
-  const int64_t hw = (int64_t)B * m->nh, ow = (int64_t)B * m->nout;
-  float** targets[] = {&m->Z1, &m->H1, &m->Z2, &m->H2, &m->dA, &m->dB};
-  for (float** t : targets) {
-    if (cudaMalloc(t, sizeof(float) * hw) != cudaSuccess) {
+  const size_t hw = sizeof(float) * (size_t)B * m->nh, ow = sizeof(float) * (size_t)B * m->nout;
+  const struct {
+    float** p;
+    size_t bytes;
+  } bufs[] = {{&m->Z1, hw}, {&m->H1, hw}, {&m->Z2, hw}, {&m->H2, hw}, {&m->dA, hw}, {&m->dB, hw}, {&m->Y, ow}, {&m->dY, ow}};
+  auto release = [&] {
+    for (const auto& b : bufs) {
+      if (*b.p) cudaFree(*b.p);
+      *b.p = nullptr;
+    }
+    m->cap = 0;
+  };
+  release();
+  for (const auto& b : bufs) {
+    if (cudaMalloc(b.p, b.bytes) != cudaSuccess) {
       cudaGetLastError();
+      *b.p = nullptr;
+      release();
       return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: activation allocation failed");
     }
   }
-  const int64_t np = max_splits(m->nh, m->nin, B, ctx->num_sms) * m->oW2 +
-                     max_splits(m->nh, m->nh, B, ctx->num_sms) * (m->oW3 - m->oW2) +
-                     max_splits(m->nout, m->nh, B, ctx->num_sms) * (m->nparam - m->oW3);
-  if (cudaMalloc(&m->Y, sizeof(float) * ow) != cudaSuccess || cudaMalloc(&m->dY, sizeof(float) * ow) != cudaSuccess ||
-      cudaMalloc(&m->part, sizeof(float) * np) != cudaSuccess) {
-    cudaGetLastError();
-    return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: activation allocation failed");
-  }
   m->cap = B;
+  return MG_OK;
+}
+
+// Partial weight gradients of the batches up to B rows.
+int ensure_partials(mg_context* ctx, mg_mlp* m, int64_t B) {
+  if (B <= m->part_cap) return MG_OK;
+  if (m->part) cudaFree(m->part);
+  m->part = nullptr;
+  m->part_cap = 0;
+  const int sms = ctx->num_sms;
+  const int64_t np = max_splits(m->nh, m->nin, B, sms) * m->oW2 + max_splits(m->nh, m->nh, B, sms) * (m->oW3 - m->oW2) +
+                     max_splits(m->nout, m->nh, B, sms) * (m->nparam - m->oW3);
+  if (cudaMalloc(&m->part, sizeof(float) * np) != cudaSuccess) {
+    cudaGetLastError();
+    m->part = nullptr;
+    return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: gradient allocation failed");
+  }
+  m->part_cap = B;
   return MG_OK;
 }
 
@@ -738,7 +761,7 @@ int mg_mlp_gradients(mg_context* ctx, mg_mlp* m, const float* X, const float* Yt
   if (!ctx) return MG_ERR_ARG;
   MG_CHECK_ARG(m && X && Yt && B > 0 && B < (int64_t)1 << 31, "mg_mlp_gradients: bad arguments");
   int rc = ensure_capacity(ctx, m, B);
-  if (rc != MG_OK) return rc;
+  if (rc != MG_OK || (rc = ensure_partials(ctx, m, B)) != MG_OK) return rc;
   if ((rc = forward(ctx, m, X, B)) != MG_OK) return rc;
   if ((rc = backward(ctx, m, X, Yt, B)) != MG_OK) return rc;
   if (grad)
@@ -757,7 +780,7 @@ int mg_mlp_train_step(mg_context* ctx, mg_mlp* m, const float* X, const float* Y
   if (!ctx) return MG_ERR_ARG;
   MG_CHECK_ARG(m && X && Yt && B > 0 && lr > 0.0f, "mg_mlp_train_step: bad arguments");
   int rc = ensure_capacity(ctx, m, B);
-  if (rc != MG_OK) return rc;
+  if (rc != MG_OK || (rc = ensure_partials(ctx, m, B)) != MG_OK) return rc;
   if ((rc = forward(ctx, m, X, B)) != MG_OK) return rc;
   if ((rc = backward(ctx, m, X, Yt, B)) != MG_OK) return rc;
   m->step += 1;
