@@ -856,6 +856,13 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
 }
 
 
+constexpr int kMaxK = 112;
+constexpr size_t solve_bytes(size_t kp) {
+  return sizeof(double) * (2 * kp * (kp + 1) + 6 * kp) + sizeof(int) * (kp + 8) + 64;
+}
+constexpr size_t update_elems(size_t k) { return k * k + 32 * (k + 1); }
+static_assert(solve_bytes(kMaxK) <= 227 * 1024 && update_elems(kMaxK) * sizeof(double) <= 227 * 1024,
+              "a CTA's shared memory");
 constexpr size_t rebuild_bytes(int kmax) { return sizeof(float) * ((size_t)kmax * (kmax + 1) + 2 * 32 * (size_t)kmax); }
 
 // Enqueues the batch (no allocation, no host synchronisation: capturable).
@@ -959,11 +966,9 @@ int enqueue(mg_context* ctx, mg_etkf_batch* b) {
     batch_gram_kernel<double, 128><<<(unsigned)b->gram_cnt[2], kThreads, 0, s>>>(b->dcases, b->items + b->gram_off[2]);
     MG_COUNT_LAUNCH();
   }
-  const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
-  batch_solve_kernel<<<(unsigned)b->ncases, kThreads, smem, s>>>(b->dcases, b->order, b->flags, b->status);
+  batch_solve_kernel<<<(unsigned)b->ncases, kThreads, solve_bytes(kp), s>>>(b->dcases, b->order, b->flags, b->status);
   MG_COUNT_LAUNCH();
-  const size_t te = f64 ? 8 : 4;
-  const size_t usmem = te * ((size_t)b->maxk * b->maxk + 32 * (size_t)(b->maxk + 1));
+  const size_t usmem = (f64 ? sizeof(double) : sizeof(float)) * update_elems(b->maxk);
   if (f64)
     batch_update_kernel<double><<<(unsigned)b->n_update_items, kThreads, usmem, s>>>(b->dcases, b->items + b->update_off,
                                                                                      b->counters, b->times);
@@ -975,34 +980,28 @@ int enqueue(mg_context* ctx, mg_etkf_batch* b) {
   return MG_OK;
 }
 
+// The dynamic shared memory limit belongs to a kernel, not to a launch or a
+// plan: it is set to what the largest k needs, so that a plan of small cases
+// never lowers it under one of large cases.
 int set_attributes(mg_context* ctx, const mg_etkf_batch* b) {
-  const int kp = b->maxk + (b->maxk & 1);
-  const size_t smem = sizeof(double) * (2 * (size_t)kp * (kp + 1) + 6 * (size_t)kp) + sizeof(int) * (kp + 8) + 64;
-  const size_t te = b->precision == MG_PREC_FP64 ? 8 : 4;
-  const size_t usmem = te * ((size_t)b->maxk * b->maxk + 32 * (size_t)(b->maxk + 1));
-  if (smem > 227 * 1024 || usmem > 227 * 1024) return mg::fail(ctx, MG_ERR_ARG, "mg_etkf_batch: k too large");
-  MG_TRY_CUDA(cudaFuncSetAttribute(batch_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto limit = [](const void* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  constexpr size_t kp = kMaxK, f = sizeof(float);
   if (mixed_hunt(b)) {
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_solve1_kernel<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(float) * solve1_floats(kp))));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_solve1_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(float) * solve1_floats(kp))));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_solve2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(float) * solve2_floats(kp))));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_rebuild_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)rebuild_bytes(32)));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_rebuild_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)rebuild_bytes(64)));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_rebuild_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)rebuild_bytes(128)));
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_update_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)mg::upd_bytes(b->maxk)));
+    MG_TRY_CUDA(limit((const void*)batch_solve1_kernel<kThreads>, f * solve1_floats(kp)));
+    MG_TRY_CUDA(limit((const void*)batch_solve1_kernel<512>, f * solve1_floats(kp)));
+    MG_TRY_CUDA(limit((const void*)batch_solve2_kernel, f * solve2_floats(kp)));
+    MG_TRY_CUDA(limit((const void*)batch_rebuild_kernel<32>, rebuild_bytes(32)));
+    MG_TRY_CUDA(limit((const void*)batch_rebuild_kernel<64>, rebuild_bytes(64)));
+    MG_TRY_CUDA(limit((const void*)batch_rebuild_kernel<128>, rebuild_bytes(128)));
+    MG_TRY_CUDA(limit((const void*)batch_update_mixed_kernel, mg::upd_bytes(kMaxK)));
     return MG_OK;
   }
-  if (te == 8)
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem));
-  else
-    MG_TRY_CUDA(cudaFuncSetAttribute(batch_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem));
+  MG_TRY_CUDA(limit((const void*)batch_solve_kernel, solve_bytes(kp)));
+  MG_TRY_CUDA(b->precision == MG_PREC_FP64
+                  ? limit((const void*)batch_update_kernel<double>, update_elems(kMaxK) * sizeof(double))
+                  : limit((const void*)batch_update_kernel<float>, update_elems(kMaxK) * sizeof(float)));
   return MG_OK;
 }
 
@@ -1017,7 +1016,7 @@ int mg_etkf_batch_create(mg_context* ctx, const mg_etkf_case* cases, int32_t nca
   MG_CHECK_ARG(precision == MG_PREC_FP64 || precision == MG_PREC_MIXED, "mg_etkf_batch_create: bad precision");
   for (int i = 0; i < ncases; ++i) {
     const mg_etkf_case& c = cases[i];
-    MG_CHECK_ARG(c.X && c.n > 0 && c.ld >= c.n && c.k >= 2 && c.k <= 112 && c.p >= 1 && (c.HX || c.obs_node) &&
+    MG_CHECK_ARG(c.X && c.n > 0 && c.ld >= c.n && c.k >= 2 && c.k <= kMaxK && c.p >= 1 && (c.HX || c.obs_node) &&
                      c.yo && c.rvar && c.rho > 0.0,
                  "mg_etkf_batch_create: bad case " + std::to_string(i) + " (k must be 2..112, p >= 1)");
   }
