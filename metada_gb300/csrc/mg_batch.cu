@@ -99,11 +99,11 @@ struct mg_etkf_batch {
   void* ws = nullptr;
   size_t ws_bytes = 0;
   unsigned long long* counters = nullptr;  // per-case finished update tiles
-  unsigned long long* times = nullptr;     // [0] start, [1 + c] case finish (ns)
+  unsigned long long* times = nullptr;     // [0] start (mixed path: its complement), [1 + c] case finish (ns)
   int* status = nullptr;
   const int* order = nullptr;  // case indices, largest k first (one CTA per case kernels)
   CaseGroup grp[kGroups];
-  cudaStream_t side[kGroups - 1] = {};  // the later groups' chains
+  cudaStream_t side[kGroups - 1] = {};  // the chains beside the first group's, where there are several groups
   cudaEvent_t fork = nullptr, join[kGroups - 1] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) batch_prep_obs_mixed_kernel(const De
                                                                         unsigned long long* times) {
   const WorkItem it = items[blockIdx.x];
   const DevCase& c = cases[it.c];
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(times, globaltimer());  // the groups' first
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(times, ~globaltimer());  // the groups' first
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = c.k;
   const int64_t ob = it.a + (int64_t)warp * kObsWarp;
@@ -657,6 +657,31 @@ bool mixed_hunt(const mg_etkf_batch* b) {
   return b->precision == MG_PREC_MIXED && !(b->flags & MG_SQRT_CHOLESKY);
 }
 
+// Tile counters, the status (two words) and the start's time: one memset.
+size_t zeroed_words(const mg_etkf_batch* b) { return (size_t)b->ncases + 3; }
+
+int home_group(const mg_etkf_batch* b) {
+  int q = 0;
+  while (q < kGroups - 1 && !b->grp[q].ncases) ++q;
+  return q;
+}
+
+// Streams and events of the groups beside the first (none for a plan of one
+// group; creating a pair takes some 10 us).
+cudaError_t side_streams(mg_etkf_batch* b) {
+  int low = 0, high = 0;
+  cudaError_t e = cudaSuccess;
+  for (int q = home_group(b) + 1; q < kGroups && e == cudaSuccess; ++q) {
+    if (!b->grp[q].ncases || b->side[q - 1]) continue;
+    if (!b->fork) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&low, &high);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[q - 1], cudaEventDisableTiming);
+    if (e == cudaSuccess)
+      e = cudaStreamCreateWithPriority(&b->side[q - 1], cudaStreamNonBlocking, std::max(high, low - q));
+  }
+  return e;
+}
+
 // Builds the item tables and workspace for the current tuning.
 int build(mg_context* ctx, mg_etkf_batch* b) {
   const bool f64 = b->precision == MG_PREC_FP64;
@@ -788,9 +813,7 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
   b->n_update_items = (int64_t)up_items.size();
   cv.reserve<DevCase>(b->ncases);
   cv.reserve<WorkItem>(all.size());
-  cv.reserve<unsigned long long>(b->ncases);
-  cv.reserve<unsigned long long>(b->ncases + 1);
-  cv.reserve<int>(4);
+  cv.reserve<unsigned long long>(zeroed_words(b) + b->ncases);
   cv.reserve<int>(b->ncases);
   if (cv.off > b->ws_bytes) {
     if (b->ws) cudaFree(b->ws);
@@ -831,9 +854,9 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
   }
   b->dcases = cv.take<DevCase>(b->ncases);
   b->items = cv.take<WorkItem>(all.size());
-  b->counters = cv.take<unsigned long long>(b->ncases);
-  b->times = cv.take<unsigned long long>(b->ncases + 1);
-  b->status = cv.take<int>(4);
+  b->counters = cv.take<unsigned long long>(zeroed_words(b) + b->ncases);
+  b->status = reinterpret_cast<int*>(b->counters + b->ncases);
+  b->times = b->counters + b->ncases + 2;
   int* order = cv.take<int>(b->ncases);
   b->order = order;
   std::vector<int> ord(b->ncases);
@@ -844,6 +867,7 @@ int build(mg_context* ctx, mg_etkf_batch* b) {
   MG_TRY_CUDA(cudaMemcpy(b->dcases, dc.data(), sizeof(DevCase) * dc.size(), cudaMemcpyHostToDevice));
   MG_TRY_CUDA(cudaMemcpy(b->items, all.data(), sizeof(WorkItem) * all.size(), cudaMemcpyHostToDevice));
   MG_TRY_CUDA(cudaMemcpy(order, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
+  MG_TRY_CUDA(side_streams(b));
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
@@ -921,8 +945,7 @@ int enqueue_group(mg_context* ctx, mg_etkf_batch* b, int gi, cudaStream_t s) {
 int enqueue(mg_context* ctx, mg_etkf_batch* b) {
   cudaStream_t s = ctx->stream;
   const bool f64 = b->precision == MG_PREC_FP64;
-  MG_TRY_CUDA(cudaMemsetAsync(b->counters, 0, sizeof(unsigned long long) * b->ncases, s));
-  MG_TRY_CUDA(cudaMemsetAsync(b->status, 0, sizeof(int) * 4, s));
+  MG_TRY_CUDA(cudaMemsetAsync(b->counters, 0, sizeof(unsigned long long) * zeroed_words(b), s));
   if (b->n_state_items) {
     if (f64)
       batch_prep_state_kernel<double><<<(unsigned)b->n_state_items, kStateTile, 0, s>>>(b->dcases, b->items + b->state_off, b->times);
@@ -931,22 +954,26 @@ int enqueue(mg_context* ctx, mg_etkf_batch* b) {
     MG_COUNT_LAUNCH();
   }
   if (mixed_hunt(b)) {
-    MG_TRY_CUDA(cudaMemsetAsync(b->times, 0xff, sizeof(unsigned long long), s));
     // The largest cases' chain is the longest: it goes first, on the stream of
     // the highest priority.  The first group there is stays on this stream.
-    int home = 0;
-    while (!b->grp[home].ncases) ++home;
-    MG_TRY_CUDA(cudaEventRecord(b->fork, s));
+    // Whatever fails, a stream that was forked is joined.
+    const int home = home_group(b);
     int rc = MG_OK;
+    if (b->fork) MG_TRY_CUDA(cudaEventRecord(b->fork, s));
+    bool forked[kGroups] = {};
+    auto ok = [&](cudaError_t e) {
+      if (e != cudaSuccess && rc == MG_OK)
+        rc = mg::fail(ctx, MG_ERR_CUDA, std::string("mg_etkf_batch: ") + cudaGetErrorString(e));
+      return e == cudaSuccess;
+    };
     for (int q = kGroups - 1; q > home && rc == MG_OK; --q) {
-      if (!b->grp[q].ncases) continue;
-      MG_TRY_CUDA(cudaStreamWaitEvent(b->side[q - 1], b->fork, 0));
+      if (!b->grp[q].ncases || !ok(cudaStreamWaitEvent(b->side[q - 1], b->fork, 0))) continue;
+      forked[q] = true;
       rc = enqueue_group(ctx, b, q, b->side[q - 1]);
-      MG_TRY_CUDA(cudaEventRecord(b->join[q - 1], b->side[q - 1]));
     }
     if (rc == MG_OK) rc = enqueue_group(ctx, b, home, s);
     for (int q = kGroups - 1; q > home; --q)
-      if (b->grp[q].ncases) MG_TRY_CUDA(cudaStreamWaitEvent(s, b->join[q - 1], 0));
+      if (forked[q] && ok(cudaEventRecord(b->join[q - 1], b->side[q - 1]))) ok(cudaStreamWaitEvent(s, b->join[q - 1], 0));
     return rc;
   }
   if (b->n_obs_items) {
@@ -1026,21 +1053,7 @@ int mg_etkf_batch_create(mg_context* ctx, const mg_etkf_case* cases, int32_t nca
   b->precision = precision;
   b->host_cases.assign(cases, cases + ncases);
   int rc = build(ctx, b.get());
-  if (rc != MG_OK) return rc;
-  if (mixed_hunt(b.get())) {
-    int low = 0, high = 0;
-    cudaError_t e = cudaDeviceGetStreamPriorityRange(&low, &high);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-    for (int q = 0; q < kGroups - 1 && e == cudaSuccess; ++q) {
-      e = cudaStreamCreateWithPriority(&b->side[q], cudaStreamNonBlocking, std::max(high, low - 1 - q));
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming);
-    }
-    if (e != cudaSuccess) {
-      mg_etkf_batch_destroy(b.release());
-      return mg::fail(ctx, MG_ERR_CUDA, std::string("mg_etkf_batch_create: ") + cudaGetErrorString(e));
-    }
-  }
-  rc = set_attributes(ctx, b.get());
+  if (rc == MG_OK) rc = set_attributes(ctx, b.get());
   if (rc != MG_OK) {
     mg_etkf_batch_destroy(b.release());
     return rc;
@@ -1105,6 +1118,7 @@ int mg_etkf_batch_finish(mg_context* ctx, mg_etkf_batch* b, double* case_ms) {
     MG_TRY_CUDA(cudaMemcpyAsync(t.data(), b->times, sizeof(unsigned long long) * t.size(), cudaMemcpyDeviceToHost,
                                 ctx->stream));
   MG_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (case_ms && mixed_hunt(b)) t[0] = ~t[0];
   if (case_ms)
     for (int i = 0; i < b->ncases; ++i) case_ms[i] = (double)(t[1 + i] - t[0]) * 1e-6;
   if (st) return mg::fail(ctx, MG_ERR_NUMERIC, "mg_etkf_batch: case " + std::to_string(st - 1) +
