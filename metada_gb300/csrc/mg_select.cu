@@ -210,11 +210,11 @@ struct CellObs {
   double2* half;  // two per obs
 };
 
-// Obs into their cells (positions from the cell starts).
-__global__ void cell_scatter_kernel(const double* __restrict__ lat, const double* __restrict__ lon,
-                                    int64_t p, const int64_t* __restrict__ start,
-                                    unsigned long long* __restrict__ cursor, CellObs co) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+// Obs into their cells (positions from the cell starts), by the first `blocks` CTAs.
+__device__ __forceinline__ void cell_scatter(const double* __restrict__ lat, const double* __restrict__ lon,
+                                             int64_t p, const int64_t* __restrict__ start,
+                                             unsigned long long* __restrict__ cursor, const CellObs& co, int blocks) {
+  const int64_t stride = (int64_t)blocks * blockDim.x;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p; o += stride) {
     const int c = cell_of(lat[o], lon[o]);
     const int64_t pos = start[c] + (int64_t)atomicAdd(&cursor[c], 1ull);
@@ -273,11 +273,21 @@ struct GeoPlan {
 };
 constexpr uint32_t kNoWindow = 0xffffffffu;
 
-// Four threads per column, each every fourth band.
-__global__ void __launch_bounds__(256) geo_plan_kernel(const double* __restrict__ col_lat,
-                                                       const double* __restrict__ col_lon, int64_t ncol,
-                                                       const __grid_constant__ GeoRule g, GeoPlan pl) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The scatter and, by the CTAs after its own, the columns' plans (in a launch
+// of their own a small search took one launch more than it has to): four
+// threads per column, each every fourth band.
+__global__ void __launch_bounds__(256) scatter_plan_kernel(const double* __restrict__ obs_lat,
+                                                           const double* __restrict__ obs_lon, int64_t p,
+                                                           const int64_t* __restrict__ start,
+                                                           unsigned long long* __restrict__ cursor, CellObs co,
+                                                           int scatter_blocks, const double* __restrict__ col_lat,
+                                                           const double* __restrict__ col_lon, int64_t ncol,
+                                                           const __grid_constant__ GeoRule g, GeoPlan pl) {
+  if ((int)blockIdx.x < scatter_blocks) {
+    cell_scatter(obs_lat, obs_lon, p, start, cursor, co, scatter_blocks);
+    return;
+  }
+  const int64_t t = (int64_t)((int)blockIdx.x - scatter_blocks) * blockDim.x + threadIdx.x;
   const int64_t col = t >> 2;
   const int q = (int)(t & 3);
   if (col >= ncol) return;
@@ -750,21 +760,20 @@ int mg_select_geo(mg_context* ctx, const double* col_lat, const double* col_lon,
   MG_TRY_CUDA(cudaMemsetAsync(nborder, 0, sizeof(unsigned long long) * 2, s));
   MG_TRY_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int) * 2, s));
   MG_TRY_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * (ncol + 1), s));
+  const unsigned gb = (unsigned)std::min<int64_t>((p + 255) / 256, 152 * 16);
   if (p > 0) {
-    const unsigned gb = (unsigned)std::min<int64_t>((p + 255) / 256, 152 * 16);
     cell_count_kernel<<<gb, 256, 0, s>>>(obs_lat, obs_lon, p, ccount);
     MG_COUNT_LAUNCH();
     MG_TRY_CUDA(cudaGetLastError());
     MG_TRY_CUDA(mg::exclusive_scan(reinterpret_cast<const int64_t*>(ccount), cstart, kNCell, tmp,
                                    tmpb, s));
-    cell_scatter_kernel<<<gb, 256, 0, s>>>(obs_lat, obs_lon, p, cstart, ccursor, co);
-    MG_COUNT_LAUNCH();
-    MG_TRY_CUDA(cudaGetLastError());
   } else {
     MG_TRY_CUDA(cudaMemsetAsync(cstart, 0, sizeof(int64_t) * (kNCell + 1), s));
   }
   // Pass 1: counts (near-threshold pairs counted and recorded).
-  geo_plan_kernel<<<(unsigned)((4 * ncol + 255) / 256), 256, 0, s>>>(col_lat, col_lon, ncol, rule, plan);
+  scatter_plan_kernel<<<gb + (unsigned)((4 * ncol + 255) / 256), 256, 0, s>>>(obs_lat, obs_lon, p, cstart, ccursor, co,
+                                                                              (int)gb, col_lat, col_lon, ncol, rule,
+                                                                              plan);
   MG_COUNT_LAUNCH();
   MG_TRY_CUDA(cudaGetLastError());
   geo_count_kernel<<<(unsigned)ncol, 256, 0, s>>>(col_lat, col_lon, rule, plan, cstart, co, obs_lat, obs_lon, counts,
