@@ -14,8 +14,8 @@
 // GB300 runs two FP64 lanes per clock per SM, so a warp instruction takes
 // its scheduler's FP64 unit 64 cycles, whatever the lanes hold: the kernel is
 // laid out for few FP64 warp instructions and no idle lanes.  One analysis
-// belongs to a group of one warp (k <= 32) or four warps (k <= 96), its
-// threads a TI x TJ grid of interleaved register tiles of A's lower triangle
+// belongs to a group of one warp (k <= 32) or four warps (k <= 96, and fewer
+// members where the points are few), its threads a TI x TJ grid of interleaved register tiles of A's lower triangle
 // (tiles above the diagonal are not formed), several groups per SM covering
 // each other's latencies.  The root-free factorisation needs one reciprocal
 // per column, from an FP32 seed and one third-order Newton step (three FP64
@@ -36,9 +36,8 @@ using mg::gaspari_cohn;
 
 constexpr int kThreads = 128;
 
-template <int KMAX>
+template <int KMAX, int NW>  // NW: warps per analysis
 struct Cfg {
-  static constexpr int NW = KMAX <= 32 ? 1 : 4;       // warps per analysis
   static constexpr int TI = NW == 1 ? 8 : 16, TJ = TI / 2;  // thread grid
   static constexpr int RA = KMAX / TI;                 // tile rows; tile columns of row a: 2 (a + 1)
   static constexpr int NT = RA * (RA + 1);             // tiles of the lower triangle
@@ -53,10 +52,10 @@ struct Cfg {
   static constexpr size_t BYTES = GROUPS * (sizeof(double) * DOUBLES + sizeof(int) * (SEL + 8));
 };
 
-template <int KMAX>
+template <int KMAX, int NW>
 __global__ void __launch_bounds__(kThreads, KMAX <= 64 ? 5 : 2) letkf_chol_kernel(LetkfParams prm) {
-  using C = Cfg<KMAX>;
-  constexpr int NW = C::NW, TI = C::TI, TJ = C::TJ, RA = C::RA, NV = C::NV, LDS = C::LDS, SEL = C::SEL, CH = C::CH;
+  using C = Cfg<KMAX, NW>;
+  constexpr int TI = C::TI, TJ = C::TJ, RA = C::RA, NV = C::NV, LDS = C::LDS, SEL = C::SEL, CH = C::CH;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   const int gid = threadIdx.x / (32 * NW);          // group in the CTA
@@ -360,17 +359,17 @@ __global__ void __launch_bounds__(kThreads, KMAX <= 64 ? 5 : 2) letkf_chol_kerne
   }
 }
 
-template <int KMAX>
+template <int KMAX, int NW>
 cudaError_t launch(const LetkfParams& prm, int num_sms, cudaStream_t s) {
-  const size_t smem = Cfg<KMAX>::BYTES;
-  cudaError_t e = cudaFuncSetAttribute(letkf_chol_kernel<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = Cfg<KMAX, NW>::BYTES;
+  cudaError_t e = cudaFuncSetAttribute(letkf_chol_kernel<KMAX, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, letkf_chol_kernel<KMAX>, kThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, letkf_chol_kernel<KMAX, NW>, kThreads, smem);
   if (e != cudaSuccess) return e;
-  const int64_t want = (prm.npoints + Cfg<KMAX>::GROUPS - 1) / Cfg<KMAX>::GROUPS;
+  const int64_t want = (prm.npoints + Cfg<KMAX, NW>::GROUPS - 1) / Cfg<KMAX, NW>::GROUPS;
   const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)std::max(per_sm, 1) * num_sms, want));
-  letkf_chol_kernel<KMAX><<<(unsigned)grid, kThreads, smem, s>>>(prm);
+  letkf_chol_kernel<KMAX, NW><<<(unsigned)grid, kThreads, smem, s>>>(prm);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -380,10 +379,18 @@ cudaError_t launch(const LetkfParams& prm, int num_sms, cudaStream_t s) {
 namespace mg {
 
 cudaError_t letkf_chol_launch(const LetkfParams& prm, int num_sms, cudaStream_t s) {
-  if (prm.k <= 16) return launch<16>(prm, num_sms, s);
-  if (prm.k <= 32) return launch<32>(prm, num_sms, s);
-  if (prm.k <= 64) return launch<64>(prm, num_sms, s);
-  return launch<96>(prm, num_sms, s);
+  // Up to two points per SM, four warps an analysis: with one, a point has a
+  // single scheduler and the others idle (304 points, k = 20, 3000 local obs:
+  // 2901 us by one warp, 1552 by four; 28 local obs 53 and 36).  From three per
+  // SM the idle lanes of the wider grid cost more than they bring where the
+  // lists are short (456 points, k = 9, 4 local obs: 15.8 and 17.9 us; 608 points,
+  // 28 local obs: 26 and 28), and more points always favour one warp (5000 points,
+  // k = 32, 28 local obs: 337 and 458 us).
+  const bool few = prm.npoints <= 2 * num_sms;
+  if (prm.k <= 16) return few ? launch<16, 4>(prm, num_sms, s) : launch<16, 1>(prm, num_sms, s);
+  if (prm.k <= 32) return few ? launch<32, 4>(prm, num_sms, s) : launch<32, 1>(prm, num_sms, s);
+  if (prm.k <= 64) return launch<64, 4>(prm, num_sms, s);
+  return launch<96, 4>(prm, num_sms, s);
 }
 
 }  // namespace mg
