@@ -25,12 +25,16 @@
 // (100 members that span 25 directions well observed: condition number 300).
 // A2 is graded by then, and Jacobi on a graded matrix is accurate relative to
 // sqrt(d_i d_j): a second pass rotates V on by an FP32 Jacobi of A2 and goes
-// back to step 2, where the caller can supply A once more (the global
-// analyses).  What is left (or not SPD) goes to the caller's FP64 Jacobi.
+// back to step 2 with A as the caller kept it.  What is left (or not SPD) goes
+// to the caller's FP64 Jacobi.  Two passes end at condition numbers of about a
+// million (kHuntMaxCond), as V has FP32 entries: its rounding puts about
+// eps32 / 2 sqrt(condition number) into E between the ends of the spectrum.  The
+// smallest eigenvalue is known, the prior term's (the mean of the members has
+// no obs-space anomaly), and ||A||_F^2 / trace A is a bound of the largest from
+// below, so that most systems beyond go back before the first rotation.
 #pragma once
 
 #include <cstddef>
-#include <type_traits>
 
 #include "mg_dense.cuh"
 #include "mg_fp64.cuh"
@@ -40,6 +44,9 @@ namespace mg {
 constexpr int kHuntThreads = 256;
 constexpr float kHuntTol = 1e-5f;   // FP32 Jacobi: off-diagonal threshold relative to sqrt(a_pp a_qq)
 constexpr float kHuntGate = 3e-5f;  // largest |E_ij| / sqrt(d_i d_j) accepted
+// Condition numbers beyond are not tried (k = 16 .. 100: 1.1e6 passes, 1.5e6
+// does not; one pass costs a fifteenth of the FP64 Jacobi, the second as much).
+constexpr float kHuntMaxCond = 1.2e6f;
 
 // float -> double by integer operations (conversions run on the FP64 unit);
 // FP32 subnormals become zero.
@@ -59,6 +66,15 @@ __device__ __forceinline__ float leading(const double* p) {
 }
 
 __device__ __forceinline__ int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
+
+// The second pass's rotations out of line: inline they take registers from the
+// rest of the local kernel (96 members, no second pass: 2.4 % slower) and of
+// the global one at 112 slots (2342 against 2320 us), but not at 64 (686
+// against 696 us).
+template <int KP>
+__device__ __noinline__ int jacobi_on(float* A, int lda, float* V, int ldv, int kp, float4* rot) {
+  return cta_jacobi_ahead<KP, kHuntThreads, true>(A, lda, V, ldv, kp, kHuntTol, 20, rot);
+}
 
 template <int KP>
 struct Hunt {
@@ -139,11 +155,10 @@ struct Hunt {
   }
 
   // A <- Ws with A^-1/2 = scale V Ws V^T.  False: left to the caller (A is
-  // destroyed).  All threads; ends synchronised.  reload() fills A as on entry
-  // for the second pass; nullptr: no second pass.
-  template <typename Reload>
-  __device__ bool transform(int k, double* scale, int* sweeps, Reload reload) {
-    constexpr bool kTwice = !std::is_same<Reload, std::nullptr_t>::value;
+  // destroyed).  All threads; ends synchronised.  prior: the multiple of I in
+  // A; reload() fills A as on entry for the second pass.
+  template <bool kInline, typename Reload>
+  __device__ bool transform(int k, double prior, double* scale, int* sweeps, Reload reload) {
     const int tid = threadIdx.x, ti = tid / 16, tj = tid % 16;
     const int kp = k + (k & 1);
     // ---- scale, FP32 copy, FP32 Jacobi ----
@@ -162,13 +177,31 @@ struct Hunt {
     *scale = __hiloint2double((1023 - e2 / 2) << 20, 0);
     for (int e = tid; e < KP * LDA; e += kHuntThreads) A32[e] = 0.0f;
     __syncthreads();
+    float fro = 0.0f, tr = 0.0f;
     lower(ti, tj, k, [&](int, int i, int j) {
       const double a = A[tri(i, j)] * down;
       A[tri(i, j)] = a;
-      A32[j * LDA + i] = (float)a;
+      const float f = (float)a;
+      A32[j * LDA + i] = f;
+      fro += (i == j ? 1.0f : 2.0f) * f * f;
+      tr += i == j ? f : 0.0f;
     });
     if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      fro += __shfl_xor_sync(0xffffffffu, fro, off);
+      tr += __shfl_xor_sync(0xffffffffu, tr, off);
+    }
+    if ((tid & 31) == 0) rot[tid >> 5] = make_float4(fro, tr, 0.0f, 0.0f);
     __syncthreads();
+    const float most = kHuntMaxCond * (float)(prior * down);  // largest eigenvalue, scaled
+    fro = tr = 0.0f;
+#pragma unroll
+    for (int q = 0; q < kHuntThreads / 32; ++q) {
+      fro += rot[q].x;
+      tr += rot[q].y;
+    }
+    if (fro > most * tr) return false;
     *sweeps = cta_jacobi_ahead<KP, kHuntThreads>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
     __syncthreads();
     double w[NL];
@@ -354,21 +387,22 @@ struct Hunt {
       __syncthreads();
       if (flag[0]) return false;
       if (!flag[1]) break;
-      if constexpr (kTwice) {
-        if (pass > 0) return false;
-        for (int e = tid; e < KP * LDA; e += kHuntThreads) A32[e] = 0.0f;
-        __syncthreads();
-        lower(ti, tj, k, [&](int, int i, int j) { A32[j * LDA + i] = (float)A[tri(i, j)]; });
-        if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
-        __syncthreads();
-        *sweeps += cta_jacobi_ahead<KP, kHuntThreads, true>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
-        reload();
-        __syncthreads();
-        lower(ti, tj, k, [&](int, int i, int j) { A[tri(i, j)] *= down; });
-        __syncthreads();
-      } else {
-        return false;
-      }
+      if (pass > 0) return false;
+      float top = 0.0f;
+      for (int i = 0; i < k; ++i) top = fmaxf(top, leading(d + i));
+      if (top > most) return false;
+      for (int e = tid; e < KP * LDA; e += kHuntThreads) A32[e] = 0.0f;
+      __syncthreads();
+      lower(ti, tj, k, [&](int, int i, int j) { A32[j * LDA + i] = (float)A[tri(i, j)]; });
+      if (tid == 0 && kp > k) A32[k * LDA + k] = 1.0f;
+      __syncthreads();
+      if constexpr (kInline) *sweeps += cta_jacobi_ahead<KP, kHuntThreads, true>(A32, LDA, V, LDV, kp, kHuntTol, 20, rot);
+      else *sweeps += jacobi_on<KP>(A32, LDA, V, LDV, kp, rot);
+      __syncthreads();
+      reload();
+      __syncthreads();
+      lower(ti, tj, k, [&](int, int i, int j) { A[tri(i, j)] *= down; });
+      __syncthreads();
     }
     float* T1 = reinterpret_cast<float*>(blk);
 #pragma unroll 1

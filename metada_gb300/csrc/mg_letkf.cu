@@ -752,6 +752,9 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   cv.reserve<int32_t>(bucket ? (size_t)d->ncol * (d->nlev + 1) : 1);       // bucket starts
   cv.reserve<int32_t>(bucket ? (size_t)n_entries + 1 : 1);                 // sorted obs indices
   cv.reserve<double>(bucket && d->loc_dist ? (size_t)n_entries + 1 : 1);   // sorted distances
+  const bool hunt64 = fp64 && !(d->flags & (MG_SQRT_CHOLESKY | MG_WARM_START));
+  const size_t hunt_doubles = hunt64 ? mg::letkf_hunt_doubles(k, ctx->num_sms) : 1;
+  cv.reserve<double>(hunt_doubles);                                        // systems of the CTAs at work
   void* ws = mg::workspace(ctx, cv.off);
   if (!ws) return MG_ERR_NOMEM;
   cv = mg::Carver{static_cast<char*>(ws), 0};
@@ -769,6 +772,7 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   int32_t* lev_boff = cv.take<int32_t>(bucket ? (size_t)d->ncol * (d->nlev + 1) : 1);
   int32_t* bidx = cv.take<int32_t>(bucket ? (size_t)n_entries + 1 : 1);
   double* bdist = cv.take<double>(bucket && d->loc_dist ? (size_t)n_entries + 1 : 1);
+  double* gram = cv.take<double>(hunt_doubles);
   cudaStream_t s = ctx->stream;
 
   MG_TRY_CUDA(cudaEventRecord(ctx->ev[0], s));
@@ -824,6 +828,7 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   prm.tol = fp64 ? 1e-14 : 1e-6;
   prm.sweep_cap = fp64 ? 30 : 20;
   prm.warm_start = (d->flags & MG_WARM_START) ? 1 : 0;
+  prm.gram = gram;
   prm.redo_out = redo;
   prm.n_redo = cnt + 6;
   prm.max_resid_bits = reinterpret_cast<unsigned*>(cnt + 7);
@@ -833,7 +838,6 @@ int mg_letkf_batched(mg_context* ctx, const mg_letkf_desc* d) {
   const bool tensor = !fp64 && !(d->flags & MG_SOLVE_SIMT) && mg::letkf_tc_supported(prm);
   int64_t n_fallback = 0;
   int tc_ctas = 0;
-  const bool hunt64 = fp64 && !(d->flags & MG_SQRT_CHOLESKY) && !prm.warm_start;
   if (tensor) {
     // Tensor-core local analyses; the few whose residual test fails are
     // re-run by the SIMT kernel over the list the first kernel wrote.

@@ -38,6 +38,7 @@ struct LetkfParams {
   double tol;
   int sweep_cap;
   int warm_start;  // levels of a column run in sequence, each Jacobi warm-started
+  double* gram;  // FP64 symmetric square root: letkf_hunt_doubles, a system per CTA
   // Tensor-core path: analyses it hands back (points col * nlev + lev) and
   // their count; the largest first-order residual seen (float bits).
   int32_t* redo_out;
@@ -105,5 +106,6 @@ cudaError_t letkf_chol_launch(const LetkfParams& prm, int num_sms, cudaStream_t 
 // FP64 local analyses with the symmetric square root, k <= 96; points that
 // it leaves to the FP64 Jacobi go to prm.redo_out / n_redo.
 cudaError_t letkf_hunt_launch(const LetkfParams& prm, int num_sms, cudaStream_t s);
+size_t letkf_hunt_doubles(int k, int num_sms);
 
 }  // namespace mg

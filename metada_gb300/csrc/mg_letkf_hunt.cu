@@ -6,9 +6,10 @@
 // in FP64 (the oracle's operation order), the whitened rows of Y' are
 // gathered 32 at a time and Y'^T R^-1 Y' and Y'^T R^-1 d accumulated on the
 // tensor cores by exact splitting (mg_ozaki.cuh), and the inverse square root
-// comes from an FP32 eigenbasis corrected in FP64 (mg_hunt.cuh).  A point
-// whose correction does not apply is handed back (redo list) to the FP64
-// Jacobi kernel.  What bounds it: the FP32 Jacobi's shared-memory rounds and
+// comes from an FP32 eigenbasis corrected in FP64 (mg_hunt.cuh), in a second
+// pass where the system is graded (the CTA keeps it in global memory for that).
+// A point whose correction does not apply is handed back (redo list) to the
+// FP64 Jacobi kernel.  What bounds it: the FP32 Jacobi's shared-memory rounds and
 // the 2.3 k^3 FP64 multiply-adds of the correction, which CTAs of one SM
 // overlap (three at k <= 64).  60 x 30 x 10 points, k = 64, about 290 local
 // obs: 782 ms with the FP64 Jacobi (ten sweeps on the FP64 units) -> 56 ms.
@@ -284,9 +285,14 @@ __global__ void __launch_bounds__(kThreads, Cfg<KP>::CTAS) letkf_hunt_kernel(Let
       }
     }
     __syncthreads();
+    const int npack = k * (k + 1) / 2;
+    for (int e = tid; e < npack; e += kThreads) prm.gram[(size_t)blockIdx.x * H::PACKED + e] = h.A[e];
     double scale;
     int sweeps = 0;
-    if (!h.transform(k, &scale, &sweeps, nullptr)) {
+    auto reload = [&] {  // each thread what it wrote
+      for (int e = tid; e < npack; e += kThreads) h.A[e] = prm.gram[(size_t)blockIdx.x * H::PACKED + e];
+    };
+    if (!h.template transform<false>(k, diag, &scale, &sweeps, reload)) {
       if (tid == 0) prm.redo_out[atomicAdd(prm.n_redo, 1ull)] = (int32_t)(col * prm.nlev + lev);
       __syncthreads();
       continue;
@@ -378,7 +384,8 @@ cudaError_t launch(const LetkfParams& prm, int num_sms, cudaStream_t s) {
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, letkf_hunt_kernel<KP>, kThreads, smem);
   if (e != cudaSuccess) return e;
-  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)std::max(per_sm, 1) * num_sms, prm.npoints));
+  per_sm = std::max(1, std::min(per_sm, Cfg<KP>::CTAS));  // prm.gram has a system for each
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * num_sms, prm.npoints));
   letkf_hunt_kernel<KP><<<(unsigned)grid, kThreads, smem, s>>>(prm);
   MG_COUNT_LAUNCH();
   return cudaGetLastError();
@@ -408,7 +415,7 @@ __global__ void __launch_bounds__(kThreads) hunt_factor_kernel(const double* __r
   __syncthreads();
   double scale = 0.0;
   int sweeps = 0;
-  const bool ok = h.transform(k, &scale, &sweeps, load);
+  const bool ok = h.template transform<(KP <= 64)>(k, diag, &scale, &sweeps, load);
   if (tid == 0) info[0] = ok ? scale : 0.0;
   if (!ok) return;
   for (int e = tid; e < k * H::LDV; e += kThreads) Vout[e] = h.V[e];
@@ -486,6 +493,12 @@ cudaError_t letkf_hunt_launch(const LetkfParams& prm, int num_sms, cudaStream_t 
   if (prm.k <= 32) return launch<32>(prm, num_sms, s);
   if (prm.k <= 64) return launch<64>(prm, num_sms, s);
   return launch<96>(prm, num_sms, s);
+}
+
+size_t letkf_hunt_doubles(int k, int num_sms) {
+  const size_t per_sm = k <= 32 ? Cfg<32>::CTAS * Hunt<32>::PACKED
+                                : (k <= 64 ? Cfg<64>::CTAS * Hunt<64>::PACKED : Cfg<96>::CTAS * Hunt<96>::PACKED);
+  return per_sm * num_sms;
 }
 
 size_t hunt_global_bytes(int k) {
