@@ -13,9 +13,10 @@
 // and weighted (Gaspari-Cohn x 1/sigma^2, or 1 for the reference's R = I),
 // the local rows of Y' are gathered chunk by chunk into shared memory and
 // the k x k Gram Y'^T R^-1 Y' accumulated in a 16 x 16 grid of register
-// tiles; the k x k transform comes from a Cholesky path (reference) or the
-// parallel Jacobi eigen-solver (Hunt), and the update is applied to every
-// variable of the point.
+// tiles; the k x k transform comes from a Cholesky path (reference, FP32) or
+// the parallel Jacobi eigen-solver (Hunt), and the update is applied to every
+// variable of the point.  FP64 points come here with MG_WARM_START, and those
+// that mg_letkf_hunt.cu hands back.
 //
 // TE is the arithmetic type of the Gram, eigen-solve and update: double for
 // the FP64 path, float for the mixed path (means, innovations and outputs
@@ -180,7 +181,8 @@ __global__ void __launch_bounds__(kThreads, (sizeof(TE) == 4 && KMAX <= 64) ? 4 
   const int k = prm.k, kp = prm.kp;
   const TE* Xp = static_cast<const TE*>(prm.Xp);
   const int ti = tid / 16, tj = tid % 16;
-  const bool use_chol = prm.flags & MG_SQRT_CHOLESKY;
+  // FP64 analyses with the Cholesky root have a kernel of their own (mg_letkf_chol.cu).
+  const bool use_chol = sizeof(TE) == 4 && (prm.flags & MG_SQRT_CHOLESKY);
   const bool infl_compat = prm.flags & MG_INFL_COMPAT;
   const bool upd_compat = prm.flags & MG_UPDATE_COMPAT;
   const bool rtps = prm.flags & MG_RTPS;
