@@ -46,8 +46,7 @@ struct mg_mlp {
   float* dA = nullptr;  // nh-wide scratch
   float* dB = nullptr;
   float* loss = nullptr;
-  float* part = nullptr;  // partial weight gradients of the split batch (up to part_cap rows), all layers
-  int64_t part_cap = 0;
+  float* part = nullptr;  // partial weight gradients of the split batch, all layers
   // BF16 activations of the tensor-core inference path, up to tc_cap rows,
   // and its error flag (a bounded wait that gave up).
   int64_t tc_cap = 0;
@@ -469,15 +468,21 @@ inline unsigned grid_for(int64_t n, int threads = kThreads) {
   return (unsigned)b;
 }
 
-// Activations for batches up to B rows.  Where an allocation fails, the handle
-// holds none and no capacity.
+// Buffers for batches up to B rows, those of the gradients included, so that a
+// call of one kind makes room for the other (a training step may be captured
+// after a forward pass).  Where an allocation fails, the handle holds none and
+// no capacity.
 int ensure_capacity(mg_context* ctx, mg_mlp* m, int64_t B) {
   if (B <= m->cap) return MG_OK;
   const size_t hw = sizeof(float) * (size_t)B * m->nh, ow = sizeof(float) * (size_t)B * m->nout;
+  const int sms = ctx->num_sms;
+  const int64_t np = max_splits(m->nh, m->nin, B, sms) * m->oW2 + max_splits(m->nh, m->nh, B, sms) * (m->oW3 - m->oW2) +
+                     max_splits(m->nout, m->nh, B, sms) * (m->nparam - m->oW3);
   const struct {
     float** p;
     size_t bytes;
-  } bufs[] = {{&m->Z1, hw}, {&m->H1, hw}, {&m->Z2, hw}, {&m->H2, hw}, {&m->dA, hw}, {&m->dB, hw}, {&m->Y, ow}, {&m->dY, ow}};
+  } bufs[] = {{&m->Z1, hw}, {&m->H1, hw}, {&m->Z2, hw}, {&m->H2, hw},          {&m->dA, hw},
+              {&m->dB, hw}, {&m->Y, ow},  {&m->dY, ow}, {&m->part, sizeof(float) * np}};
   auto release = [&] {
     for (const auto& b : bufs) {
       if (*b.p) cudaFree(*b.p);
@@ -495,24 +500,6 @@ int ensure_capacity(mg_context* ctx, mg_mlp* m, int64_t B) {
     }
   }
   m->cap = B;
-  return MG_OK;
-}
-
-// Partial weight gradients of the batches up to B rows.
-int ensure_partials(mg_context* ctx, mg_mlp* m, int64_t B) {
-  if (B <= m->part_cap) return MG_OK;
-  if (m->part) cudaFree(m->part);
-  m->part = nullptr;
-  m->part_cap = 0;
-  const int sms = ctx->num_sms;
-  const int64_t np = max_splits(m->nh, m->nin, B, sms) * m->oW2 + max_splits(m->nh, m->nh, B, sms) * (m->oW3 - m->oW2) +
-                     max_splits(m->nout, m->nh, B, sms) * (m->nparam - m->oW3);
-  if (cudaMalloc(&m->part, sizeof(float) * np) != cudaSuccess) {
-    cudaGetLastError();
-    m->part = nullptr;
-    return mg::fail(ctx, MG_ERR_NOMEM, "mg_mlp: gradient allocation failed");
-  }
-  m->part_cap = B;
   return MG_OK;
 }
 
@@ -761,7 +748,7 @@ int mg_mlp_gradients(mg_context* ctx, mg_mlp* m, const float* X, const float* Yt
   if (!ctx) return MG_ERR_ARG;
   MG_CHECK_ARG(m && X && Yt && B > 0 && B < (int64_t)1 << 31, "mg_mlp_gradients: bad arguments");
   int rc = ensure_capacity(ctx, m, B);
-  if (rc != MG_OK || (rc = ensure_partials(ctx, m, B)) != MG_OK) return rc;
+  if (rc != MG_OK) return rc;
   if ((rc = forward(ctx, m, X, B)) != MG_OK) return rc;
   if ((rc = backward(ctx, m, X, Yt, B)) != MG_OK) return rc;
   if (grad)
@@ -780,7 +767,7 @@ int mg_mlp_train_step(mg_context* ctx, mg_mlp* m, const float* X, const float* Y
   if (!ctx) return MG_ERR_ARG;
   MG_CHECK_ARG(m && X && Yt && B > 0 && lr > 0.0f, "mg_mlp_train_step: bad arguments");
   int rc = ensure_capacity(ctx, m, B);
-  if (rc != MG_OK || (rc = ensure_partials(ctx, m, B)) != MG_OK) return rc;
+  if (rc != MG_OK) return rc;
   if ((rc = forward(ctx, m, X, B)) != MG_OK) return rc;
   if ((rc = backward(ctx, m, X, Yt, B)) != MG_OK) return rc;
   m->step += 1;
