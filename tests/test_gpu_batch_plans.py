@@ -42,3 +42,28 @@ def test_small_plan_beside_a_large_one(dev, precision, flags, graph):
         assert torch.equal(c["X"], w)
     small.run(graph=graph)
     small.finish()
+
+
+@pytest.mark.parametrize("ks", [[20, 9], [112, 20, 70, 100, 3]])
+def test_run_captured_by_the_caller(dev, ks):
+    """The chains' streams join the caller's capture and leave it."""
+    dc = _cases(ks, dev)
+    X0 = [c["X"].clone() for c in dc]
+    plan = K.EtkfBatch(dc, flags=0, precision=_lib.MG_PREC_MIXED)
+    plan.run(graph=False)
+    plan.finish()
+    want = [c["X"].clone() for c in dc]
+    for c, x in zip(dc, X0):
+        c["X"].copy_(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        K.context(dev.index)  # the capturing stream
+        plan.run(graph=False)
+    K.context(dev.index)
+    assert all(torch.equal(c["X"], x) for c, x in zip(dc, X0))  # captured, not run
+    for _ in range(2):
+        for c, x in zip(dc, X0):
+            c["X"].copy_(x)
+        graph.replay()
+        plan.finish()
+        assert all(torch.equal(c["X"], w) for c, w in zip(dc, want))
