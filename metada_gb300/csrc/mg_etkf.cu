@@ -1,14 +1,16 @@
 // Global ETKF (ETKF.hpp:100-179).
 //
-//   1. mean + perturbations (Ensemble.hpp:105-151), member-major;
+//   1. the ensemble mean (Ensemble.hpp:105-151; the mixed path also its
+//      perturbations, member-major);
 //   2. obs-space prior ym, Y' = HX - ym, d = yo - ym (ETKF.hpp:128-141) and
 //   3. Gram G = Y'^T R^-1 Y' and b = Y'^T R^-1 d by obs ranges, partials
 //      summed in a fixed order (deterministic), FP64 by exact splitting on
 //      the tensor cores (mg_fp64gemm.cu);
 //   4. the k x k system: the reference's inverse + llt by one factorisation
 //      (mg_solve.cu), or the symmetric square root (mg_letkf_hunt.cu, FP64
-//      Jacobi where that does not apply), into the transform T (T_ji = rho (wa_j + W_ji) for the reference, whose
-//      perturbations carry the inflation, ETKF.hpp:125);
+//      Jacobi where that does not apply), into the transform T
+//      (T_ji = rho (wa_j + W_ji) for the reference, whose perturbations carry
+//      the inflation, ETKF.hpp:125);
 //   5. Xa_i = xm + sum_j X'_j T_ji over state tiles (mg_fp64gemm.cu).
 // The Gram and the k x k solve are FP64 on both paths; the mixed path stores
 // X' in FP32 and runs the O(n k^2) update in FP32.

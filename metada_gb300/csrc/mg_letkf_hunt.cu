@@ -12,7 +12,7 @@
 // FP64 Jacobi kernel.  What bounds it: the FP32 Jacobi's shared-memory rounds and
 // the 2.3 k^3 FP64 multiply-adds of the correction, which CTAs of one SM
 // overlap (three at k <= 64).  60 x 30 x 10 points, k = 64, about 290 local
-// obs: 782 ms with the FP64 Jacobi (ten sweeps on the FP64 units) -> 56 ms.
+// obs: 782 ms with the FP64 Jacobi (ten sweeps on the FP64 units) -> 57 ms.
 #include <algorithm>
 
 #include "mg_hunt.cuh"
